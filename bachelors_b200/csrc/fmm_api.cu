@@ -110,11 +110,8 @@ fmm_status Plan::init(const fmm_config& c)
    if(const char* e = getenv("FMM_TC_DRAINMODE")) tcDrainMode = std::min(3, std::max(0, atoi(e)));
    if(const char* e = getenv("FMM_TC_GROUP")) tcGroup = std::min(2, std::max(0, atoi(e)));
    if(const char* e = getenv("FMM_L2P_SPLIT")) l2pSplit = atoi(e) != 0;
-   if(const char* e = getenv("FMM_SIMT_TILED")) simtTiled = std::min(2, std::max(0, atoi(e)));
-   if(const char* e = getenv("FMM_SIMT_KC")) simtKc = atoi(e) == 32 ? 32 : 16;
    if(const char* e = getenv("FMM_TC_TRANSLATE")) tcTranslate = atoi(e) & 3;
    if(const char* e = getenv("FMM_TC_TRDRAIN")) tcTrDrainItems = std::max(0, atoi(e));
-   if(const char* e = getenv("FMM_L2L_CHILD")) l2lChildMajor = atoi(e) != 0;
    if(const char* e = getenv("FMM_TC_TRNP_UP")) tcTrPiecesUp = std::min(3, std::max(0, atoi(e)));
    if(const char* e = getenv("FMM_TC_TRNP_DN")) tcTrPiecesDn = std::min(3, std::max(0, atoi(e)));
 
@@ -155,8 +152,8 @@ void Plan::release()
    }
    DevBuf* bufs[] = {&srcXYZb, &srcWb, &srcJb, &tgtXYZb, &rootb, &sKeys, &tKeys, &sIdx, &tIdx, &sPos, &sQ, &tPos,
                      &cubTmp, &scratch, &lvlBounds, &lvlCnt, &lvlOff, &p2pOff, &p2pList, &parList, &m2lTargets, &m2lKeys, &errb,
-                     &mult, &local, &outB, &outA, &opM2M64, &opL2L64, &opM2L64, &opM2Mw, &opL2Lw, &opM2Lw, &opM2Lbf, &multBf, &tcCounters,
-                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf};
+                     &mult, &local, &outB, &outA, &opM2M64, &opL2L64, &opM2L64, &opM2Lbf, &multBf, &tcCounters,
+                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &rotOps, &rotQuarter, &rotTasks, &rotWs};
    for(DevBuf* b : bufs) b->release();
    for(auto& b : nodeBufs) b.release();
    for(auto& b : listBufs) b.release();
@@ -1150,7 +1147,7 @@ fmm_status fmm_get_operator(fmm_plan* plan, int kind, int index, double* out)
       slot = k;
    }
    else if(index < 0 || index > 7) return setError(FMM_E_INVALID, "octant must be 0..7");
-   FMM_TRY(buildOperators(P, 0));
+   FMM_TRY(buildDenseOperators(P, 0));
    const DevBuf& b = kind == 0 ? P.opM2M64 : kind == 1 ? P.opL2L64 : P.opM2L64;
    FMM_CUDA(cudaMemcpy(out, (const double*)b.ptr + int64_t(slot) * L * L, sizeof(double) * L * L,
                        cudaMemcpyDeviceToHost));

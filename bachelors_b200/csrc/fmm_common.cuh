@@ -147,6 +147,34 @@ __device__ inline void realIrregular(int q, T x, T y, T z, T* out)
    }
 }
 
+// Packed FP32 pairs (sm_100 f32x2 arithmetic): two floats in one 64-bit register, low half first.
+typedef unsigned long long f2p;
+__device__ __forceinline__ f2p pk2(float a, float b)
+{
+   f2p r;
+   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+   return r;
+}
+__device__ __forceinline__ void upk2(f2p v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2p sub2(f2p a, f2p b)
+{
+   f2p d;
+   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+   return d;
+}
+__device__ __forceinline__ f2p mul2(f2p a, f2p b)
+{
+   f2p d;
+   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+   return d;
+}
+__device__ __forceinline__ f2p fma2(f2p a, f2p b, f2p c)
+{
+   f2p d;
+   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+   return d;
+}
+
 template <class T> struct Vec4;
 template <> struct Vec4<float> { typedef float4 type; };
 template <> struct Vec4<double> { typedef double4 type; };

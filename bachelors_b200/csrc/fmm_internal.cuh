@@ -182,7 +182,6 @@ struct Plan
    int tcTranslate = 1;                  // M2M (1) / L2L (2) on the tensor cores in tensor-core M2L plans
    int tcTrDrainItems = 0;               // their drains: every this many pipeline items (0: per drainEvery offsets)
    int tcTrPiecesUp = 0, tcTrPiecesDn = 3;   // their bf16 pieces (0: as the M2L mode)
-   int l2lChildMajor = 1;                // CUDA-core L2L over the sorted child lists (kL2LChild)
    bool tcTranslations(int which = 3) const
    {
       return !fp64 && cfg.m2l_mode != FMM_M2L_SIMT && (tcTranslate & which) != 0;
@@ -195,14 +194,19 @@ struct Plan
    DevBuf errb;
    // expansions [node][3][Lp] and outputs
    DevBuf mult, local, outB, outA;
-   // operator tables (scaled basis): FP64 masters and the working-precision copies
+   // dense operator tables (scaled basis), tensor-core plans and fmm_get_operator
    DevBuf opM2M64, opL2L64, opM2L64;     // [8][L][L], [8][L][L], [316][L][L] FP64 row-major
-   DevBuf opM2Mw, opL2Lw, opM2Lw;        // transposed working copies, see fmm_kernels.cu
    DevBuf curlTab;                       // L2P: the curl expansion as <= 4 terms of the local, see kL2PWarp
    std::vector<unsigned char> curlHost;  // its host copy (kept alive for the asynchronous upload)
    DevBuf opM2Lbf;                       // bf16 hi/lo split for the tensor-core M2L
    DevBuf multBf;                        // multipoles split into bf16 pieces for the tensor-core M2L
    int opOrder = -1;
+   int denseOrder = -1;
+   // translations through the z axis (fmm_rotate.cu): operator tables for degree cutoff rotCut, the quarter
+   // turn they are made from, partial sums of split tiles
+   DevBuf rotOps, rotQuarter, rotTasks, rotWs;
+   std::vector<unsigned char> rotTaskHost;   // host copy of rotTasks (kept for the asynchronous upload)
+   int rotCut = -1;
    // tensor-core M2L tile choices (autotuned per order and leaf capacity, or set by environment)
    int tcKChunk = 0;                     // K chunk width 32 or 64 (0: 64 for BF16X3, 32 for BF16X6)
    int tcDrainFar = 8;                   // the same through the first (far) half of a tile's offsets
@@ -232,8 +236,6 @@ struct Plan
    DevBuf levelState;                    // its barrier, work queues and level starts
    int tcGroup = 2;                      // M2L target boxes grouped by octant, then 0: in node order,
                                          // 1: by list length, 2: by partner pattern (rarest offsets first)
-   int simtKc = 16;                      // its K chunk (16 or 32)
-   int simtTiled = 1;                    // FP32 CUDA-core M2L: register-tiled kernel (0: the row-broadcast form)
    int l2pSplit = 1;                     // 1: L2P in kL2PWarp, then the near field; 0: both in kL2PNear
    int nearTile = 256;                   // near-field source tile, points (128 or 256)
    int p2mChunk = 0;                     // P2M: 0 one warp per leaf; 16 or 32: one block per leaf, that many
@@ -311,6 +313,12 @@ template <class T> fmm_status downwardT(Plan& P, cudaStream_t st);
 template <class T> fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st);
 template <class T> fmm_status directT(Plan& P, double current, int want, cudaStream_t st);
 fmm_status buildOperators(Plan& P, cudaStream_t st);
+fmm_status buildDenseOperators(Plan& P, cudaStream_t st);
+template <class T> fmm_status ensureRotations(Plan& P, cudaStream_t st);
+template <class T> fmm_status reserveRotations(Plan& P);
+template <class T> fmm_status rotM2L(Plan& P, cudaStream_t st);
+template <class T> fmm_status rotM2M(Plan& P, cudaStream_t st);
+template <class T> fmm_status rotL2L(Plan& P, cudaStream_t st);
 fmm_status initOffsetTables();
 fmm_status m2lTensorCore(Plan& P, cudaStream_t st);
 fmm_status m2mTensorCore(Plan& P, cudaStream_t st);

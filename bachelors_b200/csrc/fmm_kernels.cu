@@ -1,5 +1,5 @@
-// FMM kernels for sm_100a: translation-operator tables (FP64), P2M, M2M, M2L (CUDA-core
-// form), L2L, and the fused L2P + direct near field.
+// FMM kernels for sm_100a: dense translation-operator tables (FP64), P2M, and the L2P and direct near field.
+// (The translations are in fmm_rotate.cu and fmm_m2l_tc.cu.)
 //
 // Every expansion is stored box-size scaled: a node of side h keeps M~_l = M_l / h^l and
 // L~_l = L_l h^(l+1). With that scaling the M2M, L2L and M2L operators do not depend on the
@@ -172,21 +172,6 @@ __global__ void kBuildOperators(int p, int lim, int first, int count, double* m2
    }
 }
 
-// Working copies: transposed [op][j (input)][k (output, padded to Lp)] in T.
-template <class T>
-__global__ void kTransposeOps(const double* __restrict__ src, int nops, int L, int Lp, T* dst)
-{
-   int64_t total = int64_t(nops) * L * Lp;
-   for(int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x)
-   {
-      int k = int(e % Lp);
-      int64_t r = e / Lp;
-      int j = int(r % L);
-      int op = int(r / L);
-      dst[e] = k < L ? T(src[(int64_t(op) * L + k) * L + j]) : T(0);
-   }
-}
-
 // The gradient coefficients of kL2PNear's gradCoeff as terms: its value is sum_i c[i] Lv[idx[i]]
 // (the same case analysis, for tables).
 struct GradTerms
@@ -232,11 +217,13 @@ struct CurlEntry
    T c[4];
 };
 
-fmm_status buildOperators(Plan& P, cudaStream_t st)
+// The dense FP64 operator tables: the tensor-core operator images are made from them, and fmm_get_operator
+// returns them. The CUDA-core translations (fmm_rotate.cu) have tables of their own.
+fmm_status buildDenseOperators(Plan& P, cudaStream_t st)
 {
-   if(P.opOrder == P.p) return FMM_OK;
+   if(P.denseOrder == P.p) return FMM_OK;
    FMM_TRY(initOffsetTables());
-   const int p = P.p, L = P.L, Lp = P.Lp;
+   const int p = P.p, L = P.L;
    const int lim = P.cfg.m2l_truncate ? p : 2 * p;
    FMM_TRY(P.opM2M64.reserve(sizeof(double) * 8 * L * L));
    FMM_TRY(P.opL2L64.reserve(sizeof(double) * 8 * L * L));
@@ -246,29 +233,20 @@ fmm_status buildOperators(Plan& P, cudaStream_t st)
                                                (double*)P.opM2L64.ptr);
    FMM_TRY(launched(P, "kBuildOperators", st));
    FMM_CHECK_LAUNCH();
-   size_t es = P.fp64 ? sizeof(double) : sizeof(float);
-   FMM_TRY(P.opM2Mw.reserve(es * 8 * L * Lp));
-   FMM_TRY(P.opL2Lw.reserve(es * 8 * L * Lp));
-   FMM_TRY(P.opM2Lw.reserve(es * 316 * L * Lp));
-   if(P.fp64)
-   {
-      kTransposeOps<double><<<1024, 256, 0, st>>>((const double*)P.opM2M64.ptr, 8, L, Lp, (double*)P.opM2Mw.ptr);
-      FMM_TRY(launched(P, "kTransposeOps", st));
-      kTransposeOps<double><<<1024, 256, 0, st>>>((const double*)P.opL2L64.ptr, 8, L, Lp, (double*)P.opL2Lw.ptr);
-      FMM_TRY(launched(P, "kTransposeOps", st));
-      kTransposeOps<double><<<4096, 256, 0, st>>>((const double*)P.opM2L64.ptr, 316, L, Lp, (double*)P.opM2Lw.ptr);
-      FMM_TRY(launched(P, "kTransposeOps", st));
-   }
-   else
-   {
-      kTransposeOps<float><<<1024, 256, 0, st>>>((const double*)P.opM2M64.ptr, 8, L, Lp, (float*)P.opM2Mw.ptr);
-      FMM_TRY(launched(P, "kTransposeOps", st));
-      kTransposeOps<float><<<1024, 256, 0, st>>>((const double*)P.opL2L64.ptr, 8, L, Lp, (float*)P.opL2Lw.ptr);
-      FMM_TRY(launched(P, "kTransposeOps", st));
-      kTransposeOps<float><<<4096, 256, 0, st>>>((const double*)P.opM2L64.ptr, 316, L, Lp, (float*)P.opM2Lw.ptr);
-      FMM_TRY(launched(P, "kTransposeOps", st));
-   }
-   FMM_CHECK_LAUNCH();
+   P.denseOrder = p;
+   P.opImgOrder = -1;
+   return FMM_OK;
+}
+
+// What every solve of the plan's order needs, built once: the rotation tables, the L2P's curl table and, in
+// tensor-core plans, the dense operators.
+fmm_status buildOperators(Plan& P, cudaStream_t st)
+{
+   if(P.opOrder == P.p) return FMM_OK;
+   FMM_TRY(initOffsetTables());
+   const int p = P.p, Lp = P.Lp;
+   if(!P.fp64 && P.cfg.m2l_mode != FMM_M2L_SIMT) FMM_TRY(buildDenseOperators(P, st));
+   FMM_TRY(P.fp64 ? ensureRotations<double>(P, st) : ensureRotations<float>(P, st));
    // the L2P curl table in the plan's precision
    {
       const int Lb = nharm(p - 1);
@@ -309,177 +287,7 @@ fmm_status buildOperators(Plan& P, cudaStream_t st)
       FMM_CUDA(cudaMemcpyAsync(P.curlTab.ptr, P.curlHost.data(), P.curlHost.size(), cudaMemcpyHostToDevice, st));
    }
    P.opOrder = p;
-   P.opImgOrder = -1;
    return FMM_OK;
-}
-
-// ====================================================================================
-// M2M and L2L as tiled GEMMs over the parents of one level. A block takes 32 parents (96 rows:
-// parent x component) and 64 output coefficients; for each child octant o it streams the rows
-// (children's multipoles, or the parents' locals) and the operator T_o through shared memory in
-// K slices of 32, 6 x 4 outputs per thread. Operator elements are loaded once per tile instead of
-// once per parent. K is limited to the triangle each translation needs: an output of degree l
-// takes inputs of degree <= l (M2M) or >= l (L2L).
-//   M2M: parent = sum_o T_o child_o          (one writer per parent: stored)
-//   L2L: child_o += T_o parent               (one writer per child: load-add-store)
-// ====================================================================================
-constexpr int TG_P = 32, TG_ROWS = 96, TG_N = 64, TG_K = 32;
-
-__device__ __forceinline__ void load4(const float* p, float* v)
-{
-   const float4 x = *reinterpret_cast<const float4*>(p);
-   v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-}
-__device__ __forceinline__ void load4(const double* p, double* v)
-{
-   const double2 x = reinterpret_cast<const double2*>(p)[0], y = reinterpret_cast<const double2*>(p)[1];
-   v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
-}
-__device__ __forceinline__ void load2(const float* p, float* v)
-{
-   const float2 x = *reinterpret_cast<const float2*>(p);
-   v[0] = x.x; v[1] = x.y;
-}
-__device__ __forceinline__ void load2(const double* p, double* v)
-{
-   const double2 x = *reinterpret_cast<const double2*>(p);
-   v[0] = x.x; v[1] = x.y;
-}
-
-__device__ __forceinline__ int degreeOf(int k)
-{
-   int l = int(sqrtf(float(k)));
-   while(l * l > k) l--;
-   while((l + 1) * (l + 1) <= k) l++;
-   return l;
-}
-
-template <class T, bool UP>
-__global__ void __launch_bounds__(256, 2) kTranslateLevel(Tree t, const int* __restrict__ parList, int pBeg, int pEnd,
-                                                          int p, int Lp, const T* __restrict__ opw, T* __restrict__ X)
-{
-   __shared__ __align__(16) T As[TG_K][TG_ROWS + 1];
-   __shared__ __align__(16) T Bs[TG_K][TG_N];
-   __shared__ int childOf[TG_P][8];
-   __shared__ int parentOf[TG_P];
-   const int tid = threadIdx.x;
-   const int L = nharm(p);
-   const int pt0 = pBeg + blockIdx.x * TG_P;
-   const int n0 = blockIdx.y * TG_N;
-   if(tid < TG_P)
-   {
-      const int par = pt0 + tid < pEnd ? parList[pt0 + tid] : -1;
-      parentOf[tid] = par;
-      for(int o = 0; o < 8; o++) childOf[tid][o] = -1;
-      if(par >= 0)
-      {
-         const int c0 = t.child0[par], nc = t.nchild[par];
-         for(int c = 0; c < nc; c++)
-         {
-            const int ch = c0 + c;
-            // M2M needs children with sources, L2L children with targets
-            const bool use = UP ? t.s1[ch] > t.s0[ch] : t.t1[ch] > t.t0[ch];
-            if(use) childOf[tid][int(t.key[ch] & 7)] = ch;
-         }
-      }
-   }
-   __syncthreads();
-   const int lLo = degreeOf(min(n0, L - 1)), lHi = degreeOf(min(n0 + TG_N - 1, L - 1));
-   const int kLo = UP ? 0 : lLo * lLo;
-   const int kHi = UP ? (lHi + 1) * (lHi + 1) : L;
-   const int tr = tid >> 4, tc = tid & 15;
-   T acc[6][4];
-#pragma unroll
-   for(int i = 0; i < 6; i++)
-#pragma unroll
-      for(int j = 0; j < 4; j++) acc[i][j] = T(0);
-   // steps (octant o, K slice) in order; each step's rows and operator slice are loaded into
-   // registers one step ahead, so the global loads overlap the previous step's arithmetic.
-   // Element q of a thread: row (tid / 32) + 8 q at K offset tid % 32 (k fastest across a warp:
-   // coalesced row reads), and operator row (tid / 64) + 4 q at column tid % 64.
-   const int nK = (kHi - kLo + TG_K - 1) / TG_K;
-   const int nSteps = 8 * nK;
-   constexpr int QA = TG_K * TG_ROWS / 256, QB = TG_K * TG_N / 256;
-   T ra[QA], rb[QB];
-   const int aK = tid & 31, aR = tid >> 5;
-   const int bN = tid & 63, bK = tid >> 6;
-   auto load = [&](int step) {
-      const int o = step / nK, k0 = kLo + (step % nK) * TG_K;
-      const T* op = opw + int64_t(o) * L * Lp + n0 + bN;
-      const bool aIn = k0 + aK < kHi;
-#pragma unroll
-      for(int q = 0; q < QA; q++)
-      {
-         const int r = aR + 8 * q;
-         const int i = r / 3, c = r - 3 * i;
-         const int src = UP ? childOf[i][o] : parentOf[i];
-         ra[q] = (src >= 0 && aIn) ? X[(int64_t(src) * 3 + c) * Lp + k0 + aK] : T(0);
-      }
-      const bool bIn = n0 + bN < Lp;
-#pragma unroll
-      for(int q = 0; q < QB; q++)
-      {
-         const int k = k0 + bK + 4 * q;
-         rb[q] = (k < kHi && bIn) ? op[int64_t(k) * Lp] : T(0);
-      }
-   };
-   if(nSteps > 0) load(0);
-   for(int step = 0; step < nSteps; step++)
-   {
-      __syncthreads();
-#pragma unroll
-      for(int q = 0; q < QA; q++) As[aK][aR + 8 * q] = ra[q];
-#pragma unroll
-      for(int q = 0; q < QB; q++) Bs[bK + 4 * q][bN] = rb[q];
-      __syncthreads();
-      if(step + 1 < nSteps) load(step + 1);
-#pragma unroll 8
-      for(int kk = 0; kk < TG_K; kk++)
-      {
-         T a[6], b[4];
-#pragma unroll
-         for(int i = 0; i < 6; i++) a[i] = As[kk][tr * 6 + i];
-         load4(&Bs[kk][tc * 4], b);
-#pragma unroll
-         for(int i = 0; i < 6; i++)
-#pragma unroll
-            for(int j = 0; j < 4; j++) acc[i][j] += a[i] * b[j];
-      }
-      if(!UP && step % nK == nK - 1)
-      {
-         // this octant's children: child += acc, then a fresh accumulator for the next octant
-         const int o = step / nK;
-#pragma unroll
-         for(int i = 0; i < 6; i++)
-         {
-            const int r = tr * 6 + i, pi = r / 3, c = r % 3;
-            const int ch = childOf[pi][o];
-            if(ch >= 0)
-               for(int j = 0; j < 4; j++)
-               {
-                  const int n = n0 + tc * 4 + j;
-                  if(n < Lp) X[(int64_t(ch) * 3 + c) * Lp + n] += acc[i][j];
-               }
-#pragma unroll
-            for(int j = 0; j < 4; j++) acc[i][j] = T(0);
-         }
-      }
-   }
-   if(UP)
-   {
-#pragma unroll
-      for(int i = 0; i < 6; i++)
-      {
-         const int r = tr * 6 + i, pi = r / 3, c = r % 3;
-         const int par = parentOf[pi];
-         if(par < 0 || t.s1[par] == t.s0[par]) continue;
-         for(int j = 0; j < 4; j++)
-         {
-            const int n = n0 + tc * 4 + j;
-            if(n < Lp) X[(int64_t(par) * 3 + c) * Lp + n] = acc[i][j];
-         }
-      }
-   }
 }
 
 // ====================================================================================
@@ -794,446 +602,10 @@ __global__ void __launch_bounds__(32 * P2MW_WARPS) kP2MWarp(Tree t, const RootBo
          }
 }
 
-// ====================================================================================
-// M2M, one level: one block per node of the level with children; the parent sums the
-// translated multipoles of its children. Output coefficient k of degree l only needs input
-// coefficients j < (l+1)^2.
-// ====================================================================================
-
-// ====================================================================================
-// L2L, one level: one block per node of the level holding targets; adds the parent's
-// translated local expansion. Output coefficient of degree l needs inputs of degree >= l.
-// ====================================================================================
-
-// ====================================================================================
-// L2L, one level, child-major: the level's children with targets come sorted by octant, and a
-// block takes 32 children of one octant (blockIdx.z), so every row of its tile uses the same
-// operator T_o and none is computed for a child that does not exist. Rows are the parents' locals
-// (parent x component), gathered; the K range per 64-column group is the L2L triangle (inputs of
-// degree >= the output's); the result is added to the children's locals (one writer per child).
-// ====================================================================================
-struct L2LSeg
-{
-   int start[9];   // the octants' ranges in the sorted child list
-};
-
-template <class T>
-__global__ void __launch_bounds__(256, 2) kL2LChild(Tree t, const int* __restrict__ list, L2LSeg seg, int p, int Lp,
-                                                    const T* __restrict__ opw, T* __restrict__ X)
-{
-   const int o = blockIdx.z;
-   const int s0 = seg.start[o] + blockIdx.x * TG_P, s1 = seg.start[o + 1];
-   if(s0 >= s1) return;
-   // rows padded by two: the transposed stores meet two-way bank conflicts, and each thread reads its
-   // six rows as three aligned pairs
-   __shared__ __align__(16) T As[TG_K][TG_ROWS + 2];
-   __shared__ __align__(16) T Bs[TG_K][TG_N];
-   __shared__ int childOf[TG_P], parentOf[TG_P];
-   const int tid = threadIdx.x;
-   const int L = nharm(p);
-   const int n0 = blockIdx.y * TG_N;
-   if(tid < TG_P)
-   {
-      const int ch = s0 + tid < s1 ? list[s0 + tid] : -1;
-      childOf[tid] = ch;
-      parentOf[tid] = ch >= 0 ? t.parent[ch] : -1;
-   }
-   __syncthreads();
-   const int lLo = degreeOf(min(n0, L - 1));
-   const int kLo = lLo * lLo, kHi = L;
-   const int tr = tid >> 4, tc = tid & 15;
-   T acc[6][4];
-#pragma unroll
-   for(int i = 0; i < 6; i++)
-#pragma unroll
-      for(int j = 0; j < 4; j++) acc[i][j] = T(0);
-   const int nK = (kHi - kLo + TG_K - 1) / TG_K;
-   constexpr int QA = TG_K * TG_ROWS / 256, QB = TG_K * TG_N / 256;
-   T ra[QA], rb[QB];
-   const int aK = tid & 31, aR = tid >> 5;
-   const int bN = tid & 63, bK = tid >> 6;
-   const T* op = opw + int64_t(o) * L * Lp + n0 + bN;
-   const bool bIn = n0 + bN < Lp;
-   auto load = [&](int step) {
-      const int k0 = kLo + step * TG_K;
-      const bool aIn = k0 + aK < kHi;
-#pragma unroll
-      for(int q = 0; q < QA; q++)
-      {
-         const int r = aR + 8 * q;
-         const int i = r / 3, c = r - 3 * i;
-         const int src = parentOf[i];
-         ra[q] = (src >= 0 && aIn) ? X[(int64_t(src) * 3 + c) * Lp + k0 + aK] : T(0);
-      }
-#pragma unroll
-      for(int q = 0; q < QB; q++)
-      {
-         const int k = k0 + bK + 4 * q;
-         rb[q] = (k < kHi && bIn) ? op[int64_t(k) * Lp] : T(0);
-      }
-   };
-   if(nK > 0) load(0);
-   for(int step = 0; step < nK; step++)
-   {
-      __syncthreads();
-#pragma unroll
-      for(int q = 0; q < QA; q++) As[aK][aR + 8 * q] = ra[q];
-#pragma unroll
-      for(int q = 0; q < QB; q++) Bs[bK + 4 * q][bN] = rb[q];
-      __syncthreads();
-      if(step + 1 < nK) load(step + 1);
-#pragma unroll 8
-      for(int kk = 0; kk < TG_K; kk++)
-      {
-         T a[6], b[4];
-#pragma unroll
-         for(int i = 0; i < 6; i += 2) load2(&As[kk][tr * 6 + i], a + i);
-         load4(&Bs[kk][tc * 4], b);
-#pragma unroll
-         for(int i = 0; i < 6; i++)
-#pragma unroll
-            for(int j = 0; j < 4; j++) acc[i][j] += a[i] * b[j];
-      }
-   }
-#pragma unroll
-   for(int i = 0; i < 6; i++)
-   {
-      const int r = tr * 6 + i, ci = r / 3, c = r % 3;
-      const int ch = childOf[ci];
-      if(ch < 0) continue;
-      for(int j = 0; j < 4; j++)
-      {
-         const int n = n0 + tc * 4 + j;
-         if(n < Lp) X[(int64_t(ch) * 3 + c) * Lp + n] += acc[i][j];
-      }
-   }
-}
-
-// ====================================================================================
-// M2L on the CUDA cores (FP32 or FP64 FMA). A block owns TT target boxes from the octant-grouped
-// list of boxes with an M2L list (3 TT rows: box x component) and all output coefficients; it
-// walks only the offsets present in its tile and, per offset, the K chunks of the operator. The
-// gathered source rows and the operator slice of an item are brought to shared memory with
-// cp.async, double-buffered so that the next item's copies run under this item's arithmetic.
-// Warp w owns rows RPT w .. RPT w + RPT - 1 (its A reads are broadcasts), lane c the columns
-// c + 32 n. With the degree cutoff l + lambda <= P, a K chunk whose lowest input degree is
-// lambda_min only reaches the first (P - lambda_min + 1)^2 columns; the rest are skipped.
-// ====================================================================================
-constexpr int SM_NC = 10;              // 10 x 32 = 320 >= Lp for p <= 16
-
-template <class T> struct SimtShape;
-template <> struct SimtShape<float> { static constexpr int RPT = 12, KC = 32; };
-template <> struct SimtShape<double> { static constexpr int RPT = 6, KC = 16; };
-
-struct SimtCols
-{
-   int n[32];   // output columns of each K chunk (0: chunk unused)
-};
-
 __device__ __forceinline__ void cpAsync16Simt(void* dst, const void* src, uint32_t srcBytes)
 {
    const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(srcBytes) : "memory");
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) kM2LSimt(const int* __restrict__ targets, int nTargets,
-                                                const int* __restrict__ vtab, int p, int Lp, int nChunks,
-                                                const SimtCols cols, const T* __restrict__ opw,
-                                                const T* __restrict__ M, T* __restrict__ Lc)
-{
-   constexpr int RPT = SimtShape<T>::RPT, KC = SimtShape<T>::KC;
-   constexpr int ROWS = 8 * RPT, TT = ROWS / 3;
-   constexpr int NCOL = 32 * SM_NC;
-   extern __shared__ __align__(16) unsigned char smraw[];
-   T* As = (T*)smraw;                       // [2][ROWS][KC]
-   T* Bs = As + 2 * ROWS * KC;              // [2][KC][NCOL]
-   __shared__ int tileNode[TT];
-   __shared__ uint32_t present[10];
-   __shared__ int offs[316];
-   __shared__ int nOffS;
-   __shared__ int colTab[32];
-   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-   const int L = nharm(p);
-   const int first = blockIdx.x * TT;
-   if(tid < TT) tileNode[tid] = first + tid < nTargets ? targets[first + tid] : -1;
-   if(tid < 10) present[tid] = 0;
-   if(tid == 0)
-   {
-#pragma unroll
-      for(int g = 0; g < 32; g++) colTab[g] = cols.n[g];
-   }
-   __syncthreads();
-   for(int e = tid; e < TT * 316; e += 256)
-   {
-      const int t = tileNode[e / 316], o = e % 316;
-      if(t >= 0 && vtab[int64_t(t) * 316 + o] >= 0) atomicOr(&present[o >> 5], 1u << (o & 31));
-   }
-   __syncthreads();
-   if(tid == 0)
-   {
-      int k = 0;
-      for(int o = 0; o < 316; o++)
-         if(present[o >> 5] & (1u << (o & 31))) offs[k++] = o;
-      nOffS = k;
-   }
-   __syncthreads();
-   const int nItems = nOffS * nChunks;
-   // copies of item it into buffer b: source rows (A) and operator rows k0 .. k0 + KC (B)
-   auto issue = [&](int it, int b) {
-      const int o = offs[it / nChunks], c = it % nChunks;
-      const int k0 = c * KC;
-      const int nCol = colTab[c];
-      T* A = As + b * ROWS * KC;
-      T* B = Bs + b * KC * NCOL;
-      constexpr int ACH = KC * int(sizeof(T)) / 16;          // 16-byte chunks per row
-      for(int e = tid; e < ROWS * ACH; e += 256)
-      {
-         const int r = e / ACH, q = e % ACH;
-         const int t = tileNode[r / 3];
-         const int src = t >= 0 ? vtab[int64_t(t) * 316 + o] : -1;
-         // K positions past the row (k0 + KC can exceed Lp) are zero-filled, never read
-         const int k = k0 + q * (16 / int(sizeof(T)));
-         const bool in = src >= 0 && k < Lp;
-         const T* g = M + (int64_t(in ? src : 0) * 3 + r % 3) * Lp + (in ? k : 0);
-         cpAsync16Simt(A + r * KC + q * (16 / int(sizeof(T))), g, in ? 16u : 0u);
-      }
-      constexpr int BCH = NCOL * int(sizeof(T)) / 16;        // 16-byte chunks per operator row
-      const T* op = opw + int64_t(o) * L * Lp;
-      for(int e = tid; e < KC * BCH; e += 256)
-      {
-         const int kk = e / BCH, q = e % BCH;
-         const int col = q * (16 / int(sizeof(T)));
-         const int k = k0 + kk;
-         const bool in = k < L && col < nCol;
-         cpAsync16Simt(B + kk * NCOL + col, op + (in ? int64_t(k) * Lp + col : 0), in ? 16u : 0u);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-   };
-   T acc[RPT][SM_NC];
-#pragma unroll
-   for(int r = 0; r < RPT; r++)
-#pragma unroll
-      for(int n = 0; n < SM_NC; n++) acc[r][n] = T(0);
-   if(nItems > 0) issue(0, 0);
-   for(int it = 0; it < nItems; it++)
-   {
-      const int b = it & 1;
-      if(it + 1 < nItems)
-      {
-         issue(it + 1, b ^ 1);
-         asm volatile("cp.async.wait_group 1;" ::: "memory");
-      }
-      else
-         asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();
-      const T* A = As + b * ROWS * KC + warp * RPT * KC;
-      const T* B = Bs + b * KC * NCOL + lane;
-      const int nCol = colTab[it % nChunks];
-#pragma unroll 2
-      for(int kk = 0; kk < KC; kk++)
-      {
-         T a[RPT], bv[SM_NC];
-#pragma unroll
-         for(int r = 0; r < RPT; r++) a[r] = A[r * KC + kk];
-#pragma unroll
-         for(int n = 0; n < SM_NC; n++) bv[n] = 32 * n < nCol ? B[kk * NCOL + 32 * n] : T(0);
-#pragma unroll
-         for(int r = 0; r < RPT; r++)
-#pragma unroll
-            for(int n = 0; n < SM_NC; n++)
-               if(32 * n < nCol) acc[r][n] += a[r] * bv[n];
-      }
-      __syncthreads();
-   }
-#pragma unroll
-   for(int r = 0; r < RPT; r++)
-   {
-      const int row = RPT * warp + r;
-      const int node = tileNode[row / 3];
-      if(node < 0) continue;
-#pragma unroll
-      for(int n = 0; n < SM_NC; n++)
-      {
-         const int col = lane + 32 * n;
-         if(col < Lp) Lc[(int64_t(node) * 3 + row % 3) * Lp + col] = col < L ? acc[r][n] : T(0);
-      }
-   }
-}
-
-// ====================================================================================
-// M2L on the CUDA cores in FP32, register-tiled (the plain FP32 form of FP32 plans). The same GEMM
-// sum as kM2LTc: a tile of 42 target boxes = 126 rows (box, component) of a 128-row block, and for each
-// offset present in the tile and each 16-wide K chunk C[128 x 160] += A_o[128 x 16] T_o[16 x 160], with
-// C the block's 160 output columns (two column blocks cover the 304 of p = 16; the second skips the K
-// chunks whose degree cutoff ends below its first column). Thread (ty, tx) of 256 owns rows 8 ty .. + 7
-// and the column pairs 2 tx + 32 j (j < 5): per K element it reads its 8 rows as two 16-byte loads from a
-// transposed copy of A and its 10 columns as five 8-byte loads, for 80 FMAs. A (gathered source rows)
-// and the operator slice arrive by cp.async, double-buffered.
-// ====================================================================================
-constexpr int ST_TT = 42, ST_ROWS = 128, ST_CB = 160, ST_TPAD = ST_ROWS + 4;
-
-template <int KC>
-constexpr size_t simtTiledSmem()
-{
-   return sizeof(float) * (2 * ST_ROWS * KC + KC * ST_TPAD + 2 * KC * ST_CB);
-}
-
-template <int MINB, int ST_KC>
-__global__ void __launch_bounds__(256, MINB) kM2LSimtTiled(const int* __restrict__ targets, int nTargets,
-                                                        const int* __restrict__ vtab, int L, int Lp, int nChunks,
-                                                        const SimtCols cols, const float* __restrict__ opw,
-                                                        const float* __restrict__ M, float* __restrict__ Lc)
-{
-   extern __shared__ __align__(16) float smf[];
-   // gathered rows, row-major (cp.async target) [2][ROWS][KC]; the current item's rows, K-major [KC][TPAD];
-   // the operator slice [2][KC][CB]
-   float (*As)[ST_ROWS][ST_KC] = reinterpret_cast<float (*)[ST_ROWS][ST_KC]>(smf);
-   float (*At)[ST_TPAD] = reinterpret_cast<float (*)[ST_TPAD]>(smf + 2 * ST_ROWS * ST_KC);
-   float (*Bs)[ST_KC][ST_CB] = reinterpret_cast<float (*)[ST_KC][ST_CB]>(smf + 2 * ST_ROWS * ST_KC + ST_KC * ST_TPAD);
-   __shared__ int tileNode[ST_TT];
-   __shared__ uint32_t present[10];
-   __shared__ int offs[316];
-   __shared__ int nOffS;
-   __shared__ int chunkList[32], nChunkS;
-   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-   const int first = blockIdx.x * ST_TT;
-   const int cb = blockIdx.y, col0 = cb * ST_CB;
-   if(tid < ST_TT) tileNode[tid] = first + tid < nTargets ? targets[first + tid] : -1;
-   if(tid < 10) present[tid] = 0;
-   __syncthreads();
-   for(int e = tid; e < ST_TT * 316; e += 256)
-   {
-      const int t = tileNode[e / 316], o = e % 316;
-      if(t >= 0 && vtab[int64_t(t) * 316 + o] >= 0) atomicOr(&present[o >> 5], 1u << (o & 31));
-   }
-   __syncthreads();
-   if(tid == 0)
-   {
-      int k = 0;
-      for(int o = 0; o < 316; o++)
-         if(present[o >> 5] & (1u << (o & 31))) offs[k++] = o;
-      nOffS = k;
-      // the K chunks that reach this column block (the degree cutoff narrows later chunks)
-      int nc = 0;
-      for(int c = 0; c < nChunks; c++)
-         if(cols.n[c] > col0) chunkList[nc++] = c;
-      nChunkS = nc;
-   }
-   __syncthreads();
-   const int nCh = nChunkS, nOff = nOffS, nItems = nOff * nCh;
-   // A: 128 rows x KC floats in 16-byte chunks; thread tid copies chunks (tid & 3) + 4 i of rows tid >> 2
-   // and (tid >> 2) + 64 for every item, so it keeps those rows' source boxes for the current offset and
-   // loads the next offset's one offset ahead (the V table read is off the copies' critical path)
-   const int rA = tid >> 2, qA = tid & 3;
-   int tA[2];
-   for(int h = 0; h < 2; h++)
-   {
-      const int r = rA + 64 * h;
-      tA[h] = r < 3 * ST_TT ? tileNode[r / 3] : -1;
-   }
-   int srcCur[2] = {-1, -1}, srcNxt[2] = {-1, -1};
-   int oiCur = -1;
-   auto loadSrc = [&](int oi, int* out) {
-      const int o = offs[oi];
-      for(int h = 0; h < 2; h++) out[h] = tA[h] >= 0 ? vtab[int64_t(tA[h]) * 316 + o] : -1;
-   };
-   auto issue = [&](int it, int b) {
-      const int oi = it / nCh;
-      const int o = offs[oi], c = chunkList[it - oi * nCh];
-      const int k0 = c * ST_KC;
-      if(oi != oiCur)
-      {
-         if(oi == oiCur + 1 && oiCur >= 0) { srcCur[0] = srcNxt[0]; srcCur[1] = srcNxt[1]; }
-         else loadSrc(oi, srcCur);
-         oiCur = oi;
-         if(oi + 1 < nOff) loadSrc(oi + 1, srcNxt);
-      }
-      for(int h = 0; h < 2; h++)
-#pragma unroll
-         for(int i = 0; i < ST_KC / 16; i++)
-         {
-            const int r = rA + 64 * h, src = srcCur[h];
-            const int q = qA + 4 * i, k = k0 + 4 * q;
-            const bool in = src >= 0 && k < Lp;
-            const float* g = M + (int64_t(in ? src : 0) * 3 + r % 3) * Lp + (in ? k : 0);
-            cpAsync16Simt(&As[b][r][4 * q], g, in ? 16u : 0u);
-         }
-      // B: 16 K rows x 160 columns = 640 chunks
-      const float* op = opw + int64_t(o) * L * Lp;
-      const int nCol = cols.n[c];
-      for(int e = tid; e < ST_KC * (ST_CB / 4); e += 256)
-      {
-         const int kk = e / (ST_CB / 4), q = e % (ST_CB / 4);
-         const int col = col0 + 4 * q, k = k0 + kk;
-         const bool in = k < L && col < nCol;
-         cpAsync16Simt(&Bs[b][kk][4 * q], op + (in ? int64_t(k) * Lp + col : 0), in ? 16u : 0u);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-   };
-   float acc[8][10];
-#pragma unroll
-   for(int r = 0; r < 8; r++)
-#pragma unroll
-      for(int n = 0; n < 10; n++) acc[r][n] = 0.f;
-   if(nItems > 0) issue(0, 0);
-   for(int it = 0; it < nItems; it++)
-   {
-      const int b = it & 1;
-      if(it + 1 < nItems)
-      {
-         issue(it + 1, b ^ 1);
-         asm volatile("cp.async.wait_group 1;" ::: "memory");
-      }
-      else
-         asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();
-      // transpose this item's rows into At[k][row]
-#pragma unroll
-      for(int q = 0; q < (ST_ROWS * ST_KC) / 256; q++)
-      {
-         const int e = tid + 256 * q;
-         const int r = e / ST_KC, k = e % ST_KC;
-         At[k][r] = As[b][r][k];
-      }
-      __syncthreads();
-#pragma unroll 4
-      for(int k = 0; k < ST_KC; k++)
-      {
-         const float4 a0 = *reinterpret_cast<const float4*>(&At[k][8 * ty]);
-         const float4 a1 = *reinterpret_cast<const float4*>(&At[k][8 * ty + 4]);
-         const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-         float bv[10];
-#pragma unroll
-         for(int j = 0; j < 5; j++)
-         {
-            const float2 v = *reinterpret_cast<const float2*>(&Bs[b][k][2 * tx + 32 * j]);
-            bv[2 * j] = v.x;
-            bv[2 * j + 1] = v.y;
-         }
-#pragma unroll
-         for(int r = 0; r < 8; r++)
-#pragma unroll
-            for(int n = 0; n < 10; n++) acc[r][n] = fmaf(a[r], bv[n], acc[r][n]);
-      }
-      __syncthreads();
-   }
-#pragma unroll
-   for(int r = 0; r < 8; r++)
-   {
-      const int row = 8 * ty + r;
-      if(row >= 3 * ST_TT) continue;
-      const int node = tileNode[row / 3];
-      if(node < 0) continue;
-      float* out = Lc + (int64_t(node) * 3 + row % 3) * Lp;
-#pragma unroll
-      for(int j = 0; j < 5; j++)
-      {
-         const int col = col0 + 2 * tx + 32 * j;
-         if(col < Lp) out[col] = col < L ? acc[r][2 * j] : 0.f;
-         if(col + 1 < Lp) out[col + 1] = col + 1 < L ? acc[r][2 * j + 1] : 0.f;
-      }
-   }
 }
 
 // ====================================================================================
@@ -1279,33 +651,6 @@ __device__ __forceinline__ float rsqrtApprox(float x)
    float y;
    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
    return y;
-}
-// Packed FP32 pairs (sm_100 f32x2 arithmetic): two floats in one 64-bit register, low half first.
-typedef unsigned long long f2p;
-__device__ __forceinline__ f2p pk2(float a, float b)
-{
-   f2p r;
-   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-   return r;
-}
-__device__ __forceinline__ void upk2(f2p v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2p sub2(f2p a, f2p b)
-{
-   f2p d;
-   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-   return d;
-}
-__device__ __forceinline__ f2p mul2(f2p a, f2p b)
-{
-   f2p d;
-   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-   return d;
-}
-__device__ __forceinline__ f2p fma2(f2p a, f2p b, f2p c)
-{
-   f2p d;
-   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-   return d;
 }
 __device__ __forceinline__ void cpAsync4(void* dst, const void* src, uint32_t srcBytes)
 {
@@ -1942,77 +1287,7 @@ fmm_status upwardT(Plan& P, cudaStream_t st)
    FMM_TRY(launched(P, "kP2M", st));
    FMM_CHECK_LAUNCH();
    if(P.tcTranslations(1)) return m2mTensorCore(P, st);
-   const int nCol = (Lp + TG_N - 1) / TG_N;
-   for(int level = P.tree.nLevels - 2; level >= 0; level--)
-   {
-      const int a = P.parStart[level], b = P.parStart[level + 1];
-      if(b <= a) continue;
-      kTranslateLevel<T, true><<<dim3((b - a + TG_P - 1) / TG_P, nCol), 256, 0, st>>>(
-         P.tree, (const int*)P.parList.ptr, a, b, P.p, Lp, (const T*)P.opM2Mw.ptr, (T*)P.mult.ptr);
-      FMM_TRY(launched(P, "kTranslateLevel<M2M>", st));
-   }
-   FMM_CHECK_LAUNCH();
-   return FMM_OK;
-}
-
-template <class T>
-fmm_status m2lSimt(Plan& P, cudaStream_t st)
-{
-   const int count = P.nM2LTargets;
-   if(count <= 0) return FMM_OK;
-   constexpr int RPT = SimtShape<T>::RPT, KC = SimtShape<T>::KC;
-   constexpr int TT = 8 * RPT / 3;
-   const int L = P.L, Lp = P.Lp;
-   const int nChunks = (L + KC - 1) / KC;
-   if(Lp > 32 * SM_NC || nChunks > 32) return setError(FMM_E_INVALID, "CUDA-core M2L supports p <= 16");
-   // degree cutoff (see fmm_config.m2l_tc_degree_cutoff): FP32 plans default to p + 8, FP64 plans
-   // to the full operator
-   const int c = P.cfg.m2l_tc_degree_cutoff;
-   const int cut = c < 0 || (c == 0 && P.fp64) ? 2 * P.p : (c == 0 ? P.p + 8 : std::max(c, P.p));
-   SimtCols cols{};
-   for(int g = 0; g < nChunks; g++)
-   {
-      const int k = KC * g;
-      int lmin = 0;
-      while((lmin + 1) * (lmin + 1) <= k) lmin++;
-      const int n = cut - lmin >= 0 ? std::min(L, (cut - lmin + 1) * (cut - lmin + 1)) : 0;
-      cols.n[g] = std::min(Lp, (n + 3) / 4 * 4);
-   }
-   if(sizeof(T) == 4 && P.simtTiled)
-   {
-      // FP32: the register-tiled kernel, K chunks of 16 (or 32) with the same degree cutoff
-      const int ST_KC = P.simtKc;
-      SimtCols c16{};
-      const int n16 = (L + ST_KC - 1) / ST_KC;
-      if(n16 > 32) return setError(FMM_E_INVALID, "CUDA-core M2L supports p <= 16");
-      for(int g = 0; g < n16; g++)
-      {
-         const int k = ST_KC * g;
-         int lmin = 0;
-         while((lmin + 1) * (lmin + 1) <= k) lmin++;
-         const int n = cut - lmin >= 0 ? std::min(L, (cut - lmin + 1) * (cut - lmin + 1)) : 0;
-         c16.n[g] = std::min(Lp, (n + 3) / 4 * 4);
-      }
-      const dim3 grid((count + ST_TT - 1) / ST_TT, (Lp + ST_CB - 1) / ST_CB);
-      // two blocks per SM (registers capped at 128) or one with all the registers it wants
-      auto kern = P.simtTiled == 2 ? (ST_KC == 32 ? kM2LSimtTiled<1, 32> : kM2LSimtTiled<1, 16>)
-                                   : (ST_KC == 32 ? kM2LSimtTiled<2, 32> : kM2LSimtTiled<2, 16>);
-      const size_t smemT = ST_KC == 32 ? simtTiledSmem<32>() : simtTiledSmem<16>();
-      FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemT)));
-      kern<<<grid, 256, smemT, st>>>((const int*)P.m2lTargets.ptr, count, P.lists.vtab, L, Lp, n16, c16,
-                                     (const float*)P.opM2Lw.ptr, (const float*)P.mult.ptr, (float*)P.local.ptr);
-      FMM_TRY(launched(P, "kM2LSimtTiled", st));
-      FMM_CHECK_LAUNCH();
-      return FMM_OK;
-   }
-   const size_t smem = sizeof(T) * 2 * (size_t(8 * RPT) * KC + size_t(KC) * 32 * SM_NC);
-   FMM_CUDA(cudaFuncSetAttribute(kM2LSimt<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-   const int blocks = (count + TT - 1) / TT;
-   kM2LSimt<T><<<blocks, 256, smem, st>>>((const int*)P.m2lTargets.ptr, count, P.lists.vtab, P.p, Lp, nChunks, cols,
-                                          (const T*)P.opM2Lw.ptr, (const T*)P.mult.ptr, (T*)P.local.ptr);
-   FMM_TRY(launched(P, "kM2LSimt", st));
-   FMM_CHECK_LAUNCH();
-   return FMM_OK;
+   return rotM2M<T>(P, st);
 }
 
 template <class T>
@@ -2023,36 +1298,10 @@ fmm_status downwardT(Plan& P, cudaStream_t st)
    FMM_TRY(P.local.reserve(sizeof(T) * N * 3 * Lp));
    FMM_CUDA(cudaMemsetAsync(P.local.ptr, 0, sizeof(T) * N * 3 * Lp, st));
    if(sizeof(T) == 4 && P.cfg.m2l_mode != FMM_M2L_SIMT) FMM_TRY(m2lTensorCore(P, st));
-   else FMM_TRY(m2lSimt<T>(P, st));
+   else FMM_TRY(rotM2L<T>(P, st));
    if(P.eventsMade && !P.capturing) cudaEventRecord(P.ev[3], st);
    if(P.tcTranslations(2)) return l2lTensorCore(P, st);
-   const int nCol = (Lp + TG_N - 1) / TG_N;
-   if(P.l2lChildMajor)
-   {
-      for(int level = 0; level + 1 < P.tree.nLevels; level++)
-      {
-         L2LSeg seg;
-         int maxTiles = 0;
-         for(int o = 0; o <= 8; o++) seg.start[o] = P.l2lStart[8 * (level + 1) + o];
-         for(int o = 0; o < 8; o++) maxTiles = std::max(maxTiles, (seg.start[o + 1] - seg.start[o] + TG_P - 1) / TG_P);
-         if(maxTiles == 0) continue;
-         kL2LChild<T><<<dim3(maxTiles, nCol, 8), 256, 0, st>>>(P.tree, (const int*)P.l2lTargets.ptr, seg, P.p, Lp,
-                                                                (const T*)P.opL2Lw.ptr, (T*)P.local.ptr);
-         FMM_TRY(launched(P, "kL2LChild", st));
-      }
-      FMM_CHECK_LAUNCH();
-      return FMM_OK;
-   }
-   for(int level = 0; level + 1 < P.tree.nLevels; level++)
-   {
-      const int a = P.parStart[level], b = P.parStart[level + 1];
-      if(b <= a) continue;
-      kTranslateLevel<T, false><<<dim3((b - a + TG_P - 1) / TG_P, nCol), 256, 0, st>>>(
-         P.tree, (const int*)P.parList.ptr, a, b, P.p, Lp, (const T*)P.opL2Lw.ptr, (T*)P.local.ptr);
-      FMM_TRY(launched(P, "kTranslateLevel<L2L>", st));
-   }
-   FMM_CHECK_LAUNCH();
-   return FMM_OK;
+   return rotL2L<T>(P, st);
 }
 
 template <class T>

@@ -1,0 +1,992 @@
+// Translations through the z axis (M2L, M2M and L2L on the CUDA cores, FP32 and FP64).
+//
+// A translation by a vector v is a rotation that takes v to the z axis, a translation along z, and the
+// rotation back. Rotations keep the degree l and, split into an azimuth turn (2 x 2 blocks on (m, -m)) and
+// a turn about y (which keeps the cosine and the sine coefficients apart), cost sum (l+1)^2 + l^2
+// multiply-adds; a z translation keeps m and costs as much. One box pair and component takes about 3 x (2/3) p^3
+// multiply-adds instead of the (p+1)^4 of the dense operator (p = 12: 4.4k instead of 28.6k, p = 16: 9.8k
+// instead of 83.5k), with the same truncation: degrees are kept by the rotations, so a cutoff on
+// l + lambda keeps the same terms. (The method is White and Head-Gordon's, J. Chem. Phys. 105, 5061, 1996.)
+//
+// With D the rotation of the solid harmonics, R(rot x) = D R(x), N = diag sqrt((l-m)! (l+m)!) and D^ = N D N^-1,
+// which is orthogonal:
+//   M2L  L_out = D^T Tz D M                  Tz[l, lambda] = (-1)^(l+m) (l+lambda)! / r^(l+lambda+1)
+//   M2M  M_out = N^-1 D^^T N  Tz  D M        Tz[l, lambda] = (-r)^(l-lambda) / (l-lambda)!
+//   L2L  L_out = D^T  Tz  N D^ N^-1 L        Tz[l, lambda] = r^(lambda-l) / (lambda-l)!
+// with the box-size scaling's powers of two in the last factor. Tz depends on l and lambda only through their
+// sum or difference, so an operator is two sets of rotation blocks and a vector of 2p + 1 numbers.
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+#include <type_traits>
+#include <vector>
+
+#include "fmm_internal.cuh"
+
+namespace fmm {
+
+namespace rot {
+
+// ------------------------------------------------------------------------------ operator tables
+// Coefficients in two orders. Degree-major: (l, cos m = 0..l) and (l, sin m = 1..l) blocks, each contiguous in
+// m. Order-major: (m, cos l = m..p) and (m, sin) blocks, contiguous in l. Blocks of n coefficients are products with
+// n x n matrices, taken four outputs at a time: a group's table is [k < n rounded up to even][4], 16-byte loads in
+// the kernel (the odd n's last row is zero; it meets the next block's first coefficient).
+//
+// One operator's table in T: the forward groups, the backward groups (both: for n = 1..p+1 the ceil(n/4) groups of
+// the cosine block of degree n - 1, then of the sine block of degree n), H[s][4] for s = 0..2p+1 (four
+// neighbouring entries of the z translation's vector: s, s+1, .. for M2L, s, s-1, .. otherwise; no translation has a
+// term at the entry an odd block's last row adds, but its coefficient is the next block's, see kRotTranslate) and
+// (cos, sin)(m phi).
+__host__ __device__ constexpr int grp(int n) { return (n + 3) >> 2; }
+__host__ __device__ constexpr int even(int n) { return (n + 1) & ~1; }
+__host__ __device__ constexpr int groupBase(int n)   // elements before the groups of blocks of n
+{
+   int s = 0;
+   for(int i = 1; i < n; i++) s += 8 * grp(i) * even(i);
+   return s;
+}
+struct Blob
+{
+   int half, hOff, zOff, size;
+   Blob() = default;
+   __host__ __device__ Blob(int p)
+   {
+      half = groupBase(p + 1) + 4 * grp(p + 1) * even(p + 1);
+      hOff = 2 * half;
+      zOff = hOff + 4 * (2 * p + 2);
+      size = zOff + ((2 * (p + 1) + 3) & ~3);
+   }
+};
+// element offset of group g of the cosine (degree n - 1) or sine (degree n) block
+__host__ __device__ inline int groupOff(int n, int sine, int g) { return groupBase(n) + (sine * grp(n) + g) * 4 * even(n); }
+
+// positions in the two orders; order-major blocks are padded to an even number of coefficients
+__host__ __device__ inline int degPos(int l, int m) { return l * l + (m >= 0 ? m : l - m); }   // cos 0..l, then sin 1..l
+__host__ __device__ inline int ordBase(int p, int m)   // first position of order |m|'s cosine (m < 0: sine) block
+{
+   const int a = m < 0 ? -m : m;
+   int s = 0;
+   for(int b = 0; b < a; b++) s += (b ? 2 : 1) * even(p + 1 - b);
+   return s + (m < 0 ? even(p + 1 - a) : 0);
+}
+__host__ __device__ inline int ordPos(int p, int l, int m) { return ordBase(p, m) + l - (m < 0 ? -m : m); }
+__host__ __device__ inline int ordSize(int p) { return ordBase(p, p + 1); }
+
+// D^ of the quarter turn about x that takes e_z to e_y, degree blocks [2l+1][2l+1] one after the other, by
+// integrating products of the orthonormal harmonics over the sphere (Gauss-Legendre x trapezoid, exact for
+// these degrees): R_i(Q x) against R_j(x).
+static int quarterOff(int l) { return l * (4 * l * l - 1) / 3; }   // sum of (2i+1)^2, i < l
+static const std::vector<double>& quarterTurn()
+{
+   static std::vector<double> tab;
+   static std::once_flag once;
+   std::call_once(once, [] {
+      const int p = MAXORDER, L = nharm(p), nz = p + 1, na = 2 * p + 1;
+      // Gauss-Legendre nodes by Newton's method on P_nz
+      std::vector<double> zs(nz), ws(nz);
+      for(int i = 0; i < nz; i++)
+      {
+         double x = std::cos(M_PI * (i + 0.75) / (nz + 0.5)), dp = 1;
+         for(int it = 0; it < 100; it++)
+         {
+            double a = 1, b = x;
+            for(int n = 2; n <= nz; n++) { const double c = ((2 * n - 1) * x * b - (n - 1) * a) / n; a = b; b = c; }
+            dp = nz * (x * b - a) / (x * x - 1);
+            const double dx = b / dp;
+            x -= dx;
+            if(std::fabs(dx) < 1e-16) break;
+         }
+         zs[i] = x;
+         ws[i] = 2 / ((1 - x * x) * dp * dp);
+      }
+      // orthogonal-basis regular harmonics N R at a unit vector, by the recurrence of visitRegular
+      std::vector<double> norm(L);
+      for(int l = 0; l <= p; l++)
+         for(int m = -l; m <= l; m++)
+         {
+            double f = 1;
+            for(int k = 2; k <= l - std::abs(m); k++) f *= k;
+            double g = 1;
+            for(int k = 2; k <= l + std::abs(m); k++) g *= k;
+            norm[hidx(l, m)] = std::sqrt(f) * std::sqrt(g);
+         }
+      auto harm = [&](double x, double y, double z, double* out) {
+         double dre = 1, dim = 0;
+         for(int m = 0; m <= p; m++)
+         {
+            if(m > 0)
+            {
+               const double s = 1.0 / (2 * m), nre = (dre * x - dim * y) * s, nim = (dre * y + dim * x) * s;
+               dre = nre; dim = nim;
+            }
+            double are = dre, aim = dim, bre = 0, bim = 0;
+            for(int l = m; l <= p; l++)
+            {
+               const double s = (l & 1) ? -1 : 1, q = std::sqrt(2.0);
+               if(m == 0) out[hidx(l, 0)] = s * are * norm[hidx(l, 0)];
+               else
+               {
+                  out[hidx(l, m)] = s * q * are * norm[hidx(l, m)];
+                  out[hidx(l, -m)] = s * q * aim * norm[hidx(l, m)];
+               }
+               const double inv = 1.0 / ((l - m + 1.0) * (l + m + 1.0));
+               const double cre = ((2 * l + 1) * z * are - bre) * inv, cim = ((2 * l + 1) * z * aim - bim) * inv;
+               bre = are; bim = aim; are = cre; aim = cim;
+            }
+         }
+      };
+      tab.assign(quarterOff(p + 1), 0.0);
+      std::vector<double> a(L), b(L);
+      for(int i = 0; i < nz; i++)
+         for(int j = 0; j < na; j++)
+         {
+            const double s = std::sqrt(1 - zs[i] * zs[i]), f = 2 * M_PI * j / na;
+            const double x = s * std::cos(f), y = s * std::sin(f), z = zs[i];
+            harm(x, y, z, b.data());
+            harm(x, z, -y, a.data());   // Q x: e_z -> e_y, e_y -> -e_z
+            const double w = ws[i] * 2 * M_PI / na / (4 * M_PI);
+            for(int l = 0; l <= p; l++)
+               for(int u = 0; u <= 2 * l; u++)
+                  for(int v = 0; v <= 2 * l; v++)
+                     tab[quarterOff(l) + u * (2 * l + 1) + v] += w * (2 * l + 1) * a[l * l + u] * b[l * l + v];
+         }
+   });
+   return tab;
+}
+
+// One block per operator: 0..7 M2M octants, 8..15 L2L octants, 16.. the M2L offset slots.
+// The turn about y by -theta is Q Z(-theta) Q^T with Q the quarter turn and Z the azimuth turn.
+template <class T>
+__global__ void kBuildRotations(int p, int cut, const double* __restrict__ quarter, T* __restrict__ out)
+{
+   constexpr int M1 = MAXORDER + 1;
+   const Blob B(p);
+   const int op = blockIdx.x;
+   const int kind = op < 8 ? 0 : (op < 16 ? 1 : 2);
+   double v[3];
+   if(kind == 2)
+   {
+      const int o = d_m2lOffset[op - 16];
+      v[0] = o % 7 - 3; v[1] = (o / 7) % 7 - 3; v[2] = o / 49 - 3;
+   }
+   else
+      for(int d = 0; d < 3; d++) v[d] = (((op >> d) & 1) - 0.5) * (kind == 0 ? 0.5 : -0.5);
+   const double r = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+   const double theta = acos(fmin(1.0, fmax(-1.0, v[2] / r)));
+   const double phi = v[0] == 0 && v[1] == 0 ? 0.0 : atan2(v[1], v[0]);
+   __shared__ double norm[M1 * M1];   // N of (l, m), m >= 0, at l M1 + m
+   __shared__ double ct[M1], sn[M1];
+   for(int e = threadIdx.x; e < M1 * M1; e += blockDim.x)
+   {
+      const int l = e / M1, m = e % M1;
+      double f = 1, g = 1;
+      for(int k = 2; k <= l - m; k++) f *= k;
+      for(int k = 2; k <= l + m; k++) g *= k;
+      norm[e] = sqrt(f) * sqrt(g);
+   }
+   if(threadIdx.x <= p) { ct[threadIdx.x] = cos(threadIdx.x * theta); sn[threadIdx.x] = sin(threadIdx.x * theta); }
+   T* o = out + int64_t(op) * B.size;
+   for(int e = threadIdx.x; e < B.size; e += blockDim.x) o[e] = T(0);
+   __syncthreads();
+   for(int l = 0; l <= p; l++)
+   {
+      const int w = 2 * l + 1;
+      int q0 = 0;
+      for(int i = 0; i < l; i++) q0 += (2 * i + 1) * (2 * i + 1);
+      const double* Q = quarter + q0;
+      // entries (a, b) of D^'s cosine (a, b = 0..l) and sine (a, b = 1..l) blocks
+      for(int e = threadIdx.x; e < (l + 1) * (l + 1) + l * l; e += blockDim.x)
+      {
+         const int sine = e < (l + 1) * (l + 1) ? 0 : 1;
+         const int f = sine ? e - (l + 1) * (l + 1) : e, n = sine ? l : l + 1;
+         const int i = f / n, j = f % n;
+         const int ma = i + sine, mb = j + sine;
+         const int a = sine ? -ma : ma, b = sine ? -mb : mb;
+         // sum over c of Q[a, c] (Z(-theta) Q^T)[c, b], Z on (m, -m): x_m' = cos x_m + sin x_-m, x_-m' = cos x_-m - sin x_m
+         double s = Q[(l + a) * w + l] * Q[(l + b) * w + l];
+         for(int m = 1; m <= l; m++)
+         {
+            const double ap = Q[(l + a) * w + l + m], an = Q[(l + a) * w + l - m];
+            const double bp = Q[(l + b) * w + l + m], bn = Q[(l + b) * w + l - m];
+            s += ap * (ct[m] * bp + sn[m] * bn) + an * (ct[m] * bn - sn[m] * bp);
+         }
+         const double nab = norm[l * M1 + mb] / norm[l * M1 + ma];   // N_b / N_a
+         // forward, output a from input b: D = N^-1 D^ N for multipoles, N D^ N^-1 for locals
+         o[groupOff(n, sine, i >> 2) + 4 * j + (i & 3)] = T(kind == 1 ? s / nab : s * nab);
+         // backward, output b from input a: D^T with M2L's sign, N^-1 D^^T N (M2M), N D^^T N^-1 = D^T (L2L)
+         double t = kind == 0 ? s / nab : s * nab;
+         if(kind == 2) { if((l + ma) & 1) t = -t; }
+         else t = ldexp(t, kind == 0 ? -l : -(l + 1));
+         o[B.half + groupOff(n, sine, j >> 2) + 4 * i + (j & 3)] = T(t);
+      }
+   }
+   // the z translation's vector: entry l + lambda (M2L), lambda - l + p (M2M, L2L)
+   for(int e = threadIdx.x; e < 4 * (2 * p + 2); e += blockDim.x)
+   {
+      const int i = kind == 2 ? (e >> 2) + (e & 3) : (e >> 2) - (e & 3);
+      double s = 0;
+      if(kind == 2)
+      {
+         if(i <= cut)
+         {
+            s = 1 / r;
+            for(int k = 1; k <= i; k++) s *= k / r;
+         }
+      }
+      else
+      {
+         const int d = kind == 0 ? p - i : i - p;
+         if(i >= 0 && d > 0)   // (d = 0, the coefficient itself, is added exactly: see kRotTranslate)
+         {
+            s = 1;
+            for(int k = 1; k <= d; k++) s *= (kind == 0 ? -2 * r : r) / k;   // M2M: 2^-lambda = 2^-l 2^(l - lambda)
+         }
+      }
+      o[B.hOff + e] = T(s);
+   }
+   for(int m = threadIdx.x; m <= p; m += blockDim.x)
+   {
+      o[B.zOff + 2 * m] = T(cos(m * phi));
+      o[B.zOff + 2 * m + 1] = T(sin(m * phi));
+   }
+}
+
+// ------------------------------------------------------------------------------ kernel
+// A task of one quarter-warp: four outputs of a block of K coefficients.
+struct __align__(16) Task
+{
+   unsigned short in, K, op, pad;   // first input position, inputs (even), operator offset / 4
+   unsigned short out[4];           // output positions (0xFFFF: none)
+};
+constexpr int MAXTASK = 88;         // quarter-warp tasks of one step (p = 16)
+struct TaskTable
+{
+   int n[3];                        // warp tasks (four tasks of equal K) of each step
+   Task t[3][MAXTASK];
+};
+
+// The tasks of the three steps, longest first.
+static void makeTasks(int p, int mode, TaskTable& tab)
+{
+   const Blob B(p);
+   for(int step = 0; step < 3; step++)
+   {
+      std::vector<Task> v;
+      for(int K = even(p + 1); K >= 2; K -= 2)
+      {
+         for(int n = K; n >= K - 1; n--)
+         {
+            if(n > p + 1) continue;
+            for(int g = 0; g < grp(n); g++)
+               for(int sine = 0; sine < 2; sine++)
+               {
+                  // the two blocks of n coefficients: cosine of degree n - 1 and sine of degree n (rotations),
+                  // cosine and sine of order p + 1 - n (z translation)
+                  if(sine && n == p + 1) continue;
+                  Task t{};
+                  t.K = (unsigned short)K;
+                  const int l = n - 1 + sine, m = p + 1 - n;
+                  if(step == 1)
+                  {
+                     t.in = (unsigned short)ordBase(p, sine ? -m : m);
+                     t.op = (unsigned short)((B.hOff + 4 * (mode == 0 ? 2 * m + 4 * g : p - 4 * g)) / 4);
+                  }
+                  else
+                  {
+                     t.in = (unsigned short)degPos(l, sine ? -1 : 0);
+                     t.op = (unsigned short)(((step == 2 ? B.half : 0) + groupOff(n, sine, g)) / 4);
+                  }
+                  for(int q = 0; q < 4; q++)
+                  {
+                     const int i = 4 * g + q;
+                     int pos = 0xFFFF;
+                     if(i < n)
+                     {
+                        const int mm = sine ? -(i + 1) : i;
+                        pos = step == 1 ? degPos(m + i, sine ? -m : m) : step == 0 ? ordPos(p, l, mm) : degPos(l, mm);
+                     }
+                     t.out[q] = (unsigned short)pos;
+                  }
+                  v.push_back(t);
+               }
+         }
+         while(v.size() & 3)
+         {
+            Task t = v.back();
+            for(int q = 0; q < 4; q++) t.out[q] = 0xFFFF;
+            v.push_back(t);
+         }
+      }
+      tab.n[step] = int(v.size() / 4);
+      std::copy(v.begin(), v.end(), tab.t[step]);
+   }
+}
+
+// A lane's rows of one coefficient: R groups of V (FP32: 4, as two packed pairs; FP64: 2) consecutive rows, 8 V
+// rows apart.
+template <class T> constexpr int laneRows() { return 16 / int(sizeof(T)); }
+template <class T> constexpr int chunkPairs() { return sizeof(T) == 4 ? 20 : 10; }
+template <class T> constexpr int rowStride() { return 3 * chunkPairs<T>(); }   // 60 (FP64: 30): a multiple of V, 2-way conflicts transposed
+
+template <class T, int R> struct Rows;
+template <int R> struct Rows<float, R>
+{
+   f2p v[2 * R];
+   __device__ __forceinline__ void zero()
+   {
+#pragma unroll
+      for(int i = 0; i < 2 * R; i++) v[i] = 0;
+   }
+   __device__ __forceinline__ void load(const float* p)
+   {
+#pragma unroll
+      for(int g = 0; g < R; g++)
+      {
+         const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(p + 32 * g);
+         v[2 * g] = x.x; v[2 * g + 1] = x.y;
+      }
+   }
+   // (the last group's last lane has no rows)
+   __device__ __forceinline__ void store(float* p, bool all) const
+   {
+#pragma unroll
+      for(int g = 0; g < R; g++)
+         if(g == 0 || all) *reinterpret_cast<ulonglong2*>(p + 32 * g) = make_ulonglong2(v[2 * g], v[2 * g + 1]);
+   }
+   __device__ __forceinline__ void mac(float a, const Rows& x)
+   {
+      const f2p aa = pk2(a, a);
+#pragma unroll
+      for(int i = 0; i < 2 * R; i++) v[i] = fma2(aa, x.v[i], v[i]);
+   }
+   // a x + b y
+   __device__ __forceinline__ void comb(float a, const Rows& x, float b, const Rows& y)
+   {
+      const f2p aa = pk2(a, a), bb = pk2(b, b);
+#pragma unroll
+      for(int i = 0; i < 2 * R; i++) v[i] = fma2(bb, y.v[i], mul2(aa, x.v[i]));
+   }
+};
+template <int R> struct Rows<double, R>
+{
+   double v[2 * R];
+   __device__ __forceinline__ void zero()
+   {
+#pragma unroll
+      for(int i = 0; i < 2 * R; i++) v[i] = 0;
+   }
+   __device__ __forceinline__ void load(const double* p)
+   {
+#pragma unroll
+      for(int g = 0; g < R; g++)
+      {
+         const double2 x = *reinterpret_cast<const double2*>(p + 16 * g);
+         v[2 * g] = x.x; v[2 * g + 1] = x.y;
+      }
+   }
+   __device__ __forceinline__ void store(double* p, bool all) const
+   {
+#pragma unroll
+      for(int g = 0; g < R; g++)
+         if(g == 0 || all) *reinterpret_cast<double2*>(p + 16 * g) = make_double2(v[2 * g], v[2 * g + 1]);
+   }
+   __device__ __forceinline__ void mac(double a, const Rows& x)
+   {
+#pragma unroll
+      for(int i = 0; i < 2 * R; i++) v[i] = fma(a, x.v[i], v[i]);
+   }
+   __device__ __forceinline__ void comb(double a, const Rows& x, double b, const Rows& y)
+   {
+#pragma unroll
+      for(int i = 0; i < 2 * R; i++) v[i] = fma(b, y.v[i], a * x.v[i]);
+   }
+};
+__device__ __forceinline__ void loadOps(const float* p, float (&e)[4])
+{
+   const float4 x = *reinterpret_cast<const float4*>(p);
+   e[0] = x.x; e[1] = x.y; e[2] = x.z; e[3] = x.w;
+}
+__device__ __forceinline__ void loadOps(const double* p, double (&e)[4])
+{
+   const double2 x = reinterpret_cast<const double2*>(p)[0], y = reinterpret_cast<const double2*>(p)[1];
+   e[0] = x.x; e[1] = x.y; e[2] = y.x; e[3] = y.y;
+}
+
+// One step: the quarter-warps of every warp task compute four outputs of a block for their 8 lanes' rows.
+template <class T, int R>
+__device__ __forceinline__ void runStep(const Task* tasks, int nTasks, int warp, int NW, int lane, const T* ops, const T* Win, T* Wout)
+{
+   constexpr int RS = rowStride<T>();
+   const int hl = lane & 7, quarter = lane >> 3;
+   const bool all = hl < 7;
+   Win += laneRows<T>() * hl;
+   Wout += laneRows<T>() * hl;
+   // dealt out back and forth: the tasks come longest first
+   for(int t0 = 0, t = warp; t0 < nTasks; t0 += NW, t = t0 + ((t0 / NW) & 1 ? NW - 1 - warp : warp))
+   {
+      if(t >= nTasks) continue;
+      const uint4 d = *reinterpret_cast<const uint4*>(tasks + 4 * t + quarter);
+      const T* x = Win + int(d.x & 0xFFFF) * RS;
+      const T* o = ops + 4 * int(d.y & 0xFFFF);
+      const int K = int(d.x >> 16);
+      Rows<T, R> acc[4];
+#pragma unroll
+      for(int q = 0; q < 4; q++) acc[q].zero();
+#pragma unroll 2
+      for(int k = 0; k < K; k += 2)
+      {
+#pragma unroll
+         for(int h = 0; h < 2; h++)
+         {
+            Rows<T, R> xv;
+            xv.load(x + (k + h) * RS);
+            T e[4];
+            loadOps(o + 4 * (k + h), e);
+#pragma unroll
+            for(int q = 0; q < 4; q++) acc[q].mac(e[q], xv);
+         }
+      }
+      const int out[4] = {int(d.z & 0xFFFF), int(d.z >> 16), int(d.w & 0xFFFF), int(d.w >> 16)};
+#pragma unroll
+      for(int q = 0; q < 4; q++)
+         if(out[q] != 0xFFFF) acc[q].store(Wout + out[q] * RS, all);
+   }
+}
+
+// Azimuth turn of the pairs (l, m), (l, -m) in degree-major order, in place: into the z frame (back = false) or out of it.
+template <class T, int R>
+__device__ __forceinline__ void turn(const unsigned* pairs, int nPairs, int warp, int NW, int lane, const T* Z, T* W, bool back)
+{
+   constexpr int RS = rowStride<T>();
+   const int hl = lane & 7, quarter = lane >> 3;
+   W += laneRows<T>() * hl;
+   for(int i = 4 * warp + quarter; i < nPairs; i += 4 * NW)
+   {
+      const unsigned d = pairs[i];
+      T* wc = W + int(d & 0x3FF) * RS;
+      T* ws = W + int(d >> 10 & 0x3FF) * RS;
+      const T c = Z[2 * (d >> 20)], s0 = Z[2 * (d >> 20) + 1], s = back ? -s0 : s0;
+      Rows<T, R> x, y, u, v;
+      x.load(wc);
+      y.load(ws);
+      u.comb(c, x, s, y);
+      v.comb(c, y, -s, x);
+      u.store(wc, hl < 7);
+      v.store(ws, hl < 7);
+   }
+}
+
+constexpr int MAXT = 40;      // target boxes of an M2L or M2M tile at most
+constexpr int MAXTL = 160;    // of an L2L tile
+template <class T>
+struct Smem   // byte offsets in the block's dynamic shared memory
+{
+   int w0, w1, tasks, pairs, pos, pads, total;
+   __host__ __device__ explicit Smem(int p)
+   {
+      constexpr int RS = rowStride<T>();
+      const int L = nharm(p);
+      int b = int(sizeof(T)) * Blob(p).size;
+      // one more position after the last block, and the last lane's reads past the last row
+      w0 = b; b += int(sizeof(T)) * (L + 2) * RS;
+      w1 = b; b += int(sizeof(T)) * (ordSize(p) + 1) * RS;
+      b = (b + 15) & ~15;
+      tasks = b; b += 3 * MAXTASK * int(sizeof(Task));
+      pairs = b; b += 4 * (p * (p + 1) / 2);
+      pads = b; b += 4 * (MAXORDER + 2);
+      pos = b; b += 2 * (padded(L));
+      total = (b + 15) & ~15;
+   }
+};
+
+__device__ __forceinline__ void cpAsync16(void* dst, const void* src)
+{
+   const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+// 2^-l of coefficient k's degree l (half that with `less`): a coefficient's own term in the M2M (L2L)
+template <class T>
+__device__ __forceinline__ T boxScale(int k, bool less)
+{
+   const int e = int(sqrtf(float(k) + 0.5f)) + (less ? 1 : 0);
+   if constexpr(sizeof(T) == 4) return __int_as_float((127 - e) << 23);
+   else return __longlong_as_double((1023ll - e) << 52);
+}
+
+struct L2LSegR { int start[9]; };
+
+// One tile of TT target boxes (blockIdx.x) and one part of its operators (blockIdx.y of gridDim.y). For every
+// operator with a source for some box of the tile the pairs are taken a chunk at a time, 20 (FP64: 10) pairs of 3
+// vectors, none of them empty: their source rows are gathered into shared memory [coefficient][vector],
+// turned about z in place, then the three steps (rotation, z translation, rotation back) alternate between two
+// such buffers, and the result is turned back and added to the targets' rows in global memory (one block owns
+// them; they stay in L2). A lane holds 8 (FP64: 4) vectors, a quarter-warp four outputs: per input
+// coefficient and lane three (FP64: four) 16-byte shared loads for 32 (16) multiply-adds, FP32 ones in
+// packed pairs. 16 warps an SM (two blocks of 8, one of 16 from p = 13 on, where one block fills the shared memory).
+// What bounds it (p = 12): ~17,000 warp instructions and ~3,000 shared-memory wavefronts a full chunk, 55 % of the issue
+// slots used; fewer warps were slower (8 an SM: 23.0 ms a solve of 2^20 points and targets, 12: 20.3, 16: 19.1), as was
+// a lane per vector with the inputs in registers and every block size unrolled (31.4 ms, instruction fetch).
+// Measured, dense operators on the CUDA cores -> this: M2L of 2^20 torus points, p = 12, FP32 55.4 -> 17.9 ms; 2^19
+// points, p = 16, 61.5 -> 23.6 ms; 65,536 points, p = 12, FP64 24.1 -> 2.6 ms; 2,000 points, p = 10, 3.4 -> 0.05 ms; L2L
+// of 2^24 points, p = 16, 13.4 -> 9.3 ms.
+//   MODE 0: M2L, X = multipoles, Y = locals (zero before); vtab[box][316], the tile's boxes are targets[..]
+//   MODE 1: M2M, X = Y = multipoles, the boxes are parents (zero before), vtab[parent][8] their children with sources
+//   MODE 2: L2L, X = Y = locals, one octant's operator (blockIdx.z); the boxes are its children, the source their parent
+// In the M2M and L2L a coefficient's own term (lambda = l) is the coefficient times a power of two: it is added as
+// it is, and only the other, smaller terms go through the rotations and their rounding (with it among them the
+// 2^24-point solve at p = 16 was 8.5e-7 off, without 7.7e-7 as with the dense operators).
+// gridDim.y > 1: the parts' sums go to ws[part][3 nTargets][Lp] (zero before) for kSumParts.
+template <class T, int MODE>
+__global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ targets, int nTargets,
+                                                    const int* __restrict__ vtab, const int* __restrict__ parent,
+                                                    const L2LSegR seg, int TT, int p, int Lp, const TaskTable* __restrict__ tasks,
+                                                    const T* __restrict__ ops, const T* X, T* Y, T* ws)
+{
+   constexpr int NOP = MODE == 0 ? 316 : 8;
+   constexpr int RS = rowStride<T>(), CH = chunkPairs<T>(), V = laneRows<T>();
+   extern __shared__ __align__(16) unsigned char smraw[];
+   constexpr int MT = MODE == 2 ? MAXTL : MAXT;
+   __shared__ int tileNode[MT];
+   __shared__ uint32_t present[10];
+   __shared__ int offs[NOP];
+   __shared__ int nOffS;
+   __shared__ int slotT[2][MAXT], slotS[2][MT], nSlot[2];
+   __shared__ int srcRow[2][RS], dstRow[2][RS];
+   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+   const int NT = blockDim.x, NW = NT >> 5;
+   const int L = nharm(p);
+   const Blob B(p);
+   int first = blockIdx.x * TT, end = nTargets;
+   if(MODE == 2)
+   {
+      first = seg.start[blockIdx.z] + blockIdx.x * TT;
+      end = seg.start[blockIdx.z + 1];
+      if(first >= end) return;
+   }
+   const int nTile = min(TT, end - first);
+   const Smem<T> sm(p);
+   T* D = reinterpret_cast<T*>(smraw);
+   T* W0 = reinterpret_cast<T*>(smraw + sm.w0);
+   T* W1 = reinterpret_cast<T*>(smraw + sm.w1);
+   Task* task = reinterpret_cast<Task*>(smraw + sm.tasks);
+   unsigned* pairs = reinterpret_cast<unsigned*>(smraw + sm.pairs);       // positions of (l, m), (l, -m), and m
+   int* pads = reinterpret_cast<int*>(smraw + sm.pads);                   // order-major pad positions, their number at [MAXORDER + 1]
+   unsigned short* pos = reinterpret_cast<unsigned short*>(smraw + sm.pos);   // degree-major position of k (L: none)
+   for(int t = tid; t < nTile; t += NT) tileNode[t] = targets[first + t];
+   if(tid < 10) present[tid] = 0;
+   const int nTask[3] = {tasks->n[0], tasks->n[1], tasks->n[2]};
+   for(int e = tid; e < 3 * MAXTASK; e += NT)
+      reinterpret_cast<uint4*>(task)[e] = reinterpret_cast<const uint4*>(&tasks->t[0][0])[e];
+   for(int k = tid; k < Lp; k += NT)
+   {
+      int l = int(sqrtf(float(k)));
+      while(l * l > k) l--;
+      while((l + 1) * (l + 1) <= k) l++;
+      const int m = k - l * l - l;
+      pos[k] = (unsigned short)(k < L ? degPos(l, m) : 0xFFFF);
+      if(k < L && m > 0) pairs[l * (l - 1) / 2 + m - 1] = unsigned(degPos(l, m)) | unsigned(degPos(l, -m)) << 10 | unsigned(m) << 20;
+   }
+   if(tid == 0)
+   {
+      int n = 0;
+      for(int a = 0; a <= p; a++)
+         if((p + 1 - a) & 1)
+         {
+            pads[n++] = ordBase(p, a) + p + 1 - a;
+            if(a) pads[n++] = ordBase(p, -a) + p + 1 - a;
+         }
+      pads[MAXORDER + 1] = n;
+   }
+   // (a zero operator row meets these: they must be numbers)
+   for(int e = tid; e < 2 * RS; e += NT) W0[L * RS + e] = T(0);
+   for(int e = tid; e < RS; e += NT) W1[ordSize(p) * RS + e] = T(0);
+   __syncthreads();
+   int o0 = 0, o1 = 1;
+   if(MODE == 2)
+   {
+      // every box has its pair: its parent
+      if(tid == 0) { offs[0] = blockIdx.z; nSlot[0] = nTile; }
+      for(int t = tid; t < nTile; t += NT) slotS[0][t] = parent[tileNode[t]];
+      __syncthreads();
+   }
+   else
+   {
+      // a warp per box, its table row in loads that are all in flight
+      constexpr int NWORD = (NOP + 31) / 32;
+      uint32_t have[NWORD] = {};
+      for(int t = warp; t < nTile; t += NW)
+      {
+         const int* row = vtab + int64_t(tileNode[t]) * NOP;
+         int v[NWORD];
+#pragma unroll
+         for(int w = 0; w < NWORD; w++) v[w] = lane + 32 * w < NOP ? row[lane + 32 * w] : -1;
+#pragma unroll
+         for(int w = 0; w < NWORD; w++) have[w] |= __ballot_sync(0xffffffffu, v[w] >= 0);
+      }
+      if(lane == 0)
+#pragma unroll
+         for(int w = 0; w < NWORD; w++)
+            if(have[w]) atomicOr(&present[w], have[w]);
+      __syncthreads();
+      if(warp == 0)
+      {
+         // the operators present, in order
+         int base = 0;
+         for(int w = 0; w * 32 < NOP; w++)
+         {
+            const uint32_t bits = present[w];
+            if(bits >> lane & 1) offs[base + __popc(bits & ((1u << lane) - 1))] = 32 * w + lane;
+            base += __popc(bits);
+         }
+         if(lane == 0) nOffS = base;
+      }
+      __syncthreads();
+      const int nOff = nOffS, parts = gridDim.y, part = blockIdx.y;
+      o0 = int(int64_t(nOff) * part / parts);
+      o1 = int(int64_t(nOff) * (part + 1) / parts);
+   }
+   if(o0 >= o1) return;
+   // source of the tile's box t for operator o
+   auto sourceOf = [&](int t, int o) {
+      if(t >= nTile) return -1;
+      return vtab[int64_t(tileNode[t]) * NOP + o];
+   };
+   // warp 0: the pairs of operator oi, compacted; the sources were loaded one operator earlier
+   int ahead[2] = {-1, -1};
+   auto loadAhead = [&](int oi) {
+      ahead[0] = sourceOf(lane, offs[oi]);
+      ahead[1] = sourceOf(lane + 32, offs[oi]);
+   };
+   auto compact = [&](int b) {
+      int n = 0;
+#pragma unroll
+      for(int h = 0; h < 2; h++)
+      {
+         const uint32_t bits = __ballot_sync(0xffffffffu, ahead[h] >= 0);
+         if(ahead[h] >= 0)
+         {
+            const int k = n + __popc(bits & ((1u << lane) - 1));
+            slotT[b][k] = lane + 32 * h;
+            slotS[b][k] = ahead[h];
+         }
+         n += __popc(bits);
+      }
+      if(lane == 0) nSlot[b] = n;
+   };
+   const bool toParts = gridDim.y > 1 && MODE != 2;
+   T* out = toParts ? ws + (int64_t(blockIdx.y) * nTargets + first) * 3 * Lp : Y;
+   // the rows of X a chunk's vectors come from and the rows of Y (or of this part's sums) they are added to
+   auto setRows = [&](int b, int c0, int nr, int db) {
+      if(tid < nr)
+      {
+         const int t = c0 + tid / 3, cmp = tid % 3;
+         srcRow[db][tid] = 3 * slotS[b][t] + cmp;
+         dstRow[db][tid] = 3 * (MODE == 2 ? tileNode[t] : toParts ? slotT[b][t] : tileNode[slotT[b][t]]) + cmp;
+      }
+   };
+   // rows and coefficients move between global and shared memory with 4 lanes of V consecutive coefficients
+   // by 8 rows
+   const int kl = V * (lane & 3), rl = lane >> 2, nkb = (Lp + 4 * V - 1) / (4 * V);
+   typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type VT;
+   auto gather = [&](const int* rows, int nr) {
+      for(int j = warp; j < nkb; j += NW)
+      {
+         const int k = 4 * V * j + kl;
+         int w[V];
+#pragma unroll
+         for(int i = 0; i < V; i++) w[i] = pos[k + i];
+         for(int r0 = rl; r0 < nr; r0 += 32)
+         {
+            VT x[4];
+#pragma unroll
+            for(int h = 0; h < 4; h++)
+               if(r0 + 8 * h < nr) x[h] = *reinterpret_cast<const VT*>(X + int64_t(rows[r0 + 8 * h]) * Lp + k);
+#pragma unroll
+            for(int h = 0; h < 4; h++)
+               if(r0 + 8 * h < nr)
+               {
+                  const T* xs = reinterpret_cast<const T*>(&x[h]);
+#pragma unroll
+                  for(int i = 0; i < V; i++)
+                     if(w[i] != 0xFFFF) W0[w[i] * RS + r0 + 8 * h] = xs[i];
+               }
+         }
+      }
+   };
+   auto addOut = [&](int db, int nr) {
+      const int* rows = dstRow[db];
+      for(int j = warp; j < nkb; j += NW)
+      {
+         const int k = 4 * V * j + kl;
+         int w[V];
+#pragma unroll
+         for(int i = 0; i < V; i++) w[i] = pos[k + i];
+         for(int r0 = rl; r0 < nr; r0 += 32)
+         {
+            VT y[4], id[4];
+            VT* q[4];
+#pragma unroll
+            for(int h = 0; h < 4; h++)
+               if(r0 + 8 * h < nr)
+               {
+                  q[h] = reinterpret_cast<VT*>(out + int64_t(rows[r0 + 8 * h]) * Lp + k);
+                  y[h] = *q[h];
+                  if(MODE != 0) id[h] = *reinterpret_cast<const VT*>(X + int64_t(srcRow[db][r0 + 8 * h]) * Lp + k);
+               }
+#pragma unroll
+            for(int h = 0; h < 4; h++)
+               if(r0 + 8 * h < nr)
+               {
+                  T* ys = reinterpret_cast<T*>(&y[h]);
+#pragma unroll
+                  for(int i = 0; i < V; i++)
+                     if(w[i] != 0xFFFF)
+                     {
+                        T v = W1[w[i] * RS + r0 + 8 * h];
+                        if(MODE != 0) v = fma(reinterpret_cast<const T*>(&id[h])[i], boxScale<T>(k + i, MODE == 2), v);
+                        ys[i] += v;
+                     }
+                  *q[h] = y[h];
+               }
+         }
+      }
+   };
+   if(MODE != 2 && warp == 0)
+   {
+      loadAhead(o0);
+      compact(0);
+      if(o0 + 1 < o1) loadAhead(o0 + 1);
+   }
+   __syncthreads();
+   int oi = o0, b = 0, c0 = 0, nPairs = nSlot[0], nr = 3 * min(CH, nPairs), prevRows = 0, chunk = 0;
+   setRows(0, 0, nr, 0);
+   __syncthreads();
+   const T* Z = D + B.zOff;
+   const int nTurn = p * (p + 1) / 2;
+   while(true)
+   {
+      if(c0 == 0)
+      {
+         const T* src = ops + int64_t(offs[oi]) * B.size;
+         for(int e = tid * V; e < B.size; e += NT * V) cpAsync16(D + e, src + e);
+         asm volatile("cp.async.commit_group;" ::: "memory");
+      }
+      if(chunk) addOut((chunk - 1) & 1, prevRows);
+      gather(srcRow[chunk & 1], nr);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      if(MODE != 2 && c0 == 0 && warp == 0 && oi + 1 < o1)
+      {
+         compact(b ^ 1);
+         if(oi + 2 < o1) loadAhead(oi + 2);
+      }
+      for(int e = tid; e < pads[MAXORDER + 1] * RS; e += NT) W1[pads[e / RS] * RS + e % RS] = T(0);
+      if(nr > 8 * V)
+      {
+         turn<T, 2>(pairs, nTurn, warp, NW, lane, Z, W0, false);
+         __syncthreads();
+         runStep<T, 2>(task, nTask[0], warp, NW, lane, D, W0, W1);
+         __syncthreads();
+         runStep<T, 2>(task + MAXTASK, nTask[1], warp, NW, lane, D, W1, W0);
+         __syncthreads();
+         runStep<T, 2>(task + 2 * MAXTASK, nTask[2], warp, NW, lane, D, W0, W1);
+         __syncthreads();
+         turn<T, 2>(pairs, nTurn, warp, NW, lane, Z, W1, true);
+      }
+      else
+      {
+         // at most one group of rows
+         turn<T, 1>(pairs, nTurn, warp, NW, lane, Z, W0, false);
+         __syncthreads();
+         runStep<T, 1>(task, nTask[0], warp, NW, lane, D, W0, W1);
+         __syncthreads();
+         runStep<T, 1>(task + MAXTASK, nTask[1], warp, NW, lane, D, W1, W0);
+         __syncthreads();
+         runStep<T, 1>(task + 2 * MAXTASK, nTask[2], warp, NW, lane, D, W0, W1);
+         __syncthreads();
+         turn<T, 1>(pairs, nTurn, warp, NW, lane, Z, W1, true);
+      }
+      // the next chunk
+      prevRows = nr;
+      chunk++;
+      c0 += CH;
+      if(c0 >= nPairs)
+      {
+         c0 = 0;
+         b ^= 1;
+         if(++oi < o1) nPairs = nSlot[b];
+      }
+      if(oi < o1)
+      {
+         nr = 3 * min(CH, nPairs - c0);
+         setRows(b, c0, nr, chunk & 1);
+      }
+      __syncthreads();
+      if(oi >= o1) break;
+   }
+   addOut((chunk - 1) & 1, prevRows);
+}
+
+// Y of every target row = the parts' sums in order.
+template <class T>
+__global__ void kSumParts(const int* __restrict__ targets, int nTargets, int parts, int Lp, const T* __restrict__ ws,
+                          T* __restrict__ Y)
+{
+   const int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+   const int64_t rowElems = 3 * int64_t(nTargets) * Lp;
+   if(e >= rowElems) return;
+   const int64_t row = e / Lp;
+   T s = T(0);
+   for(int q = 0; q < parts; q++) s += ws[q * rowElems + e];
+   Y[(int64_t(targets[row / 3]) * 3 + row % 3) * Lp + int(e % Lp)] = s;
+}
+
+}  // namespace rot
+
+// The rotation tables of the plan's order and degree cutoff, all 332 operators.
+template <class T>
+fmm_status ensureRotations(Plan& P, cudaStream_t st)
+{
+   // the full operator by default: a cutoff saves nothing here (fmm_config.m2l_tc_degree_cutoff); m2l_truncate
+   // stops at l + lambda = p
+   const int c = P.cfg.m2l_tc_degree_cutoff;
+   int cut = c <= 0 ? 2 * P.p : std::max(c, P.p);
+   if(P.cfg.m2l_truncate) cut = std::min(cut, P.p);
+   cut = std::min(cut, 2 * P.p);
+   if(P.rotCut == cut) return FMM_OK;
+   const rot::Blob B(P.p);
+   const std::vector<double>& q = rot::quarterTurn();
+   FMM_TRY(P.rotQuarter.reserve(sizeof(double) * q.size()));
+   FMM_TRY(P.rotOps.reserve(sizeof(T) * size_t(B.size) * (16 + 316)));
+   // the step tasks of the M2L and of the M2M / L2L
+   P.rotTaskHost.resize(2 * sizeof(rot::TaskTable));
+   for(int mode = 0; mode < 2; mode++)
+      rot::makeTasks(P.p, mode, reinterpret_cast<rot::TaskTable*>(P.rotTaskHost.data())[mode]);
+   FMM_TRY(P.rotTasks.reserve(P.rotTaskHost.size()));
+   FMM_CUDA(cudaMemcpyAsync(P.rotTasks.ptr, P.rotTaskHost.data(), P.rotTaskHost.size(), cudaMemcpyHostToDevice, st));
+   FMM_CUDA(cudaMemcpyAsync(P.rotQuarter.ptr, q.data(), sizeof(double) * q.size(), cudaMemcpyHostToDevice, st));
+   rot::kBuildRotations<T><<<16 + 316, 256, 0, st>>>(P.p, cut, (const double*)P.rotQuarter.ptr, (T*)P.rotOps.ptr);
+   FMM_TRY(launched(P, "kBuildRotations", st));
+   P.rotCut = cut;
+   return FMM_OK;
+}
+
+// Boxes of a tile, and into how many parts the operators of a tile are split (a part is a block; their sums meet
+// in kSumParts). FP32 tiles of one chunk's boxes and of two measured within 2 % of each other (2^20 points, p = 12:
+// 19.1 and 19.6 ms a solve), FP64 ones 4.13 and 4.05 ms (65,536 points, p = 10). Parts: four rounds of
+// resident blocks, so that small trees fill the chip (2,000 points, p = 10: M2L 54 us; one block a tile took over 1 ms)
+// and larger ones have no long last round.
+template <class T> static int rotTile(int mode) { return rot::chunkPairs<T>() * (mode == 0 && sizeof(T) == 8 ? 4 : 1); }
+template <class T>
+static int rotPerSM(const Plan& P) { return std::max(1, std::min(2, (227 * 1024) / (rot::Smem<T>(P.p).total + 6 * 1024))); }
+template <class T>
+static int rotParts(const Plan& P, int mode, int count)
+{
+   const int tile = rotTile<T>(mode), tiles = (count + tile - 1) / tile;
+   if(tiles == 0) return 1;
+   return std::max(1, std::min(mode == 0 ? 64 : 8, 4 * 148 * rotPerSM<T>(P) / tiles));
+}
+
+// Room for the parts' sums of every launch on the current tree, so that none of them allocates.
+template <class T>
+fmm_status reserveRotations(Plan& P)
+{
+   const bool tc = !P.fp64 && P.cfg.m2l_mode != FMM_M2L_SIMT;   // M2L (and M2M) on the tensor cores
+   if(tc && P.tcTranslations(1)) return FMM_OK;
+   size_t rows = 0;
+   auto need = [&](int mode, int count) {
+      const int parts = rotParts<T>(P, mode, count);
+      if(parts > 1) rows = std::max(rows, size_t(parts) * 3 * size_t(count));
+   };
+   if(!tc) need(0, P.nM2LTargets);
+   for(int level = 0; level + 1 < P.tree.nLevels; level++) need(1, P.parStart[level + 1] - P.parStart[level]);
+   return rows ? P.rotWs.reserve(sizeof(T) * rows * P.Lp) : FMM_OK;
+}
+
+template <class T, int MODE>
+static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int count, const int* vtab, const rot::L2LSegR& seg,
+                            int most, const T* X, T* Y)
+{
+   const rot::Blob B(P.p);
+   const size_t smem = rot::Smem<T>(P.p).total;
+   const int THREADS = rotPerSM<T>(P) == 1 ? 512 : 256;   // 16 warps an SM either way
+   auto kern = rot::kRotTranslate<T, MODE>;
+   FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+   const T* ops = (const T*)P.rotOps.ptr + size_t(B.size) * (MODE == 0 ? 16 : MODE == 1 ? 0 : 8);
+   const rot::TaskTable* tasks = (const rot::TaskTable*)P.rotTasks.ptr + (MODE == 0 ? 0 : 1);
+   const int tile = rotTile<T>(MODE);
+   if(MODE == 2)
+   {
+      // up to eight chunks a block, which loads the octant's tables once, while that leaves four rounds of blocks
+      const int chunk = rot::chunkPairs<T>(), all = seg.start[8] - seg.start[0];
+      const int tl = chunk * std::max(1, std::min(rot::MAXTL / chunk, all / (chunk * 4 * 148 * rotPerSM<T>(P))));
+      kern<<<dim3((most + tl - 1) / tl, 1, 8), THREADS, smem, st>>>(targets, 0, nullptr, P.tree.parent, seg, tl, P.p, P.Lp,
+                                                                   tasks, ops, X, Y, nullptr);
+      return launched(P, "kRotTranslate<L2L>", st);
+   }
+   const int tiles = (count + tile - 1) / tile, parts = rotParts<T>(P, MODE, count);
+   const int64_t n = 3 * int64_t(count) * P.Lp;
+   if(parts > 1) FMM_CUDA(cudaMemsetAsync(P.rotWs.ptr, 0, sizeof(T) * size_t(parts) * n, st));
+   kern<<<dim3(tiles, parts), THREADS, smem, st>>>(targets, count, vtab, P.tree.parent, seg, tile, P.p, P.Lp, tasks, ops, X, Y,
+                                                   (T*)P.rotWs.ptr);
+   FMM_TRY(launched(P, MODE == 0 ? "kRotTranslate<M2L>" : "kRotTranslate<M2M>", st));
+   if(parts > 1)
+   {
+      rot::kSumParts<T><<<int((n + 255) / 256), 256, 0, st>>>(targets, count, parts, P.Lp, (const T*)P.rotWs.ptr, Y);
+      FMM_TRY(launched(P, "kSumParts", st));
+   }
+   return FMM_OK;
+}
+
+template <class T>
+fmm_status rotM2L(Plan& P, cudaStream_t st)
+{
+   if(P.nM2LTargets <= 0) return FMM_OK;
+   return launchRot<T, 0>(P, st, (const int*)P.m2lTargets.ptr, P.nM2LTargets, P.lists.vtab, rot::L2LSegR{}, 0,
+                          (const T*)P.mult.ptr, (T*)P.local.ptr);
+}
+
+template <class T>
+fmm_status rotM2M(Plan& P, cudaStream_t st)
+{
+   for(int level = P.tree.nLevels - 2; level >= 0; level--)
+   {
+      const int a = P.parStart[level], b = P.parStart[level + 1];
+      if(b <= a) continue;
+      FMM_TRY((launchRot<T, 1>(P, st, (const int*)P.parList.ptr + a, b - a, (const int*)P.vtabUp.ptr, rot::L2LSegR{}, 0,
+                               (const T*)P.mult.ptr, (T*)P.mult.ptr)));
+   }
+   FMM_CHECK_LAUNCH();
+   return FMM_OK;
+}
+
+template <class T>
+fmm_status rotL2L(Plan& P, cudaStream_t st)
+{
+   for(int level = 0; level + 1 < P.tree.nLevels; level++)
+   {
+      rot::L2LSegR seg;
+      int most = 0;
+      for(int o = 0; o <= 8; o++) seg.start[o] = P.l2lStart[8 * (level + 1) + o];
+      for(int o = 0; o < 8; o++) most = std::max(most, seg.start[o + 1] - seg.start[o]);
+      if(most == 0) continue;
+      FMM_TRY((launchRot<T, 2>(P, st, (const int*)P.l2lTargets.ptr, 0, nullptr, seg, most, (const T*)P.local.ptr, (T*)P.local.ptr)));
+   }
+   FMM_CHECK_LAUNCH();
+   return FMM_OK;
+}
+
+template fmm_status ensureRotations<float>(Plan&, cudaStream_t);
+template fmm_status ensureRotations<double>(Plan&, cudaStream_t);
+template fmm_status reserveRotations<float>(Plan&);
+template fmm_status reserveRotations<double>(Plan&);
+template fmm_status rotM2L<float>(Plan&, cudaStream_t);
+template fmm_status rotM2L<double>(Plan&, cudaStream_t);
+template fmm_status rotM2M<float>(Plan&, cudaStream_t);
+template fmm_status rotM2M<double>(Plan&, cudaStream_t);
+template fmm_status rotL2L<float>(Plan&, cudaStream_t);
+template fmm_status rotL2L<double>(Plan&, cudaStream_t);
+
+}  // namespace fmm

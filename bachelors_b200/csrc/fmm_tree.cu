@@ -905,7 +905,7 @@ __global__ void kTranslateTables(Tree t, int nNodes, int* __restrict__ up, int* 
    if(par < 0) return;
    const int o = int(t.key[i] & 7);
    if(t.s1[i] > t.s0[i]) up[int64_t(par) * 8 + o] = i;
-   if(t.t1[i] > t.t0[i]) dn[int64_t(i) * 8 + o] = par;
+   if(dn && t.t1[i] > t.t0[i]) dn[int64_t(i) * 8 + o] = par;
 }
 // Keys (level, octant) of the nodes with targets below the roots; the rest sort last.
 __global__ void kL2LTargetKeys(Tree t, int nNodes, unsigned* keys, int* vals)
@@ -1340,15 +1340,16 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
    // M2M / L2L tables: the L2L child lists always (both L2L forms use them), the octant tables
    // for the tensor-core forms
    {
-      if(P.tcTranslations())
+      const bool dn = P.tcTranslations(2);
+      FMM_TRY(P.vtabUp.reserve(sizeof(int) * 8 * size_t(nn)));
+      FMM_CUDA(cudaMemsetAsync(P.vtabUp.ptr, 0xff, sizeof(int) * 8 * size_t(nn), st));
+      if(dn)
       {
-         FMM_TRY(P.vtabUp.reserve(sizeof(int) * 8 * size_t(nn)));
          FMM_TRY(P.vtabDn.reserve(sizeof(int) * 8 * size_t(nn)));
-         FMM_CUDA(cudaMemsetAsync(P.vtabUp.ptr, 0xff, sizeof(int) * 8 * size_t(nn), st));
          FMM_CUDA(cudaMemsetAsync(P.vtabDn.ptr, 0xff, sizeof(int) * 8 * size_t(nn), st));
-         kTranslateTables<<<(nn + 255) / 256, 256, 0, st>>>(t, nn, (int*)P.vtabUp.ptr, (int*)P.vtabDn.ptr);
-         FMM_TRY(launched(P, "kTranslateTables", st));
       }
+      kTranslateTables<<<(nn + 255) / 256, 256, 0, st>>>(t, nn, (int*)P.vtabUp.ptr, dn ? (int*)P.vtabDn.ptr : nullptr);
+      FMM_TRY(launched(P, "kTranslateTables", st));
       FMM_TRY(P.l2lTargets.reserve(2 * sizeof(int) * nn));
       FMM_TRY(P.l2lKeys.reserve(2 * sizeof(unsigned) * nn));
       unsigned* kk = (unsigned*)P.l2lKeys.ptr;
@@ -1378,7 +1379,7 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_TRY(launched(P, "kGatherSources", st));
       FMM_CHECK_LAUNCH();
    }
-   return FMM_OK;
+   return reserveRotations<T>(P);
 }
 
 template fmm_status buildTreeT<float>(Plan&, cudaStream_t);

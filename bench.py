@@ -640,7 +640,7 @@ def main():
             # the comparator's own roofline: the same executed M2L operator on the CUDA cores (FP32 FMA)
             fp32_peak = fp32_core_peak_tflops(peaks.get("sm_max_mhz", 1965.0))
             ach32 = flops_m2l / (pf["ms_m2l"] / 1000.0) / 1e12
-            pf["roofline"] = {"kernel": "M2L (simt, kM2LSimt)", "bound": "fp32", "achieved": ach32, "peak": fp32_peak,
+            pf["roofline"] = {"kernel": "M2L (CUDA cores, kRotTranslate; FLOPs of the dense operator)", "bound": "fp32", "achieved": ach32, "peak": fp32_peak,
                               "unit": "TFLOP/s", "frac": ach32 / fp32_peak,
                               "note": "peak = nominal FP32 FMA rate of the CUDA cores, 148 SMs x 128 lanes x 2 x "
                                       "max SM clock (not in MEASURED_PEAKS.json); same FLOP count as the headline"}
