@@ -270,6 +270,9 @@ struct Plan
    Plan* adj = nullptr;
    DevBuf adjG, adjOut;
    DevBuf tcPts, tcOut;                  // fmm_treecode: staging of host query points and results
+   DevBuf tcCurl, tcSort;                // its curl table (order tcCurlOrder) and the sorted points' keys and order
+   std::vector<unsigned char> tcCurlHost;   // host copy of tcCurl (kept for the asynchronous upload)
+   int tcCurlOrder = -1;
    bool adjointDone = false;
 
    // fmm_set_sources_async: the host inputs cross the bus on copyStream while the solve runs; the

@@ -7,218 +7,420 @@
 // acceptance test), any other box through its children; a leaf that fails the test is summed directly
 // (by default) or contributes nothing (FMM_TREECODE_REFERENCE_NEAR, as the reference, which loses
 // 10-19 % near its sources). With box-size scaled multipoles (a box of side h keeps M~_l = M_l / h^l)
-// a box's potential at x is (1/h) sum_k M~_k I_k(u), u = (x - c) / h; its gradient, for B = curl A,
-// comes from the same irregular-harmonic recurrence run on dual numbers (value and three partial
-// derivatives), or by central differences of A with step 1e-3 as the reference does
-// (FMM_TREECODE_FD_CURL).
+// a box's potential at x is (1/h) sum_k M~_k I_k(u), u = (x - c) / h. B = curl A is again a sum of irregular
+// harmonics, one degree higher: with T_l^m the complex irregular harmonic of fmm_common.cuh,
+//   d/dz T_l^m = -T_{l+1}^m,   (d/dx + i d/dy) T_l^m = -T_{l+1}^{m+1},   (d/dx - i d/dy) T_l^m = T_{l+1}^{m-1} (m >= 1),
+// so a box's curl expansion is a fixed combination of at most four multipole coefficients per entry, made
+// once per box and group of points, and a point costs one harmonic recurrence. Or B comes by central differences of
+// A with step 1e-3 as the reference does (FMM_TREECODE_FD_CURL).
 //
-// One thread per query point, an explicit stack of boxes in local memory.
+// A block takes W query points (1..32, neighbours in Morton order where W > 1) and walks the tree for all of them
+// at once: a box on the block's stack carries the mask of the points that reached it. A batch of boxes is tested a
+// thread per box; the points a box is far from meet it as one entry of the far list, a leaf's others as
+// one of the near list, and the rest go to its children. The far entries are dealt out to the warps (curl
+// expansion into shared memory, then a point per lane, 32 / W lanes sharing a point's orders), the near leaves'
+// sources are staged in shared memory in FP64 and split over all lanes. The sums meet in a fixed order.
+//
+// What bounds it: the FP64 near sum (~30 FP64 instructions a pair) and the FP32 far evaluation (~18 instructions a
+// harmonic). With a thread per point walking alone, evaluating value and gradient by dual numbers and reading
+// its boxes' multipoles itself, the few points near the sources kept their warps for the whole call. Measured, that ->
+// this, 262,144 sources, p = 10, FP32: leaves of 1000, 65,536 points 23.4 -> 2.65 ms, 1,000 points 16.6 -> 0.45 ms, one
+// point 0.39 -> 0.03 ms; leaves of 100, 65,536 points 11.5 -> 7.3 ms, 10,000 points 8.3 -> 3.6 ms; FP64, leaves of 1000,
+// 65,536 points 40 -> 3.2 ms.
+#include <cub/cub.cuh>
+
 #include "fmm_internal.cuh"
 
 namespace fmm {
 
 namespace {
 
-// value and gradient (d/dx, d/dy, d/dz) of a scalar
+constexpr int TC_NT = 256, TC_WARPS = TC_NT / 32;
+// Boxes on a block's stack. A batch pops at most (room left - 200) / 7 boxes, at least one, and pushes at most 8 for
+// each; one box at a time adds at most 7 a level (147 in 21 levels) before the stack is shorter again.
+constexpr int TC_STACK = 1536;
+constexpr int TC_SRC = 256;     // sources staged at a time
+
+// The curl (entries of degree <= p + 1) of the expansion sum_k M_k I_k as terms of the multipole row [3][Lp], with
+// the real-basis factors (-1)^l sqrt2 folded in: entry [k'][component], at most four terms.
 template <class T>
-struct Dual
+struct CurlTerm
 {
-   T v, x, y, z;
+   int idx[4];
+   T c[4];
 };
-template <class T> __device__ __forceinline__ Dual<T> dAdd(Dual<T> a, Dual<T> b) { return {a.v + b.v, a.x + b.x, a.y + b.y, a.z + b.z}; }
-template <class T> __device__ __forceinline__ Dual<T> dSub(Dual<T> a, Dual<T> b) { return {a.v - b.v, a.x - b.x, a.y - b.y, a.z - b.z}; }
-template <class T> __device__ __forceinline__ Dual<T> dScale(Dual<T> a, T s) { return {a.v * s, a.x * s, a.y * s, a.z * s}; }
-template <class T> __device__ __forceinline__ Dual<T> dMul(Dual<T> a, Dual<T> b)
-{
-   return {a.v * b.v, a.x * b.v + a.v * b.x, a.y * b.v + a.v * b.y, a.z * b.v + a.v * b.z};
-}
-// acc += s a
-template <class T> __device__ __forceinline__ void dAxpy(Dual<T>& acc, T s, Dual<T> a)
-{
-   acc.v += s * a.v; acc.x += s * a.x; acc.y += s * a.y; acc.z += s * a.z;
-}
 
-constexpr int TC_STACK = 192;   // 7 siblings a level x 21 levels + the root, with room to spare
-constexpr int TC_NT = 128;
-
-// sum_k M~[c][k] I_k(u) for the three components c, with gradients with respect to u, in the standard
-// real irregular convention (I_l^0 = (-1)^l Re T_l^0, I_l^{+-m} = (-1)^l sqrt2 {Re, Im} T_l^m, T the
-// complex irregular harmonic of fmm_common.cuh, whose recurrence this runs on dual numbers).
-template <class T, bool GRAD>
-__device__ void irregularSum(int p, int Lp, const T* __restrict__ M, T ux, T uy, T uz, Dual<T> acc[3])
+template <class T>
+std::vector<CurlTerm<T>> curlTerms(int p, int Lp)
 {
-   const T sq2 = T(1.4142135623730950488);
-   const Dual<T> X{ux, T(1), T(0), T(0)}, Y{uy, T(0), T(1), T(0)}, Z{uz, T(0), T(0), T(1)};
-   const T r2 = ux * ux + uy * uy + uz * uz;
-   const T i2 = T(1) / r2, ir = sqrt(i2);
-   // 1 / r^2 and 1 / r as duals
-   const Dual<T> IR2{i2, -T(2) * ux * i2 * i2, -T(2) * uy * i2 * i2, -T(2) * uz * i2 * i2};
-   const T ir3 = ir * i2;
-   Dual<T> dre{ir, -ux * ir3, -uy * ir3, -uz * ir3}, dim{T(0), T(0), T(0), T(0)};   // T_m^m
-   for(int c = 0; c < 3; c++) acc[c] = {T(0), T(0), T(0), T(0)};
-   for(int m = 0; m <= p; m++)
+   const int q = p + 1;
+   std::vector<CurlTerm<T>> tab(size_t(nharm(q)) * 4);
+   // A = sum a_lm Re T_l^m + b_lm Im T_l^m; a (im = 0) or b (im = 1) of degree l, order m as a multiple of a coefficient
+   auto put = [&](CurlTerm<T>& e, int& n, double f, int comp, int l, int m, int im) {
+      if(l < 0 || m > l || m < 0 || (im && m == 0)) return;
+      e.idx[n] = comp * Lp + hidx(l, im ? -m : m);
+      e.c[n] = T(f * ((l & 1) ? -1.0 : 1.0) * (m ? 1.4142135623730950488 : 1.0));
+      n++;
+   };
+   for(int k = 0; k < nharm(q); k++)
    {
-      if(m > 0)
-      {
-         // T_m^m = (2m - 1) (x + i y) T_{m-1}^{m-1} / r^2
-         const T f = T(2 * m - 1);
-         const Dual<T> nre = dMul(dSub(dMul(X, dre), dMul(Y, dim)), IR2);
-         const Dual<T> nim = dMul(dAdd(dMul(X, dim), dMul(Y, dre)), IR2);
-         dre = dScale(nre, f);
-         dim = dScale(nim, f);
-      }
-      Dual<T> are = dre, aim = dim, bre{T(0), T(0), T(0), T(0)}, bim{T(0), T(0), T(0), T(0)};
-      for(int l = m; l <= p; l++)
-      {
-         const T s = (l & 1) ? T(-1) : T(1);
-         if(m == 0)
+      int l = 0;
+      while((l + 1) * (l + 1) <= k) l++;
+      const int mu = abs(k - l * l - l), im = k - l * l - l < 0;   // entry: Re (im = 0) or Im T_l^mu
+      // its coefficient in d/dx_j of component c (times f), from degree l - 1
+      auto deriv = [&](CurlTerm<T>& e, int& n, double f, int c, int j) {
+         if(j == 2) put(e, n, -f, c, l - 1, mu, im);
+         else if(j == 0)
          {
-            const int k = l * l + l;
-            for(int c = 0; c < 3; c++) dAxpy(acc[c], s * M[c * Lp + k], are);
+            if(mu >= 1) put(e, n, mu == 1 && !im ? -f : -0.5 * f, c, l - 1, mu - 1, im);
+            put(e, n, 0.5 * f, c, l - 1, mu + 1, im);
+         }
+         else if(im)
+         {
+            put(e, n, mu == 1 ? -f : -0.5 * f, c, l - 1, mu - 1, 0);
+            put(e, n, -0.5 * f, c, l - 1, mu + 1, 0);
          }
          else
          {
-            const int kp = l * l + l + m, km = l * l + l - m;
-            for(int c = 0; c < 3; c++)
-            {
-               dAxpy(acc[c], s * sq2 * M[c * Lp + kp], are);
-               dAxpy(acc[c], s * sq2 * M[c * Lp + km], aim);
-            }
+            put(e, n, 0.5 * f, c, l - 1, mu - 1, 1);
+            put(e, n, 0.5 * f, c, l - 1, mu + 1, 1);
          }
-         if(l == p) break;
-         Dual<T> cre, cim;
-         if(l == m)
-         {
-            const T f = T(2 * m + 1);
-            cre = dScale(dMul(dMul(Z, are), IR2), f);
-            cim = dScale(dMul(dMul(Z, aim), IR2), f);
-         }
-         else
-         {
-            const T f = T(2 * l + 1), g = T((l + m) * (l - m));
-            cre = dMul(dSub(dScale(dMul(Z, are), f), dScale(bre, g)), IR2);
-            cim = dMul(dSub(dScale(dMul(Z, aim), f), dScale(bim, g)), IR2);
-         }
-         bre = are; bim = aim; are = cre; aim = cim;
+      };
+      for(int c = 0; c < 3; c++)
+      {
+         CurlTerm<T>& e = tab[4 * size_t(k) + c];
+         e = CurlTerm<T>{};
+         int n = 0;
+         deriv(e, n, 1.0, (c + 2) % 3, (c + 1) % 3);
+         deriv(e, n, -1.0, (c + 1) % 3, (c + 2) % 3);
       }
+      tab[4 * size_t(k) + 3] = CurlTerm<T>{};
    }
-   (void)GRAD;
+   return tab;
 }
+
+// Walks T_l^m(ux, uy, uz) for m = g, g + G, .. <= q and l = m..q and calls f(k of (l, m), k of (l, -m), re, im, l). The
+// recurrence's integer factors are kept as running sums in T.
+template <class T, class F>
+__device__ __forceinline__ void visitIrregular(int q, int g, int G, T ux, T uy, T uz, F&& f)
+{
+   const T r2 = ux * ux + uy * uy + uz * uz;
+   const T i2 = T(1) / r2;
+   const T zi = uz * i2, xi = ux * i2, yi = uy * i2;
+   T dre = sqrt(i2), dim = T(0);   // T_m^m
+   int m = 0;
+   T odd = T(1);                   // 2 m + 1
+   auto diag = [&]() {
+      const T nre = odd * (xi * dre - yi * dim), nim = odd * (xi * dim + yi * dre);
+      dre = nre; dim = nim;
+      odd += T(2);
+      m++;
+   };
+   while(m < g && m < q) diag();
+   if(m < g) return;
+   while(true)
+   {
+      T are = dre, aim = dim, bre = T(0), bim = T(0);
+      T c1 = odd, c2 = T(0);       // 2 l + 1, l^2 - m^2
+      for(int l = m, k0 = m * m + 2 * m, k1 = m * m;; l++)
+      {
+         f(k0, k1, are, aim, l);
+         if(l == q) break;
+         const T az = c1 * zi, bz = c2 * i2;
+         const T cre = az * are - bz * bre, cim = az * aim - bz * bim;
+         bre = are; bim = aim; are = cre; aim = cim;
+         c2 += c1;
+         c1 += T(2);
+         k0 += 2 * l + 2; k1 += 2 * l + 2;
+      }
+      if(m + G > q) break;
+      for(int j = 0; j < G; j++) diag();
+   }
+}
+
+template <class T>
+struct TcSmem
+{
+   int stackN, stackM, farN, farM, nearN, nearM, pts, src, warp0, perWarp, total;
+   __host__ __device__ TcSmem(int p, bool wantA)
+   {
+      int b = 0;
+      auto take = [&](int bytes) { const int at = b; b += (bytes + 15) & ~15; return at; };
+      stackN = take(4 * TC_STACK);
+      stackM = take(4 * TC_STACK);
+      farN = take(4 * TC_NT);
+      farM = take(4 * TC_NT);
+      nearN = take(4 * TC_NT);
+      nearM = take(4 * TC_NT);
+      pts = take(8 * 3 * 32);
+      src = take(8 * 8 * TC_SRC);            // also the warps' sums at the end: [TC_WARPS][32][6]
+      warp0 = b;
+      // per warp: the curl expansion [(p + 2)^2][4] and the potential's [(p + 1)^2][4]
+      perWarp = int(sizeof(T)) * (4 * nharm(p + 1) + (wantA ? 4 * nharm(p) : 0));
+      perWarp = (perWarp + 31) & ~31;
+      b = (b + 31) & ~31;
+      warp0 = b;
+      total = warp0 + TC_WARPS * perWarp;
+   }
+};
 
 template <class T>
 __global__ void __launch_bounds__(TC_NT) kTreecode(Tree t, const RootBox* __restrict__ rootp, int p, int Lp,
-                                                   const T* __restrict__ mult, const typename Vec4<T>::type* __restrict__ spos,
+                                                   const T* __restrict__ mult, const CurlTerm<T>* __restrict__ curl,
+                                                   const typename Vec4<T>::type* __restrict__ spos,
                                                    const typename Vec4<T>::type* __restrict__ sq, const T* __restrict__ pts,
-                                                   int64_t m, int flags, T scaleB, T scaleA, int want, int bem,
-                                                   T* __restrict__ outB, T* __restrict__ outA, int* err)
+                                                   const int* __restrict__ order, int64_t m, int W, int flags, T scaleB,
+                                                   T scaleA, int want, int bem, T* __restrict__ outB, T* __restrict__ outA)
 {
-   const int64_t qi = blockIdx.x * int64_t(TC_NT) + threadIdx.x;
-   if(qi >= m) return;
+   typedef typename Vec4<T>::type V4;
+   typedef cub::BlockScan<int, TC_NT> Scan;
+   extern __shared__ __align__(32) unsigned char smraw[];
+   __shared__ typename Scan::TempStorage scanTmp;
    const bool refNear = flags & 1, fdCurl = flags & 2;
+   const bool wantB = want & 1, wantA = (want & 2) != 0, curlB = wantB && !fdCurl, potA = wantA || fdCurl;
+   const TcSmem<T> sm(p, potA);
+   int* stackN = reinterpret_cast<int*>(smraw + sm.stackN);
+   unsigned* stackM = reinterpret_cast<unsigned*>(smraw + sm.stackM);
+   int* farN = reinterpret_cast<int*>(smraw + sm.farN);
+   unsigned* farM = reinterpret_cast<unsigned*>(smraw + sm.farM);
+   int* nearN = reinterpret_cast<int*>(smraw + sm.nearN);
+   unsigned* nearM = reinterpret_cast<unsigned*>(smraw + sm.nearM);
+   double* P = reinterpret_cast<double*>(smraw + sm.pts);       // [3][32]
+   double* S = reinterpret_cast<double*>(smraw + sm.src);       // [TC_SRC][8]
+   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+   V4* Cs = reinterpret_cast<V4*>(smraw + sm.warp0 + warp * sm.perWarp);
+   V4* As = Cs + nharm(p + 1);
+   const int64_t q0 = int64_t(blockIdx.x) * W;
+   const int nq = int(min(int64_t(W), m - q0));
+   const int G = 32 / W, j = lane % W, g = lane / W;
+   if(tid < 32)
+   {
+      const int64_t i = q0 + min(tid, nq - 1);
+      const int64_t src = order ? order[i] : i;
+      for(int d = 0; d < 3; d++) P[32 * d + tid] = double(pts[3 * src + d]);
+   }
    const RootBox rb = rootp[0];
-   const double x = double(pts[3 * qi]), y = double(pts[3 * qi + 1]), z = double(pts[3 * qi + 2]);
-   double A[3] = {0, 0, 0}, G[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};   // A_c and dA_c / dx_j
-   double Bn[3] = {0, 0, 0};                                              // direct near-field B
-   int stack[TC_STACK];
-   int top = 0;
-   for(int r = t.levelStart[0]; r < t.levelStart[1]; r++) stack[top++] = r;
+   const unsigned all = nq == 32 ? 0xffffffffu : (1u << nq) - 1u;
+   int count = 0;
+   for(int r = t.levelStart[0]; r < t.levelStart[1]; r++)
+   {
+      if(tid == 0) { stackN[count] = r; stackM[count] = all; }
+      count++;
+   }
+   __syncthreads();
+   const double x = P[j], y = P[32 + j], z = P[64 + j];
+   double A[3] = {0, 0, 0}, B[3] = {0, 0, 0};
    const T eps = T(1e-3);   // the reference's math::eps for the central differences
-   while(top > 0)
+   auto centre = [&](int node, double& h, double& cx, double& cy, double& cz) {
+      h = 2.0 * rb.H / double(int64_t(1) << t.level[node]);
+      cx = rb.center[0] - rb.H + (double(t.ix[node]) + 0.5) * h;
+      cy = rb.center[1] - rb.H + (double(t.iy[node]) + 0.5) * h;
+      cz = rb.center[2] - rb.H + (double(t.iz[node]) + 0.5) * h;
+   };
+   while(count > 0)
    {
-      const int node = stack[--top];
-      const int level = t.level[node];
-      const double h = 2.0 * rb.H / double(int64_t(1) << level);
-      const double cx = rb.center[0] - rb.H + (double(t.ix[node]) + 0.5) * h;
-      const double cy = rb.center[1] - rb.H + (double(t.iy[node]) + 0.5) * h;
-      const double cz = rb.center[2] - rb.H + (double(t.iz[node]) + 0.5) * h;
-      const double dx = x - cx, dy = y - cy, dz = z - cz;
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      const double r2 = 3.0 * 0.25 * h * h;   // half-diagonal^2: three half-widths h / 2
-      if(4.0 * r2 < d2)
+      // a batch from the top of the stack, a thread per box
+      const int batch = min(count, max(1, min(TC_NT, (TC_STACK - 200 - count) / 7)));
+      const int base = count - batch;
+      int node = -1, c0 = 0, nc = 0;
+      unsigned farMask = 0, rest = 0;
+      if(tid < batch)
       {
-         const T* M = mult + int64_t(node) * 3 * Lp;
-         const double ih = 1.0 / h;
-         if(!fdCurl)
+         node = stackN[base + tid];
+         const unsigned mask = stackM[base + tid];
+         if(t.s1[node] > t.s0[node])
          {
-            Dual<T> acc[3];
-            irregularSum<T, true>(p, Lp, M, T(dx * ih), T(dy * ih), T(dz * ih), acc);
-            for(int c = 0; c < 3; c++)
+            double h, cx, cy, cz;
+            centre(node, h, cx, cy, cz);
+            const double r2 = 3.0 * 0.25 * h * h;   // half-diagonal^2: three half-widths h / 2
+            for(unsigned left = mask; left; left &= left - 1)
             {
-               A[c] += double(acc[c].v) * ih;
-               G[c][0] += double(acc[c].x) * ih * ih;
-               G[c][1] += double(acc[c].y) * ih * ih;
-               G[c][2] += double(acc[c].z) * ih * ih;
+               const int i = __ffs(left) - 1;
+               const double dx = P[i] - cx, dy = P[32 + i] - cy, dz = P[64 + i] - cz;
+               const double d2 = dx * dx + dy * dy + dz * dz;
+               if(4.0 * r2 < d2) farMask |= 1u << i;
             }
+            rest = mask & ~farMask;
+            if(rest) { nc = t.nchild[node]; c0 = t.child0[node]; }
          }
-         else
+      }
+      const bool near = rest && nc == 0 && !refNear;
+      // far entries, near leaves and children in one scan: 9, 9 and 12 bits
+      int at, total;
+      Scan(scanTmp).ExclusiveSum((farMask ? 1 : 0) | (near ? 1 << 9 : 0) | (rest ? nc << 18 : 0), at, total);
+      if(farMask) { farN[at & 511] = node; farM[at & 511] = farMask; }
+      if(near) { nearN[at >> 9 & 511] = node; nearM[at >> 9 & 511] = rest; }
+      if(rest)
+         for(int c = 0; c < nc; c++)
          {
-            Dual<T> acc[3];
-            irregularSum<T, false>(p, Lp, M, T(dx * ih), T(dy * ih), T(dz * ih), acc);
-            for(int c = 0; c < 3; c++) A[c] += double(acc[c].v) * ih;
-            if(want & 1)
-               for(int j = 0; j < 3; j++)
+            stackN[base + (at >> 18) + c] = c0 + c;
+            stackM[base + (at >> 18) + c] = rest;
+         }
+      count = base + (total >> 18);
+      const int nFar = total & 511, nNear = total >> 9 & 511;
+      __syncthreads();
+      // far boxes, one a warp at a time
+      for(int e = warp; e < nFar; e += TC_WARPS)
+      {
+         const int box = farN[e];
+         const bool on = farM[e] >> j & 1;
+         const T* row = mult + int64_t(box) * 3 * Lp;
+         __syncwarp();
+         if(curlB)
+            for(int i = lane; i < 4 * nharm(p + 1); i += 32)
+            {
+               const CurlTerm<T> ce = curl[i];
+               reinterpret_cast<T*>(Cs)[i] =
+                  ce.c[0] * row[ce.idx[0]] + ce.c[1] * row[ce.idx[1]] + ce.c[2] * row[ce.idx[2]] + ce.c[3] * row[ce.idx[3]];
+            }
+         if(potA)
+            for(int i = lane; i < 4 * nharm(p); i += 32)
+            {
+               const int k = i >> 2, c = i & 3;
+               int l = int(sqrtf(float(k) + 0.5f));
+               const T f = ((l & 1) ? T(-1) : T(1)) * (k != l * l + l ? T(1.4142135623730950488) : T(1));
+               reinterpret_cast<T*>(As)[i] = c < 3 ? f * row[c * Lp + k] : T(0);
+            }
+         __syncwarp();
+         double h, cx, cy, cz;
+         centre(box, h, cx, cy, cz);
+         const double dx = x - cx, dy = y - cy, dz = z - cz, ih = 1.0 / h;
+         T b[3] = {T(0), T(0), T(0)}, a[3] = {T(0), T(0), T(0)};
+         // (for m = 0 the imaginary part is zero, so its k1 = k0 term adds nothing)
+         auto addA = [&](int k0, int k1, T re, T im) {
+            const V4 u = As[k0], v = As[k1];
+            a[0] += u.x * re + v.x * im; a[1] += u.y * re + v.y * im; a[2] += u.z * re + v.z * im;
+         };
+         const T ux = T(dx * ih), uy = T(dy * ih), uz = T(dz * ih);
+         if(curlB)
+            visitIrregular<T>(p + 1, g, G, ux, uy, uz, [&](int k0, int k1, T re, T im, int l) {
+               const V4 u = Cs[k0], v = Cs[k1];
+               b[0] += u.x * re + v.x * im; b[1] += u.y * re + v.y * im; b[2] += u.z * re + v.z * im;
+               if(wantA && l <= p) addA(k0, k1, re, im);
+            });
+         else if(wantA)
+            visitIrregular<T>(p, g, G, ux, uy, uz, [&](int k0, int k1, T re, T im, int) { addA(k0, k1, re, im); });
+         if(on)
+            for(int c = 0; c < 3; c++) { B[c] += double(b[c]) * ih * ih; A[c] += double(a[c]) * ih; }
+         if(wantB && fdCurl)
+         {
+            // central differences of this box's A: dA_c / dx_j
+            double D[3][3];
+            for(int d = 0; d < 3; d++)
+            {
+               T s[2][3];
+               for(int side = 0; side < 2; side++)
                {
-                  Dual<T> ap[3], am[3];
-                  const double e = double(eps) * ih;
-                  irregularSum<T, false>(p, Lp, M, T(dx * ih + (j == 0 ? e : 0.0)), T(dy * ih + (j == 1 ? e : 0.0)),
-                                         T(dz * ih + (j == 2 ? e : 0.0)), ap);
-                  irregularSum<T, false>(p, Lp, M, T(dx * ih - (j == 0 ? e : 0.0)), T(dy * ih - (j == 1 ? e : 0.0)),
-                                         T(dz * ih - (j == 2 ? e : 0.0)), am);
-                  for(int c = 0; c < 3; c++) G[c][j] += double(ap[c].v - am[c].v) * ih / (2.0 * double(eps));
+                  const double sh = (side ? -1.0 : 1.0) * (double(eps) * ih);
+                  for(int c = 0; c < 3; c++) a[c] = T(0);
+                  visitIrregular<T>(p, g, G, T(dx * ih + (d == 0 ? sh : 0.0)), T(dy * ih + (d == 1 ? sh : 0.0)),
+                                    T(dz * ih + (d == 2 ? sh : 0.0)), [&](int k0, int k1, T re, T im, int) { addA(k0, k1, re, im); });
+                  for(int c = 0; c < 3; c++) s[side][c] = a[c];
                }
-         }
-         continue;
-      }
-      const int nc = t.nchild[node];
-      if(nc == 0)
-      {
-         if(refNear) continue;
-         // direct sum over the leaf's sources (coincident points skipped)
-         for(int i = t.s0[node]; i < t.s1[node]; i++)
-         {
-            const auto q = spos[i];
-            const auto s = sq[i];
-            const double ex = x - double(q.x), ey = y - double(q.y), ez = z - double(q.z);
-            const double e2 = ex * ex + ey * ey + ez * ez;
-            if(e2 == 0.0) continue;
-            const double ri = 1.0 / sqrt(e2), ri3 = ri * ri * ri;
-            if(bem)
-            {
-               // the BEM kernel sigma d / |d|^3 + d x s / |d|^3 with d = q - x = -(ex, ey, ez) (fmm_bem.cu)
-               const double sg = double(s.w);
-               A[0] -= (sg * ex + (ey * double(s.z) - ez * double(s.y))) * ri3;
-               A[1] -= (sg * ey + (ez * double(s.x) - ex * double(s.z))) * ri3;
-               A[2] -= (sg * ez + (ex * double(s.y) - ey * double(s.x))) * ri3;
-               continue;
+               for(int c = 0; c < 3; c++)
+               {
+                  // the lanes of a point hold different orders: their sums first, then the difference
+                  for(int off = W; off < 32; off <<= 1)
+                  {
+                     s[0][c] += __shfl_xor_sync(0xffffffffu, s[0][c], off);
+                     s[1][c] += __shfl_xor_sync(0xffffffffu, s[1][c], off);
+                  }
+                  D[c][d] = double(s[0][c] - s[1][c]) * ih / (2.0 * double(eps));
+               }
             }
-            Bn[0] += (double(s.y) * ez - double(s.z) * ey) * ri3;
-            Bn[1] += (double(s.z) * ex - double(s.x) * ez) * ri3;
-            Bn[2] += (double(s.x) * ey - double(s.y) * ex) * ri3;
-            A[0] += double(s.x) * ri;
-            A[1] += double(s.y) * ri;
-            A[2] += double(s.z) * ri;
+            if(on && g == 0)
+            {
+               B[0] += D[2][1] - D[1][2];
+               B[1] += D[0][2] - D[2][0];
+               B[2] += D[1][0] - D[0][1];
+            }
          }
-         continue;
       }
-      if(top + nc > TC_STACK)
+      // near leaves: their sources staged in FP64, every lane takes every (8 G)-th one
+      for(int e = 0; e < nNear; e++)
       {
-         atomicOr(err, ERR_DFS);
-         break;
+         const int leaf = nearN[e];
+         const bool on = nearM[e] >> j & 1;
+         const int s1 = t.s1[leaf];
+         for(int sb = t.s0[leaf]; sb < s1; sb += TC_SRC)
+         {
+            const int n = min(TC_SRC, s1 - sb);
+            __syncthreads();
+            if(tid < n)
+            {
+               const V4 a = spos[sb + tid], b = sq[sb + tid];
+               double* d = S + 8 * tid;
+               d[0] = double(a.x); d[1] = double(a.y); d[2] = double(a.z); d[3] = double(b.w);
+               d[4] = double(b.x); d[5] = double(b.y); d[6] = double(b.z);
+            }
+            __syncthreads();
+            if(!on) continue;
+#pragma unroll 2
+            for(int i = warp * G + g; i < n; i += TC_WARPS * G)
+            {
+               const double* d = S + 8 * i;
+               const double2 d0 = *reinterpret_cast<const double2*>(d), d1 = *reinterpret_cast<const double2*>(d + 2);
+               const double2 d2 = *reinterpret_cast<const double2*>(d + 4);
+               const double sx = d2.x, sy = d2.y, sz = d[6];
+               const double ex = x - d0.x, ey = y - d0.y, ez = z - d1.x;
+               const double e2 = ex * ex + ey * ey + ez * ez;
+               const double ri = e2 > 0.0 ? rsqrt(e2) : 0.0, ri3 = ri * ri * ri;   // (coincident points skipped)
+               if(bem)
+               {
+                  // the BEM kernel sigma d / |d|^3 + d x s / |d|^3 with d = q - x = -(ex, ey, ez) (fmm_bem.cu)
+                  const double sg = d1.y;
+                  A[0] -= (sg * ex + (ey * sz - ez * sy)) * ri3;
+                  A[1] -= (sg * ey + (ez * sx - ex * sz)) * ri3;
+                  A[2] -= (sg * ez + (ex * sy - ey * sx)) * ri3;
+                  continue;
+               }
+               if(wantB)
+               {
+                  B[0] += (sy * ez - sz * ey) * ri3;
+                  B[1] += (sz * ex - sx * ez) * ri3;
+                  B[2] += (sx * ey - sy * ex) * ri3;
+               }
+               if(wantA) { A[0] += sx * ri; A[1] += sy * ri; A[2] += sz * ri; }
+            }
+         }
       }
-      const int c0 = t.child0[node];
-      for(int c = 0; c < nc; c++) stack[top++] = c0 + c;
+      __syncthreads();
    }
-   if(want & 1)
+   // the lanes of a point, then the warps
+   double s[6] = {B[0], B[1], B[2], A[0], A[1], A[2]};
+   for(int off = W; off < 32; off <<= 1)
+      for(int c = 0; c < 6; c++) s[c] += __shfl_xor_sync(0xffffffffu, s[c], off);
+   for(int c = 0; c < 6; c++) S[(warp * 6 + c) * 32 + lane] = s[c];
+   __syncthreads();
+   if(tid < nq)
    {
-      const double B0 = G[2][1] - G[1][2] + Bn[0];
-      const double B1 = G[0][2] - G[2][0] + Bn[1];
-      const double B2 = G[1][0] - G[0][1] + Bn[2];
-      outB[3 * qi] = T(B0 * double(scaleB));
-      outB[3 * qi + 1] = T(B1 * double(scaleB));
-      outB[3 * qi + 2] = T(B2 * double(scaleB));
+      for(int w = 1; w < TC_WARPS; w++)
+         for(int c = 0; c < 6; c++) s[c] += S[(w * 6 + c) * 32 + tid];
+      const int64_t q = order ? order[q0 + tid] : q0 + tid;
+      for(int c = 0; c < 3; c++)
+      {
+         if(wantB) outB[3 * q + c] = T(s[c] * double(scaleB));
+         if(wantA) outA[3 * q + c] = T(s[3 + c] * double(scaleA));
+      }
    }
-   if(want & 2)
-      for(int c = 0; c < 3; c++) outA[3 * qi + c] = T(A[c] * double(scaleA));
+}
+
+// Morton keys of the query points, 10 bits an axis over twice the root cube (points outside clamp to its faces).
+template <class T>
+__global__ void kQueryKeys(const T* __restrict__ pts, int64_t m, const RootBox* __restrict__ rootp, unsigned* keys, int* idx)
+{
+   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+   if(i >= m) return;
+   const RootBox rb = rootp[0];
+   unsigned key = 0;
+   for(int d = 0; d < 3; d++)
+   {
+      const double u = (double(pts[3 * i + d]) - rb.center[d]) / (4.0 * rb.H) + 0.5;
+      const unsigned v = unsigned(fmin(1023.0, fmax(0.0, u * 1024.0)));
+      for(int b = 0; b < 10; b++) key |= (v >> b & 1u) << (3 * b + d);
+   }
+   keys[i] = key;
+   idx[i] = int(i);
 }
 
 }  // namespace
@@ -232,16 +434,43 @@ fmm_status treecodeT(Plan& P, double current, int want, const void* pts, int64_t
    // A (and, for BEM sources, the BEM integral) times current / (4 pi), as MultipoleSolver::calcA
    // (multipole_solver.cpp:686-692) scales both
    const T scaleB = T(REF_MU0 / (4 * REF_PI) * current), scaleA = T(1.0 / (4 * REF_PI) * current);
-   FMM_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
-   const int blocks = int((m + TC_NT - 1) / TC_NT);
-   kTreecode<T><<<blocks, TC_NT, 0, st>>>(P.tree, P.root, P.p, P.Lp, (const T*)P.mult.ptr, (const V4*)P.sPos.ptr,
-                                          (const V4*)P.sQ.ptr, (const T*)pts, m, flags, scaleB, scaleA, want, P.bem ? 1 : 0, (T*)outB,
-                                          (T*)outA, P.err);
+   if(P.tcCurlOrder != P.p)
+   {
+      const std::vector<CurlTerm<T>> tab = curlTerms<T>(P.p, P.Lp);
+      const size_t bytes = tab.size() * sizeof(CurlTerm<T>);
+      FMM_TRY(P.tcCurl.reserve(bytes));
+      P.tcCurlHost.resize(bytes);
+      std::copy_n(reinterpret_cast<const unsigned char*>(tab.data()), bytes, P.tcCurlHost.data());
+      FMM_CUDA(cudaMemcpyAsync(P.tcCurl.ptr, P.tcCurlHost.data(), bytes, cudaMemcpyHostToDevice, st));
+      P.tcCurlOrder = P.p;
+   }
+   // Points a block: as many as share a leaf's neighbourhood on average, so that a block's points want mostly the
+   // same boxes; few points, or points sparse among the leaves, walk alone (then a point has 256 threads).
+   const int64_t dense = m / std::max<int64_t>(1, P.tree.nNodes);
+   int W = 1;
+   while(W < 32 && 2 * W <= dense && m / (2 * W) >= 2 * 148) W *= 2;
+   const int* order = nullptr;
+   if(W > 1)
+   {
+      // keys, sorted keys, indexes, sorted indexes
+      FMM_TRY(P.tcSort.reserve(sizeof(unsigned) * 4 * size_t(m)));
+      unsigned* k = (unsigned*)P.tcSort.ptr;
+      int* ix = (int*)(k + 2 * m);
+      kQueryKeys<T><<<int((m + 255) / 256), 256, 0, st>>>((const T*)pts, m, P.root, k, ix);
+      FMM_TRY(launched(P, "kQueryKeys", st));
+      size_t tmp = 0;
+      cub::DeviceRadixSort::SortPairs(nullptr, tmp, k, k + m, ix, ix + m, int(m), 0, 30, st);
+      FMM_TRY(P.cubTmp.reserve(tmp));
+      tmp = P.cubTmp.bytes;
+      FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, k, k + m, ix, ix + m, int(m), 0, 30, st));
+      order = ix + m;
+   }
+   const TcSmem<T> sm(P.p, (want & 2) || (flags & 2));
+   FMM_CUDA(cudaFuncSetAttribute(kTreecode<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm.total));
+   kTreecode<T><<<unsigned((m + W - 1) / W), TC_NT, sm.total, st>>>(
+      P.tree, P.root, P.p, P.Lp, (const T*)P.mult.ptr, (const CurlTerm<T>*)P.tcCurl.ptr, (const V4*)P.sPos.ptr,
+      (const V4*)P.sQ.ptr, (const T*)pts, order, m, W, flags, scaleB, scaleA, want, P.bem ? 1 : 0, (T*)outB, (T*)outA);
    FMM_TRY(launched(P, "kTreecode", st));
-   int herr = 0;
-   FMM_CUDA(cudaMemcpyAsync(&herr, P.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-   FMM_CUDA(cudaStreamSynchronize(st));
-   if(herr) return setError(FMM_E_LIMIT, "fmm_treecode: the descent stack overflowed (code %d)", herr);
    return FMM_OK;
 }
 
