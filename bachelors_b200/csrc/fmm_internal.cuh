@@ -215,11 +215,9 @@ struct Plan
    int tcProf = 0;                       // FMM_TC_PROF=1: per-role cycle counts of the M2L launch to stderr
    DevBuf tcProfBuf;
    int tcCorrLam = 5;                    // ... and only in K steps whose lowest input degree is <= this (-1: any)
-   int tcAsyncArrive = 0;                // tensor-core pipelines: 0: each producer waits for its copies, fences
+   int tcAsyncArrive = -1;               // tensor-core pipelines: 0: each producer waits for its copies, fences
                                          // and arrives; 1: producers arrive through cp.async.mbarrier and
-                                         // the MMA thread fences (up to NS items in flight, but the MMA
-                                         // thread loses ~400-600 cycles per item after such a barrier:
-                                         // M2L 159 ms against 137 ms at 2^24)
+                                         // the MMA warp fences; -1: by the K chunk (asyncArrivals)
    int tcKeepTail = 1;                   // tensor-core M2L: accumulator columns >= 256 (the top degrees) are
                                          // drained once per tile, not with the others
    int tcPair = 1;                       // tensor-core M2L: K chunks without correction products travel

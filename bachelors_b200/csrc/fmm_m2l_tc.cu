@@ -16,7 +16,7 @@
 // kind::tf32, 4-byte elements); all are accumulated in FP32 in tensor memory.
 //
 // Warp roles (576 threads):
-//   warp 0      TMEM allocation; lane 0 issues the tcgen05.mma instructions
+//   warp 0      TMEM allocation; issues the tcgen05.mma instructions (one elected lane)
 //   warp 1      lane 0 streams the pre-swizzled operator image with cp.async.bulk (no multicast)
 //   warps 2..9  gather the source rows, already split into bf16 pieces once per solve
 //               (kSplitMultipoles), with 16-byte cp.async copies into the swizzled K-major layout
@@ -158,6 +158,13 @@ __device__ __forceinline__ void cpAsyncArriveNoinc(uint32_t bar)
    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void cpAsyncWaitAll() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// waits until at most n of this thread's copy groups are still in flight (n = 0, 1 or 2)
+__device__ __forceinline__ void cpAsyncWaitGroups(int n)
+{
+   if(n <= 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+   else if(n == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+   else asm volatile("cp.async.wait_group 2;" ::: "memory");
+}
 
 __device__ __forceinline__ void bulkLoad(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
 {
@@ -176,13 +183,29 @@ __host__ __device__ constexpr uint32_t instrDescBf16(int M, int N)
           | (uint32_t(M >> 4) << 24);  // M
 }
 
-__device__ __forceinline__ void mmaBf16(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate)
+// (executed by a whole warp, issued by the lane whose `elected` is set: the operands then stay in the warp's uniform
+// registers, which the instruction takes)
+__device__ __forceinline__ void mmaBf16(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate,
+                                        uint32_t elected)
 {
    asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate));
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate), "r"(elected));
+}
+
+// 1 in one lane of the (converged) warp, 0 in the others
+__device__ __forceinline__ uint32_t electOne()
+{
+   uint32_t e;
+   asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+   return e;
 }
 
 // Instruction descriptor: tf32 x tf32 -> f32, A and B K-major, shape M x N.
@@ -195,13 +218,15 @@ __host__ __device__ constexpr uint32_t instrDescTf32(int M, int N)
           | (uint32_t(M >> 4) << 24);  // M
 }
 
-__device__ __forceinline__ void mmaTf32(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void mmaTf32(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate,
+                                        uint32_t elected)
 {
    asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate));
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate), "r"(elected));
 }
 
 // x rounded to tf32 (10 explicit mantissa bits, round to nearest, ties away), as its fp32 bit pattern
@@ -378,6 +403,23 @@ struct M2LCols
    int nItems;              // items per offset
 };
 
+// The MMAs of every item, in issue order, as the instruction takes them: passed by value, so that the issuing warp
+// reads them through the constant bank into uniform registers.
+struct __align__(16) MmaOp
+{
+   uint32_t idesc;     // instruction descriptor (type, M, N)
+   uint16_t a, b;      // operand offsets / 16 in the item's A and B stage
+   uint16_t d;         // first accumulator column
+   uint16_t fresh;     // 1: starts the accumulation unless it goes on from the previous item, 2: the same for the kept tail
+   uint32_t pad;
+};
+constexpr int MAXMMA = 256;     // 240 with six products (p = 16)
+struct MmaProgram
+{
+   MmaOp op[MAXMMA];
+   int first[MAXITEMS + 1];
+};
+
 // Control area after the stages: barriers, the accumulator's address, the abort flag, the offsets present,
 // then the per-tile tables (16-bit where they fit, so that a third A stage fits at p = 16)
 constexpr int CTRL_HEAD = 256;
@@ -484,6 +526,46 @@ struct PipeCursor
    }
 };
 
+// Which offsets have a source for some box of the tile: a warp per box, its table row in loads that are all in
+// flight. (A row entry at a time per thread, with the list below made by one thread, the prologue took 52k cycles of a
+// 1.03M-cycle tile at p = 16. Functions of their own: inlined, they cost the pipeline's warps registers.)
+__device__ __noinline__ void markOffsets(const int* __restrict__ vtab, const int* tileNode, int nTile, int nOps, uint32_t* present,
+                                         int warp, int lane)
+{
+   uint32_t mine = 0;
+   for(int t = warp; t < nTile; t += tc::NTHREADS / 32)
+   {
+      const int* row = vtab + int64_t(tileNode[t]) * nOps;
+      int v[10];
+#pragma unroll
+      for(int w = 0; w < 10; w++) v[w] = lane + 32 * w < nOps ? row[lane + 32 * w] : -1;
+#pragma unroll
+      for(int w = 0; w < 10; w++)
+      {
+         const uint32_t bits = __ballot_sync(0xffffffffu, v[w] >= 0);
+         if(lane == w) mine |= bits;
+      }
+   }
+   if(lane < 10 && mine) atomicOr(&present[lane], mine);
+}
+
+// The offsets present, by one warp; returns their number. M2L: far offsets first, so the smaller contributions enter
+// the accumulator before the large ones; the 8 child octants of M2M / L2L in order.
+__device__ __noinline__ int listOffsets(int nOps, const uint32_t* present, uint16_t* itemOffset, int lane)
+{
+   int k = 0;
+   for(int i0 = 0; i0 < nOps; i0 += 32)
+   {
+      const int i = i0 + lane;
+      const int o = i < nOps ? (nOps == 316 ? d_m2lFarFirst[i] : i) : 0;
+      const bool on = i < nOps && (present[o >> 5] >> (o & 31) & 1u);
+      const uint32_t bits = __ballot_sync(0xffffffffu, on);
+      if(on) itemOffset[k + __popc(bits & ((1u << lane) - 1u))] = uint16_t(o);
+      k += __popc(bits);
+   }
+   return k;
+}
+
 // 18 warps: five of them share one SM sub-partition's 16K registers, so 96 per thread at most.
 // PIECES: the final outputs are also stored as operand pieces (Mout); the M2M's form.
 template <int NP, class Lay, bool PIECES = false>
@@ -492,19 +574,13 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
        int nChunks, const uint8_t* __restrict__ img, const uint8_t* __restrict__ Mbf, float* __restrict__ Lc,
        int addOut, uint8_t* __restrict__ Mout, int drainEvery, int drainFar, int drainItems, int nStagesA, int nStagesB,
        uint32_t bStage, int drainMode, int keepTail,
-       const M2LCols cols, unsigned long long* counters, int* err, uint64_t waitNs, int asyncArrive,
+       const M2LCols cols, const MmaProgram prog, unsigned long long* counters, int* err, uint64_t waitNs, int asyncArrive,
        unsigned long long* prof)
 {
    // prof (developer switch): SM cycles per role, summed over CTAs, see TcProf
    const long long tStart = prof ? clock64() : 0;
    using namespace tc;
    constexpr int KCH = Lay::KC;
-   constexpr int NPASS = NP == 1 ? 1 : (NP == 2 ? 3 : 6);
-   // (A piece, B piece) of every product kept: hi*hi, hi*lo, lo*hi  /  down to 2^-16 with three pieces
-   constexpr int PA[6] = {0, 0, 1, 1, 0, 2};
-   constexpr int PB[6] = {0, 1, 0, 1, 2, 0};
-   constexpr int PA2[3] = {0, 0, 1};
-   constexpr int PB2[3] = {0, 1, 0};
    extern __shared__ uint8_t smraw[];
    const int N = Lp;                                   // output columns (<= 320)
    const uint32_t aBytes = ROWS * Lay::RB;             // one A piece
@@ -540,24 +616,22 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
 
    if(tid < 10) present[tid] = 0;
    if(tid < TT) tileNode[tid] = tid < nTile ? targets[first + tid] : -1;
-   if(tid == 0)
+   if(tid == 64)
+   for(int i = 0; i < cols.nItems; i++)
    {
-      for(int i = 0; i < cols.nItems; i++)
+      uint16_t* r = recTab + REC * i;
+      const int c0 = cols.first[i], m = cols.count[i];
+      for(int k = 0; k < REC; k++) r[k] = 0;
+      r[Rec::FIRST] = uint16_t(c0);
+      r[Rec::COUNT] = uint16_t(m);
+      for(int j = 0; j < NP; j++)
       {
-         uint16_t* r = recTab + REC * i;
-         const int c0 = cols.first[i], m = cols.count[i];
-         for(int k = 0; k < REC; k++) r[k] = 0;
-         r[Rec::FIRST] = uint16_t(c0);
-         r[Rec::COUNT] = uint16_t(m);
-         for(int j = 0; j < NP; j++)
-         {
-            r[Rec::BOFF + j] = uint16_t(cols.bOff[i][j]);
-            if(j < m)
-               for(int ks = 0; ks < KPC; ks++) r[Rec::NCOL + KPC * j + ks] = uint16_t(cols.n[(c0 + j) * KPC + ks]);
-         }
-         if(m == 1)
-            for(int ks = 0; ks < KPC; ks++) r[Rec::NCOR + ks] = uint16_t(cols.nc[c0 * KPC + ks]);
+         r[Rec::BOFF + j] = uint16_t(cols.bOff[i][j]);
+         if(j < m)
+            for(int ks = 0; ks < KPC; ks++) r[Rec::NCOL + KPC * j + ks] = uint16_t(cols.n[(c0 + j) * KPC + ks]);
       }
+      if(m == 1)
+         for(int ks = 0; ks < KPC; ks++) r[Rec::NCOR + ks] = uint16_t(cols.nc[c0 * KPC + ks]);
    }
    if(tid == 0)
    {
@@ -580,31 +654,22 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
    }
    __syncthreads();
-   // which offsets have a source for some box of the tile
-   for(int e = tid; e < TT * nOps; e += NTHREADS)
-   {
-      const int t = tileNode[e / nOps], o = e % nOps;
-      if(t >= 0 && vtab[int64_t(t) * nOps + o] >= 0) atomicOr(&present[o >> 5], 1u << (o & 31));
-   }
+   markOffsets(vtab, tileNode, nTile, nOps, present, warp, lane);
    fenceBeforeSync();
    __syncthreads();
    fenceAfterSync();
-   if(tid == 0)
+   if(warp == 0)
    {
-      // M2L: far offsets first, so the smaller contributions enter the accumulator before the large
-      // ones; the 8 child octants of M2M / L2L in order
-      int k = 0;
-      for(int i = 0; i < nOps; i++)
+      const int k = listOffsets(nOps, present, itemOffset, lane);
+      if(lane == 0)
       {
-         const int o = nOps == 316 ? d_m2lFarFirst[i] : i;
-         if(present[o >> 5] & (1u << (o & 31))) itemOffset[k++] = uint16_t(o);
-      }
-      *offCount = k;
-      // work accounting: pipeline items and tile-offset pairs
-      if(counters)
-      {
-         atomicAdd(counters, (unsigned long long)(k * cols.nItems));
-         atomicAdd(counters + 1, (unsigned long long)k);
+         *offCount = k;
+         // work accounting: pipeline items and tile-offset pairs
+         if(counters)
+         {
+            atomicAdd(counters, (unsigned long long)(k * cols.nItems));
+            atomicAdd(counters + 1, (unsigned long long)k);
+         }
       }
    }
    __syncthreads();
@@ -620,34 +685,31 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
 
    if(warp == 0)
    {
-      if(lane == 0)
+      // The whole warp runs the loop and one lane issues: every operand of an MMA (stage descriptors, the item's
+      // program from the kernel's parameters) is then a uniform value. An MMA of N columns takes max(45, N / 2)
+      // cycles; issued by one thread with widths read from shared memory it took 105-120 whatever N, for the moves into
+      // the uniform registers. What bounds the tile now is the shared memory: per offset at p = 16 the MMAs read 290 KB
+      // and the copies write 225 KB, 4.0k cycles at 128 B a cycle, of the 6.2k a (tile, offset) step takes (7.6k before;
+      // M2L of 2^24 points 112 -> 95 ms, of 2^20, p = 12, 3.76 -> 3.1 ms).
       {
-         bool firstMma = true;
-         bool tailFirst = true;   // keepTail: the columns >= split accumulate through the whole tile
-         // an MMA covers at most 256 columns; a wider K step is split at 256, with keepTail where the kept
-         // columns start
-         const int split = keepTail ? tailSplit(1, N) : 256;
+         const uint32_t el = electOne();
+         const int nItemsU = __shfl_sync(0xffffffffu, nItems, 0), nOffU = __shfl_sync(0xffffffffu, nOff, 0);
+         const uint32_t tmemU = __shfl_sync(0xffffffffu, tmem, 0);
+         uint32_t accOn = 0;      // 0: the next MMA starts a fresh accumulation
+         uint32_t tailOn = 0;     // the same for the kept tail, which accumulates through the whole tile
          int drains = 0;
          long long tw0 = 0, tw1 = 0, tw2 = 0;
-         long long tIssue[6] = {0, 0, 0, 0, 0, 0};   // per K chunk: from the stage's arrival to the commit
+         long long tIssue = 0;   // from the stages' arrival to the commit
          const long long tl = prof ? clock64() : 0;
-         DrainSchedule sched(nOff, drainEvery, drainFar);
+         DrainSchedule sched(nOffU, drainEvery, drainFar);
          PipeCursor cur;
          int sinceDrain = 0;
-         // item records are read one item ahead: the loads land while the thread waits for the stages
-         Rec next;
-         next.load(rec4, 0);
-         for(int it = 0; it < nItems; it++, cur.next(NA, NB, nPer))
+         for(int it = 0; it < nItemsU; it++, cur.next(NA, NB, nPer))
          {
-            const Rec rc = next;
-            {
-               next.load(rec4, cur.c + 1 == nPer ? 0 : cur.c + 1);
-            }
-            const int m = rc[Rec::COUNT];
             long long t0 = prof ? clock64() : 0;
-            if(!mbarWait(fullBar0 + 8 * cur.sa, cur.pha, err, abortFlag, waitNs)) break;
+            if(!__all_sync(0xffffffffu, mbarWait(fullBar0 + 8 * cur.sa, cur.pha, err, abortFlag, waitNs))) break;
             long long t1 = prof ? clock64() : 0;
-            if(!mbarWait(opBar0 + 8 * cur.sb, cur.phb, err, abortFlag, waitNs)) break;
+            if(!__all_sync(0xffffffffu, mbarWait(opBar0 + 8 * cur.sb, cur.phb, err, abortFlag, waitNs))) break;
             long long t2 = 0;
             if(prof)
             {
@@ -657,58 +719,27 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
             }
             // the producers' cp.async writes (generic proxy), observed through the barrier, before
             // the tensor core reads the stage (async proxy)
-            if(asyncArrive) fenceProxyAsync();
+            if(asyncArrive && el) fenceProxyAsync();
             fenceAfterSync();
             const uint32_t aSt = base + cur.sa * aStage, bSt = bRing + cur.sb * bStage;
             // descriptors of the stages; an MMA's operand is the stage's descriptor plus the slot's
-            // byte offset / 16 (the start-address field, bits 0-13, holds every shared-memory address)
+            // byte offset / 16 (the start-address field, bits 0-13, holds every shared-memory address, so the sum
+            // stays in the low word)
             const uint64_t dA = smemDescT<Lay>(aSt), dB = smemDescT<Lay>(bSt);
-#pragma unroll
-            for(int j = 0; j < NP; j++)
+            const int i1 = prog.first[cur.c + 1];
+#pragma unroll 4
+            for(int i = prog.first[cur.c]; i < i1; i++)
             {
-               if(j >= m) break;
-#pragma unroll
-               for(int ks = 0; ks < KPC; ks++)
-               {
-                  const uint32_t koff = ks * 32;
-                  // this K step's output columns in one MMA (<= 256) or two (split at 256 or at the kept
-                  // tail); the correction products over the first nCor of them (a chunk alone: j = 0). K steps
-                  // past the last coefficient (the last chunk is partly padding) have no columns.
-                  const int nCol = rc[Rec::NCOL + KPC * j + ks];
-                  if(nCol == 0) break;
-                  const int nCor = rc[Rec::NCOR + ks];
-#pragma unroll
-                  for(int pass = 0; pass < NPASS; pass++)
-                  {
-                     const int w = pass == 0 ? nCol : nCor;
-                     if(w == 0) break;
-                     const int nA = min(w, split), nB = w - nA;
-                     const uint32_t idA = Lay::TF32 ? instrDescTf32(ROWS, nA) : instrDescBf16(ROWS, nA);
-                     const uint32_t idB = Lay::TF32 ? instrDescTf32(ROWS, nB > 0 ? nB : 16) : instrDescBf16(ROWS, nB > 0 ? nB : 16);
-                     // piece slots: pa, pb for a chunk alone, slot j (pass 0 only) for a shared stage
-                     const int pa = j + (NP == 1 ? 0 : (NP == 2 ? PA2[pass] : PA[pass]));
-                     const int pb = j + (NP == 1 ? 0 : (NP == 2 ? PB2[pass] : PB[pass]));
-                     const uint64_t da = dA + ((pa * aBytes + koff) >> 4);
-                     const uint64_t db = dB + uint64_t(rc[Rec::BOFF + pb]) + (koff >> 4);
-                     const uint32_t acc = firstMma ? 0u : 1u;
-                     const uint32_t accT = keepTail ? (tailFirst ? 0u : 1u) : acc;
-                     if constexpr(Lay::TF32)
-                     {
-                        mmaTf32(tmem, da, db, idA, acc);
-                        if(nB > 0) mmaTf32(tmem + nA, da, db + ((nA * Lay::RB) >> 4), idB, accT);
-                     }
-                     else
-                     {
-                        mmaBf16(tmem, da, db, idA, acc);
-                        if(nB > 0) mmaBf16(tmem + nA, da, db + ((nA * Lay::RB) >> 4), idB, accT);
-                     }
-                     firstMma = false;
-                     if(nB > 0) tailFirst = false;
-                  }
-               }
+               const MmaOp o = prog.op[i];
+               const uint64_t da = dA + o.a, db = dB + o.b;
+               const uint32_t acc = o.fresh == 0 ? 1u : (o.fresh == 1 ? accOn : tailOn);
+               if constexpr(Lay::TF32) mmaTf32(tmemU + o.d, da, db, o.idesc, acc, el);
+               else mmaBf16(tmemU + o.d, da, db, o.idesc, acc, el);
             }
-            mmaCommit(emptyBar0 + 8 * cur.sa);
-            if(prof && cur.c < 6) tIssue[cur.c] += clock64() - t2;
+            accOn = 1;
+            tailOn = 1;
+            if(el) mmaCommit(emptyBar0 + 8 * cur.sa);
+            if(prof) tIssue += clock64() - t2;
             // every drainEvery offsets (and after the last) hand the accumulator to the drain warps
             // and start a fresh one: the tensor cores' FP32 accumulation truncates, so long chains
             // of accumulations into one TMEM value drift; the running sum is kept in FP32 instead
@@ -717,35 +748,34 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
             bool drainNow;
             if(drainItems > 0)
             {
-               drainNow = ++sinceDrain == drainItems || it == nItems - 1;
+               drainNow = ++sinceDrain == drainItems || it == nItemsU - 1;
                if(drainNow) sinceDrain = 0;
             }
             else
                drainNow = cur.c == nPer - 1 && sched.after(cur.oi);
+            if(drainNow)
             {
-               if(drainNow)
+               if(el) mmaCommit(drainFull);
+               if(it != nItemsU - 1)
                {
-                  mmaCommit(drainFull);
-                  if(it != nItems - 1)
-                  {
-                     const long long t3 = prof ? clock64() : 0;
-                     if(!mbarWait(drainEmpty, drains & 1, err, abortFlag, waitNs)) break;
-                     if(prof) tw2 += clock64() - t3;
-                     fenceAfterSync();
-                  }
-                  drains++;
-                  firstMma = true;
+                  const long long t3 = prof ? clock64() : 0;
+                  if(!__all_sync(0xffffffffu, mbarWait(drainEmpty, drains & 1, err, abortFlag, waitNs))) break;
+                  if(prof) tw2 += clock64() - t3;
+                  fenceAfterSync();
                }
+               drains++;
+               accOn = 0;
             }
          }
-         mmaCommit(doneBar);
-         if(prof)
+         __syncwarp();
+         if(el) mmaCommit(doneBar);
+         if(prof && lane == 0)
          {
             atomicAdd(prof + 0, (unsigned long long)tw0);
             atomicAdd(prof + 1, (unsigned long long)tw1);
             atomicAdd(prof + 2, (unsigned long long)tw2);
             atomicAdd(prof + 3, (unsigned long long)(clock64() - tl));
-            for(int c = 0; c < 6; c++) atomicAdd(prof + 16 + c, (unsigned long long)tIssue[c]);
+            atomicAdd(prof + 16, (unsigned long long)tIssue);
          }
       }
       __syncwarp();
@@ -975,9 +1005,9 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
    else
    {
       // producers (warps 2..9): two threads per row, KCH / 2 K-elements (KCH / 8 chunks of 16 bytes)
-      // of every piece each. Item it - 1 is signalled as soon as its copies have landed, then the
-      // copies of item it are issued once its stage is free: one item's gather is in flight while
-      // the tensor cores work on the previous one, and issuing never delays a signal.
+      // of every piece each. Up to three items' copies are in flight per thread, fewer than the stages; an item is
+      // signalled when its copies have landed, at the latest before the thread blocks on a stage that is not yet free
+      // (with one item in flight the gather's latency set the pace: 2.2k cycles an item at p = 16).
       constexpr int PER = KCH / 2;                   // K elements per thread and chunk
       constexpr int EPC = 16 / Lay::ES;              // elements per 16-byte copy
       const int ptid = tid - 64;
@@ -986,7 +1016,16 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
       const int tgt = row < 3 * TT ? tileNode[slot] : -1;
       int src = (tgt >= 0 && nItems > 0) ? vtab[int64_t(tgt) * nOps + itemOffset[0]] : -1;
       int srcNext = -1;
-      int pending = -1;   // stage of the item whose copies are still to be signalled (synchronous form)
+      int pending = 0;            // items whose copies are still to be signalled (synchronous form) ...
+      int pendStage = 0;          // ... from this stage on
+      const int maxPending = min(3, NA - 1);
+      auto signalOldest = [&]() {
+         cpAsyncWaitGroups(pending - 1);
+         fenceProxyAsync();
+         mbarArrive(fullBar0 + 8 * pendStage);
+         pending--;
+         if(++pendStage == NA) pendStage = 0;
+      };
       long long twp = 0;
       const long long tpl = prof ? clock64() : 0;
       PipeCursor cur;
@@ -996,16 +1035,12 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
          const int oi = cur.oi, c = cur.c;
          if(c == 0 && oi + 1 < nOff)
             srcNext = tgt >= 0 ? vtab[int64_t(tgt) * nOps + itemOffset[oi + 1]] : -1;
-         if(pending >= 0)
-         {
-            // (synchronous form: this thread waits for its previous item's copies, then arrives)
-            cpAsyncWaitAll();
-            fenceProxyAsync();
-            mbarArrive(fullBar0 + 8 * pending);
-            pending = -1;
-         }
          const long long t0 = prof ? clock64() : 0;
-         if(it >= NA && !mbarWait(emptyBar0 + 8 * s, cur.pha ^ 1, err, abortFlag, waitNs)) break;
+         if(it >= NA)
+         {
+            while(pending > 0 && !mbarTryWait(emptyBar0 + 8 * s, cur.pha ^ 1)) signalOldest();
+            if(!mbarWait(emptyBar0 + 8 * s, cur.pha ^ 1, err, abortFlag, waitNs)) break;
+         }
          if(prof) twp += clock64() - t0;
          const uint32_t aSt = base + s * aStage;
          Rec rc;
@@ -1037,16 +1072,12 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
          else
          {
             cpAsyncCommit();
-            pending = s;
+            if(++pending == maxPending) signalOldest();
          }
          if(c == nPer - 1) src = srcNext;
       }
+      while(pending > 0 && !*abortFlag) signalOldest();
       cpAsyncWaitAll();
-      if(pending >= 0 && !*abortFlag)
-      {
-         fenceProxyAsync();
-         mbarArrive(fullBar0 + 8 * pending);
-      }
       if(prof && tid == 64)
       {
          atomicAdd(prof + 5, (unsigned long long)twp);
@@ -1133,6 +1164,62 @@ static fmm_status planStages(M2LCols& cols, int NP, int stepsPerChunk, int rowBy
    return FMM_OK;
 }
 
+// Producer arrivals: through cp.async.mbarrier with the MMA warp's proxy fence (every stage's copies in flight), or
+// each producer's own after waiting for its copies. The first pays where an item's MMAs outlast the fence, with
+// 64-wide K chunks (M2L of 2^24 points, p = 16: 92.3 against 97.1 ms), not with 32-wide ones (BF16X6, 2^19 points, p = 16:
+// 4.46 against 4.11 ms).
+template <class Lay>
+static int asyncArrivals(const Plan& P) { return P.tcAsyncArrive >= 0 ? P.tcAsyncArrive : (Lay::KC == 64 ? 1 : 0); }
+
+// The MMAs of each item (planStages must have run). An MMA covers at most 256 columns; a wider K step is split at 256,
+// with keepTail where the kept columns start.
+template <int NP, class Lay>
+static fmm_status planMmas(const M2LCols& cols, int N, int keepTail, MmaProgram& prog)
+{
+   constexpr int NPASS = NP == 1 ? 1 : (NP == 2 ? 3 : 6);
+   // (A piece, B piece) of every product kept: hi*hi, hi*lo, lo*hi  /  down to 2^-16 with three pieces
+   constexpr int PA[3][6] = {{0}, {0, 0, 1}, {0, 0, 1, 1, 0, 2}};
+   constexpr int PB[3][6] = {{0}, {0, 1, 0}, {0, 1, 0, 1, 2, 0}};
+   constexpr int KPC = Lay::KC / Lay::KSTEP;
+   const int split = keepTail ? tailSplit(1, N) : 256;
+   int n = 0;
+   for(int c = 0; c < cols.nItems; c++)
+   {
+      prog.first[c] = n;
+      const int c0 = cols.first[c], m = cols.count[c];
+      for(int j = 0; j < m; j++)
+         for(int ks = 0; ks < KPC; ks++)
+         {
+            // K steps past the last coefficient (the last chunk is partly padding) have no columns
+            const int step = (c0 + j) * KPC + ks, nCol = cols.n[step], nCor = m == 1 ? cols.nc[step] : 0;
+            if(nCol == 0) break;
+            for(int pass = 0; pass < NPASS; pass++)
+            {
+               const int w = pass == 0 ? nCol : nCor;
+               if(w == 0) break;
+               // piece slots: pa, pb for a chunk alone, slot j (pass 0 only) for a shared stage
+               const int pa = j + PA[NP - 1][pass], pb = j + PB[NP - 1][pass];
+               const int nA = std::min(w, split);
+               for(int part = 0; part < (w > nA ? 2 : 1); part++)
+               {
+                  if(n == MAXMMA) return setError(FMM_E_INVALID, "tensor-core pipeline: more than %d MMAs an offset", MAXMMA);
+                  MmaOp& o = prog.op[n++];
+                  const int cnt = part ? w - nA : nA;
+                  o.idesc = Lay::TF32 ? tc::instrDescTf32(tc::ROWS, cnt) : tc::instrDescBf16(tc::ROWS, cnt);
+                  o.a = uint16_t((size_t(pa) * tc::ROWS * Lay::RB + ks * 32) / 16);
+                  o.b = uint16_t(cols.bOff[c][pb] + (ks * 32 + (part ? nA * Lay::RB : 0)) / 16);
+                  o.d = uint16_t(part ? nA : 0);
+                  // possibly the first over its columns since a drain: those of an item's first leading product
+                  o.fresh = uint16_t(j == 0 && ks == 0 && pass == 0 ? (part && keepTail ? 2 : 1) : 0);
+                  o.pad = 0;
+               }
+            }
+         }
+   }
+   prog.first[cols.nItems] = n;
+   return FMM_OK;
+}
+
 template <int NP, class Lay>
 static fmm_status launchM2LTc(Plan& P, cudaStream_t st)
 {
@@ -1184,6 +1271,8 @@ static fmm_status launchM2LTc(Plan& P, cudaStream_t st)
    FMM_TRY(planItems(cols, nChunks, Lay::KC / Lay::KSTEP, NP, P.tcPair != 0));
    StagePlan sp;
    FMM_TRY(planStages(cols, NP, Lay::KC / Lay::KSTEP, Lay::RB, "tensor-core M2L", sp));
+   MmaProgram prog{};
+   FMM_TRY((planMmas<NP, Lay>(cols, Lp, P.tcKeepTail, prog)));
    // (the attribute is the budget, not this launch's size: the translations share the kernel and a graph
    // replays every launch with its own size)
    FMM_CUDA(cudaFuncSetAttribute(kM2LTc<NP, Lay>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BUDGET)));
@@ -1206,7 +1295,7 @@ static fmm_status launchM2LTc(Plan& P, cudaStream_t st)
    kM2LTc<NP, Lay><<<blocks, tc::NTHREADS, sp.smem, st>>>((const int*)P.m2lTargets.ptr, count, P.lists.vtab, 316, L, Lp,
                                                       nChunks, (const uint8_t*)P.opM2Lbf.ptr, (const uint8_t*)P.multBf.ptr,
                                                       (float*)P.local.ptr, 0, nullptr, (NP == 2 ? P.tcDrainEvery : std::max(1, P.tcDrainEvery / 2)),
-                                                      (NP == 2 ? P.tcDrainFar : std::max(1, P.tcDrainFar / 2)), 0, sp.na, sp.nb, sp.bStage, P.tcDrainMode, P.tcKeepTail, cols, (unsigned long long*)P.tcCounters.ptr, P.pipeErr, P.tcWaitNs, P.tcAsyncArrive,
+                                                      (NP == 2 ? P.tcDrainFar : std::max(1, P.tcDrainFar / 2)), 0, sp.na, sp.nb, sp.bStage, P.tcDrainMode, P.tcKeepTail, cols, prog, (unsigned long long*)P.tcCounters.ptr, P.pipeErr, P.tcWaitNs, asyncArrivals<Lay>(P),
                                                       prof);
    FMM_TRY(launched(P, "kM2LTc", st));
    if(prof)
@@ -1222,9 +1311,7 @@ static fmm_status launchM2LTc(Plan& P, cudaStream_t st)
               blocks, it, h[9] / b, h[10] / b, h[3] / b, h[0] / b, h[1] / b, h[2] / b, h[4] / b, h[6] / b, h[5] / b,
               h[8] / b, h[7] / b);
       fprintf(stderr, "kM2LTc profile, drains per CTA %.1f\n", double(h[23]) / b);
-      fprintf(stderr, "kM2LTc profile, MMA thread cycles per item from the stage's arrival to its commit, by item:");
-      for(int c = 0; c < std::min(cols.nItems, 6); c++) fprintf(stderr, " %.0f", h[16 + c] * double(cols.nItems) / double(h[11]));
-      fprintf(stderr, "\n");
+      fprintf(stderr, "kM2LTc profile, MMA warp cycles per item from its stages' arrival to the commit: %.0f\n", h[16] / double(h[11]));
    }
    // a timed-out wait raises the pipeline error word, which the calling phase reads once at its end
    return FMM_OK;
@@ -1265,6 +1352,8 @@ static fmm_status translateTc(Plan& P, cudaStream_t st, bool up)
    FMM_TRY(planItems(cols, nChunks, Lay::KC / Lay::KSTEP, NP, false));
    StagePlan sp;
    FMM_TRY(planStages(cols, NP, Lay::KC / Lay::KSTEP, Lay::RB, "tensor-core translation", sp));
+   MmaProgram prog{};
+   FMM_TRY((planMmas<NP, Lay>(cols, Lp, 0, prog)));
    const size_t smem = sp.smem;
    FMM_CUDA(cudaFuncSetAttribute(kM2LTc<NP, Lay>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BUDGET)));
    FMM_CUDA(cudaFuncSetAttribute(kM2LTc<NP, Lay, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BUDGET)));
@@ -1295,7 +1384,7 @@ static fmm_status translateTc(Plan& P, cudaStream_t st, bool up)
          kern<<<(b - a + tc::TT - 1) / tc::TT, tc::NTHREADS, smem, st>>>(
             (const int*)P.parList.ptr + a, b - a, (const int*)P.vtabUp.ptr, 8, L, Lp, nChunks,
             (const uint8_t*)P.opM2Mbf.ptr, (const uint8_t*)P.multBf.ptr, (float*)P.mult.ptr, 0,
-            (uint8_t*)P.multBf.ptr, drainEvery, drainEvery, P.tcTrDrainItems, sp.na, sp.nb, sp.bStage, P.tcDrainMode, 0, cols, nullptr, P.pipeErr, P.tcWaitNs, P.tcAsyncArrive, nullptr);
+            (uint8_t*)P.multBf.ptr, drainEvery, drainEvery, P.tcTrDrainItems, sp.na, sp.nb, sp.bStage, P.tcDrainMode, 0, cols, prog, nullptr, P.pipeErr, P.tcWaitNs, asyncArrivals<Lay>(P), nullptr);
          FMM_TRY(launched(P, "kM2LTc<M2M>", st));
       }
       P.multBfTag = NP * 2 + (Lay::TF32 ? 1 : 0);
@@ -1311,7 +1400,7 @@ static fmm_status translateTc(Plan& P, cudaStream_t st, bool up)
             (const int*)P.l2lTargets.ptr + a, b - a, (const int*)P.vtabDn.ptr, 8, L, Lp, nChunks,
             (const uint8_t*)P.opL2Lbf.ptr, (const uint8_t*)P.multBf.ptr, (float*)P.local.ptr, 1, nullptr, drainEvery, drainEvery,
             P.tcTrDrainItems, sp.na, sp.nb, sp.bStage,
-            P.tcDrainMode, 0, cols, nullptr, P.pipeErr, P.tcWaitNs, P.tcAsyncArrive, nullptr);
+            P.tcDrainMode, 0, cols, prog, nullptr, P.pipeErr, P.tcWaitNs, asyncArrivals<Lay>(P), nullptr);
          FMM_TRY(launched(P, "kM2LTc<L2L>", st));
       }
       P.multBfTag = -1;
