@@ -44,6 +44,88 @@ fmm_status setError(fmm_status s, const char* fmt, ...)
    return s;
 }
 
+namespace {
+struct DevicePool
+{
+   std::once_flag once;
+   cudaMemPool_t pool = nullptr;
+   cudaStream_t stream = nullptr;
+};
+DevicePool* devicePool()
+{
+   static DevicePool pools[64];
+   int dev = 0;
+   if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+   DevicePool& d = pools[dev];
+   std::call_once(d.once, [&] {
+      int has = 0;
+      if(cudaDeviceGetAttribute(&has, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess || !has) return;
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      if(cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) { d.pool = nullptr; return; }
+      uint64_t keep = POOL_KEEP;
+      if(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+         cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking) != cudaSuccess)
+      {
+         cudaMemPoolDestroy(d.pool);
+         d.pool = nullptr;
+      }
+   });
+   cudaGetLastError();
+   return d.pool ? &d : nullptr;
+}
+}
+
+namespace {
+// Page-locked words for the plans' error reads: one page for the process (page-locking a word a plan took 2 ms with its
+// release), further ones of their own.
+constexpr int PINNED_WORDS = 1024;
+std::mutex g_pinnedMutex;
+int* g_pinned = nullptr;
+std::vector<int> g_pinnedFree;
+}
+
+cudaError_t pinnedWord(int** word)
+{
+   std::lock_guard<std::mutex> lock(g_pinnedMutex);
+   if(!g_pinned)
+   {
+      void* page = nullptr;
+      const cudaError_t e = cudaHostAlloc(&page, PINNED_WORDS * sizeof(int), cudaHostAllocPortable);
+      if(e != cudaSuccess) return e;
+      g_pinned = (int*)page;
+      for(int i = PINNED_WORDS - 1; i >= 0; i--) g_pinnedFree.push_back(i);
+   }
+   if(g_pinnedFree.empty()) return cudaMallocHost((void**)word, sizeof(int));
+   *word = g_pinned + g_pinnedFree.back();
+   g_pinnedFree.pop_back();
+   return cudaSuccess;
+}
+
+void pinnedWordFree(int* word)
+{
+   std::lock_guard<std::mutex> lock(g_pinnedMutex);
+   if(g_pinned && word >= g_pinned && word < g_pinned + PINNED_WORDS) g_pinnedFree.push_back(int(word - g_pinned));
+   else cudaFreeHost(word);
+}
+
+cudaError_t poolAlloc(void** ptr, size_t bytes)
+{
+   DevicePool* d = devicePool();
+   if(!d) return cudaErrorNotSupported;
+   cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, d->pool, d->stream);
+   if(e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
+   return e;
+}
+
+void poolFree(void* ptr)
+{
+   DevicePool* d = devicePool();
+   if(d) cudaFreeAsync(ptr, d->stream);
+}
+
 fmm_status Plan::ensureNodes(int64_t cap, cudaStream_t st)
 {
    if(cap <= nodeCap) return FMM_OK;
@@ -122,7 +204,7 @@ fmm_status Plan::init(const fmm_config& c)
    err = (int*)errb.ptr;
    pipeErr = err + 1;
    FMM_CUDA(cudaMemset(errb.ptr, 0, 2 * sizeof(int)));
-   FMM_CUDA(cudaMallocHost((void**)&hostErr, sizeof(int)));
+   FMM_CUDA(pinnedWord(&hostErr));
    *hostErr = 0;
    for(int i = 0; i < 8; i++) cudaEventCreate(&ev[i]);
    eventsMade = true;
@@ -150,14 +232,15 @@ void Plan::release()
       delete adj;
       adj = nullptr;
    }
-   DevBuf* bufs[] = {&srcXYZb, &srcWb, &srcJb, &tgtXYZb, &rootb, &sKeys, &tKeys, &sIdx, &tIdx, &sPos, &sQ, &tPos,
+   DevBuf* bufs[] = {&segb, &srcXYZb, &srcWb, &srcJb, &tgtXYZb, &rootb, &sKeys, &tKeys, &sIdx, &tIdx, &sPos, &sQ, &tPos,
                      &cubTmp, &scratch, &lvlBounds, &lvlCnt, &lvlOff, &p2pOff, &p2pList, &parList, &m2lTargets, &m2lKeys, &errb,
                      &mult, &local, &outB, &outA, &opM2M64, &opL2L64, &opM2L64, &opM2Lbf, &multBf, &tcCounters,
-                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotWs};
-   for(DevBuf* b : bufs) b->release();
-   for(auto& b : nodeBufs) b.release();
-   for(auto& b : listBufs) b.release();
-   if(hostErr) cudaFreeHost(hostErr);
+                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &directPart, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotWs};
+   cudaDeviceSynchronize();   // once for all buffers
+   for(DevBuf* b : bufs) b->release(true);
+   for(auto& b : nodeBufs) b.release(true);
+   for(auto& b : listBufs) b.release(true);
+   if(hostErr) pinnedWordFree(hostErr);
    hostErr = nullptr;
    err = pipeErr = nullptr;
    if(eventsMade)
@@ -261,6 +344,18 @@ fmm_status downwardPhase(Plan& P, cudaStream_t st)
    return FMM_OK;
 }
 
+// The packed sources of a direct sum: the tree's when there is one, else in input order.
+fmm_status directSources(Plan& P, cudaStream_t st)
+{
+   if(P.treeReady) return FMM_OK;
+   if(P.n + P.m == 0) return setError(FMM_E_INVALID, "no sources or targets set");
+   FMM_TRY(P.fp64 ? packSourcesT<double>(P, st) : packSourcesT<float>(P, st));
+   P.treeDeferred = true;
+   P.upReady = P.downReady = false;
+   P.dropGraph();
+   return FMM_OK;
+}
+
 double elapsed(cudaEvent_t a, cudaEvent_t b)
 {
    float ms = 0;
@@ -345,7 +440,7 @@ fmm_status fmm_set_sources(fmm_plan* plan, const void* xyz, const void* w, const
    P.bem = false;
    P.n = n;
    P.tgtIsSrc = false;
-   P.treeReady = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -398,7 +493,7 @@ fmm_status fmm_set_sources_async(fmm_plan* plan, const void* xyz, const void* w,
    P.bem = false;
    P.n = n;
    P.tgtIsSrc = false;
-   P.treeReady = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -451,7 +546,7 @@ fmm_status fmm_set_bem_sources(fmm_plan* plan, const void* xyz, const void* w, c
    }
    stage.release();
    P.inputsAsync = false;
-   P.treeReady = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
    P.dropGraph();
    return s;
 }
@@ -469,7 +564,7 @@ fmm_status fmm_set_targets(fmm_plan* plan, const void* xyz, int64_t m, int on_de
    if(!on_device) FMM_CUDA(cudaStreamSynchronize(st));
    P.m = m;
    P.tgtIsSrc = false;
-   P.treeReady = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -489,9 +584,15 @@ fmm_status fmm_set_targets_to_sources(fmm_plan* plan, void* stream)
    P.tgtXYZ = P.tgtXYZb.ptr;
    P.m = P.n;
    P.tgtIsSrc = true;
-   P.treeReady = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
+}
+
+// fmm_direct needs no tree and leaves it to the first call that does (those accept a plan after fmm_direct).
+static fmm_status buildDeferredTree(fmm_plan* plan, void* stream)
+{
+   return plan->P.treeDeferred && !plan->P.treeReady ? fmm_build_tree(plan, stream) : FMM_OK;
 }
 
 fmm_status fmm_build_tree(fmm_plan* plan, void* stream)
@@ -514,6 +615,7 @@ fmm_status fmm_upward(fmm_plan* plan, void* stream)
 {
    if(!plan) return setError(FMM_E_INVALID, "null plan");
    Plan& P = plan->P;
+   FMM_TRY(buildDeferredTree(plan, stream));
    if(!P.treeReady) return setError(FMM_E_INVALID, "fmm_upward: tree not built");
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
@@ -600,11 +702,11 @@ fmm_status fmm_direct(fmm_plan* plan, double current, int want, void* out_B, voi
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   if(!P.treeReady) FMM_TRY(fmm_build_tree(plan, stream));
+   FMM_TRY(directSources(P, st));
    size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    size_t bytes = es * 3 * std::max<int64_t>(P.m, 1);
-   FMM_TRY(P.outB.reserve(bytes));
-   FMM_TRY(P.outA.reserve(bytes));
+   if(want & 1) FMM_TRY(P.outB.reserve(bytes));
+   if(want & 2) FMM_TRY(P.outA.reserve(bytes));
    FMM_TRY(P.fp64 ? directT<double>(P, current, want, st) : directT<float>(P, current, want, st));
    if(want & 1) FMM_TRY(copyOut(out_B, P.outB, es * 3 * P.m, on_device, st));
    if(want & 2) FMM_TRY(copyOut(out_A, P.outA, es * 3 * P.m, on_device, st));
@@ -620,7 +722,7 @@ fmm_status fmm_direct_fp64_subset(fmm_plan* plan, double current, const double* 
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = 0;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   if(!P.treeReady) FMM_TRY(fmm_build_tree(plan, nullptr));
+   FMM_TRY(directSources(P, st));
    DevBuf t, o;
    FMM_TRY(t.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
    fmm_status s = o.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1));
@@ -923,7 +1025,7 @@ fmm_status fmm_batch_set_coils(fmm_plan* plan, int64_t ncoils, const int64_t* sr
       P.nCoils = int(ncoils);
       P.batch = true;
    }
-   P.treeReady = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -958,6 +1060,7 @@ fmm_status fmm_update_sources(fmm_plan* plan, const void* w, const void* J, int 
 {
    if(!plan) return setError(FMM_E_INVALID, "null plan");
    Plan& P = plan->P;
+   FMM_TRY(buildDeferredTree(plan, stream));
    if(!P.treeReady) return setError(FMM_E_INVALID, "fmm_update_sources: the tree is not built");
    if(P.n > 0 && !w) return setError(FMM_E_INVALID, "fmm_update_sources: null weights");
    if(P.bem) return setError(FMM_E_INVALID, "fmm_update_sources: set BEM sources again with fmm_set_bem_sources");
@@ -985,6 +1088,7 @@ fmm_status fmm_graph_capture(fmm_plan* plan, int want, void* stream)
    if(!plan) return setError(FMM_E_INVALID, "null plan");
    Plan& P = plan->P;
    const bool tcMode = !P.fp64 && P.cfg.m2l_mode != FMM_M2L_SIMT;
+   FMM_TRY(buildDeferredTree(plan, stream));
    if(!P.treeReady || P.opOrder != P.p || (tcMode && P.opImgOrder < 0))
       return setError(FMM_E_INVALID, "fmm_graph_capture: run fmm_solve first");
    if(want < 1 || want > 3) return setError(FMM_E_INVALID, "want must be 1, 2 or 3");
@@ -1079,6 +1183,12 @@ fmm_status fmm_get_stats(const fmm_plan* plan, fmm_stats* stats)
    if(!plan || !stats) return setError(FMM_E_INVALID, "null argument");
    const Plan& P = plan->P;
    DeviceGuard g(P.cfg.device);
+   if(P.treeDeferred && !P.treeReady)
+   {
+      // the tree fmm_direct left out, on the default stream after everything queued so far
+      FMM_CUDA(cudaDeviceSynchronize());
+      FMM_TRY(buildDeferredTree(const_cast<fmm_plan*>(plan), nullptr));
+   }
    fmm_stats s{};
    if(P.downReady) cudaEventSynchronize(P.ev[5]);
    s.ms_tree = elapsed(P.ev[0], P.ev[1]);

@@ -79,32 +79,53 @@ extern __constant__ int d_m2lIndex[NOFF];   // offset index (0..342) -> M2L slot
 extern __constant__ int d_m2lOffset[316];   // M2L slot -> offset index
 extern __constant__ int d_m2lFarFirst[316]; // M2L slots by decreasing offset length
 
+// Small device blocks (up to POOL_BLOCK bytes) come from a memory pool of the library, one per device, which keeps at most
+// POOL_KEEP bytes of freed blocks for later plans (the driver returns the rest): a plan has about fifty of them, and
+// cudaMalloc and cudaFree took ~5 ms for each plan a call creates and drops. A block is handed out after its pool's stream
+// has been waited for, so any stream may use it, and taken back after the device has been waited for (as cudaFree
+// does); the pool's own calls are safe from several threads. Larger blocks, and devices without memory pools, use cudaMalloc.
+constexpr size_t POOL_BLOCK = size_t(8) << 20, POOL_KEEP = size_t(128) << 20;
+cudaError_t poolAlloc(void** ptr, size_t bytes);   // cudaErrorNotSupported: no pool on the current device
+void poolFree(void* ptr);
+cudaError_t pinnedWord(int** word);   // a page-locked host word, and back
+void pinnedWordFree(int* word);
+
 // A growable device allocation.
 struct DevBuf
 {
    void* ptr = nullptr;
    size_t bytes = 0;
+   bool pooled = false;
    fmm_status reserve(size_t want)
    {
       if(want <= bytes) return FMM_OK;
-      if(ptr) cudaFree(ptr);
-      ptr = nullptr;
-      bytes = 0;
+      release();
       size_t b = std::max<size_t>(want, 256);
-      cudaError_t e = cudaMalloc(&ptr, b);
+      cudaError_t e = cudaErrorNotSupported;
+      if(b <= POOL_BLOCK) e = poolAlloc(&ptr, b);
+      pooled = e == cudaSuccess;
+      if(e == cudaErrorNotSupported) e = cudaMalloc(&ptr, b);
       if(e != cudaSuccess)
       {
          cudaGetLastError();
+         ptr = nullptr;
          return setError(FMM_E_OOM, "cudaMalloc(%zu) failed: %s", b, cudaGetErrorString(e));
       }
       bytes = b;
       return FMM_OK;
    }
-   void release()
+   // idle: the caller has waited for the device (cudaFree waits by itself)
+   void release(bool idle = false)
    {
-      if(ptr) cudaFree(ptr);
+      if(ptr && pooled)
+      {
+         if(!idle) cudaDeviceSynchronize();
+         poolFree(ptr);
+      }
+      else if(ptr) cudaFree(ptr);
       ptr = nullptr;
       bytes = 0;
+      pooled = false;
    }
 };
 
@@ -243,6 +264,7 @@ struct Plan
    int opImgOrder = -1;                  // order the tensor-core operator image was built for
    // state
    bool treeReady = false, upReady = false, downReady = false;
+   bool treeDeferred = false;            // fmm_direct has been called without a tree since the inputs were set
    fmm_stats stats{};
    cudaEvent_t ev[8];
    bool eventsMade = false;
@@ -268,6 +290,7 @@ struct Plan
    Plan* adj = nullptr;
    DevBuf adjG, adjOut;
    DevBuf tcPts, tcOut;                  // fmm_treecode: staging of host query points and results
+   DevBuf directPart;                    // fmm_direct: the sums of split sources
    DevBuf tcCurl, tcSort;                // its curl table (order tcCurlOrder) and the sorted points' keys and order
    std::vector<unsigned char> tcCurlHost;   // host copy of tcCurl (kept for the asynchronous upload)
    int tcCurlOrder = -1;
@@ -309,6 +332,7 @@ inline fmm_status launched(Plan& P, const char* name, cudaStream_t st)
 }
 
 template <class T> fmm_status buildTreeT(Plan& P, cudaStream_t st);
+template <class T> fmm_status packSourcesT(Plan& P, cudaStream_t st);   // sPos, sQ in input order, coil segments uploaded
 template <class T> fmm_status upwardT(Plan& P, cudaStream_t st);
 template <class T> fmm_status downwardT(Plan& P, cudaStream_t st);
 template <class T> fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st);

@@ -1181,25 +1181,35 @@ __global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 
 }
 
 // ====================================================================================
-// Direct sums over all sources (fmm_direct): one thread per target, sources staged through
-// shared memory.
+// Direct sums over all sources (fmm_direct): one thread per target, sources staged through shared memory in the
+// arithmetic's type. The sources of a coil are split over blockIdx.z where the targets alone leave the chip
+// idle; a part's sums then go to part[z][6][targets] and kDirectSum adds the parts in order.
+// Bound: the FP64 (FP32) pipe, about 30 FP64 instructions a pair with the library's rsqrt. With 1 / sqrt, the
+// potential summed whether wanted or not and no split, 38,400 sources x 10,000 targets in FP64 took 6.5 ms.
 // ====================================================================================
-template <class T, class U, int NT>
+template <class U> __device__ __forceinline__ U rsqrtOf(U x);
+template <> __device__ __forceinline__ float rsqrtOf<float>(float x) { return rsqrtf(x); }
+template <> __device__ __forceinline__ double rsqrtOf<double>(double x) { return rsqrt(x); }
+
+template <class T, class U, int NT, bool WANTB, bool WANTA>
 __global__ void __launch_bounds__(NT) kDirect(const typename Vec4<T>::type* __restrict__ spos,
                                               const typename Vec4<T>::type* __restrict__ sq, int n,
                                               const U* __restrict__ tgt, int m, const int* __restrict__ sseg,
-                                              const int* __restrict__ tseg, U scaleB, U scaleA, int want,
-                                              U* __restrict__ outB, U* __restrict__ outA)
+                                              const int* __restrict__ tseg, U scaleB, U scaleA, U* __restrict__ outB,
+                                              U* __restrict__ outA, U* __restrict__ part)
 {
-   __shared__ U Sp[NT][4];
-   __shared__ U Sq[NT][3];
+   typedef typename Vec4<U>::type U4;
+   __shared__ U4 Sp[NT];          // x, y, z, s_x
+   __shared__ U Sy[NT][2];        // s_y, s_z
    // blockIdx.y selects a coil: its targets [tseg[c], tseg[c+1]) see only its sources
    // [sseg[c], sseg[c+1]); without segments every target sees every source
    const int c = blockIdx.y;
    const int tBeg = tseg ? tseg[c] : 0, tEnd = tseg ? tseg[c + 1] : m;
-   const int sBeg = sseg ? sseg[c] : 0, sEnd = sseg ? sseg[c + 1] : n;
+   const int s0 = sseg ? sseg[c] : 0, s1 = sseg ? sseg[c + 1] : n;
    const int ti = tBeg + blockIdx.x * NT + threadIdx.x;
    if(tBeg + int(blockIdx.x) * NT >= tEnd) return;
+   const int sBeg = s0 + int(int64_t(s1 - s0) * blockIdx.z / gridDim.z);
+   const int sEnd = s0 + int(int64_t(s1 - s0) * (blockIdx.z + 1) / gridDim.z);
    const bool active = ti < tEnd;
    U x = 0, y = 0, z = 0;
    if(active) { x = tgt[3 * int64_t(ti)]; y = tgt[3 * int64_t(ti) + 1]; z = tgt[3 * int64_t(ti) + 2]; }
@@ -1212,31 +1222,55 @@ __global__ void __launch_bounds__(NT) kDirect(const typename Vec4<T>::type* __re
       {
          const auto a = spos[sb + threadIdx.x];
          const auto b = sq[sb + threadIdx.x];
-         Sp[threadIdx.x][0] = U(a.x); Sp[threadIdx.x][1] = U(a.y); Sp[threadIdx.x][2] = U(a.z);
-         Sq[threadIdx.x][0] = U(b.x); Sq[threadIdx.x][1] = U(b.y); Sq[threadIdx.x][2] = U(b.z);
+         Sp[threadIdx.x] = U4{U(a.x), U(a.y), U(a.z), U(b.x)};
+         Sy[threadIdx.x][0] = U(b.y);
+         Sy[threadIdx.x][1] = U(b.z);
       }
       __syncthreads();
       if(active)
+#pragma unroll 4
          for(int i = 0; i < cnt; i++)
          {
-            const U dx = x - Sp[i][0], dy = y - Sp[i][1], dz = z - Sp[i][2];
+            const U4 p = Sp[i];
+            const U sx = p.w, sy = Sy[i][0], sz = Sy[i][1];
+            const U dx = x - p.x, dy = y - p.y, dz = z - p.z;
             const U r2 = dx * dx + dy * dy + dz * dz;
-            if(r2 == U(0)) continue;
-            U ri;
-            if constexpr(sizeof(U) == 4) ri = rsqrtf(r2);
-            else ri = U(1) / sqrt(r2);
-            const U ri3 = ri * ri * ri;
-            B[0] += (Sq[i][1] * dz - Sq[i][2] * dy) * ri3;
-            B[1] += (Sq[i][2] * dx - Sq[i][0] * dz) * ri3;
-            B[2] += (Sq[i][0] * dy - Sq[i][1] * dx) * ri3;
-            A[0] += Sq[i][0] * ri; A[1] += Sq[i][1] * ri; A[2] += Sq[i][2] * ri;
+            const U ri = r2 == U(0) ? U(0) : rsqrtOf<U>(r2);   // (coincident pairs skipped)
+            if constexpr(WANTB)
+            {
+               const U ri3 = ri * ri * ri;
+               B[0] += (sy * dz - sz * dy) * ri3;
+               B[1] += (sz * dx - sx * dz) * ri3;
+               B[2] += (sx * dy - sy * dx) * ri3;
+            }
+            if constexpr(WANTA) { A[0] += sx * ri; A[1] += sy * ri; A[2] += sz * ri; }
          }
    }
-   if(active)
+   if(!active) return;
+   if(gridDim.z > 1)
    {
-      if(want & 1) for(int d = 0; d < 3; d++) outB[3 * int64_t(ti) + d] = B[d] * scaleB;
-      if(want & 2) for(int d = 0; d < 3; d++) outA[3 * int64_t(ti) + d] = A[d] * scaleA;
+      U* o = part + int64_t(blockIdx.z) * 6 * m + ti;
+      for(int d = 0; d < 3; d++)
+      {
+         if constexpr(WANTB) o[int64_t(d) * m] = B[d];
+         if constexpr(WANTA) o[int64_t(3 + d) * m] = A[d];
+      }
+      return;
    }
+   if constexpr(WANTB) for(int d = 0; d < 3; d++) outB[3 * int64_t(ti) + d] = B[d] * scaleB;
+   if constexpr(WANTA) for(int d = 0; d < 3; d++) outA[3 * int64_t(ti) + d] = A[d] * scaleA;
+}
+
+// out[3 i + d] = scale * the parts' sums of quantity d (0..2) of target i, first = 0 (B) or 3 (A)
+template <class U>
+__global__ void kDirectSum(const U* __restrict__ part, int parts, int m, int first, U scale, U* __restrict__ out)
+{
+   const int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+   if(e >= 3 * int64_t(m)) return;
+   const int d = int(e / m), i = int(e % m);
+   U s = U(0);
+   for(int q = 0; q < parts; q++) s += part[(int64_t(q) * 6 + first + d) * m + i];
+   out[3 * int64_t(i) + d] = s * scale;
 }
 
 // ====================================================================================
@@ -1377,47 +1411,61 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
    return FMM_OK;
 }
 
-template <class T>
-fmm_status directT(Plan& P, double current, int want, cudaStream_t st)
+// kDirect over coils of at most maxT targets and maxS sources (m targets in all), the sources split so that the
+// launch has about eight blocks a SM and a part keeps at least 512 sources.
+template <class T, class U>
+static fmm_status launchDirect(Plan& P, int coils, int maxT, int maxS, const U* tgt, int m, const int* sseg, const int* tseg,
+                               U scaleB, U scaleA, int want, U* outB, U* outA, cudaStream_t st)
 {
    typedef typename Vec4<T>::type V4;
    constexpr int NT = 128;
-   T scaleB = T(REF_MU0 / (4 * REF_PI) * current), scaleA = T(1.0 / (4 * REF_PI) * current);
-   if(P.bem) return bemDirectT<T>(P, st);
-   int maxT = 0;
-   for(int c = 0; c < P.nCoils; c++) maxT = std::max(maxT, P.tgtOff[c + 1] - P.tgtOff[c]);
    const int blocks = (maxT + NT - 1) / NT;
    if(blocks == 0) return FMM_OK;
-   const int* seg = (const int*)P.segb.ptr;   // srcOff then tgtOff, uploaded by the tree build
-   kDirect<T, T, NT><<<dim3(blocks, P.nCoils), NT, 0, st>>>((const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, int(P.n),
-                                                           (const T*)P.tgtXYZ, int(P.m), seg, seg + P.nCoils + 1,
-                                                           scaleB, scaleA, want, (T*)P.outB.ptr, (T*)P.outA.ptr);
+   const int64_t wantParts = (8 * 148 + int64_t(blocks) * coils - 1) / (int64_t(blocks) * coils);
+   const int parts = int(std::max<int64_t>(1, std::min<int64_t>(wantParts, maxS / 512)));
+   if(parts > 1) FMM_TRY(P.directPart.reserve(sizeof(U) * 6 * size_t(parts) * size_t(m)));
+   U* part = (U*)P.directPart.ptr;
+   auto run = [&](auto kern) {
+      kern<<<dim3(blocks, coils, parts), NT, 0, st>>>((const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, int(P.n), tgt, m, sseg, tseg,
+                                                      scaleB, scaleA, outB, outA, part);
+   };
+   if(want == 1) run(kDirect<T, U, NT, true, false>);
+   else if(want == 2) run(kDirect<T, U, NT, false, true>);
+   else run(kDirect<T, U, NT, true, true>);
    FMM_TRY(launched(P, "kDirect", st));
+   if(parts > 1)
+   {
+      const int sumBlocks = int((3 * int64_t(m) + 255) / 256);
+      if(want & 1) kDirectSum<U><<<sumBlocks, 256, 0, st>>>(part, parts, m, 0, scaleB, outB);
+      if(want & 2) kDirectSum<U><<<sumBlocks, 256, 0, st>>>(part, parts, m, 3, scaleA, outA);
+      FMM_TRY(launched(P, "kDirectSum", st));
+   }
    FMM_CHECK_LAUNCH();
    return FMM_OK;
 }
 
+template <class T>
+fmm_status directT(Plan& P, double current, int want, cudaStream_t st)
+{
+   T scaleB = T(REF_MU0 / (4 * REF_PI) * current), scaleA = T(1.0 / (4 * REF_PI) * current);
+   if(P.bem) return bemDirectT<T>(P, st);
+   int maxT = 0, maxS = 0;
+   for(int c = 0; c < P.nCoils; c++)
+   {
+      maxT = std::max(maxT, P.tgtOff[c + 1] - P.tgtOff[c]);
+      maxS = std::max(maxS, P.srcOff[c + 1] - P.srcOff[c]);
+   }
+   const int* seg = (const int*)P.segb.ptr;   // srcOff then tgtOff, uploaded by the tree build
+   return launchDirect<T, T>(P, P.nCoils, maxT, maxS, (const T*)P.tgtXYZ, int(P.m), seg, seg + P.nCoils + 1, scaleB, scaleA,
+                             want, (T*)P.outB.ptr, (T*)P.outA.ptr, st);
+}
+
 fmm_status directFp64Subset(Plan& P, double current, const double* tgtDev, int k, double* outDev, cudaStream_t st)
 {
-   constexpr int NT = 128;
-   int blocks = (k + NT - 1) / NT;
-   if(blocks == 0) return FMM_OK;
-   double scaleB = REF_MU0 / (4 * REF_PI) * current;
+   const double scaleB = REF_MU0 / (4 * REF_PI) * current;
    if(P.fp64)
-   {
-      kDirect<double, double, NT><<<blocks, NT, 0, st>>>((const double4*)P.sPos.ptr, (const double4*)P.sQ.ptr,
-                                                         int(P.n), tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1,
-                                                         outDev, nullptr);
-      FMM_TRY(launched(P, "kDirect", st));
-   }
-   else
-   {
-      kDirect<float, double, NT><<<blocks, NT, 0, st>>>((const float4*)P.sPos.ptr, (const float4*)P.sQ.ptr, int(P.n),
-                                                        tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1, outDev, nullptr);
-      FMM_TRY(launched(P, "kDirect", st));
-   }
-   FMM_CHECK_LAUNCH();
-   return FMM_OK;
+      return launchDirect<double, double>(P, 1, k, int(P.n), tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1, outDev, nullptr, st);
+   return launchDirect<float, double>(P, 1, k, int(P.n), tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1, outDev, nullptr, st);
 }
 
 // New strengths w J for the same source positions, in the tree's sorted order.

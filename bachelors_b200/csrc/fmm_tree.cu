@@ -173,7 +173,7 @@ __global__ void kGatherSources(const T* __restrict__ xyz, const T* __restrict__ 
 {
    int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
    if(i >= n) return;
-   int64_t s = order[i];
+   int64_t s = order ? order[i] : i;
    T x = xyz[3 * s], y = xyz[3 * s + 1], z = xyz[3 * s + 2];
    T jx, jy, jz;
    if(J) { jx = J[3 * s]; jy = J[3 * s + 1]; jz = J[3 * s + 2]; }
@@ -1004,12 +1004,10 @@ static fmm_status buildLevelsPersistent(Plan& P, cudaStream_t st, int64_t& capNo
    return setError(FMM_E_LIMIT, "kBuildLevels: node capacity did not converge");
 }
 
-template <class T>
-fmm_status buildTreeT(Plan& P, cudaStream_t st)
+// The coils' offsets (one coil by default), checked and uploaded: srcOff then tgtOff in segb.
+static fmm_status uploadCoils(Plan& P, cudaStream_t st)
 {
    const int64_t n = P.n, m = P.m;
-   const int threads = 256;
-   // coils: one by default; the key keeps ceil(log2(coils)) bits above the Morton bits
    const int K = P.nCoils;
    if(!P.batch)
    {
@@ -1020,15 +1018,49 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       return setError(FMM_E_INVALID, "coil offsets do not match the source/target counts (%lld, %lld); "
                                      "call fmm_batch_set_coils after setting sources and targets",
                       (long long)n, (long long)m);
-   P.coilBits = 0;
-   while((int64_t(1) << P.coilBits) < K) P.coilBits++;
-   P.maxLevel = std::min(MAXLEVEL, (63 - P.coilBits) / 3);
-   FMM_TRY(P.waitSourcePoints(st));   // points copied by fmm_set_sources_async
    FMM_TRY(P.segb.reserve(sizeof(int) * 2 * (K + 1)));
    int* dSrcOff = (int*)P.segb.ptr;
    int* dTgtOff = dSrcOff + K + 1;
    FMM_CUDA(cudaMemcpyAsync(dSrcOff, P.srcOff.data(), sizeof(int) * (K + 1), cudaMemcpyHostToDevice, st));
    FMM_CUDA(cudaMemcpyAsync(dTgtOff, P.tgtOff.data(), sizeof(int) * (K + 1), cudaMemcpyHostToDevice, st));
+   return FMM_OK;
+}
+
+template <class T>
+fmm_status packSourcesT(Plan& P, cudaStream_t st)
+{
+   typedef typename Vec4<T>::type V4;
+   const int64_t n = P.n;
+   FMM_TRY(uploadCoils(P, st));
+   FMM_TRY(P.sPos.reserve(sizeof(V4) * std::max<int64_t>(n, 1)));
+   FMM_TRY(P.sQ.reserve(sizeof(V4) * std::max<int64_t>(n, 1)));
+   if(n)
+   {
+      kGatherSources<T><<<int((n + 255) / 256), 256, 0, st>>>(
+         (const T*)P.srcXYZ, (const T*)P.srcW, (const T*)(P.hasJ ? P.srcJ : nullptr),
+         (const T*)(P.bem ? P.srcSigma : nullptr), nullptr, n, (V4*)P.sPos.ptr, (V4*)P.sQ.ptr);
+      FMM_TRY(launched(P, "kGatherSources", st));
+   }
+   return FMM_OK;
+}
+
+template fmm_status packSourcesT<float>(Plan&, cudaStream_t);
+template fmm_status packSourcesT<double>(Plan&, cudaStream_t);
+
+template <class T>
+fmm_status buildTreeT(Plan& P, cudaStream_t st)
+{
+   const int64_t n = P.n, m = P.m;
+   const int threads = 256;
+   // the key keeps ceil(log2(coils)) bits above the Morton bits
+   const int K = P.nCoils;
+   FMM_TRY(uploadCoils(P, st));
+   int* dSrcOff = (int*)P.segb.ptr;
+   int* dTgtOff = dSrcOff + K + 1;
+   P.coilBits = 0;
+   while((int64_t(1) << P.coilBits) < K) P.coilBits++;
+   P.maxLevel = std::min(MAXLEVEL, (63 - P.coilBits) / 3);
+   FMM_TRY(P.waitSourcePoints(st));   // points copied by fmm_set_sources_async
    // root cubes
    FMM_TRY(P.rootb.reserve(sizeof(RootBox) * K));
    P.root = (RootBox*)P.rootb.ptr;

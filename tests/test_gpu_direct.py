@@ -1,0 +1,79 @@
+"""The direct sum with its sources split over blocks and without a tree: sizes around the block (128 targets) and the
+smallest part (512 sources), both precisions, B and A, coils, and what a plan accepts after fmm_direct."""
+import numpy as np
+import pytest
+
+from bachelors_b200 import FmmError, Plan, geometry as G
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(xyz, w, J, tgt, dtype=np.float64):
+    """B and A in FP64 from strengths w J rounded to the plan's type, as the plan packs them."""
+    d = tgt[:, None, :] - xyz[None, :, :]
+    r2 = (d ** 2).sum(-1)
+    ri = np.where(r2 > 0, 1 / np.sqrt(np.where(r2 > 0, r2, 1)), 0)
+    q = (w.astype(dtype)[:, None] * J.astype(dtype)).astype(np.float64)
+    B = np.cross(q[None], d)
+    c = 4 * 3.14159265359
+    return 1.2566370614e-6 / c * (B * (ri ** 3)[..., None]).sum(1), (q[None] * ri[..., None]).sum(1) / c
+
+
+def rel(a, b):
+    return np.linalg.norm(np.asarray(a, np.float64) - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (511, 127), (512, 128), (1023, 129), (1024, 5), (5003, 300)])
+# FP32: n terms of 2^-24 each in blocks of at most a few thousand, against the same FP32 inputs
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("fp32", 3e-5)])
+def test_direct_sizes(n, m, precision, tol):
+    rng = np.random.default_rng(n + m)
+    xyz, w, J = rng.uniform(-1, 1, (n, 3)), rng.uniform(0.5, 1, n), rng.normal(size=(n, 3))
+    tgt = rng.uniform(-1.5, 1.5, (m, 3))
+    if m > 1:
+        tgt[0] = xyz[0]                                  # a coincident pair
+    if precision == "fp32":
+        xyz, w, J, tgt = (v.astype(np.float32).astype(np.float64) for v in (xyz, w, J, tgt))
+    plan = Plan(order=2, leaf_capacity=64, precision=precision)
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    Bo, Ao = reference(xyz, w, J, tgt, np.float32 if precision == "fp32" else np.float64)
+    for want in (1, 2, 3):
+        B, A = plan.direct(1.0, want)
+        assert B is None or rel(B, Bo) < tol
+        assert A is None or rel(A, Ao) < tol
+    assert rel(plan.direct_fp64(tgt), Bo) < 1e-12
+    plan.solve(1.0, 1)                                  # the same sums over the tree's order of the sources
+    assert rel(plan.direct(1.0, 1)[0], Bo) < tol
+    plan.close()
+
+
+def test_after_direct():
+    xyz, w, J = G.torus(16, 8, 4)
+    tgt = G.uniform_points(100, -3, 3, 1)
+    plan = Plan(order=4, leaf_capacity=16, precision="fp64")
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    with pytest.raises(FmmError):
+        plan.upward()                                   # no tree
+    plan.direct(1.0, 1)
+    nodes = plan.stats()["nodes"]
+    plan.upward()                                       # fmm_direct stands for the tree build
+    plan.downward()
+    B, _ = plan.evaluate(1.0, 1)
+    S, _ = plan.solve(1.0, 1)
+    assert np.array_equal(B, S) and plan.stats()["nodes"] == nodes
+    plan.set_targets(tgt[:50])
+    with pytest.raises(FmmError):
+        plan.upward()                                   # new inputs: not any more
+    plan.close()
+    # coils see only their own sources
+    plan = Plan(order=2, precision="fp64")
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    plan.set_coils([0, 200, 200, len(w)], [0, 30, 60, 100])
+    B, _ = plan.direct(1.0, 1)
+    assert rel(B[:30], reference(xyz[:200], w[:200], J[:200], tgt[:30])[0]) < 1e-12
+    assert not B[30:60].any()
+    assert rel(B[60:], reference(xyz[200:], w[200:], J[200:], tgt[60:])[0]) < 1e-12
+    plan.close()
