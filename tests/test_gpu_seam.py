@@ -92,3 +92,33 @@ def test_seam_rejects_bad_arguments():
     from bachelors_b200._lib import FmmError
     with pytest.raises(FmmError):
         K.translateAllGPU(np.zeros((1, 34 ** 2)), np.zeros((1, 34 ** 2, 3)))   # order 33 > 32
+
+
+@pytest.mark.parametrize("p,count", [(0, 1), (1, 31), (3, 32), (6, 33), (10, 65), (13, 40), (14, 3), (19, 2), (20, 2)])
+def test_translate_all_block_edges(p, count):
+    """Blocks of 32 items (full, one short, one over, a single item) and the orders where an item's entries stop
+    fitting the shared memory (FP64 above 13, FP32 above 19)."""
+    import torch
+    rng = np.random.default_rng(p + count)
+    L = (p + 1) ** 2
+    fall = 0.7 ** np.floor(np.sqrt(np.arange(L)))
+    a = rng.normal(size=(count, L)) * fall
+    b = rng.normal(size=(count, L, 3)) * fall[:, None]
+    ref = O.translate_all(p, a, b)
+    for dt, tol in ((torch.float64, 1e-12), (torch.float32, 1e-5)):
+        got = K.translateAllGPU(torch.tensor(a, dtype=dt, device="cuda"), torch.tensor(b, dtype=dt, device="cuda"))
+        assert rel(got, ref) < tol
+
+
+@pytest.mark.parametrize("L,count,batch", [(4, 127, 1), (64, 128, 2), (121, 129, 1), (144, 3, 3), (1089, 40, 1)])
+def test_translate_all_matrix_tiles(L, count, batch):
+    """Tiles of 128 rows and 128 (FP64: 64) columns, 16-deep slices: full, with remainders, smaller than one."""
+    import torch
+    rng = np.random.default_rng(L * count)
+    a, b = rng.normal(size=(batch, count, L)), rng.normal(size=(L, L)) / np.sqrt(L)
+    ref = a @ b
+    p = int(round(L ** 0.5)) - 1
+    for dt, tol in ((torch.float64, 1e-12), (torch.float32, 1e-5)):
+        got = K.translateAllGPUMatrixCuBLAS(torch.tensor(a, dtype=dt, device="cuda"), torch.tensor(b, dtype=dt, device="cuda"),
+                                            harmonicOrder=p)
+        assert rel(got, ref) < tol
