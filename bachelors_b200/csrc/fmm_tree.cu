@@ -65,17 +65,26 @@ __device__ void setRootBox(const double lo[3], const double hi[3], int maxLevel,
    root->scale = double(int64_t(1) << maxLevel) / (2.0 * H);
 }
 
-__global__ void kRootFromBBox(const double* partial, int nblocks, int maxLevel, RootBox* root)
+// (one block of 256 threads; a single thread over up to 1024 partial boxes took 0.22 ms)
+__global__ void __launch_bounds__(256) kRootFromBBox(const double* partial, int nblocks, int maxLevel, RootBox* root)
 {
-   if(threadIdx.x != 0 || blockIdx.x != 0) return;
    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-   for(int b = 0; b < nblocks; b++)
+   for(int b = threadIdx.x; b < nblocks; b += 256)
       for(int d = 0; d < 3; d++)
       {
          lo[d] = fmin(lo[d], partial[6 * b + d]);
          hi[d] = fmax(hi[d], partial[6 * b + 3 + d]);
       }
-   setRootBox(lo, hi, maxLevel, root);
+   typedef cub::BlockReduce<double, 256> BR;
+   __shared__ typename BR::TempStorage tmp;
+   for(int d = 0; d < 3; d++)
+   {
+      lo[d] = BR(tmp).Reduce(lo[d], cub::Min());
+      __syncthreads();
+      hi[d] = BR(tmp).Reduce(hi[d], cub::Max());
+      __syncthreads();
+   }
+   if(threadIdx.x == 0) setRootBox(lo, hi, maxLevel, root);
 }
 
 __global__ void kRootFromConfig(double cx, double cy, double cz, double H, int maxLevel, RootBox* root)
@@ -214,15 +223,33 @@ __global__ void kInitRoots(Tree t, int nCoils, const int* __restrict__ srcOff, c
    t.parent[c] = -1; t.child0[c] = -1; t.nchild[c] = 0;
 }
 
-__device__ __forceinline__ int lowerBound(const uint64_t* __restrict__ keys, int a, int b, uint64_t v)
+// The first positions in keys[a, b) whose key is >= first + c step, c = 1..7: the seven searches halve the same range
+// together, so that their loads are in flight at once (one after the other, the level build waited for 14 searches
+// of a node in a row: 1.0 ms of tree phase at 2^20 points and targets, 0.51 this way).
+__device__ __forceinline__ void lowerBounds7(const uint64_t* __restrict__ keys, int a, int b, uint64_t first, uint64_t step,
+                                             int (&pos)[7])
 {
-   while(a < b)
+#pragma unroll
+   for(int c = 0; c < 7; c++) pos[c] = a;
+   int len = b - a;
+   while(len > 1)
    {
-      int mid = (a + b) >> 1;
-      if(keys[mid] < v) a = mid + 1;
-      else b = mid;
+      const int half = len >> 1;
+      uint64_t k[7];
+#pragma unroll
+      for(int c = 0; c < 7; c++) k[c] = keys[pos[c] + half - 1];
+#pragma unroll
+      for(int c = 0; c < 7; c++) pos[c] += k[c] < first + uint64_t(c + 1) * step ? half : 0;
+      len -= half;
    }
-   return a;
+   if(len == 1)
+   {
+      uint64_t k[7];
+#pragma unroll
+      for(int c = 0; c < 7; c++) k[c] = keys[pos[c]];
+#pragma unroll
+      for(int c = 0; c < 7; c++) pos[c] += k[c] < first + uint64_t(c + 1) * step ? 1 : 0;
+   }
 }
 
 // Node i (the j-th of its level): decide the split and find the 8 children's ranges (bounds row j);
@@ -236,15 +263,18 @@ __device__ int childBounds(Tree& t, int i, int j, int level, int maxLevel, int c
    if(!((s1 - s0 > cap || t1 - t0 > capT) && level < maxLevel)) return 0;
    uint64_t key = t.key[i];
    int shift = 3 * (maxLevel - level - 1);
-   int sb[9], tb[9];
-   for(int c = 0; c < 8; c++)
-   {
-      uint64_t bound = ((key << 3) + uint64_t(c)) << shift;
-      sb[c] = c == 0 ? s0 : lowerBound(skeys, s0, s1, bound);
-      tb[c] = c == 0 ? t0 : lowerBound(tkeys, t0, t1, bound);
-   }
+   int sb[9], tb[9], found[7];
+   const uint64_t first = (key << 3) << shift, step = uint64_t(1) << shift;
+   lowerBounds7(skeys, s0, s1, first, step, found);
+#pragma unroll
+   for(int c = 0; c < 7; c++) sb[c + 1] = found[c];
+   lowerBounds7(tkeys, t0, t1, first, step, found);
+#pragma unroll
+   for(int c = 0; c < 7; c++) tb[c + 1] = found[c];
+   sb[0] = s0; tb[0] = t0;
    sb[8] = s1; tb[8] = t1;
    int k = 0;
+#pragma unroll
    for(int c = 0; c < 8; c++)
    {
       bounds[18 * j + c] = sb[c];
@@ -394,7 +424,7 @@ __device__ __forceinline__ unsigned long long lbWord(int level, int state, int v
    return (unsigned long long)(level + 1) << 40 | (unsigned long long)state << 32 | unsigned(value);
 }
 
-__global__ void __launch_bounds__(LB_T, 6) kBuildLevels(Tree t, int maxLevel, int cap, int capT,
+__global__ void __launch_bounds__(LB_T, 4) kBuildLevels(Tree t, int maxLevel, int cap, int capT,
                                                         const uint64_t* __restrict__ skeys,
                                                         const uint64_t* __restrict__ tkeys, int* bounds,
                                                         unsigned long long* look, int64_t capNodes,
@@ -698,8 +728,88 @@ __global__ void kNearCounts(Tree t, int nNodes, const int* __restrict__ off, con
    }
 }
 
-// Direct-interaction source nodes of every target leaf (count pass when out == nullptr).
-__global__ void kP2PLists(Tree t, Lists L, int nNodes, const int* __restrict__ off, int* cnt, int* out, int* err)
+// Direct-interaction source nodes of every target leaf (count pass when out == nullptr), a warp per node: the
+// same-level leaf colleagues (the leaf itself among them) and coarser adjacent leaves; below the colleagues that are no leaves
+// the adjacent leaves and the non-adjacent nodes whose parent is adjacent (the duals of A and X); the
+// coarser non-adjacent leaves of the node and its ancestors. The nodes below colleagues wait on a stack in shared
+// memory, from which the lanes take up to 32 at a time: a batch of b nodes pushes at most 8 b, and is small enough
+// that the stack then holds the descent of one node (at most 7 more a level) as well. Entries are appended in lane
+// order, so the lists are the same from run to run. Both passes, a thread per leaf with a stack in local memory
+// (kP2PListsThread) -> this: 187 leaves 113 -> 15 us, 2^20 points and targets 0.34 -> 0.11 ms; the 256-coil batch 1.7
+// -> 2.2 ms (3.8 with eight lanes a node), so batches keep the thread per leaf.
+constexpr int PL_WARPS = 4, PL_STACK = 768;
+
+__global__ void __launch_bounds__(32 * PL_WARPS) kP2PLists(Tree t, Lists L, int nNodes, const int* __restrict__ off, int* cnt,
+                                                           int* out)
+{
+   __shared__ int stackS[PL_WARPS][PL_STACK];
+   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+   const int T = blockIdx.x * PL_WARPS + w;
+   if(T >= nNodes) return;
+   if(t.nchild[T] != 0 || t.t1[T] == t.t0[T])
+   {
+      if(!out && lane == 0) cnt[T] = 0;
+      return;
+   }
+   int* stack = stackS[w];
+   const unsigned below = (1u << lane) - 1u;
+   int k = 0, sp = 0;
+   const int base = out ? off[T] : 0;
+   // appends the lanes' nodes (those with sources) in lane order
+   auto emit = [&](bool has, int S) {
+      has = has && t.s1[S] > t.s0[S];
+      const unsigned m = __ballot_sync(0xffffffffu, has);
+      if(has && out) out[base + k + __popc(m & below)] = S;
+      k += __popc(m);
+   };
+   // pushes the children of the lanes' nodes (nc of them from c0)
+   auto push = [&](int nc, int c0) {
+      int incl = nc;
+      for(int d = 1; d < 32; d <<= 1)
+      {
+         const int v = __shfl_up_sync(0xffffffffu, incl, d);
+         if(lane >= d) incl += v;
+      }
+      for(int c = 0; c < nc; c++) stack[sp + incl - nc + c] = c0 + c;
+      sp += __shfl_sync(0xffffffffu, incl, 31);
+      __syncwarp();
+   };
+   // colleagues and their children (at most 27 and 216)
+   const int nc = L.ncol[T];
+   for(int e0 = 0; e0 < nc; e0 += 32)
+   {
+      const bool in = e0 + lane < nc;
+      const int C = in ? L.col[int64_t(T) * COLCAP + e0 + lane] : 0;
+      const int kids = in ? t.nchild[C] : 0;
+      emit(in && kids == 0, C);
+      push(kids, kids ? t.child0[C] : 0);
+   }
+   for(int e0 = 0; e0 < L.na[T]; e0 += 32)
+      emit(e0 + lane < L.na[T], e0 + lane < L.na[T] ? L.acoarse[int64_t(T) * ACAP + e0 + lane] : 0);
+   while(sp > 0)
+   {
+      // n nodes off the top: sp + 7 n <= PL_STACK - 160 while n > 1, and one node's descent adds at most 7 a level
+      const int n = min(sp, max(1, min(32, (PL_STACK - 160 - sp) / 7)));
+      sp -= n;
+      const int Q = lane < n ? stack[sp + lane] : 0;
+      __syncwarp();
+      const bool adj = lane < n && adjacentNodes(t, Q, T);
+      const int kids = adj ? t.nchild[Q] : 0;
+      emit(lane < n && (!adj || kids == 0), Q);
+      push(kids, kids ? t.child0[Q] : 0);
+   }
+   for(int a = T; a >= 0; a = t.parent[a])
+   {
+      const int nx = L.nx[a];
+      for(int e0 = 0; e0 < nx; e0 += 32)
+         emit(e0 + lane < nx, e0 + lane < nx ? L.xl[int64_t(a) * XCAP + e0 + lane] : 0);
+   }
+   if(!out && lane == 0) cnt[T] = k;
+}
+
+// kP2PLists with a thread per node, for batches: their leaves have few candidates, and a group of lanes waits for the
+// longest of them.
+__global__ void kP2PListsThread(Tree t, Lists L, int nNodes, const int* __restrict__ off, int* cnt, int* out, int* err)
 {
    int T = blockIdx.x * blockDim.x + threadIdx.x;
    if(T >= nNodes) return;
@@ -1083,7 +1193,7 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_TRY(P.scratch.reserve(sizeof(double) * 6 * nb));
       kBBox<T><<<nb, threads, 0, st>>>((const T*)P.srcXYZ, n, (const T*)P.tgtXYZ, m, (double*)P.scratch.ptr);
       FMM_TRY(launched(P, "kBBox", st));
-      kRootFromBBox<<<1, 1, 0, st>>>((const double*)P.scratch.ptr, nb, P.maxLevel, P.root);
+      kRootFromBBox<<<1, 256, 0, st>>>((const double*)P.scratch.ptr, nb, P.maxLevel, P.root);
       FMM_TRY(launched(P, "kRootFromBBox", st));
    }
    FMM_CHECK_LAUNCH();
@@ -1250,7 +1360,11 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
    FMM_TRY(P.lvlCnt.reserve(sizeof(int) * (nn + 1)));
    int* pc = (int*)P.lvlCnt.ptr;
    int* po = (int*)P.p2pOff.ptr;
-   kP2PLists<<<(nn + 127) / 128, 128, 0, st>>>(t, Ls, nn, nullptr, pc, nullptr, P.err);
+   auto p2pLists = [&](const int* offs, int* counts, int* list) {
+      if(K == 1) kP2PLists<<<(nn + PL_WARPS - 1) / PL_WARPS, 32 * PL_WARPS, 0, st>>>(t, Ls, nn, offs, counts, list);
+      else kP2PListsThread<<<(nn + 127) / 128, 128, 0, st>>>(t, Ls, nn, offs, counts, list, P.err);
+   };
+   p2pLists(nullptr, pc, nullptr);
    FMM_TRY(launched(P, "kP2PLists", st));
    FMM_CUDA(cudaMemsetAsync(pc + nn, 0, sizeof(int), st));
    tmp = 0;
@@ -1274,7 +1388,7 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
    FMM_CUDA(cudaStreamSynchronize(st));
    if(herr) return setError(FMM_E_LIMIT, "interaction list capacity exceeded (code %d)", herr);
    FMM_TRY(P.p2pList.reserve(sizeof(int) * std::max(nP2P, 1)));
-   kP2PLists<<<(nn + 127) / 128, 128, 0, st>>>(t, Ls, nn, po, nullptr, (int*)P.p2pList.ptr, P.err);
+   p2pLists(po, nullptr, (int*)P.p2pList.ptr);
    FMM_TRY(launched(P, "kP2PLists", st));
    FMM_CHECK_LAUNCH();
    P.nP2P = nP2P;
