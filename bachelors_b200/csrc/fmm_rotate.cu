@@ -477,7 +477,7 @@ __device__ __forceinline__ void turn(const unsigned* pairs, int nPairs, int warp
    }
 }
 
-constexpr int MAXT = 40;      // target boxes of an M2L or M2M tile at most
+constexpr int MAXT = 100;     // target boxes of an M2L or M2M tile at most
 constexpr int MAXTL = 160;    // of an L2L tile
 template <class T>
 struct Smem   // byte offsets in the block's dynamic shared memory
@@ -506,6 +506,18 @@ __device__ __forceinline__ void cpAsync16(void* dst, const void* src)
    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
+// one element, asynchronously
+__device__ __forceinline__ void cpAsyncElem(float* dst, const float* src)
+{
+   const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cpAsyncElem(double* dst, const double* src)
+{
+   const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+
 // 2^-l of coefficient k's degree l (half that with `less`): a coefficient's own term in the M2M (L2L)
 template <class T>
 __device__ __forceinline__ T boxScale(int k, bool less)
@@ -524,12 +536,13 @@ struct L2LSegR { int start[9]; };
 // such buffers, and the result is turned back and added to the targets' rows in global memory (one block owns
 // them; they stay in L2). A lane holds 8 (FP64: 4) vectors, a quarter-warp four outputs: per input
 // coefficient and lane three (FP64: four) 16-byte shared loads for 32 (16) multiply-adds, FP32 ones in
-// packed pairs. 16 warps an SM (two blocks of 8, one of 16 from p = 13 on, where one block fills the shared memory).
-// What bounds it (p = 12): ~17,000 warp instructions and ~3,000 shared-memory wavefronts a full chunk, 55 % of the issue
-// slots used; fewer warps were slower (8 an SM: 23.0 ms a solve of 2^20 points and targets, 12: 20.3, 16: 19.1), as was
-// a lane per vector with the inputs in registers and every block size unrolled (31.4 ms, instruction fetch).
-// Measured, dense operators on the CUDA cores -> this: M2L of 2^20 torus points, p = 12, FP32 55.4 -> 17.9 ms; 2^19
-// points, p = 16, 61.5 -> 23.6 ms; 65,536 points, p = 12, FP64 24.1 -> 2.6 ms; 2,000 points, p = 10, 3.4 -> 0.05 ms; L2L
+// packed pairs. 16 warps an SM, in one to four blocks.
+// What bounds it (p = 12): ~17,000 warp instructions and ~3,500 shared-memory wavefronts a full chunk, half of the issue
+// slots used, the rest fixed latencies and barriers; fewer warps were slower (8 an SM: 23.0 ms a solve of 2^20 points and targets,
+// 12: 20.3, 16: 19.1), as was a lane per vector with the inputs in registers and every block size unrolled (31.4 ms,
+// instruction fetch).
+// Measured, dense operators on the CUDA cores -> this: M2L of 2^20 torus points, p = 12, FP32 55.4 -> 15.1 ms; 2^19
+// points, p = 16, 61.5 -> 20.1 ms; 65,536 points, p = 12, FP64 24.1 -> 2.3 ms; 2,000 points, p = 10, 3.4 -> 0.05 ms; L2L
 // of 2^24 points, p = 16, 13.4 -> 9.3 ms.
 //   MODE 0: M2L, X = multipoles, Y = locals (zero before); vtab[box][316], the tile's boxes are targets[..]
 //   MODE 1: M2M, X = Y = multipoles, the boxes are parents (zero before), vtab[parent][8] their children with sources
@@ -654,15 +667,16 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
       return vtab[int64_t(tileNode[t]) * NOP + o];
    };
    // warp 0: the pairs of operator oi, compacted; the sources were loaded one operator earlier
-   int ahead[2] = {-1, -1};
+   constexpr int AH = (MAXT + 31) / 32;
+   int ahead[AH];
    auto loadAhead = [&](int oi) {
-      ahead[0] = sourceOf(lane, offs[oi]);
-      ahead[1] = sourceOf(lane + 32, offs[oi]);
+#pragma unroll
+      for(int h = 0; h < AH; h++) ahead[h] = sourceOf(lane + 32 * h, offs[oi]);
    };
    auto compact = [&](int b) {
       int n = 0;
 #pragma unroll
-      for(int h = 0; h < 2; h++)
+      for(int h = 0; h < AH; h++)
       {
          const uint32_t bits = __ballot_sync(0xffffffffu, ahead[h] >= 0);
          if(ahead[h] >= 0)
@@ -686,70 +700,61 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
          dstRow[db][tid] = 3 * (MODE == 2 ? tileNode[t] : toParts ? slotT[b][t] : tileNode[slotT[b][t]]) + cmp;
       }
    };
-   // rows and coefficients move between global and shared memory with 4 lanes of V consecutive coefficients
-   // by 8 rows
-   const int kl = V * (lane & 3), rl = lane >> 2, nkb = (Lp + 4 * V - 1) / (4 * V);
-   typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type VT;
+   // Gather: element copies that all stay in flight while the previous chunk's sums are added, 8 consecutive
+   // coefficients (a 32-byte sector in FP32) of 4 rows a warp.
+   const int nk8 = (L + 7) >> 3, k8 = lane & 7, r4 = lane >> 3;
    auto gather = [&](const int* rows, int nr) {
-      for(int j = warp; j < nkb; j += NW)
+      const int nq = (nr + 3) >> 2;
+      for(int j = warp; j < nk8; j += NW)
       {
-         const int k = 4 * V * j + kl;
-         int w[V];
-#pragma unroll
-         for(int i = 0; i < V; i++) w[i] = pos[k + i];
-         for(int r0 = rl; r0 < nr; r0 += 32)
-         {
-            VT x[4];
-#pragma unroll
-            for(int h = 0; h < 4; h++)
-               if(r0 + 8 * h < nr) x[h] = *reinterpret_cast<const VT*>(X + int64_t(rows[r0 + 8 * h]) * Lp + k);
-#pragma unroll
-            for(int h = 0; h < 4; h++)
-               if(r0 + 8 * h < nr)
-               {
-                  const T* xs = reinterpret_cast<const T*>(&x[h]);
-#pragma unroll
-                  for(int i = 0; i < V; i++)
-                     if(w[i] != 0xFFFF) W0[w[i] * RS + r0 + 8 * h] = xs[i];
-               }
-         }
+         const int k = 8 * j + k8;
+         if(k >= L) continue;
+         T* w = W0 + int(pos[k]) * RS + r4;
+         const T* src = X + k;
+#pragma unroll 4
+         for(int q = 0; q < nq; q++)
+            if(4 * q + r4 < nr) cpAsyncElem(w + 4 * q, src + int64_t(rows[4 * q + r4]) * Lp);
       }
    };
+   // Sums: 4 lanes of V consecutive coefficients by 8 rows a warp and item, BT items' loads in flight together.
+   const int kl = V * (lane & 3), rl = lane >> 2, nkb = (Lp + 4 * V - 1) / (4 * V);
+   typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type VT;
+   constexpr int BT = MODE == 0 ? 6 : 4;
    auto addOut = [&](int db, int nr) {
       const int* rows = dstRow[db];
-      for(int j = warp; j < nkb; j += NW)
+      const int nItems = nkb * ((nr + 7) >> 3);
+      for(int i0 = warp; i0 < nItems; i0 += BT * NW)
       {
-         const int k = 4 * V * j + kl;
-         int w[V];
+         VT y[BT], id[BT];
+         T* q[BT];
 #pragma unroll
-         for(int i = 0; i < V; i++) w[i] = pos[k + i];
-         for(int r0 = rl; r0 < nr; r0 += 32)
+         for(int h = 0; h < BT; h++)
          {
-            VT y[4], id[4];
-            VT* q[4];
+            const int it = i0 + h * NW, r = 8 * (it / nkb) + rl, k = 4 * V * (it % nkb) + kl;
+            q[h] = nullptr;
+            if(it < nItems && r < nr)
+            {
+               q[h] = out + int64_t(rows[r]) * Lp + k;
+               y[h] = *reinterpret_cast<const VT*>(q[h]);
+               if(MODE != 0) id[h] = *reinterpret_cast<const VT*>(X + int64_t(srcRow[db][r]) * Lp + k);
+            }
+         }
 #pragma unroll
-            for(int h = 0; h < 4; h++)
-               if(r0 + 8 * h < nr)
-               {
-                  q[h] = reinterpret_cast<VT*>(out + int64_t(rows[r0 + 8 * h]) * Lp + k);
-                  y[h] = *q[h];
-                  if(MODE != 0) id[h] = *reinterpret_cast<const VT*>(X + int64_t(srcRow[db][r0 + 8 * h]) * Lp + k);
-               }
+         for(int h = 0; h < BT; h++)
+         {
+            if(!q[h]) continue;
+            const int it = i0 + h * NW, r = 8 * (it / nkb) + rl, k = 4 * V * (it % nkb) + kl;
+            T* ys = reinterpret_cast<T*>(&y[h]);
 #pragma unroll
-            for(int h = 0; h < 4; h++)
-               if(r0 + 8 * h < nr)
-               {
-                  T* ys = reinterpret_cast<T*>(&y[h]);
-#pragma unroll
-                  for(int i = 0; i < V; i++)
-                     if(w[i] != 0xFFFF)
-                     {
-                        T v = W1[w[i] * RS + r0 + 8 * h];
-                        if(MODE != 0) v = fma(reinterpret_cast<const T*>(&id[h])[i], boxScale<T>(k + i, MODE == 2), v);
-                        ys[i] += v;
-                     }
-                  *q[h] = y[h];
-               }
+            for(int i = 0; i < V; i++)
+            {
+               const int w = pos[k + i];
+               if(w == 0xFFFF) continue;
+               T v = W1[w * RS + r];
+               if(MODE != 0) v = fma(reinterpret_cast<const T*>(&id[h])[i], boxScale<T>(k + i, MODE == 2), v);
+               ys[i] += v;
+            }
+            *reinterpret_cast<VT*>(q[h]) = y[h];
          }
       }
    };
@@ -773,8 +778,9 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
          for(int e = tid * V; e < B.size; e += NT * V) cpAsync16(D + e, src + e);
          asm volatile("cp.async.commit_group;" ::: "memory");
       }
-      if(chunk) addOut((chunk - 1) & 1, prevRows);
       gather(srcRow[chunk & 1], nr);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      if(chunk) addOut((chunk - 1) & 1, prevRows);
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncthreads();
       if(MODE != 2 && c0 == 0 && warp == 0 && oi + 1 < o1)
@@ -873,20 +879,26 @@ fmm_status ensureRotations(Plan& P, cudaStream_t st)
    return FMM_OK;
 }
 
-// Boxes of a tile, and into how many parts the operators of a tile are split (a part is a block; their sums meet
-// in kSumParts). FP32 tiles of one chunk's boxes and of two measured within 2 % of each other (2^20 points, p = 12:
-// 19.1 and 19.6 ms a solve), FP64 ones 4.13 and 4.05 ms (65,536 points, p = 10). Parts: four rounds of
-// resident blocks, so that small trees fill the chip (2,000 points, p = 10: M2L 54 us; one block a tile took over 1 ms)
-// and larger ones have no long last round.
-template <class T> static int rotTile(int mode) { return rot::chunkPairs<T>() * (mode == 0 && sizeof(T) == 8 ? 4 : 1); }
+// Boxes of a tile, into how many parts the operators of a tile are split (a part is a block; their sums meet in
+// kSumParts), and the block's threads. An M2L tile has five chunks' boxes (FP64: six): an operator has partners for about half of
+// them, so its chunks are mostly full (tiles of one chunk: M2L of 2^19 points and targets, p = 12, 9.3 ms, of five 7.5;
+// FP64, 131,072, p = 12, 4.3 and 3.6). Parts: eight rounds of resident blocks (four: 8.3 and 3.6 ms), so that small trees
+// fill the chip and larger ones have no long last round. Threads: 16 warps an SM (the registers' limit) as two blocks,
+// from p = 13 on as one; for the M2L blocks of 4 warps where three or four fit, p <= 9 in FP32 (8 warps a block at p = 4: 2.4 ms,
+// 4 warps 1.7; at p = 8 4.3 and 3.9; at p = 10, where two fit, 6.0 and 7.4).
+template <class T> static int rotTile(int mode) { return rot::chunkPairs<T>() * (mode == 0 ? (sizeof(T) == 8 ? 6 : 5) : 1); }
 template <class T>
-static int rotPerSM(const Plan& P) { return std::max(1, std::min(2, (227 * 1024) / (rot::Smem<T>(P.p).total + 6 * 1024))); }
+static int rotPerSM(const Plan& P, int mode)
+{
+   const int fit = (227 * 1024) / (rot::Smem<T>(P.p).total + 6 * 1024);
+   return fit >= 3 && mode == 0 ? std::min(fit, 4) : (fit >= 2 ? 2 : 1);
+}
 template <class T>
 static int rotParts(const Plan& P, int mode, int count)
 {
    const int tile = rotTile<T>(mode), tiles = (count + tile - 1) / tile;
    if(tiles == 0) return 1;
-   return std::max(1, std::min(mode == 0 ? 64 : 8, 4 * 148 * rotPerSM<T>(P) / tiles));
+   return std::max(1, std::min(mode == 0 ? 64 : 8, 8 * 148 * rotPerSM<T>(P, mode) / tiles));
 }
 
 // Room for the parts' sums of every launch on the current tree, so that none of them allocates.
@@ -911,7 +923,7 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
 {
    const rot::Blob B(P.p);
    const size_t smem = rot::Smem<T>(P.p).total;
-   const int THREADS = rotPerSM<T>(P) == 1 ? 512 : 256;   // 16 warps an SM either way
+   const int perSM = rotPerSM<T>(P, MODE), THREADS = perSM >= 3 ? 128 : 512 / perSM;
    auto kern = rot::kRotTranslate<T, MODE>;
    FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
    const T* ops = (const T*)P.rotOps.ptr + size_t(B.size) * (MODE == 0 ? 16 : MODE == 1 ? 0 : 8);
@@ -921,7 +933,7 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
    {
       // up to eight chunks a block, which loads the octant's tables once, while that leaves four rounds of blocks
       const int chunk = rot::chunkPairs<T>(), all = seg.start[8] - seg.start[0];
-      const int tl = chunk * std::max(1, std::min(rot::MAXTL / chunk, all / (chunk * 4 * 148 * rotPerSM<T>(P))));
+      const int tl = chunk * std::max(1, std::min(rot::MAXTL / chunk, all / (chunk * 4 * 148 * rotPerSM<T>(P, MODE))));
       kern<<<dim3((most + tl - 1) / tl, 1, 8), THREADS, smem, st>>>(targets, 0, nullptr, P.tree.parent, seg, tl, P.p, P.Lp,
                                                                    tasks, ops, X, Y, nullptr);
       return launched(P, "kRotTranslate<L2L>", st);
