@@ -235,7 +235,7 @@ void Plan::release()
    DevBuf* bufs[] = {&segb, &srcXYZb, &srcWb, &srcJb, &tgtXYZb, &rootb, &sKeys, &tKeys, &sIdx, &tIdx, &sPos, &sQ, &tPos,
                      &cubTmp, &scratch, &lvlBounds, &lvlCnt, &lvlOff, &p2pOff, &p2pList, &parList, &m2lTargets, &m2lKeys, &errb,
                      &mult, &local, &outB, &outA, &opM2M64, &opL2L64, &opM2L64, &opM2Lbf, &multBf, &tcCounters,
-                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &directPart, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotWs};
+                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &directPart, &nearPart, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotWs};
    cudaDeviceSynchronize();   // once for all buffers
    for(DevBuf* b : bufs) b->release(true);
    for(auto& b : nodeBufs) b.release(true);

@@ -290,6 +290,7 @@ struct Plan
    Plan* adj = nullptr;
    DevBuf adjG, adjOut;
    DevBuf tcPts, tcOut;                  // fmm_treecode: staging of host query points and results
+   DevBuf nearPart;                      // near field: the sums of split direct lists
    DevBuf directPart;                    // fmm_direct: the sums of split sources
    DevBuf tcCurl, tcSort;                // its curl table (order tcCurlOrder) and the sorted points' keys and order
    std::vector<unsigned char> tcCurlHost;   // host copy of tcCurl (kept for the asynchronous upload)
@@ -333,6 +334,7 @@ inline fmm_status launched(Plan& P, const char* name, cudaStream_t st)
 
 template <class T> fmm_status buildTreeT(Plan& P, cudaStream_t st);
 template <class T> fmm_status packSourcesT(Plan& P, cudaStream_t st);   // sPos, sQ in input order, coil segments uploaded
+int nearParts(const Plan& P);         // blocks a leaf's direct list is split into
 template <class T> fmm_status upwardT(Plan& P, cudaStream_t st);
 template <class T> fmm_status downwardT(Plan& P, cudaStream_t st);
 template <class T> fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st);

@@ -454,7 +454,9 @@ inline size_t p2mWarpSmem(int p, int Lp)
    return sizeof(T) * (size_t(P2MW_STEPS) * 32 * 4 + P2MW_WARPS * perWarp);
 }
 
-template <class T>
+// SPLIT: the block's warps share one leaf, warp w taking every P2MW_WARPS-th group of 32 points, and their sums meet in
+// shared memory in warp order (few large leaves: 38,400 points in leaves of up to 1000, p = 10, 270 -> 80 us).
+template <class T, bool SPLIT>
 __global__ void __launch_bounds__(32 * P2MW_WARPS) kP2MWarp(Tree t, const RootBox* __restrict__ rootp,
                                                           const typename Vec4<T>::type* __restrict__ pos,
                                                           const typename Vec4<T>::type* __restrict__ q, int p,
@@ -492,7 +494,7 @@ __global__ void __launch_bounds__(32 * P2MW_WARPS) kP2MWarp(Tree t, const RootBo
       AB[e] = V4{a, b, ee, T(0)};
    }
    __syncthreads();
-   const int node = blockIdx.x * P2MW_WARPS + warp;
+   const int node = SPLIT ? int(blockIdx.x) : int(blockIdx.x) * P2MW_WARPS + warp;
    if(node >= t.nNodes || t.nchild[node] != 0) return;
    const int s0 = t.s0[node], s1 = t.s1[node];
    if(s1 == s0) return;
@@ -503,7 +505,7 @@ __global__ void __launch_bounds__(32 * P2MW_WARPS) kP2MWarp(Tree t, const RootBo
    T accR[P2MW_STEPS], accI[P2MW_STEPS];
 #pragma unroll
    for(int j = 0; j < P2MW_STEPS; j++) { accR[j] = T(0); accI[j] = T(0); }
-   for(int base = s0; base < s1; base += 32)
+   for(int base = s0 + (SPLIT ? 32 * warp : 0); base < s1; base += SPLIT ? 32 * P2MW_WARPS : 32)
    {
       const int cnt = min(32, s1 - base);
       if(lane < cnt)
@@ -589,6 +591,20 @@ __global__ void __launch_bounds__(32 * P2MW_WARPS) kP2MWarp(Tree t, const RootBo
    }
    __syncwarp();
    T* out = M + int64_t(node) * 3 * Lp;
+   if(SPLIT)
+   {
+      // the warps' sums into the first warp's
+      __syncthreads();
+      T* first = (T*)(AB + P2MW_STEPS * 32) + 32 * 8;
+      for(int e = threadIdx.x; e < 3 * Lp; e += 32 * P2MW_WARPS)
+      {
+         T v = first[e];
+         for(int w = 1; w < P2MW_WARPS; w++) v += first[w * perWarp + e];
+         first[e] = v;
+      }
+      __syncthreads();
+      if(warp) return;
+   }
    for(int e = lane; e < 3 * Lp; e += 32) out[e] = Mst[e];
    // the same coefficients as tensor-core operand pieces (the M2M's and M2L's input format), so the
    // upward pass needs no separate split of the leaves
@@ -900,11 +916,14 @@ __global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 
                                                const typename Vec4<T>::type* __restrict__ sq,
                                                const int* __restrict__ p2pOff, const int* __restrict__ p2pList,
                                                const int* __restrict__ tOrder, T scaleB, T scaleA, int want,
-                                               T* __restrict__ outB, T* __restrict__ outA)
+                                               T* __restrict__ outB, T* __restrict__ outA, double* __restrict__ part,
+                                               int mTargets)
 {
    typedef typename Vec4<T>::type V4;
    extern __shared__ __align__(32) unsigned char smraw[];
    const int node = blockIdx.x;
+   // the tiles of a leaf's list dealt out to gridDim.y blocks (!FAR); their sums then go to part
+   const int nParts = FAR ? 1 : int(gridDim.y), myPart = FAR ? 0 : int(blockIdx.y);
    if(t.nchild[node] != 0 || t.t1[node] == t.t0[node]) return;
    const int tid = threadIdx.x;
    const int L = nharm(p);
@@ -953,7 +972,7 @@ __global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 
       const int ti = base + tt;
       V4 x = inGroup ? tpos[ti] : V4{T(0), T(0), T(0), T(0)};
       double Bd[3] = {0, 0, 0}, Ad[3] = {0, 0, 0};
-      if(!FAR && inGroup && g == 0)
+      if(!FAR && inGroup && g == 0 && nParts == 1)
       {
          // the far field, already evaluated by kL2PWarp into the outputs (unscaled)
          const int o = tOrder[ti];
@@ -1074,6 +1093,7 @@ __global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 
       // the list in batches of NE entries: their point ranges are read together into shared memory
       // and prefix-summed, so every tile position finds its source by a shared-memory search and
       // all of a tile's loads are independent
+      int firstTile = myPart;   // this block's first tile of the batch
       for(int eb = e0; eb < e1; eb += NE)
       {
          const int ne = min(NE, e1 - eb);
@@ -1142,20 +1162,24 @@ __global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 
             asm volatile("cp.async.commit_group;" ::: "memory");
          };
          const int nTiles = (total + TS - 1) / TS;
-         if(nTiles > 0) issueTile(0, 0);
-         for(int k = 0; k < nTiles; k++)
+         if(firstTile < nTiles) issueTile(firstTile * TS, 0);
+         int k = firstTile;
+         for(int b = 0; k < nTiles; k += nParts, b ^= 1)
          {
-            if(k + 1 < nTiles)
+            if(k + nParts < nTiles)
             {
-               issueTile((k + 1) * TS, (k + 1) & 1);
+               issueTile((k + nParts) * TS, b ^ 1);
                asm volatile("cp.async.wait_group 1;" ::: "memory");
             }
             else
                asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
-            tileSum(min(TS, total - k * TS), k & 1);
+            tileSum(min(TS, total - k * TS), b);
             __syncthreads();
          }
+         firstTile = k - nTiles;
+         // (a block without a tile in this batch must not overwrite its prefix sums while others read them)
+         if(nParts > 1) __syncthreads();
       }
       // add the groups' partial sums in group order
       if(G > 1)
@@ -1171,12 +1195,39 @@ __global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 
                }
          __syncthreads();
       }
-      if(g == 0)
+      if(g == 0 && nParts > 1)
+      {
+         double* o = part + int64_t(myPart) * 6 * mTargets + ti;
+         for(int d = 0; d < 3; d++)
+         {
+            o[int64_t(d) * mTargets] = Bd[d];
+            if(WANTA) o[int64_t(3 + d) * mTargets] = Ad[d];
+         }
+      }
+      else if(g == 0)
       {
          const int o = tOrder[ti];
          if(want & 1) for(int d = 0; d < 3; d++) outB[3 * int64_t(o) + d] = T(Bd[d] * double(scaleB));
          if(want & 2) for(int d = 0; d < 3; d++) outA[3 * int64_t(o) + d] = T(Ad[d] * double(scaleA));
       }
+   }
+}
+
+// The outputs' far field plus the near field's parts in order, scaled (kL2PNear with gridDim.y > 1).
+template <class T>
+__global__ void kNearParts(const double* __restrict__ part, int parts, int m, const int* __restrict__ tOrder, T scaleB, T scaleA,
+                           int want, T* __restrict__ outB, T* __restrict__ outA)
+{
+   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   if(i >= m) return;
+   const int64_t o = 3 * int64_t(tOrder[i]);
+   for(int c = 0; c < 6; c++)
+   {
+      if(!(want & (c < 3 ? 1 : 2))) continue;
+      T* out = c < 3 ? outB + o + c : outA + o + c - 3;
+      double v = double(*out);
+      for(int q = 0; q < parts; q++) v += part[(int64_t(q) * 6 + c) * m + i];
+      *out = T(v * double(c < 3 ? scaleB : scaleA));
    }
 }
 
@@ -1296,14 +1347,16 @@ fmm_status upwardT(Plan& P, cudaStream_t st)
    else if(P.p2mChunk == 0)
    {
       const size_t shw = p2mWarpSmem<T>(P.p, Lp);
-      if(shw > 48 * 1024)
-         FMM_CUDA(cudaFuncSetAttribute(kP2MWarp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shw)));
+      // a warp per leaf, or a block where leaves are large and too few to fill the chip with warps
+      const bool split = N <= 16 * 148 && P.n / std::max<int64_t>(1, N) >= 64;
+      auto kern = split ? kP2MWarp<T, true> : kP2MWarp<T, false>;
+      if(shw > 48 * 1024) FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shw)));
       // tensor-core M2M plans: the leaves' multipoles also leave as the M2M's operand pieces
       int np = 0;
       if(sizeof(T) == 4 && P.tcTranslations(1) && P.tcDrainMode != 0) np = m2mPieces(P);
       if(np)
          FMM_TRY(P.multBf.reserve(size_t(np == 1 ? 4 : 2 * np) * size_t(N) * 3 * Lp));
-      kP2MWarp<T><<<int((N + P2MW_WARPS - 1) / P2MW_WARPS), 32 * P2MW_WARPS, shw, st>>>(
+      kern<<<int(split ? N : (N + P2MW_WARPS - 1) / P2MW_WARPS), 32 * P2MW_WARPS, shw, st>>>(
          P.tree, P.root, (const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, P.p, Lp, (T*)P.mult.ptr,
          np ? (uint8_t*)P.multBf.ptr : nullptr, np);
       P.p2mPiecesTag = np ? (np == 1 ? 3 : 2 * np) : -1;
@@ -1336,6 +1389,17 @@ fmm_status downwardT(Plan& P, cudaStream_t st)
    if(P.eventsMade && !P.capturing) cudaEventRecord(P.ev[3], st);
    if(P.tcTranslations(2)) return l2lTensorCore(P, st);
    return rotL2L<T>(P, st);
+}
+
+// Into how many blocks a leaf's direct list is split: with few leaves of many sources a block per leaf leaves the chip idle
+// while the longest list is summed (38,400 points in leaves of up to 1000 and 4,001 targets: near field 0.86 ms with
+// one block a leaf, 0.12 split). Two rounds of 16 blocks a SM, only where lists average two tiles, and at most 50 MB of
+// partial sums (more than 2^20 targets in so few leaves keep a block busy by themselves).
+int nearParts(const Plan& P)
+{
+   const int64_t N = std::max<int64_t>(1, P.tree.nNodes);
+   if(double(P.nP2P) / double(N) * (double(P.n) / double(N)) < 512 || P.m == 0) return 1;
+   return int(std::max<int64_t>(1, std::min({int64_t(16), int64_t(2 * 16 * 148) / N, (int64_t(1) << 20) / P.m})));
 }
 
 template <class T>
@@ -1375,12 +1439,14 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
       else FMM_TRY(runL2P(kL2PWarp<T, false>, l2pWarpSmem<T, false>(P.p)));
       FMM_TRY(launched(P, "kL2PWarp", st));
    }
+   const int parts = split ? nearParts(P) : 1;
+   if(parts > 1) FMM_TRY(P.nearPart.reserve(sizeof(double) * 6 * size_t(parts) * size_t(P.m)));
    auto run = [&](auto kernel) -> fmm_status {
       FMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
-      kernel<<<int(N), NT, shm, st>>>(P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr,
+      kernel<<<dim3(int(N), parts), NT, shm, st>>>(P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr,
                                       (const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, (const int*)P.p2pOff.ptr,
                                       (const int*)P.p2pList.ptr, (const int*)P.tIdx.ptr, scaleB, scaleA, want,
-                                      (T*)P.outB.ptr, (T*)P.outA.ptr);
+                                      (T*)P.outB.ptr, (T*)P.outA.ptr, (double*)P.nearPart.ptr, int(P.m));
       return FMM_OK;
    };
    if(split)
@@ -1407,6 +1473,12 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
       else FMM_TRY(run(kL2PNear<T, NT, 256, NE, false, true>));
    }
    FMM_TRY(launched(P, "kL2PNear", st));
+   if(parts > 1)
+   {
+      kNearParts<T><<<int((P.m + 255) / 256), 256, 0, st>>>((const double*)P.nearPart.ptr, parts, int(P.m), (const int*)P.tIdx.ptr,
+                                                            scaleB, scaleA, want, (T*)P.outB.ptr, (T*)P.outA.ptr);
+      FMM_TRY(launched(P, "kNearParts", st));
+   }
    FMM_CHECK_LAUNCH();
    return FMM_OK;
 }

@@ -1525,6 +1525,9 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_TRY(launched(P, "kGatherSources", st));
       FMM_CHECK_LAUNCH();
    }
+   // room for split sums, so that no later phase allocates
+   const int parts = nearParts(P);
+   if(parts > 1) FMM_TRY(P.nearPart.reserve(sizeof(double) * 6 * size_t(parts) * size_t(m)));
    return reserveRotations<T>(P);
 }
 
