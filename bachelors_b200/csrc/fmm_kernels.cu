@@ -443,42 +443,69 @@ __global__ void __launch_bounds__(NT) kP2M(Tree t, const RootBox* __restrict__ r
 // each chain, so no lane branches. At the end the real coefficients (-1)^l sqrt2 (Re, Im) S_l^m
 // (m > 0) and (-1)^l S_l^0 go through shared memory to one coalesced store of the leaf's
 // multipole.
+// Bound by the issue of the recurrence (a step depends on the last one, 16 warps a SM). Points go two at a time,
+// interleaved in shared memory; in FP32 a pair is one packed f32x2 operand of every step (12 instructions a step
+// against 21 for two scalar chains), the chain is one FMA deep, the table is kept by u and not by lane, and a
+// block serves many leaves per table. 2^24 points in leaves of 18, p = 16: 10.1 -> 8.0 ms; 2^23
+// points of 256 coils: 8.1 -> 5.1 ms (128 registers; a chain of scalar operands or the table kept in registers spills).
 // ====================================================================================
-constexpr int P2MW_WARPS = 4;
+constexpr int P2MW_WARPS = 4;               // a leaf each
+constexpr int P2MW_SPLIT_WARPS = 8;         // of one leaf
 constexpr int P2MW_STEPS = MAXORDER + 2;
+constexpr int P2MW_U = MAXORDER / 2 + 1;   // the step table's row
 
 template <class T>
-inline size_t p2mWarpSmem(int p, int Lp)
+constexpr size_t p2mTableBytes = (sizeof(T) * P2MW_STEPS * P2MW_U * (sizeof(T) == 4 ? 6 : 3) + 15) / 16 * 16;
+
+// Shared-memory loads that stay where they are written: the step table does not change from pair to pair, and the
+// compiler would otherwise keep as many of its rows in registers as fit, and spill.
+__device__ __forceinline__ ulonglong2 ldsPair(const void* p)
 {
-   const size_t perWarp = 32 * 8 + std::max<size_t>(size_t(32) * 2 * (p + 1), size_t(3) * Lp);
-   return sizeof(T) * (size_t(P2MW_STEPS) * 32 * 4 + P2MW_WARPS * perWarp);
+   ulonglong2 v;
+   asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(uint32_t(__cvta_generic_to_shared(p))) : "memory");
+   return v;
+}
+__device__ __forceinline__ f2p ldsOne(const void* p)
+{
+   f2p v;
+   asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(uint32_t(__cvta_generic_to_shared(p))) : "memory");
+   return v;
 }
 
-// SPLIT: the block's warps share one leaf, warp w taking every P2MW_WARPS-th group of 32 points, and their sums meet in
-// shared memory in warp order (few large leaves: 38,400 points in leaves of up to 1000, p = 10, 270 -> 80 us).
+template <class T>
+inline size_t p2mWarpSmem(int p, int Lp, int warps)
+{
+   const size_t perWarp = 32 * 8 + std::max<size_t>(size_t(32) * 2 * (p + 1), size_t(3) * Lp);
+   return p2mTableBytes<T> + sizeof(T) * (warps * perWarp);
+}
+
+// SPLIT: the block's warps share one leaf, warp w taking every eighth group of 32 points, and their sums meet in shared
+// memory in warp order (few large leaves: 38,400 points in leaves of up to 1000, p = 10, 270 -> 54 us).
 template <class T, bool SPLIT>
-__global__ void __launch_bounds__(32 * P2MW_WARPS) kP2MWarp(Tree t, const RootBox* __restrict__ rootp,
-                                                          const typename Vec4<T>::type* __restrict__ pos,
-                                                          const typename Vec4<T>::type* __restrict__ q, int p,
-                                                          int Lp, T* __restrict__ M, uint8_t* __restrict__ Mpieces,
-                                                          int np)
+__global__ void __launch_bounds__(32 * (SPLIT ? P2MW_SPLIT_WARPS : P2MW_WARPS), (sizeof(T) == 4 ? 4 : 3) / (SPLIT ? 2 : 1))
+   kP2MWarp(Tree t, const RootBox* __restrict__ rootp, const typename Vec4<T>::type* __restrict__ pos,
+            const typename Vec4<T>::type* __restrict__ q, int p, int Lp, T* __restrict__ M,
+            uint8_t* __restrict__ Mpieces, int np)
 {
    typedef typename Vec4<T>::type V4;
+   constexpr bool PK = sizeof(T) == 4;
+   constexpr int WARPS = SPLIT ? P2MW_SPLIT_WARPS : P2MW_WARPS;
    extern __shared__ __align__(16) unsigned char smraw[];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    const int U = p / 2 + 1;
-   // the step table, [step][lane] (a, b, e, 0)
-   V4* AB = (V4*)smraw;
+   // the step table, [step][u]: (a, -b), then e; FP32: each value twice, as the packed operands
+   T* AB = (T*)smraw;
+   T* EE = AB + P2MW_STEPS * P2MW_U * (PK ? 4 : 2);
    const size_t perWarp = 32 * 8 + max(32 * 2 * (p + 1), 3 * Lp);
-   T* Pt = (T*)(AB + P2MW_STEPS * 32) + warp * perWarp;   // [32][8] point: u, r^2, q
-   T* Ds = Pt + 32 * 8;                                  // [32][p + 1] (re, im) of S_m^m; later [3][Lp]
+   T* Pt0 = (T*)(smraw + p2mTableBytes<T>);
+   T* Pt = Pt0 + warp * perWarp;                         // [16 pairs][8][2] points: u, r^2, q
+   T* Ds = Pt + 32 * 8;                                  // [16][p + 1][re, im][2] S_m^m; later [3][Lp]
    const int u = lane % U, c = min(lane / U, 2);
    const int ma = u, mb = p - u;
-   const int na = p + 1 - ma;                            // terms of the m_a chain
-   for(int e = threadIdx.x; e < P2MW_STEPS * 32; e += 32 * P2MW_WARPS)
+   const int jb = p + 2 - U;                             // no lane's m_b chain starts before this step
+   for(int e = threadIdx.x; e < P2MW_STEPS * P2MW_U; e += 32 * WARPS)
    {
-      const int j = e / 32, ln = e % 32;
-      const int uu = ln % U;
+      const int j = e / P2MW_U, uu = min(e % P2MW_U, U - 1);
       const int a0 = uu, b0 = p - uu, n0 = p + 1 - a0;
       const int n = n0 + (b0 != a0 ? p + 1 - b0 : 0);
       T a = T(0), b = T(0), ee = T(0);
@@ -489,133 +516,193 @@ __global__ void __launch_bounds__(32 * P2MW_WARPS) kP2MWarp(Tree t, const RootBo
          const int l = j < n0 ? a0 + j - 1 : b0 + (j - n0) - 1;
          const T inv = T(1) / T((l - m + 1) * (l + m + 1));
          a = T(2 * l + 1) * inv;
-         b = l == m ? T(0) : inv;
+         b = l == m ? T(0) : -inv;
       }
-      AB[e] = V4{a, b, ee, T(0)};
+      if constexpr(PK)
+      {
+         AB[4 * e] = AB[4 * e + 1] = a;
+         AB[4 * e + 2] = AB[4 * e + 3] = b;
+         EE[2 * e] = EE[2 * e + 1] = ee;
+      }
+      else
+      {
+         AB[2 * e] = a;
+         AB[2 * e + 1] = b;
+         EE[e] = ee;
+      }
    }
    __syncthreads();
-   const int node = SPLIT ? int(blockIdx.x) : int(blockIdx.x) * P2MW_WARPS + warp;
-   if(node >= t.nNodes || t.nchild[node] != 0) return;
-   const int s0 = t.s0[node], s1 = t.s1[node];
-   if(s1 == s0) return;
-   const RootBox rb = rootp[rootOf(t, node)];
-   double cen[3], h;
-   nodeCenter(rb, t.level[node], t.ix[node], t.iy[node], t.iz[node], cen, h);
-   const double ih = 1.0 / h;
-   T accR[P2MW_STEPS], accI[P2MW_STEPS];
-#pragma unroll
-   for(int j = 0; j < P2MW_STEPS; j++) { accR[j] = T(0); accI[j] = T(0); }
-   for(int base = s0 + (SPLIT ? 32 * warp : 0); base < s1; base += SPLIT ? 32 * P2MW_WARPS : 32)
+   // SPLIT: the block's node; else the warp's nodes, dealt out over the grid
+   for(int node = SPLIT ? int(blockIdx.x) : int(blockIdx.x) * WARPS + warp; node < t.nNodes;
+       node += SPLIT ? t.nNodes : int(gridDim.x) * WARPS)
    {
-      const int cnt = min(32, s1 - base);
-      if(lane < cnt)
+      if(t.nchild[node] != 0) continue;
+      const int s0 = t.s0[node], s1 = t.s1[node];
+      if(s1 == s0) continue;
+      const RootBox rb = rootp[rootOf(t, node)];
+      double cen[3], h;
+      nodeCenter(rb, t.level[node], t.ix[node], t.iy[node], t.iz[node], cen, h);
+      const double ih = 1.0 / h;
+      typedef typename std::conditional<PK, f2p, T>::type Acc;   // FP32: the two points of a pair summed apart
+      Acc accR[P2MW_STEPS], accI[P2MW_STEPS];
+#pragma unroll
+      for(int j = 0; j < P2MW_STEPS; j++) { accR[j] = Acc(0); accI[j] = Acc(0); }
+      for(int base = s0 + (SPLIT ? 32 * warp : 0); base < s1; base += SPLIT ? 32 * WARPS : 32)
       {
-         const V4 xp = pos[base + lane], w = q[base + lane];
-         const T x = T((double(xp.x) - cen[0]) * ih), y = T((double(xp.y) - cen[1]) * ih),
-                 z = T((double(xp.z) - cen[2]) * ih);
-         T* pt = Pt + lane * 8;
-         pt[0] = x; pt[1] = y; pt[2] = z; pt[3] = x * x + y * y + z * z;
-         pt[4] = w.x; pt[5] = w.y; pt[6] = w.z;
-         T dre = T(1), dim = T(0);
-         T* d = Ds + lane * 2 * (p + 1);
-         d[0] = dre; d[1] = dim;
-         for(int m = 1; m <= p; m++)
+         const int cnt = min(32, s1 - base);
+         if(lane < ((cnt + 1) & ~1))
          {
-            const T sc = T(1) / T(2 * m);
-            const T nre = (dre * x - dim * y) * sc;
-            const T nim = (dre * y + dim * x) * sc;
-            dre = nre; dim = nim;
-            d[2 * m] = dre; d[2 * m + 1] = dim;
+            // (an odd count's last partner: a zero-strength point at the box centre)
+            T x = T(0), y = T(0), z = T(0);
+            V4 w{T(0), T(0), T(0), T(0)};
+            if(lane < cnt)
+            {
+               const V4 xp = pos[base + lane];
+               w = q[base + lane];
+               x = T((double(xp.x) - cen[0]) * ih);
+               y = T((double(xp.y) - cen[1]) * ih);
+               z = T((double(xp.z) - cen[2]) * ih);
+            }
+            T* pt = Pt + (lane >> 1) * 16 + (lane & 1);
+            pt[0] = x; pt[2] = y; pt[4] = z; pt[6] = x * x + y * y + z * z;
+            pt[8] = w.x; pt[10] = w.y; pt[12] = w.z;
+            T dre = T(1), dim = T(0);
+            T* d = Ds + (lane >> 1) * 4 * (p + 1) + (lane & 1);
+            d[0] = dre; d[2] = dim;
+#pragma unroll
+            for(int m = 1; m <= MAXORDER; m++)
+            {
+               if(m > p) break;
+               const T sc = T(1) / T(2 * m);
+               const T nre = (dre * x - dim * y) * sc;
+               const T nim = (dre * y + dim * x) * sc;
+               dre = nre; dim = nim;
+               d[4 * m] = dre; d[4 * m + 2] = dim;
+            }
+         }
+         __syncwarp();
+         for(int i = 0; 2 * i < cnt; i++)
+         {
+            const T* pt = Pt + i * 16;
+            const T* d = Ds + i * 4 * (p + 1);
+            if constexpr(PK)
+            {
+               const ulonglong2 da = *(const ulonglong2*)(d + 4 * ma), db = *(const ulonglong2*)(d + 4 * mb);
+               const f2p Z = *(const f2p*)(pt + 4), R2 = *(const f2p*)(pt + 6), Q = *(const f2p*)(pt + 8 + 2 * c);
+               f2p are = da.x, aim = da.y, bre = 0, bim = 0;
+               accR[0] = fma2(Q, are, accR[0]);
+               accI[0] = fma2(Q, aim, accI[0]);
+#pragma unroll
+               for(int j = 1; j < P2MW_STEPS; j++)
+               {
+                  if(j > p + 1) break;
+                  const ulonglong2 k = ldsPair(AB + 4 * (j * P2MW_U + u));
+                  const f2p az = mul2(k.x, Z), br = mul2(k.y, R2);
+                  f2p tre = mul2(br, bre), tim = mul2(br, bim);
+                  if(j >= jb)
+                  {
+                     const f2p e = ldsOne(EE + 2 * (j * P2MW_U + u));
+                     tre = fma2(e, db.x, tre);
+                     tim = fma2(e, db.y, tim);
+                  }
+                  bre = are; bim = aim;
+                  are = fma2(az, are, tre);
+                  aim = fma2(az, aim, tim);
+                  accR[j] = fma2(Q, are, accR[j]);
+                  accI[j] = fma2(Q, aim, accI[j]);
+               }
+            }
+            else
+            {
+               const T z = pt[4], r2 = pt[6], qc = pt[8 + 2 * c], z2 = pt[5], r22 = pt[7], qc2 = pt[9 + 2 * c];
+               T are = d[4 * ma], aim = d[4 * ma + 2], are2 = d[4 * ma + 1], aim2 = d[4 * ma + 3];
+               const T bdr = d[4 * mb], bdi = d[4 * mb + 2], bdr2 = d[4 * mb + 1], bdi2 = d[4 * mb + 3];
+               T bre = T(0), bim = T(0), bre2 = T(0), bim2 = T(0);
+               accR[0] += qc * are + qc2 * are2;
+               accI[0] += qc * aim + qc2 * aim2;
+#pragma unroll
+               for(int j = 1; j < P2MW_STEPS; j++)
+               {
+                  if(j > p + 1) break;
+                  const ulonglong2 kk = ldsPair(AB + 2 * (j * P2MW_U + u));
+               const T ka = __longlong_as_double(kk.x), kb = __longlong_as_double(kk.y);
+               const T ke = __longlong_as_double(ldsOne(EE + j * P2MW_U + u));
+                  const T az = ka * z, br = kb * r2;
+                  const T az2 = ka * z2, br2 = kb * r22;
+                  const T cre = ke * bdr + br * bre + az * are;
+                  const T cim = ke * bdi + br * bim + az * aim;
+                  const T cre2 = ke * bdr2 + br2 * bre2 + az2 * are2;
+                  const T cim2 = ke * bdi2 + br2 * bim2 + az2 * aim2;
+                  bre = are; bim = aim; are = cre; aim = cim;
+                  bre2 = are2; bim2 = aim2; are2 = cre2; aim2 = cim2;
+                  accR[j] += qc * are + qc2 * are2;
+                  accI[j] += qc * aim + qc2 * aim2;
+               }
+            }
+         }
+         __syncwarp();
+      }
+      auto sum = [](Acc v) -> T {
+         if constexpr(PK)
+         {
+            T a, b;
+            upk2(v, a, b);
+            return a + b;
+         }
+         else return v;
+      };
+      // real coefficients through shared memory, then one coalesced store
+      T* Mst = Ds;
+      for(int e = (p + 1) * (p + 1) + lane; e < Lp; e += 32) Mst[e] = Mst[Lp + e] = Mst[2 * Lp + e] = T(0);
+      if(lane < 3 * U)
+      {
+         int ma1 = ma;
+         asm volatile("" : "+r"(ma1));   // (else every coefficient's address is kept across the leaves)
+         const int mb1 = p - ma1, na1 = p + 1 - ma1;
+         const int nb = mb1 != ma1 ? p + 1 - mb1 : 0;
+         const T sq2 = T(1.4142135623730950488);
+#pragma unroll
+         for(int j = 0; j < P2MW_STEPS; j++)
+         {
+            if(j >= na1 + nb) break;
+            const int m = j < na1 ? ma1 : mb1;
+            const int l = j < na1 ? ma1 + j : mb1 + (j - na1);
+            const T sg = (l & 1) ? T(-1) : T(1);
+            T* mc = Mst + c * Lp;
+            if(m == 0) mc[hidx(l, 0)] = sg * sum(accR[j]);
+            else
+            {
+               mc[hidx(l, m)] = sg * sq2 * sum(accR[j]);
+               mc[hidx(l, -m)] = sg * sq2 * sum(accI[j]);
+            }
          }
       }
       __syncwarp();
-      // two points per pass (independent recurrences sharing the table loads); an odd count's
-      // partner is a zero-strength point at the box centre
-      for(int i = 0; i < cnt; i += 2)
+      T* out = M + int64_t(node) * 3 * Lp;
+      if(SPLIT)
       {
-         const bool two = i + 1 < cnt;
-         const T* pt = Pt + i * 8;
-         const T* d = Ds + i * 2 * (p + 1);
-         const T z = pt[2], r2 = pt[3], qc = pt[4 + c];
-         const T z2 = two ? pt[8 + 2] : T(0), r22 = two ? pt[8 + 3] : T(0), qc2 = two ? pt[8 + 4 + c] : T(0);
-         const T* d2 = d + 2 * (p + 1);
-         T are = d[2 * ma], aim = d[2 * ma + 1];
-         const T bdr = d[2 * mb], bdi = d[2 * mb + 1];
-         T are2 = two ? d2[2 * ma] : T(0), aim2 = two ? d2[2 * ma + 1] : T(0);
-         const T bdr2 = two ? d2[2 * mb] : T(0), bdi2 = two ? d2[2 * mb + 1] : T(0);
-         T bre = T(0), bim = T(0), bre2 = T(0), bim2 = T(0);
-         accR[0] += qc * are + qc2 * are2;
-         accI[0] += qc * aim + qc2 * aim2;
-#pragma unroll
-         for(int j = 1; j < P2MW_STEPS; j++)
+         // the warps' sums into the first warp's
+         __syncthreads();
+         T* first = Pt0 + 32 * 8;
+         for(int e = threadIdx.x; e < 3 * Lp; e += 32 * WARPS)
          {
-            if(j > p + 1) break;
-            const V4 k = AB[j * 32 + lane];
-            const T az = k.x * z, br = k.y * r2;
-            const T az2 = k.x * z2, br2 = k.y * r22;
-            const T cre = k.z * bdr + (az * are - br * bre);
-            const T cim = k.z * bdi + (az * aim - br * bim);
-            const T cre2 = k.z * bdr2 + (az2 * are2 - br2 * bre2);
-            const T cim2 = k.z * bdi2 + (az2 * aim2 - br2 * bim2);
-            bre = are; bim = aim; are = cre; aim = cim;
-            bre2 = are2; bim2 = aim2; are2 = cre2; aim2 = cim2;
-            accR[j] += qc * are + qc2 * are2;
-            accI[j] += qc * aim + qc2 * aim2;
+            T v = first[e];
+            for(int w = 1; w < WARPS; w++) v += first[w * perWarp + e];
+            first[e] = v;
          }
+         __syncthreads();
+         if(warp) return;
       }
+      for(int e = lane; e < 3 * Lp; e += 32) out[e] = Mst[e];
+      // the same coefficients as tensor-core operand pieces (the M2M's and M2L's input format), so the
+      // upward pass needs no separate split of the leaves
+      if constexpr(sizeof(T) == 4)
+         if(Mpieces)
+            for(int d = 0; d < 3; d++)
+               for(int e = 4 * lane; e < Lp; e += 128)
+                  storePieces4(Mpieces, int64_t(node) * 3 + d, e, Lp, np, *(const float4*)(Mst + d * Lp + e));
       __syncwarp();
    }
-   // real coefficients through shared memory, then one coalesced store
-   T* Mst = Ds;
-   for(int e = lane; e < 3 * Lp; e += 32)
-      if(e % Lp >= (p + 1) * (p + 1)) Mst[e] = T(0);
-   if(lane < 3 * U)
-   {
-      const int nb = mb != ma ? p + 1 - mb : 0;
-      const T sq2 = T(1.4142135623730950488);
-#pragma unroll
-      for(int j = 0; j < P2MW_STEPS; j++)
-      {
-         if(j >= na + nb) break;
-         const int m = j < na ? ma : mb;
-         const int l = j < na ? ma + j : mb + (j - na);
-         const T sg = (l & 1) ? T(-1) : T(1);
-         T* mc = Mst + c * Lp;
-         if(m == 0) mc[hidx(l, 0)] = sg * accR[j];
-         else
-         {
-            mc[hidx(l, m)] = sg * sq2 * accR[j];
-            mc[hidx(l, -m)] = sg * sq2 * accI[j];
-         }
-      }
-   }
-   __syncwarp();
-   T* out = M + int64_t(node) * 3 * Lp;
-   if(SPLIT)
-   {
-      // the warps' sums into the first warp's
-      __syncthreads();
-      T* first = (T*)(AB + P2MW_STEPS * 32) + 32 * 8;
-      for(int e = threadIdx.x; e < 3 * Lp; e += 32 * P2MW_WARPS)
-      {
-         T v = first[e];
-         for(int w = 1; w < P2MW_WARPS; w++) v += first[w * perWarp + e];
-         first[e] = v;
-      }
-      __syncthreads();
-      if(warp) return;
-   }
-   for(int e = lane; e < 3 * Lp; e += 32) out[e] = Mst[e];
-   // the same coefficients as tensor-core operand pieces (the M2M's and M2L's input format), so the
-   // upward pass needs no separate split of the leaves
-   if constexpr(sizeof(T) == 4)
-      if(Mpieces)
-         for(int e4 = lane; e4 < 3 * Lp / 4; e4 += 32)
-         {
-            const int e = 4 * e4;
-            const float4 v = make_float4(Mst[e], Mst[e + 1], Mst[e + 2], Mst[e + 3]);
-            storePieces4(Mpieces, int64_t(node) * 3 + e / Lp, e % Lp, Lp, np, v);
-         }
 }
 
 __device__ __forceinline__ void cpAsync16Simt(void* dst, const void* src, uint32_t srcBytes)
@@ -1346,17 +1433,18 @@ fmm_status upwardT(Plan& P, cudaStream_t st)
    }
    else if(P.p2mChunk == 0)
    {
-      const size_t shw = p2mWarpSmem<T>(P.p, Lp);
       // a warp per leaf, or a block where leaves are large and too few to fill the chip with warps
       const bool split = N <= 16 * 148 && P.n / std::max<int64_t>(1, N) >= 64;
       auto kern = split ? kP2MWarp<T, true> : kP2MWarp<T, false>;
+      const int warps = split ? P2MW_SPLIT_WARPS : P2MW_WARPS;
+      const size_t shw = p2mWarpSmem<T>(P.p, Lp, warps);
       if(shw > 48 * 1024) FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shw)));
       // tensor-core M2M plans: the leaves' multipoles also leave as the M2M's operand pieces
       int np = 0;
       if(sizeof(T) == 4 && P.tcTranslations(1) && P.tcDrainMode != 0) np = m2mPieces(P);
       if(np)
          FMM_TRY(P.multBf.reserve(size_t(np == 1 ? 4 : 2 * np) * size_t(N) * 3 * Lp));
-      kern<<<int(split ? N : (N + P2MW_WARPS - 1) / P2MW_WARPS), 32 * P2MW_WARPS, shw, st>>>(
+      kern<<<int(split ? N : std::min<int64_t>((N + P2MW_WARPS - 1) / P2MW_WARPS, 16 * 148)), 32 * warps, shw, st>>>(
          P.tree, P.root, (const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, P.p, Lp, (T*)P.mult.ptr,
          np ? (uint8_t*)P.multBf.ptr : nullptr, np);
       P.p2mPiecesTag = np ? (np == 1 ? 3 : 2 * np) : -1;
