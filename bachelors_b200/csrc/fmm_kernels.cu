@@ -449,6 +449,54 @@ __global__ void __launch_bounds__(NT) kP2M(Tree t, const RootBox* __restrict__ r
 // block serves many leaves per table. 2^24 points in leaves of 18, p = 16: 10.1 -> 8.0 ms; 2^23
 // points of 256 coils: 8.1 -> 5.1 ms (128 registers; a chain of scalar operands or the table kept in registers spills).
 // ====================================================================================
+// A warp's walk over the leaves that hold points: its nodes are first, first + stride, ...; 32 of them are looked at
+// together, a lane each, so a leaf's range is in a register when its turn comes and the other nodes cost nothing.
+struct LeafWalk
+{
+   int base, stride;
+   unsigned todo = 0;
+   int a = 0, b = 0;   // the lane's node
+   struct Leaf
+   {
+      int node, a, b;
+   };
+   __device__ LeafWalk(int first, int stride_) : base(first - 32 * stride_), stride(stride_) {}
+   // The next leaf with [p0, p1) not empty (node < 0: none); all lanes of the warp together.
+   __device__ __forceinline__ Leaf next(const Tree& t, const int* __restrict__ p0, const int* __restrict__ p1)
+   {
+      while(!todo)
+      {
+         base += 32 * stride;
+         if(base >= t.nNodes) return Leaf{-1, 0, 0};
+         const int64_t mine = base + int64_t(threadIdx.x & 31) * stride;
+         bool in = mine < t.nNodes && t.nchild[mine] == 0;
+         if(in)
+         {
+            a = p0[mine]; b = p1[mine];
+            in = b > a;
+         }
+         todo = __ballot_sync(0xffffffffu, in);
+      }
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      return Leaf{base + l * stride, __shfl_sync(0xffffffffu, a, l), __shfl_sync(0xffffffffu, b, l)};
+   }
+};
+
+// Blocks of a kernel whose warps walk the leaves: every SM filled four times over, so that blocks that meet small
+// leaves are replaced, and a block still sets up its tables once for many leaves.
+template <class K>
+int walkBlocks(K kernel, int threads, size_t shm, int64_t n)
+{
+   int perSM = 1;
+   if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, threads, shm) != cudaSuccess || perSM < 1)
+   {
+      cudaGetLastError();
+      perSM = 1;
+   }
+   return int(std::max<int64_t>(1, std::min<int64_t>((n + threads / 32 - 1) / (threads / 32), 4 * 148 * int64_t(perSM))));
+}
+
 constexpr int P2MW_WARPS = 4;               // a leaf each
 constexpr int P2MW_SPLIT_WARPS = 8;         // of one leaf
 constexpr int P2MW_STEPS = MAXORDER + 2;
@@ -533,15 +581,14 @@ __global__ void __launch_bounds__(32 * (SPLIT ? P2MW_SPLIT_WARPS : P2MW_WARPS), 
    }
    __syncthreads();
    // SPLIT: the block's node; else the warp's nodes, dealt out over the grid
-   for(int node = SPLIT ? int(blockIdx.x) : int(blockIdx.x) * WARPS + warp; node < t.nNodes;
-       node += SPLIT ? t.nNodes : int(gridDim.x) * WARPS)
+   LeafWalk walk(SPLIT ? int(blockIdx.x) : int(blockIdx.x) * WARPS + warp, int(gridDim.x) * (SPLIT ? 1 : WARPS));
+   for(;;)
    {
-      if(t.nchild[node] != 0) continue;
-      const int s0 = t.s0[node], s1 = t.s1[node];
-      if(s1 == s0) continue;
-      const RootBox rb = rootp[rootOf(t, node)];
+      const LeafWalk::Leaf leaf = walk.next(t, t.s0, t.s1);
+      if(leaf.node < 0) break;
+      const int node = leaf.node, s0 = leaf.a, s1 = leaf.b;
       double cen[3], h;
-      nodeCenter(rb, t.level[node], t.ix[node], t.iy[node], t.iz[node], cen, h);
+      nodeCenter(rootp[rootOf(t, node)], t.level[node], t.ix[node], t.iy[node], t.iz[node], cen, h);
       const double ih = 1.0 / h;
       typedef typename std::conditional<PK, f2p, T>::type Acc;   // FP32: the two points of a pair summed apart
       Acc accR[P2MW_STEPS], accI[P2MW_STEPS];
@@ -691,7 +738,7 @@ __global__ void __launch_bounds__(32 * (SPLIT ? P2MW_SPLIT_WARPS : P2MW_WARPS), 
             first[e] = v;
          }
          __syncthreads();
-         if(warp) return;
+         if(warp) continue;   // (no further leaf)
       }
       for(int e = lane; e < 3 * Lp; e += 32) out[e] = Mst[e];
       // the same coefficients as tensor-core operand pieces (the M2M's and M2L's input format), so the
@@ -781,6 +828,9 @@ template <> __device__ __forceinline__ double riCap<double>() { return 1.0e100; 
 // the block (visit order: m outer, l inner): 1/(2m) at l = m, else the (a, b) of
 // S_l^m = a z S_{l-1}^m - b r^2 S_{l-2}^m, so no lane divides. The far field is written to the
 // outputs unscaled; kL2PNear<..., FAR = false> adds the near field and applies the scale.
+// Bound by latency (a leaf's setup, then a recurrence with shared-memory loads in its chain): a warp walks many leaves,
+// so the table is built once, and the next leaf's local row is on its way while this one is evaluated. 2^24 targets,
+// p = 16: 12.5 -> 11.3 ms; 2^23 targets of 256 coils: 3.6 -> 2.1 ms (against four leaves a block, loaded in turn).
 constexpr int L2PW_WARPS = 4;
 
 template <class T, bool WANTA>
@@ -792,7 +842,7 @@ inline size_t l2pWarpSmem(int p)
 }
 
 template <class T, bool WANTA>
-__global__ void __launch_bounds__(32 * L2PW_WARPS) kL2PWarp(Tree t, const RootBox* __restrict__ rootp, int p,
+__global__ void __launch_bounds__(32 * L2PW_WARPS, sizeof(T) == 4 ? (WANTA ? 5 : 6) : 3) kL2PWarp(Tree t, const RootBox* __restrict__ rootp, int p,
                                                           int Lp, const T* __restrict__ Lc,
                                                           const typename Vec4<T>::type* __restrict__ tpos,
                                                           const int* __restrict__ tOrder,
@@ -828,162 +878,167 @@ __global__ void __launch_bounds__(32 * L2PW_WARPS) kL2PWarp(Tree t, const RootBo
       tab[v] = V4{a, b, T(0), T(0)};
    }
    __syncthreads();
-   const int node = blockIdx.x * L2PW_WARPS + warp;
-   if(node >= t.nNodes || t.nchild[node] != 0) return;
-   const int t0 = t.t0[node], t1 = t.t1[node];
-   if(t1 == t0) return;
-   // the box's local row staged with 16-byte loads (Lp is a multiple of 16), all issued at once
-   {
-      typedef typename Vec4<T>::type V4g;
-      const V4g* src = reinterpret_cast<const V4g*>(Lc + int64_t(node) * 3 * Lp);
-      V4g* dst = reinterpret_cast<V4g*>(Ls);
-#pragma unroll 4
-      for(int e = lane; e < 3 * Lp / 4; e += 32) dst[e] = src[e];
-   }
-   __syncwarp();
-   const T* lc = Ls;
-   // the curl expansion from the table: each entry <= 4 terms of the box's local row
-#pragma unroll 4
-   for(int e = lane; e < 4 * Lb; e += 32)
-   {
-      const CurlEntry<T> ce = curl[e];
-      ((T*)Cs)[e] = ce.c[0] * lc[ce.idx[0]] + ce.c[1] * lc[ce.idx[1]] + ce.c[2] * lc[ce.idx[2]] +
-                    ce.c[3] * lc[ce.idx[3]];
-   }
-   if(WANTA)
-   {
-      const T sq2 = T(1.4142135623730950488);
-      for(int e = lane; e < 4 * L; e += 32)
+   // a box's local row copied asynchronously (Lp is a multiple of 16): the next leaf's while this one is evaluated
+   auto fetch = [&](int node) {
+      if(node >= 0)
       {
-         const int k = e >> 2, c = e & 3;
-         int l = int(sqrtf(float(k)));
-         while(l * l > k) l--;
-         while((l + 1) * (l + 1) <= k) l++;
-         const int mu = k - l * l - l;
-         const T f = ((l & 1) ? T(-1) : T(1)) * (mu != 0 ? sq2 : T(1));
-         ((T*)As)[e] = c < 3 ? f * lc[c * Lp + k] : T(0);
+         const char* src = (const char*)(Lc + int64_t(node) * 3 * Lp);
+         for(int e = 16 * lane; e < 3 * Lp * int(sizeof(T)); e += 512) cpAsync16Simt((char*)Ls + e, src + e, 16u);
       }
-   }
-   __syncwarp();
-   const RootBox rb = rootp[rootOf(t, node)];
-   double cen[3], h;
-   nodeCenter(rb, t.level[node], t.ix[node], t.iy[node], t.iz[node], cen, h);
-   const T ih = T(1.0 / h), ih2 = T(1.0 / (h * h));
-   // G lanes per target when the leaf is small (G = 4 up to 8 targets, 2 up to 16): group g of the
-   // W = 32 / G lanes visits the orders m = g, g + G, ..., and the groups' sums meet by shuffles
-   const int nt = t1 - t0;
-   const int G = nt <= 8 ? 4 : (nt <= 16 ? 2 : 1), W = 32 / G;
-   const int g = lane / W, jl = lane % W;
-   auto vStart = [&](int m) { return m * (p + 1) - m * (m - 1) / 2; };   // first visit of order m
-   for(int base = t0; base < t1; base += W)
+   };
+   LeafWalk walk(int(blockIdx.x) * L2PW_WARPS + warp, int(gridDim.x) * L2PW_WARPS);
+   LeafWalk::Leaf leaf = walk.next(t, t.t0, t.t1);
+   fetch(leaf.node);
+   while(leaf.node >= 0)
    {
-      const int ti = base + jl;
-      const bool act = ti < t1;
-      const V4 x = act ? tpos[ti] : V4{T(0), T(0), T(0), T(0)};
-      const T ux = T((double(x.x) - cen[0]) / h), uy = T((double(x.y) - cen[1]) / h),
-              uz = T((double(x.z) - cen[2]) / h);
-      const T r2 = ux * ux + uy * uy + uz * uz;
-      T B0 = T(0), B1 = T(0), B2 = T(0), A0 = T(0), A1 = T(0), A2 = T(0);
-      T dre = T(1), dim = T(0);   // S_m^m, advanced to this group's first order
-      for(int j = 1; j <= g; j++)
+      const int node = leaf.node, t0 = leaf.a, t1 = leaf.b;
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      const T* lc = Ls;
+      // the curl expansion from the table: each entry <= 4 terms of the box's local row
+#pragma unroll 4
+      for(int e = lane; e < 4 * Lb; e += 32)
       {
-         const T sc = tab[vStart(j)].x;
-         const T nre = (dre * ux - dim * uy) * sc;
-         const T nim = (dre * uy + dim * ux) * sc;
-         dre = nre; dim = nim;
+         const CurlEntry<T> ce = curl[e];
+         ((T*)Cs)[e] = ce.c[0] * lc[ce.idx[0]] + ce.c[1] * lc[ce.idx[1]] + ce.c[2] * lc[ce.idx[2]] +
+                       ce.c[3] * lc[ce.idx[3]];
       }
-      // S_l^0 stays real (the imaginary parts are zero), so order 0 needs no case of its own: its
-      // k1 = k0 term adds zero
-      // the contribution of one visited harmonic (l, m): coefficients k0 = hidx(l, m), k1 = hidx(l, -m)
-      auto visit = [&](int l, int k0, int k1, T are, T aim) {
-         if(!WANTA || l < p)
-         {
-            const V4 c0 = Cs[k0], c1 = Cs[k1];
-            B0 += c0.x * are + c1.x * aim; B1 += c0.y * are + c1.y * aim; B2 += c0.z * are + c1.z * aim;
-         }
-         if(WANTA)
-         {
-            const V4 a0 = As[k0], a1 = As[k1];
-            A0 += a0.x * are + a1.x * aim; A1 += a0.y * are + a1.y * aim; A2 += a0.z * are + a1.z * aim;
-         }
-      };
-      // S_{j-1}^{j-1} -> S_j^j
-      auto diag = [&](T& re, T& im, int j) {
-         const T sc = tab[vStart(j)].x;
-         const T nre = (re * ux - im * uy) * sc;
-         const T nim = (re * uy + im * ux) * sc;
-         re = nre; im = nim;
-      };
-      // orders m and m2 = m + G walked together: two independent recurrences in flight per lane
-      for(int m = g; m <= q; m += 2 * G)
+      if(WANTA)
       {
-         const int m2 = m + G;
-         const bool two = m2 <= q;
-         T e2re = dre, e2im = dim;   // S_{m2}^{m2}
-         for(int j = m + 1; j <= m2 && j <= q; j++) diag(e2re, e2im, j);
-         int v = vStart(m), v2 = two ? vStart(m2) : 0;
-         T are = dre, aim = dim, bre = T(0), bim = T(0);
-         T are2 = e2re, aim2 = e2im, bre2 = T(0), bim2 = T(0);
-         int k0 = m * m + 2 * m, k1 = m * m, k02 = m2 * m2 + 2 * m2, k12 = m2 * m2;
-         visit(m, k0, k1, are, aim);
-         v++;
-         if(two)
+         const T sq2 = T(1.4142135623730950488);
+         for(int e = lane; e < 4 * L; e += 32)
          {
-            visit(m2, k02, k12, are2, aim2);
-            v2++;
+            const int k = e >> 2, c = e & 3;
+            int l = int(sqrtf(float(k)));
+            while(l * l > k) l--;
+            while((l + 1) * (l + 1) <= k) l++;
+            const int mu = k - l * l - l;
+            const T f = ((l & 1) ? T(-1) : T(1)) * (mu != 0 ? sq2 : T(1));
+            ((T*)As)[e] = c < 3 ? f * lc[c * Lp + k] : T(0);
          }
-         const int n2 = two ? q - m2 : 0;   // steps both orders take
+      }
+      __syncwarp();
+      double cen[3], h;
+      nodeCenter(rootp[rootOf(t, node)], t.level[node], t.ix[node], t.iy[node], t.iz[node], cen, h);
+      leaf = walk.next(t, t.t0, t.t1);
+      fetch(leaf.node);
+      const T ih = T(1.0 / h), ih2 = T(1.0 / (h * h));
+      // G lanes per target when the leaf is small (G = 4 up to 8 targets, 2 up to 16): group g of the
+      // W = 32 / G lanes visits the orders m = g, g + G, ..., and the groups' sums meet by shuffles
+      const int nt = t1 - t0;
+      const int G = nt <= 8 ? 4 : (nt <= 16 ? 2 : 1), W = 32 / G;
+      const int g = lane / W, jl = lane % W;
+      auto vStart = [&](int m) { return m * (p + 1) - m * (m - 1) / 2; };   // first visit of order m
+      for(int base = t0; base < t1; base += W)
+      {
+         const int ti = base + jl;
+         const bool act = ti < t1;
+         const V4 x = act ? tpos[ti] : V4{T(0), T(0), T(0), T(0)};
+         const T ux = T((double(x.x) - cen[0]) / h), uy = T((double(x.y) - cen[1]) / h),
+                 uz = T((double(x.z) - cen[2]) / h);
+         const T r2 = ux * ux + uy * uy + uz * uz;
+         T B0 = T(0), B1 = T(0), B2 = T(0), A0 = T(0), A1 = T(0), A2 = T(0);
+         T dre = T(1), dim = T(0);   // S_m^m, advanced to this group's first order
+         for(int j = 1; j <= g; j++)
+         {
+            const T sc = tab[vStart(j)].x;
+            const T nre = (dre * ux - dim * uy) * sc;
+            const T nim = (dre * uy + dim * ux) * sc;
+            dre = nre; dim = nim;
+         }
+         // S_l^0 stays real (the imaginary parts are zero), so order 0 needs no case of its own: its
+         // k1 = k0 term adds zero
+         // the contribution of one visited harmonic (l, m): coefficients k0 = hidx(l, m), k1 = hidx(l, -m)
+         auto visit = [&](int l, int k0, int k1, T are, T aim) {
+            if(!WANTA || l < p)
+            {
+               const V4 c0 = Cs[k0], c1 = Cs[k1];
+               B0 += c0.x * are + c1.x * aim; B1 += c0.y * are + c1.y * aim; B2 += c0.z * are + c1.z * aim;
+            }
+            if(WANTA)
+            {
+               const V4 a0 = As[k0], a1 = As[k1];
+               A0 += a0.x * are + a1.x * aim; A1 += a0.y * are + a1.y * aim; A2 += a0.z * are + a1.z * aim;
+            }
+         };
+         // S_{j-1}^{j-1} -> S_j^j
+         auto diag = [&](T& re, T& im, int j) {
+            const T sc = tab[vStart(j)].x;
+            const T nre = (re * ux - im * uy) * sc;
+            const T nim = (re * uy + im * ux) * sc;
+            re = nre; im = nim;
+         };
+         // orders m and m2 = m + G walked together: two independent recurrences in flight per lane
+         for(int m = g; m <= q; m += 2 * G)
+         {
+            const int m2 = m + G;
+            const bool two = m2 <= q;
+            T e2re = dre, e2im = dim;   // S_{m2}^{m2}
+            for(int j = m + 1; j <= m2 && j <= q; j++) diag(e2re, e2im, j);
+            int v = vStart(m), v2 = two ? vStart(m2) : 0;
+            T are = dre, aim = dim, bre = T(0), bim = T(0);
+            T are2 = e2re, aim2 = e2im, bre2 = T(0), bim2 = T(0);
+            int k0 = m * m + 2 * m, k1 = m * m, k02 = m2 * m2 + 2 * m2, k12 = m2 * m2;
+            visit(m, k0, k1, are, aim);
+            v++;
+            if(two)
+            {
+               visit(m2, k02, k12, are2, aim2);
+               v2++;
+            }
+            const int n2 = two ? q - m2 : 0;   // steps both orders take
 #pragma unroll 2
-         for(int st = 1; st <= n2; st++, v++, v2++)
-         {
-            const int l = m + st, l2 = m2 + st;
-            const V4 ab = tab[v], ab2 = tab[v2];
-            k0 += 2 * l; k1 += 2 * l; k02 += 2 * l2; k12 += 2 * l2;
-            const T az = ab.x * uz, br = ab.y * r2, az2 = ab2.x * uz, br2 = ab2.y * r2;
-            const T cre = az * are - br * bre, cim = az * aim - br * bim;
-            const T cre2 = az2 * are2 - br2 * bre2, cim2 = az2 * aim2 - br2 * bim2;
-            bre = are; bim = aim; are = cre; aim = cim;
-            bre2 = are2; bim2 = aim2; are2 = cre2; aim2 = cim2;
-            visit(l, k0, k1, are, aim);
-            visit(l2, k02, k12, are2, aim2);
-         }
-         // the rest of order m (all of it when m2 > q)
+            for(int st = 1; st <= n2; st++, v++, v2++)
+            {
+               const int l = m + st, l2 = m2 + st;
+               const V4 ab = tab[v], ab2 = tab[v2];
+               k0 += 2 * l; k1 += 2 * l; k02 += 2 * l2; k12 += 2 * l2;
+               const T az = ab.x * uz, br = ab.y * r2, az2 = ab2.x * uz, br2 = ab2.y * r2;
+               const T cre = az * are - br * bre, cim = az * aim - br * bim;
+               const T cre2 = az2 * are2 - br2 * bre2, cim2 = az2 * aim2 - br2 * bim2;
+               bre = are; bim = aim; are = cre; aim = cim;
+               bre2 = are2; bim2 = aim2; are2 = cre2; aim2 = cim2;
+               visit(l, k0, k1, are, aim);
+               visit(l2, k02, k12, are2, aim2);
+            }
+            // the rest of order m (all of it when m2 > q)
 #pragma unroll 4
-         for(int l = m + n2 + 1; l <= q; l++, v++)
-         {
-            const V4 ab = tab[v];
-            k0 += 2 * l; k1 += 2 * l;
-            const T az = ab.x * uz, br = ab.y * r2;
-            const T cre = az * are - br * bre, cim = az * aim - br * bim;
-            bre = are; bim = aim; are = cre; aim = cim;
-            visit(l, k0, k1, are, aim);
+            for(int l = m + n2 + 1; l <= q; l++, v++)
+            {
+               const V4 ab = tab[v];
+               k0 += 2 * l; k1 += 2 * l;
+               const T az = ab.x * uz, br = ab.y * r2;
+               const T cre = az * are - br * bre, cim = az * aim - br * bim;
+               bre = are; bim = aim; are = cre; aim = cim;
+               visit(l, k0, k1, are, aim);
+            }
+            // S_m^m -> S_{m+2G}^{m+2G}
+            dre = e2re; dim = e2im;
+            for(int j = m2 + 1; j <= m2 + G && j <= q; j++) diag(dre, dim, j);
          }
-         // S_m^m -> S_{m+2G}^{m+2G}
-         dre = e2re; dim = e2im;
-         for(int j = m2 + 1; j <= m2 + G && j <= q; j++) diag(dre, dim, j);
-      }
-      for(int off = 16; off >= W; off >>= 1)
-      {
-         B0 += __shfl_down_sync(0xffffffffu, B0, off);
-         B1 += __shfl_down_sync(0xffffffffu, B1, off);
-         B2 += __shfl_down_sync(0xffffffffu, B2, off);
-         if(WANTA)
+         for(int off = 16; off >= W; off >>= 1)
          {
-            A0 += __shfl_down_sync(0xffffffffu, A0, off);
-            A1 += __shfl_down_sync(0xffffffffu, A1, off);
-            A2 += __shfl_down_sync(0xffffffffu, A2, off);
+            B0 += __shfl_down_sync(0xffffffffu, B0, off);
+            B1 += __shfl_down_sync(0xffffffffu, B1, off);
+            B2 += __shfl_down_sync(0xffffffffu, B2, off);
+            if(WANTA)
+            {
+               A0 += __shfl_down_sync(0xffffffffu, A0, off);
+               A1 += __shfl_down_sync(0xffffffffu, A1, off);
+               A2 += __shfl_down_sync(0xffffffffu, A2, off);
+            }
          }
-      }
-      if(act && g == 0)
-      {
-         const int o = tOrder[ti];
-         if(want & 1)
+         if(act && g == 0)
          {
-            outB[3 * int64_t(o)] = B0 * ih2; outB[3 * int64_t(o) + 1] = B1 * ih2; outB[3 * int64_t(o) + 2] = B2 * ih2;
-         }
-         if(WANTA)
-         {
-            outA[3 * int64_t(o)] = A0 * ih; outA[3 * int64_t(o) + 1] = A1 * ih; outA[3 * int64_t(o) + 2] = A2 * ih;
+            const int o = tOrder[ti];
+            if(want & 1)
+            {
+               outB[3 * int64_t(o)] = B0 * ih2; outB[3 * int64_t(o) + 1] = B1 * ih2; outB[3 * int64_t(o) + 2] = B2 * ih2;
+            }
+            if(WANTA)
+            {
+               outA[3 * int64_t(o)] = A0 * ih; outA[3 * int64_t(o) + 1] = A1 * ih; outA[3 * int64_t(o) + 2] = A2 * ih;
+            }
          }
       }
    }
@@ -1444,7 +1499,7 @@ fmm_status upwardT(Plan& P, cudaStream_t st)
       if(sizeof(T) == 4 && P.tcTranslations(1) && P.tcDrainMode != 0) np = m2mPieces(P);
       if(np)
          FMM_TRY(P.multBf.reserve(size_t(np == 1 ? 4 : 2 * np) * size_t(N) * 3 * Lp));
-      kern<<<int(split ? N : std::min<int64_t>((N + P2MW_WARPS - 1) / P2MW_WARPS, 16 * 148)), 32 * warps, shw, st>>>(
+      kern<<<split ? int(N) : walkBlocks(kern, 32 * warps, shw, N), 32 * warps, shw, st>>>(
          P.tree, P.root, (const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, P.p, Lp, (T*)P.mult.ptr,
          np ? (uint8_t*)P.multBf.ptr : nullptr, np);
       P.p2mPiecesTag = np ? (np == 1 ? 3 : 2 * np) : -1;
@@ -1508,7 +1563,7 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
       // the 1 / (4 pi) of calcBEM (fast_multipole_solver.cpp:233-250; no current factor there)
       const size_t sh = l2pWarpSmem<T, true>(P.p);
       if(sh > 48 * 1024) FMM_CUDA(cudaFuncSetAttribute(kL2PWarp<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh)));
-      kL2PWarp<T, true><<<int((N + L2PW_WARPS - 1) / L2PW_WARPS), 32 * L2PW_WARPS, sh, st>>>(
+      kL2PWarp<T, true><<<walkBlocks(kL2PWarp<T, true>, 32 * L2PW_WARPS, sh, N), 32 * L2PW_WARPS, sh, st>>>(
          P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr, (const int*)P.tIdx.ptr,
          (const CurlEntry<T>*)P.curlTab.ptr, 2, (T*)P.outB.ptr, (T*)P.outA.ptr);
       FMM_TRY(launched(P, "kL2PWarp", st));
@@ -1518,7 +1573,7 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
    {
       auto runL2P = [&](auto kernel, size_t sh) -> fmm_status {
          if(sh > 48 * 1024) FMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh)));
-         kernel<<<int((N + L2PW_WARPS - 1) / L2PW_WARPS), 32 * L2PW_WARPS, sh, st>>>(
+         kernel<<<walkBlocks(kernel, 32 * L2PW_WARPS, sh, N), 32 * L2PW_WARPS, sh, st>>>(
             P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr, (const int*)P.tIdx.ptr,
             (const CurlEntry<T>*)P.curlTab.ptr, want, (T*)P.outB.ptr, (T*)P.outA.ptr);
          return FMM_OK;
