@@ -155,7 +155,7 @@ __device__ __forceinline__ int64_t quantize(double x, double lo, double scale, i
 // cell in that coil's root cube.
 template <class T>
 __global__ void kKeys(const T* __restrict__ xyz, int64_t n, const RootBox* __restrict__ roots,
-                      const int* __restrict__ off, int nCoils, int maxLevel, uint64_t* keys, int* idx)
+                      const int* __restrict__ off, int nCoils, int maxLevel, uint64_t mark, uint64_t* keys, int* idx)
 {
    int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
    if(i >= n) return;
@@ -170,9 +170,19 @@ __global__ void kKeys(const T* __restrict__ xyz, int64_t n, const RootBox* __res
    int64_t ux = quantize(double(xyz[3 * i]), rb.lo[0], rb.scale, maxLevel);
    int64_t uy = quantize(double(xyz[3 * i + 1]), rb.lo[1], rb.scale, maxLevel);
    int64_t uz = quantize(double(xyz[3 * i + 2]), rb.lo[2], rb.scale, maxLevel);
-   keys[i] = (uint64_t(lo) << (3 * maxLevel)) | spread3(uint64_t(ux)) | (spread3(uint64_t(uy)) << 1) |
+   keys[i] = mark | (uint64_t(lo) << (3 * maxLevel)) | spread3(uint64_t(ux)) | (spread3(uint64_t(uy)) << 1) |
              (spread3(uint64_t(uz)) << 2);
    idx[i] = int(i);
+}
+
+// The targets' part of a sort of sources and targets together, without its mark.
+__global__ void kUnmark(const uint64_t* __restrict__ k, const int* __restrict__ i, int64_t m, uint64_t mark,
+                        uint64_t* __restrict__ keys, int* __restrict__ idx)
+{
+   const int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+   if(j >= m) return;
+   keys[j] = k[j] & ~mark;
+   idx[j] = i[j];
 }
 
 template <class T>
@@ -1197,40 +1207,53 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_TRY(launched(P, "kRootFromBBox", st));
    }
    FMM_CHECK_LAUNCH();
-   // keys and sort
-   FMM_TRY(P.sKeys.reserve(2 * sizeof(uint64_t) * n));
+   // targets that are the sources (fmm_set_targets_to_sources, one coil): their keys, order and sorted
+   // positions are the sources', copied instead of computed and sorted again
+   const bool same = P.tgtIsSrc && K == 1 && m == n && !P.bem;
+   // keys and sort. A sort of a few thousand to some hundred thousand points is eight passes of 7 us each, whatever it
+   // sorts: sources and targets are sorted together, the targets marked by the bit above the key (38,400 sources and
+   // 4,001 targets: 123 -> 71 us). Up to about 2,300 points a sort is one launch of 11 us (2,048 of each sorted together:
+   // 56 us, so not), and from 2^19 points on two sorts cost the same as one and the room is kept.
+   const int keyBits = 3 * P.maxLevel + P.coilBits;
+   const bool joint = std::min(n, m) > 2500 && !same && n + m <= (int64_t(1) << 19);
+   const int64_t ns = joint ? n + m : n;
+   FMM_TRY(P.sKeys.reserve(2 * sizeof(uint64_t) * ns));
    FMM_TRY(P.tKeys.reserve(2 * sizeof(uint64_t) * m));
-   FMM_TRY(P.sIdx.reserve(2 * sizeof(int) * n));
+   FMM_TRY(P.sIdx.reserve(2 * sizeof(int) * ns));
    FMM_TRY(P.tIdx.reserve(2 * sizeof(int) * m));
    uint64_t* sk = (uint64_t*)P.sKeys.ptr;
    uint64_t* tk = (uint64_t*)P.tKeys.ptr;
    int* si = (int*)P.sIdx.ptr;
    int* ti = (int*)P.tIdx.ptr;
+   const uint64_t mark = joint ? uint64_t(1) << keyBits : 0;
    if(n) {
       kKeys<T><<<(n + threads - 1) / threads, threads, 0, st>>>((const T*)P.srcXYZ, n, P.root, dSrcOff, K,
-                                                                P.maxLevel, sk + n, si + n);
+                                                                P.maxLevel, 0, sk + ns, si + ns);
       FMM_TRY(launched(P, "kKeys", st));
    }
-   // targets that are the sources (fmm_set_targets_to_sources, one coil): their keys, order and sorted
-   // positions are the sources', copied instead of computed and sorted again
-   const bool same = P.tgtIsSrc && K == 1 && m == n && !P.bem;
    if(m && !same) {
-      kKeys<T><<<(m + threads - 1) / threads, threads, 0, st>>>((const T*)P.tgtXYZ, m, P.root, dTgtOff, K,
-                                                                P.maxLevel, tk + m, ti + m);
+      kKeys<T><<<(m + threads - 1) / threads, threads, 0, st>>>((const T*)P.tgtXYZ, m, P.root, dTgtOff, K, P.maxLevel, mark,
+                                                                joint ? sk + ns + n : tk + m, joint ? si + ns + n : ti + m);
       FMM_TRY(launched(P, "kKeys", st));
    }
    FMM_CHECK_LAUNCH();
-   const int keyBits = 3 * P.maxLevel + P.coilBits;
    size_t need = 0, tmp = 0;
-   cub::DeviceRadixSort::SortPairs(nullptr, tmp, sk + n, sk, si + n, si, int(n), 0, keyBits, st);
+   cub::DeviceRadixSort::SortPairs(nullptr, tmp, sk + ns, sk, si + ns, si, int(ns), 0, keyBits + (joint ? 1 : 0), st);
    need = std::max(need, tmp);
    cub::DeviceRadixSort::SortPairs(nullptr, tmp, tk + m, tk, ti + m, ti, int(m), 0, keyBits, st);
    need = std::max(need, tmp);
    FMM_TRY(P.cubTmp.reserve(need));
    tmp = P.cubTmp.bytes;
-   if(n) FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, sk + n, sk, si + n, si, int(n), 0, keyBits, st));
+   if(n) FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, sk + ns, sk, si + ns, si, int(ns), 0,
+                                                  keyBits + (joint ? 1 : 0), st));
    tmp = P.cubTmp.bytes;
-   if(m && !same) FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, tk + m, tk, ti + m, ti, int(m), 0, keyBits, st));
+   if(joint)
+   {
+      kUnmark<<<(m + threads - 1) / threads, threads, 0, st>>>(sk + n, si + n, m, mark, tk, ti);
+      FMM_TRY(launched(P, "kUnmark", st));
+   }
+   else if(m && !same)
+      FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, tk + m, tk, ti + m, ti, int(m), 0, keyBits, st));
    if(m && same)
    {
       FMM_CUDA(cudaMemcpyAsync(tk, sk, sizeof(uint64_t) * m, cudaMemcpyDeviceToDevice, st));
@@ -1398,6 +1421,13 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
    kNearCounts<<<148 * 4, 256, 0, st>>>(t, nn, po, (const int*)P.p2pList.ptr, (unsigned long long*)P.nearCounts.ptr);
    FMM_TRY(launched(P, "kNearCounts", st));
    FMM_CHECK_LAUNCH();
+   // what the host needs of the rest, read back together at the end: where each level's parents start, the boxes with an
+   // M2L list, and where each level's octants start in the L2L's order
+   FMM_TRY(P.scratch.reserve(sizeof(int) * (9 * (MAXLEVEL + 2) + 1)));
+   int* tail = (int*)P.scratch.ptr;
+   int* tailL2L = tail + MAXLEVEL + 2;
+   int* tailCount = tail + 9 * (MAXLEVEL + 2);
+   FMM_CUDA(cudaMemsetAsync(tailCount, 0, sizeof(int), st));
    // parents per level for the M2M / L2L GEMMs
    {
       int* flags = (int*)P.lvlCnt.ptr;   // nn + 1 ints, free again once the direct lists are counted
@@ -1414,13 +1444,9 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_CUDA(cub::DeviceScan::ExclusiveSum(P.cubTmp.ptr, tmp, flags, pos, nn + 1, st));
       kParentScatter<<<(nn + 255) / 256, 256, 0, st>>>(flags, pos, nn, (int*)P.parList.ptr);
       FMM_TRY(launched(P, "kParentScatter", st));
-      FMM_TRY(P.scratch.reserve(sizeof(int) * (MAXLEVEL + 2)));
       t.levelStart[nLevels] = nn;
-      kParentLevelStarts<<<1, 32, 0, st>>>(t, pos, (int*)P.scratch.ptr);
+      kParentLevelStarts<<<1, 32, 0, st>>>(t, pos, tail);
       FMM_TRY(launched(P, "kParentLevelStarts", st));
-      P.parStart.assign(nLevels + 1, 0);
-      FMM_CUDA(cudaMemcpyAsync(P.parStart.data(), P.scratch.ptr, sizeof(int) * (nLevels + 1), cudaMemcpyDeviceToHost, st));
-      FMM_CUDA(cudaStreamSynchronize(st));
    }
    // M2L targets grouped by octant, then (tcGroup 2) by partner pattern
    if(P.tcGroup == 2)
@@ -1436,13 +1462,12 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       unsigned* counts = (unsigned*)(k3 + nn + 2);
       int* rank = (int*)(counts + 320);
       int* vv = (int*)P.m2lTargets.ptr;
-      FMM_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
       FMM_CUDA(cudaMemsetAsync(counts, 0, sizeof(unsigned) * 320, st));
       kOffsetCounts<<<148 * 4, 256, 0, st>>>(Ls, nn, counts);
       FMM_TRY(launched(P, "kOffsetCounts", st));
       kOffsetRanks<<<1, 320, 0, st>>>(counts, rank);
       FMM_TRY(launched(P, "kOffsetRanks", st));
-      kM2LMaskKeys<<<148 * 8, 256, 0, st>>>(t, Ls, nn, rank, k0, k1, vv + nn, P.err);
+      kM2LMaskKeys<<<148 * 8, 256, 0, st>>>(t, Ls, nn, rank, k0, k1, vv + nn, tailCount);
       FMM_TRY(launched(P, "kM2LMaskKeys", st));
       // stable LSD order: by word 1, then by word 0
       tmp = 0;
@@ -1456,11 +1481,6 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, k2, k3, vv, vv + nn, nn, 0, 64, st));
       // the final order is in vv + nn: move it to the front
       FMM_CUDA(cudaMemcpyAsync(vv, vv + nn, sizeof(int) * nn, cudaMemcpyDeviceToDevice, st));
-      int cntT = 0;
-      FMM_CUDA(cudaMemcpyAsync(&cntT, P.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-      FMM_CUDA(cudaStreamSynchronize(st));
-      P.nM2LTargets = cntT;
-      FMM_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
    }
    else
    {
@@ -1468,19 +1488,13 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_TRY(P.m2lKeys.reserve(2 * sizeof(unsigned) * nn));
       unsigned* kk = (unsigned*)P.m2lKeys.ptr;
       int* vv = (int*)P.m2lTargets.ptr;
-      FMM_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
-      kM2LTargetKeys<<<(nn + 255) / 256, 256, 0, st>>>(t, Ls, nn, P.tcGroup == 1, kk + nn, vv + nn, P.err);
+      kM2LTargetKeys<<<(nn + 255) / 256, 256, 0, st>>>(t, Ls, nn, P.tcGroup == 1, kk + nn, vv + nn, tailCount);
       FMM_TRY(launched(P, "kM2LTargetKeys", st));
       tmp = 0;
       cub::DeviceRadixSort::SortPairs(nullptr, tmp, kk + nn, kk, vv + nn, vv, nn, 0, 13, st);
       FMM_TRY(P.cubTmp.reserve(tmp));
       tmp = P.cubTmp.bytes;
       FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, kk + nn, kk, vv + nn, vv, nn, 0, 13, st));
-      int cntT = 0;
-      FMM_CUDA(cudaMemcpyAsync(&cntT, P.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-      FMM_CUDA(cudaStreamSynchronize(st));
-      P.nM2LTargets = cntT;
-      FMM_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
    }
    P.multBfTag = -1;
    // M2M / L2L tables: the L2L child lists always (both L2L forms use them), the octant tables
@@ -1507,12 +1521,14 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
       FMM_TRY(P.cubTmp.reserve(tmp));
       tmp = P.cubTmp.bytes;
       FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, kk + nn, kk, vv + nn, vv, nn, 0, 8, st));
-      FMM_TRY(P.scratch.reserve(sizeof(int) * 8 * (MAXLEVEL + 2)));
-      kL2LLevelStarts<<<1, 8 * (MAXLEVEL + 2), 0, st>>>(kk, nn, nLevels, (int*)P.scratch.ptr);
+      kL2LLevelStarts<<<1, 8 * (MAXLEVEL + 2), 0, st>>>(kk, nn, nLevels, tailL2L);
       FMM_TRY(launched(P, "kL2LLevelStarts", st));
-      P.l2lStart.assign(8 * nLevels + 1, 0);
-      FMM_CUDA(cudaMemcpyAsync(P.l2lStart.data(), P.scratch.ptr, sizeof(int) * (8 * nLevels + 1), cudaMemcpyDeviceToHost, st));
+      int host[9 * (MAXLEVEL + 2) + 1];
+      FMM_CUDA(cudaMemcpyAsync(host, tail, sizeof(host), cudaMemcpyDeviceToHost, st));
       FMM_CUDA(cudaStreamSynchronize(st));
+      P.parStart.assign(host, host + nLevels + 1);
+      P.l2lStart.assign(host + MAXLEVEL + 2, host + MAXLEVEL + 2 + 8 * nLevels + 1);
+      P.nM2LTargets = host[9 * (MAXLEVEL + 2)];
       FMM_CHECK_LAUNCH();
    }
    if(P.inputsAsync && n)
