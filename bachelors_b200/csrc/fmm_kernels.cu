@@ -1051,7 +1051,7 @@ __global__ void __launch_bounds__(32 * L2PW_WARPS, sizeof(T) == 4 ? (WANTA ? 5 :
 // source of a tile and their partial sums are added in a fixed order at the end. Each thread
 // sums one tile in T and the tile sums in FP64, so no single-precision chain is longer than a tile.
 template <class T, int NT, int TS, int NE, bool WANTA, bool FAR>
-__global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 16) : 8)) kL2PNear(Tree t, const RootBox* __restrict__ rootp, int p, int Lp,
+__global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 16) : 8) * 64 / NT) kL2PNear(Tree t, const RootBox* __restrict__ rootp, int p, int Lp,
                                                const T* __restrict__ Lc,
                                                const typename Vec4<T>::type* __restrict__ tpos,
                                                const typename Vec4<T>::type* __restrict__ spos,
@@ -1326,14 +1326,18 @@ __global__ void __launch_bounds__(NT, FAR ? 1 : (sizeof(T) == 4 ? (WANTA ? 12 : 
       // add the groups' partial sums in group order
       if(G > 1)
       {
-         for(int d = 0; d < 3; d++) { red[d * NT + tid] = Bd[d]; red[(3 + d) * NT + tid] = Ad[d]; }
+         for(int d = 0; d < 3; d++)
+         {
+            red[d * NT + tid] = Bd[d];
+            if(WANTA) red[(3 + d) * NT + tid] = Ad[d];
+         }
          __syncthreads();
          if(g == 0)
             for(int gg = 1; gg < G; gg++)
                for(int d = 0; d < 3; d++)
                {
                   Bd[d] += red[d * NT + gg * nt + tt];
-                  Ad[d] += red[(3 + d) * NT + gg * nt + tt];
+                  if(WANTA) Ad[d] += red[(3 + d) * NT + gg * nt + tt];
                }
          __syncthreads();
       }
@@ -1545,17 +1549,29 @@ int nearParts(const Plan& P)
    return int(std::max<int64_t>(1, std::min({int64_t(16), int64_t(2 * 16 * 148) / N, (int64_t(1) << 20) / P.m})));
 }
 
+// Threads of a near-field block. 128 where lists are long (a leaf's targets fill 128 threads better than 64, and a
+// tile's fill is shared by more: 2^18 points, 478 sources a list, 0.43 -> 0.365 ms; in FP64 1.28 -> 1.02 ms with the
+// L2P; 2^24 points, 465, the same within the clock's drift) and where all blocks run at once, so that the longest one
+// counts (2,048 points 25 -> 14 us; 239 large leaves 99 -> 90 us); 64 where a block mostly pays for its set-up (256
+// coils, 31 sources a list: 6.5 ms against 7.6 with 128; 2^20 points and targets, 112: 0.48 against 0.54 ms).
+int nearThreads(const Plan& P)
+{
+   const int64_t N = std::max<int64_t>(1, P.tree.nNodes);
+   return N <= 16 * 148 || double(P.nP2P) / double(N) * (double(P.n) / double(N)) >= 256 ? 128 : 64;
+}
+
 template <class T>
 fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
 {
    typedef typename Vec4<T>::type V4;
    const int64_t N = P.tree.nNodes;
    const int L = P.L, Lb = nharm(P.p - 1);
-   constexpr int NT = 64, NE = 128;
+   constexpr int NE = 128;
    const int TS = P.nearTile == 128 ? 128 : 256;
    const bool split = P.l2pSplit != 0;
+   const int NT = split ? nearThreads(P) : 64;
    const size_t coef = split ? 0 : (sizeof(T) * (3 * L + 3 * Lb) + 31) & ~size_t(31);
-   size_t shm = coef + 2 * size_t(nearTileBytes<T>(TS)) + sizeof(double) * 6 * NT;
+   size_t shm = coef + 2 * size_t(nearTileBytes<T>(TS)) + sizeof(double) * (want & 2 || !split ? 6 : 3) * NT;
    T scaleB = T(REF_MU0 / (4 * REF_PI) * current), scaleA = T(1.0 / (4 * REF_PI) * current);
    if(P.bem)
    {
@@ -1592,29 +1608,16 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
                                       (T*)P.outB.ptr, (T*)P.outA.ptr, (double*)P.nearPart.ptr, int(P.m));
       return FMM_OK;
    };
-   if(split)
-   {
-      if(TS == 128)
-      {
-         if(want & 2) FMM_TRY(run(kL2PNear<T, NT, 128, NE, true, false>));
-         else FMM_TRY(run(kL2PNear<T, NT, 128, NE, false, false>));
-      }
-      else
-      {
-         if(want & 2) FMM_TRY(run(kL2PNear<T, NT, 256, NE, true, false>));
-         else FMM_TRY(run(kL2PNear<T, NT, 256, NE, false, false>));
-      }
-   }
-   else if(TS == 128)
-   {
-      if(want & 2) FMM_TRY(run(kL2PNear<T, NT, 128, NE, true, true>));
-      else FMM_TRY(run(kL2PNear<T, NT, 128, NE, false, true>));
-   }
-   else
-   {
-      if(want & 2) FMM_TRY(run(kL2PNear<T, NT, 256, NE, true, true>));
-      else FMM_TRY(run(kL2PNear<T, NT, 256, NE, false, true>));
-   }
+   auto pick = [&](auto nt, auto ts, auto far) -> fmm_status {
+      if(want & 2) return run(kL2PNear<T, decltype(nt)::value, decltype(ts)::value, NE, true, decltype(far)::value>);
+      return run(kL2PNear<T, decltype(nt)::value, decltype(ts)::value, NE, false, decltype(far)::value>);
+   };
+   constexpr std::integral_constant<int, 64> n64;
+   constexpr std::integral_constant<int, 128> n128, t128;
+   constexpr std::integral_constant<int, 256> t256;
+   if(!split) FMM_TRY(TS == 128 ? pick(n64, t128, std::true_type()) : pick(n64, t256, std::true_type()));
+   else if(NT == 64) FMM_TRY(TS == 128 ? pick(n64, t128, std::false_type()) : pick(n64, t256, std::false_type()));
+   else FMM_TRY(TS == 128 ? pick(n128, t128, std::false_type()) : pick(n128, t256, std::false_type()));
    FMM_TRY(launched(P, "kL2PNear", st));
    if(parts > 1)
    {
