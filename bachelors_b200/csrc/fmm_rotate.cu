@@ -5,7 +5,7 @@
 // a turn about y (which keeps the cosine and the sine coefficients apart), cost sum (l+1)^2 + l^2
 // multiply-adds; a z translation keeps m and costs as much. One box pair and component takes about 3 x (2/3) p^3
 // multiply-adds instead of the (p+1)^4 of the dense operator (p = 12: 4.4k instead of 28.6k, p = 16: 9.8k
-// instead of 83.5k), with the same truncation: degrees are kept by the rotations, so a cutoff on
+// instead of 83.5k), with the same truncation: degrees are kept by the rotations, so m2l_truncate's limit on
 // l + lambda keeps the same terms. (The method is White and Head-Gordon's, J. Chem. Phys. 105, 5061, 1996.)
 //
 // With D the rotation of the solid harmonics, R(rot x) = D R(x), N = diag sqrt((l-m)! (l+m)!) and D^ = N D N^-1,
@@ -851,16 +851,12 @@ __global__ void kSumParts(const int* __restrict__ targets, int nTargets, int par
 
 }  // namespace rot
 
-// The rotation tables of the plan's order and degree cutoff, all 332 operators.
+// The rotation tables of the plan's order, all 332 operators: the full M2L operator, or with m2l_truncate the terms up
+// to l + lambda = p. (fmm_config.m2l_tc_degree_cutoff is the tensor-core M2L's: here a cutoff would save nothing.)
 template <class T>
 fmm_status ensureRotations(Plan& P, cudaStream_t st)
 {
-   // the full operator by default: a cutoff saves nothing here (fmm_config.m2l_tc_degree_cutoff); m2l_truncate
-   // stops at l + lambda = p
-   const int c = P.cfg.m2l_tc_degree_cutoff;
-   int cut = c <= 0 ? 2 * P.p : std::max(c, P.p);
-   if(P.cfg.m2l_truncate) cut = std::min(cut, P.p);
-   cut = std::min(cut, 2 * P.p);
+   const int cut = P.cfg.m2l_truncate ? P.p : 2 * P.p;
    if(P.rotCut == cut) return FMM_OK;
    const rot::Blob B(P.p);
    const std::vector<double>& q = rot::quarterTurn();

@@ -59,3 +59,19 @@ def test_one_pair_and_uneven_levels(precision, tol):
     (B, A), st = solve(9, 8, precision, xyz, w, J, tgt)
     assert st["nodes"] == so["nodes"]
     assert rel(B, Bo) < tol and rel(A, Ao) < tol
+
+
+@pytest.mark.parametrize("p,precision", [(1, "fp32"), (1, "fp64"), (4, "fp32"), (10, "fp64")])
+@pytest.mark.parametrize("cutoff", ["p", "p + 1", "2 p", "none"])
+def test_degree_cutoff_is_the_tensor_cores(p, precision, cutoff):
+    """m2l_tc_degree_cutoff belongs to the tensor-core M2L: a CUDA-core plan applies its full operator whatever the
+    value, bit for bit."""
+    xyz, w, J = G.torus(24, 8, 5, 2.0, 0.5)
+    tgt = G.uniform_points(301, -3, 3, p)
+    if precision == "fp32":
+        xyz, w, J, tgt = (v.astype(np.float32) for v in (xyz, w, J, tgt))
+    (full,), st = solve(p, 8, precision, xyz, w, J, tgt, want=1)
+    (cut,), _ = solve(p, 8, precision, xyz, w, J, tgt, want=1,
+                      m2l_degree_cutoff={"p": p, "p + 1": p + 1, "2 p": 2 * p, "none": -1}[cutoff])
+    assert st["v_pairs"] > 0
+    np.testing.assert_array_equal(cut, full)
