@@ -829,15 +829,20 @@ fmm_status fmm_treecode(fmm_plan* plan, double current, int want, const void* pt
       dB = (want & 1) ? P.tcOut.ptr : nullptr;
       dA = (want & 2) ? (char*)P.tcOut.ptr + bytes : nullptr;
    }
-   FMM_TRY(P.fp64 ? treecodeT<double>(P, current, want, dPts, m, dB, dA, flags, st)
-                  : treecodeT<float>(P, current, want, dPts, m, dB, dA, flags, st));
-   if(!on_device)
+   fmm_status s = P.fp64 ? treecodeT<double>(P, current, want, dPts, m, dB, dA, flags, st)
+                         : treecodeT<float>(P, current, want, dPts, m, dB, dA, flags, st);
+   cudaError_t e = cudaSuccess;
+   if(s == FMM_OK && !on_device)
    {
-      if(want & 1) FMM_CUDA(cudaMemcpyAsync(out_B, dB, bytes, cudaMemcpyDeviceToHost, st));
-      if(want & 2) FMM_CUDA(cudaMemcpyAsync(out_A, dA, bytes, cudaMemcpyDeviceToHost, st));
-      FMM_CUDA(cudaStreamSynchronize(st));
+      if(want & 1) e = cudaMemcpyAsync(out_B, dB, bytes, cudaMemcpyDeviceToHost, st);
+      if(e == cudaSuccess && (want & 2)) e = cudaMemcpyAsync(out_A, dA, bytes, cudaMemcpyDeviceToHost, st);
    }
-   return FMM_OK;
+   // The points' order, the curl table and the staging belong to the plan: nothing of this call is in flight when the
+   // next one, on whatever stream, takes them (nor when the caller reuses the points or reads the results elsewhere).
+   const cudaError_t done = cudaStreamSynchronize(st);
+   if(e == cudaSuccess) e = done;
+   if(s == FMM_OK && e != cudaSuccess) s = setError(FMM_E_CUDA, "fmm_treecode: %s", cudaGetErrorString(e));
+   return s;
 }
 
 fmm_status fmm_adjoint_direct(fmm_plan* plan, double current, const void* dL_dB, void* dL_dJ, void* dL_dx,

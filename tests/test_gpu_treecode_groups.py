@@ -49,3 +49,34 @@ def test_points_on_sources_and_far_away(precision, tol):
     assert rel(got, want) < tol
     ref.close()
     s.plan.close()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_calls_on_two_streams(precision):
+    """Queries of different sizes, one after the other on two streams without a wait by the caller: the plan's scratch
+    (the points' order, the curl table) is never one call's while another's kernel reads it. The results are complete
+    when a call returns and equal those of the same calls on one stream, bit for bit."""
+    import torch
+    dt = torch.float32 if precision == "fp32" else torch.float64
+    xyz, w, J = (torch.tensor(v, dtype=dt, device="cuda") for v in G.torus(64, 24, 12, 2.0, 0.5))
+    pts = [torch.tensor(G.uniform_points(m, -3, 3, m), dtype=dt, device="cuda") for m in (4099, 30011, 9001, 50021, 7)]
+
+    def queries(streams):
+        s = MultipoleSolver((xyz, w, J), quadratureOctreeLeafCapacity=500, order=8, precision=precision)
+        s.calcMultipoleExpansionsAtLeaves()
+        torch.cuda.synchronize()
+        out, idle = [], []
+        for i, p in enumerate(pts):
+            with torch.cuda.stream(streams[i % len(streams)]):
+                out.append(s.calcB(1.0, p))
+                idle.append(streams[i % len(streams)].query())
+        torch.cuda.synchronize()
+        out = [v.cpu().numpy() for v in out]
+        s.plan.close()
+        return out, idle
+
+    one, _ = queries([torch.cuda.current_stream()])
+    two, idle = queries([torch.cuda.Stream(), torch.cuda.Stream()])
+    assert all(idle)
+    for a, b in zip(one, two):
+        np.testing.assert_array_equal(a, b)
