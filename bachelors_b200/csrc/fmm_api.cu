@@ -207,6 +207,8 @@ fmm_status Plan::init(const fmm_config& c)
    FMM_CUDA(pinnedWord(&hostErr));
    *hostErr = 0;
    for(int i = 0; i < 8; i++) cudaEventCreate(&ev[i]);
+   cudaEventCreateWithFlags(&evPacked, cudaEventDisableTiming);
+   cudaEventCreateWithFlags(&evDirect, cudaEventDisableTiming);
    eventsMade = true;
    return FMM_OK;
 }
@@ -235,7 +237,7 @@ void Plan::release()
    DevBuf* bufs[] = {&segb, &srcXYZb, &srcWb, &srcJb, &tgtXYZb, &rootb, &sKeys, &tKeys, &sIdx, &tIdx, &sPos, &sQ, &tPos,
                      &cubTmp, &scratch, &lvlBounds, &lvlCnt, &lvlOff, &p2pOff, &p2pList, &parList, &m2lTargets, &m2lKeys, &errb,
                      &mult, &local, &outB, &outA, &opM2M64, &opL2L64, &opM2L64, &opM2Lbf, &multBf, &tcCounters,
-                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &directPart, &nearPart, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotWs};
+                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &directPart, &subsetPart, &nearPart, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotWs};
    cudaDeviceSynchronize();   // once for all buffers
    for(DevBuf* b : bufs) b->release(true);
    for(auto& b : nodeBufs) b.release(true);
@@ -244,7 +246,11 @@ void Plan::release()
    hostErr = nullptr;
    err = pipeErr = nullptr;
    if(eventsMade)
+   {
       for(int i = 0; i < 8; i++) cudaEventDestroy(ev[i]);
+      cudaEventDestroy(evPacked);
+      cudaEventDestroy(evDirect);
+   }
    eventsMade = false;
 }
 
@@ -344,16 +350,42 @@ fmm_status downwardPhase(Plan& P, cudaStream_t st)
    return FMM_OK;
 }
 
-// The packed sources of a direct sum: the tree's when there is one, else in input order.
-fmm_status directSources(Plan& P, cudaStream_t st)
+// The packed sources of a direct sum: the tree's when there is one, else packed now in input order (`packed`).
+fmm_status directSources(Plan& P, cudaStream_t st, bool& packed)
 {
+   packed = false;
    if(P.treeReady) return FMM_OK;
    if(P.n + P.m == 0) return setError(FMM_E_INVALID, "no sources or targets set");
+   FMM_TRY(P.waitDirect(st));
+   packed = true;
    FMM_TRY(P.fp64 ? packSourcesT<double>(P, st) : packSourcesT<float>(P, st));
+   FMM_CUDA(cudaEventRecord(P.evPacked, st));
    P.treeDeferred = true;
    P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
+}
+
+// Ends a direct sum of status s. The next call may be on another stream: whatever puts the packed sources in another
+// order waits for this sum (waitDirect); and the inputs, which the packing reads, may change as soon as the host goes
+// on, so it waits for the packing (not for the sum, which is queued behind it). A sum that a caller captures into a
+// graph of its own leaves no event: the replays are the caller's to order.
+fmm_status directDone(Plan& P, cudaStream_t st, bool packed, fmm_status s)
+{
+   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+   cudaError_t e = cudaStreamIsCapturing(st, &cap);
+   if(e == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+   {
+      e = cudaEventRecord(P.evDirect, st);
+      P.directQueued = e == cudaSuccess;
+   }
+   if(packed)
+   {
+      const cudaError_t done = s == FMM_OK ? cudaEventSynchronize(P.evPacked) : cudaStreamSynchronize(st);
+      if(e == cudaSuccess) e = done;
+   }
+   if(s == FMM_OK && e != cudaSuccess) s = setError(FMM_E_CUDA, "direct sum: %s", cudaGetErrorString(e));
+   return s;
 }
 
 double elapsed(cudaEvent_t a, cudaEvent_t b)
@@ -702,15 +734,19 @@ fmm_status fmm_direct(fmm_plan* plan, double current, int want, void* out_B, voi
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   FMM_TRY(directSources(P, st));
-   size_t es = P.fp64 ? sizeof(double) : sizeof(float);
-   size_t bytes = es * 3 * std::max<int64_t>(P.m, 1);
-   if(want & 1) FMM_TRY(P.outB.reserve(bytes));
-   if(want & 2) FMM_TRY(P.outA.reserve(bytes));
-   FMM_TRY(P.fp64 ? directT<double>(P, current, want, st) : directT<float>(P, current, want, st));
-   if(want & 1) FMM_TRY(copyOut(out_B, P.outB, es * 3 * P.m, on_device, st));
-   if(want & 2) FMM_TRY(copyOut(out_A, P.outA, es * 3 * P.m, on_device, st));
-   return FMM_OK;
+   bool packed = false;
+   auto sum = [&]() -> fmm_status {
+      FMM_TRY(directSources(P, st, packed));
+      size_t es = P.fp64 ? sizeof(double) : sizeof(float);
+      size_t bytes = es * 3 * std::max<int64_t>(P.m, 1);
+      if(want & 1) FMM_TRY(P.outB.reserve(bytes));
+      if(want & 2) FMM_TRY(P.outA.reserve(bytes));
+      FMM_TRY(P.fp64 ? directT<double>(P, current, want, st) : directT<float>(P, current, want, st));
+      if(want & 1) FMM_TRY(copyOut(out_B, P.outB, es * 3 * P.m, on_device, st));
+      if(want & 2) FMM_TRY(copyOut(out_A, P.outA, es * 3 * P.m, on_device, st));
+      return FMM_OK;
+   };
+   return directDone(P, st, packed, sum());
 }
 
 fmm_status fmm_direct_fp64_subset(fmm_plan* plan, double current, const double* tgt, int64_t k, double* out_B)
@@ -722,19 +758,19 @@ fmm_status fmm_direct_fp64_subset(fmm_plan* plan, double current, const double* 
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = 0;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   FMM_TRY(directSources(P, st));
    DevBuf t, o;
-   FMM_TRY(t.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
-   fmm_status s = o.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1));
-   if(s != FMM_OK) { t.release(); return s; }
-   cudaMemcpyAsync(t.ptr, tgt, sizeof(double) * 3 * k, cudaMemcpyHostToDevice, st);
-   s = directFp64Subset(P, current, (const double*)t.ptr, int(k), (double*)o.ptr, st);
-   if(s == FMM_OK)
-   {
-      cudaError_t e = cudaMemcpyAsync(out_B, o.ptr, sizeof(double) * 3 * k, cudaMemcpyDeviceToHost, st);
-      if(e == cudaSuccess) e = cudaStreamSynchronize(st);
-      if(e != cudaSuccess) s = setError(FMM_E_CUDA, "fmm_direct_fp64_subset: %s", cudaGetErrorString(e));
-   }
+   bool packed = false;
+   auto sum = [&]() -> fmm_status {
+      FMM_TRY(directSources(P, st, packed));
+      FMM_TRY(t.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
+      FMM_TRY(o.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
+      FMM_CUDA(cudaMemcpyAsync(t.ptr, tgt, sizeof(double) * 3 * k, cudaMemcpyHostToDevice, st));
+      FMM_TRY(directFp64Subset(P, current, (const double*)t.ptr, int(k), (double*)o.ptr, st));
+      FMM_CUDA(cudaMemcpyAsync(out_B, o.ptr, sizeof(double) * 3 * k, cudaMemcpyDeviceToHost, st));
+      FMM_CUDA(cudaStreamSynchronize(st));
+      return FMM_OK;
+   };
+   const fmm_status s = directDone(P, st, packed, sum());
    t.release();
    o.release();
    return s;

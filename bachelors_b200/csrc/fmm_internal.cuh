@@ -267,6 +267,8 @@ struct Plan
    bool treeDeferred = false;            // fmm_direct has been called without a tree since the inputs were set
    fmm_stats stats{};
    cudaEvent_t ev[8];
+   cudaEvent_t evPacked, evDirect;       // the last direct sum's sources packed (without a tree), its kernels done
+   bool directQueued = false;            // evDirect has been recorded
    bool eventsMade = false;
 
    int64_t launches = 0;      // kernels this plan launched (all phases, cumulative)
@@ -291,7 +293,7 @@ struct Plan
    DevBuf adjG, adjOut;
    DevBuf tcPts, tcOut;                  // fmm_treecode: staging of host query points and results
    DevBuf nearPart;                      // near field: the sums of split direct lists
-   DevBuf directPart;                    // fmm_direct: the sums of split sources
+   DevBuf directPart, subsetPart;        // fmm_direct, fmm_direct_fp64_subset: the sums of split sources
    DevBuf tcCurl, tcSort;                // its curl table (order tcCurlOrder) and the sorted points' keys and order
    std::vector<unsigned char> tcCurlHost;   // host copy of tcCurl (kept for the asynchronous upload)
    int tcCurlOrder = -1;
@@ -306,6 +308,13 @@ struct Plan
    bool inputsAsync = false;
    fmm_status waitSourcePoints(cudaStream_t st) { return waitCopy(st, evPos); }
    fmm_status waitSourceInputs(cudaStream_t st) { return waitCopy(st, evInputs); }
+   // before the packed sources change: a direct sum on another stream may still read them
+   fmm_status waitDirect(cudaStream_t st)
+   {
+      const cudaError_t e = directQueued ? cudaStreamWaitEvent(st, evDirect, 0) : cudaSuccess;
+      if(e != cudaSuccess) return setError(FMM_E_CUDA, "waiting for a direct sum: %s", cudaGetErrorString(e));
+      return FMM_OK;
+   }
    fmm_status waitCopy(cudaStream_t st, cudaEvent_t ev)
    {
       const cudaError_t e = inputsAsync ? cudaStreamWaitEvent(st, ev, 0) : cudaSuccess;

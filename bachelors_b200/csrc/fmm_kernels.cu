@@ -1632,8 +1632,8 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
 // kDirect over coils of at most maxT targets and maxS sources (m targets in all), the sources split so that the
 // launch has about eight blocks a SM and a part keeps at least 512 sources.
 template <class T, class U>
-static fmm_status launchDirect(Plan& P, int coils, int maxT, int maxS, const U* tgt, int m, const int* sseg, const int* tseg,
-                               U scaleB, U scaleA, int want, U* outB, U* outA, cudaStream_t st)
+static fmm_status launchDirect(Plan& P, DevBuf& partBuf, int coils, int maxT, int maxS, const U* tgt, int m, const int* sseg,
+                               const int* tseg, U scaleB, U scaleA, int want, U* outB, U* outA, cudaStream_t st)
 {
    typedef typename Vec4<T>::type V4;
    constexpr int NT = 128;
@@ -1641,8 +1641,8 @@ static fmm_status launchDirect(Plan& P, int coils, int maxT, int maxS, const U* 
    if(blocks == 0) return FMM_OK;
    const int64_t wantParts = (8 * 148 + int64_t(blocks) * coils - 1) / (int64_t(blocks) * coils);
    const int parts = int(std::max<int64_t>(1, std::min<int64_t>(wantParts, maxS / 512)));
-   if(parts > 1) FMM_TRY(P.directPart.reserve(sizeof(U) * 6 * size_t(parts) * size_t(m)));
-   U* part = (U*)P.directPart.ptr;
+   if(parts > 1) FMM_TRY(partBuf.reserve(sizeof(U) * 6 * size_t(parts) * size_t(m)));
+   U* part = (U*)partBuf.ptr;
    auto run = [&](auto kern) {
       kern<<<dim3(blocks, coils, parts), NT, 0, st>>>((const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, int(P.n), tgt, m, sseg, tseg,
                                                       scaleB, scaleA, outB, outA, part);
@@ -1674,7 +1674,7 @@ fmm_status directT(Plan& P, double current, int want, cudaStream_t st)
       maxS = std::max(maxS, P.srcOff[c + 1] - P.srcOff[c]);
    }
    const int* seg = (const int*)P.segb.ptr;   // srcOff then tgtOff, uploaded by the tree build
-   return launchDirect<T, T>(P, P.nCoils, maxT, maxS, (const T*)P.tgtXYZ, int(P.m), seg, seg + P.nCoils + 1, scaleB, scaleA,
+   return launchDirect<T, T>(P, P.directPart, P.nCoils, maxT, maxS, (const T*)P.tgtXYZ, int(P.m), seg, seg + P.nCoils + 1, scaleB, scaleA,
                              want, (T*)P.outB.ptr, (T*)P.outA.ptr, st);
 }
 
@@ -1682,8 +1682,8 @@ fmm_status directFp64Subset(Plan& P, double current, const double* tgtDev, int k
 {
    const double scaleB = REF_MU0 / (4 * REF_PI) * current;
    if(P.fp64)
-      return launchDirect<double, double>(P, 1, k, int(P.n), tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1, outDev, nullptr, st);
-   return launchDirect<float, double>(P, 1, k, int(P.n), tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1, outDev, nullptr, st);
+      return launchDirect<double, double>(P, P.subsetPart, 1, k, int(P.n), tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1, outDev, nullptr, st);
+   return launchDirect<float, double>(P, P.subsetPart, 1, k, int(P.n), tgtDev, k, nullptr, nullptr, scaleB, 0.0, 1, outDev, nullptr, st);
 }
 
 // New strengths w J for the same source positions, in the tree's sorted order.

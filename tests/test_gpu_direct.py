@@ -77,3 +77,73 @@ def test_after_direct():
     assert not B[30:60].any()
     assert rel(B[60:], reference(xyz[200:], w[200:], J[200:], tgt[60:])[0]) < 1e-12
     plan.close()
+
+
+def _cuda(*arrays, dtype):
+    import torch
+    return [torch.tensor(a, dtype=dtype, device="cuda") for a in arrays]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("then", ["solve", "new sources", "new targets", "subset"])
+def test_next_call_on_another_stream(precision, then):
+    """A direct sum without a tree, still running on one stream when the plan's next call comes on another: that call
+    changes the sources' order (a tree build, another direct sum), the inputs, or runs a sum of its own, and the first
+    one's result stays what it is alone, bit for bit."""
+    import torch
+    dt = torch.float64 if precision == "fp64" else torch.float32
+    rng = np.random.default_rng(8)
+    n, m = 150001, 9001
+    xyz, w, J, tgt = _cuda(rng.uniform(-1, 1, (n, 3)), rng.uniform(0.5, 1, n), rng.normal(size=(n, 3)),
+                           rng.uniform(-2, 2, (m, 3)), dtype=dt)
+    other = _cuda(rng.uniform(3, 4, (n, 3)), rng.uniform(0.5, 1, n), rng.normal(size=(n, 3)), dtype=dt)
+    plan = Plan(order=3, leaf_capacity=200, precision=precision)
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    alone = plan.direct(1.0, 1)[0].clone()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(3):
+        plan.set_sources(xyz, w, J)
+        plan.set_targets(tgt)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            got = plan.direct(1.0, 1)[0]
+        with torch.cuda.stream(b):
+            if then == "solve":
+                plan.solve(1.0, 1)
+            elif then == "new sources":
+                plan.set_sources(*other)
+                plan.build_tree()
+            elif then == "new targets":
+                plan.set_targets(tgt.clone())
+                plan.build_tree()
+            else:
+                plan.direct_fp64(rng.uniform(-2, 2, (3, 3)))
+        torch.cuda.synchronize()
+        assert torch.equal(got, alone)
+    plan.close()
+
+
+def test_captured_by_the_caller():
+    """A direct sum over a plan's tree, captured into a graph of the caller's and replayed; the plan goes on."""
+    import torch
+    rng = np.random.default_rng(9)
+    xyz, w, J, tgt = _cuda(rng.uniform(-1, 1, (5000, 3)), rng.uniform(0.5, 1, 5000), rng.normal(size=(5000, 3)),
+                           rng.uniform(-2, 2, (300, 3)), dtype=torch.float64)
+    plan = Plan(order=3, leaf_capacity=100, precision="fp64")
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    plan.solve(1.0, 1)
+    want = plan.direct(1.0, 1)[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        got = plan.direct(1.0, 1)[0]
+    for _ in range(2):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    plan.build_tree()
+    assert torch.equal(plan.direct(1.0, 1)[0], want)
+    plan.close()
