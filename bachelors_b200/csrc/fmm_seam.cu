@@ -487,11 +487,18 @@ void launchTranslateAll(T* r, const T* a, const T* b, int64_t count, int p, cuda
 {
    if(count == 0) return;
    const int L = (p + 1) * (p + 1);
-   // 32 items a block where their entries fit the shared memory (FP32 p <= 19, FP64 p <= 13)
-   if(seamItemsSmem<T>(L) <= 227 * 1024 && (count + SEAM_ITEMS - 1) / SEAM_ITEMS <= INT32_MAX)
+   // 32 items a block where their entries fit the shared memory (FP32 p <= 19, FP64 p <= 13). A block takes its 32 items
+   // as long as one: at high orders longer than kTranslateAll takes a single item, which therefore keeps the counts that
+   // leave SMs idle either way, and those of orders 0 and 1, whose items do not fill a block's warps. A call of kTranslateAll
+   // and of this, us, FP32: p = 0 25 26 (64 items), p = 1 26 27 (64) 47 35 (32,768); p = 10 59 54 (128);
+   // p = 13 78 81 (128) 88 80 (512); p = 16 106 122 (128) 127 123 (512); p = 19 134 179 (128) 190 178 (512); FP64: p = 13 85 91
+   // (128) 98 90 (512).
+   const int64_t few = p < 2 ? 2048 : (p < 13 ? 0 : 448);
+   if(count > few && seamItemsSmem<T>(L) <= 227 * 1024 && (count + SEAM_ITEMS - 1) / SEAM_ITEMS <= INT32_MAX)
    {
       const size_t smem = seamItemsSmem<T>(L);
-      cudaFuncSetAttribute(kTranslateItems<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      if(smem > 48 * 1024)
+         cudaFuncSetAttribute(kTranslateItems<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
       kTranslateItems<T><<<unsigned((count + SEAM_ITEMS - 1) / SEAM_ITEMS), 32 * SEAM_WARPS, smem, st>>>(r, a, b, count, p);
       return;
    }

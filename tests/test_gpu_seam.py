@@ -122,3 +122,9 @@ def test_translate_all_matrix_tiles(L, count, batch):
         got = K.translateAllGPUMatrixCuBLAS(torch.tensor(a, dtype=dt, device="cuda"), torch.tensor(b, dtype=dt, device="cuda"),
                                             harmonicOrder=p)
         assert rel(got, ref) < tol
+
+
+@pytest.mark.parametrize("p,count", [(0, 2048), (0, 2049), (1, 2081), (2, 1), (12, 5), (13, 448), (13, 449), (16, 449), (19, 481)])
+def test_translate_all_few_items(p, count):
+    """The counts from which low and high orders take 32 items a block, on both sides of the lines."""
+    test_translate_all_block_edges(p, count)
