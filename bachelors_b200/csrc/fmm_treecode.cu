@@ -346,41 +346,54 @@ __global__ void __launch_bounds__(TC_NT) kTreecode(Tree t, const RootBox* __rest
          {
             const int n = min(TC_SRC, s1 - sb);
             __syncthreads();
+            bool odd = false;
             if(tid < n)
             {
                const V4 a = spos[sb + tid], b = sq[sb + tid];
                double* d = S + 8 * tid;
                d[0] = double(a.x); d[1] = double(a.y); d[2] = double(a.z); d[3] = double(b.w);
                d[4] = double(b.x); d[5] = double(b.y); d[6] = double(b.z);
+               odd = !(isfinite(b.x) && isfinite(b.y) && isfinite(b.z) && isfinite(b.w));
             }
-            __syncthreads();
-            if(!on) continue;
-#pragma unroll 2
-            for(int i = warp * G + g; i < n; i += TC_WARPS * G)
+            // Coincident points are skipped: by a factor of zero, but in a tile with a strength that is no number the sum
+            // goes from one such point to the next.
+            const bool skip = __syncthreads_or(odd);
+            for(int i = warp * G + g; on && i < n; i += TC_WARPS * G)
             {
-               const double* d = S + 8 * i;
-               const double2 d0 = *reinterpret_cast<const double2*>(d), d1 = *reinterpret_cast<const double2*>(d + 2);
-               const double2 d2 = *reinterpret_cast<const double2*>(d + 4);
-               const double sx = d2.x, sy = d2.y, sz = d[6];
-               const double ex = x - d0.x, ey = y - d0.y, ez = z - d1.x;
-               const double e2 = ex * ex + ey * ey + ez * ez;
-               const double ri = e2 > 0.0 ? rsqrt(e2) : 0.0, ri3 = ri * ri * ri;   // (coincident points skipped)
-               if(bem)
+               int stop = n;
+               if(skip)
+                  for(stop = i; stop < n; stop += TC_WARPS * G)
+                  {
+                     const double ex = x - S[8 * stop], ey = y - S[8 * stop + 1], ez = z - S[8 * stop + 2];
+                     if(ex * ex + ey * ey + ez * ez == 0.0) break;
+                  }
+#pragma unroll 2
+               for(; i < stop; i += TC_WARPS * G)
                {
-                  // the BEM kernel sigma d / |d|^3 + d x s / |d|^3 with d = q - x = -(ex, ey, ez) (fmm_bem.cu)
-                  const double sg = d1.y;
-                  A[0] -= (sg * ex + (ey * sz - ez * sy)) * ri3;
-                  A[1] -= (sg * ey + (ez * sx - ex * sz)) * ri3;
-                  A[2] -= (sg * ez + (ex * sy - ey * sx)) * ri3;
-                  continue;
+                  const double* d = S + 8 * i;
+                  const double2 d0 = *reinterpret_cast<const double2*>(d), d1 = *reinterpret_cast<const double2*>(d + 2);
+                  const double2 d2 = *reinterpret_cast<const double2*>(d + 4);
+                  const double sx = d2.x, sy = d2.y, sz = d[6];
+                  const double ex = x - d0.x, ey = y - d0.y, ez = z - d1.x;
+                  const double e2 = ex * ex + ey * ey + ez * ez;
+                  const double ri = e2 > 0.0 ? rsqrt(e2) : 0.0, ri3 = ri * ri * ri;   // (coincident points skipped)
+                  if(bem)
+                  {
+                     // the BEM kernel sigma d / |d|^3 + d x s / |d|^3 with d = q - x = -(ex, ey, ez) (fmm_bem.cu)
+                     const double sg = d1.y;
+                     A[0] -= (sg * ex + (ey * sz - ez * sy)) * ri3;
+                     A[1] -= (sg * ey + (ez * sx - ex * sz)) * ri3;
+                     A[2] -= (sg * ez + (ex * sy - ey * sx)) * ri3;
+                     continue;
+                  }
+                  if(wantB)
+                  {
+                     B[0] += (sy * ez - sz * ey) * ri3;
+                     B[1] += (sz * ex - sx * ez) * ri3;
+                     B[2] += (sx * ey - sy * ex) * ri3;
+                  }
+                  if(wantA) { A[0] += sx * ri; A[1] += sy * ri; A[2] += sz * ri; }
                }
-               if(wantB)
-               {
-                  B[0] += (sy * ez - sz * ey) * ri3;
-                  B[1] += (sz * ex - sx * ez) * ri3;
-                  B[2] += (sx * ey - sy * ex) * ri3;
-               }
-               if(wantA) { A[0] += sx * ri; A[1] += sy * ri; A[2] += sz * ri; }
             }
          }
       }

@@ -147,3 +147,31 @@ def test_captured_by_the_caller():
     plan.build_tree()
     assert torch.equal(plan.direct(1.0, 1)[0], want)
     plan.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_own_source_is_skipped_whatever_its_strength(precision, bad):
+    """A target on a source whose strength is no number, in a coil of its own: the pair is skipped, so the other
+    sources alone make its field; targets off that source see the value. The treecode's leaves do the same."""
+    rng = np.random.default_rng(10)
+    dt = np.float32 if precision == "fp32" else np.float64
+    xyz, w, J = rng.uniform(-1, 1, (700, 3)).astype(dt), rng.uniform(0.5, 1, 700).astype(dt), rng.normal(size=(700, 3)).astype(dt)
+    J[37] = bad
+    tgt = np.concatenate([xyz[37:38], xyz[37:38], [[2.0, 0, 0]]]).astype(dt)
+    rest = np.arange(700) != 37
+    Bo, Ao = reference(*(v.astype(np.float64) for v in (xyz[rest], w[rest], J[rest], tgt)), dt)
+    plan = Plan(order=2, leaf_capacity=1000, precision=precision)
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    tol = 1e-12 if precision == "fp64" else 3e-5
+    for want in (1, 2, 3):
+        B, A = plan.direct(1.0, want)
+        assert B is None or (rel(B[:2], Bo[:2]) < tol and not np.isfinite(B[2]).all())
+        assert A is None or (rel(A[:2], Ao[:2]) < tol and not np.isfinite(A[2]).all())
+    assert rel(plan.direct_fp64(tgt[:2]), Bo[:2]) < 1e-12
+    plan.build_tree()
+    plan.upward()
+    B, A = plan.treecode(tgt[:2], 1.0, 3)
+    assert rel(B, Bo[:2]) < tol and rel(A, Ao[:2]) < tol
+    plan.close()
