@@ -350,11 +350,12 @@ fmm_status downwardPhase(Plan& P, cudaStream_t st)
    return FMM_OK;
 }
 
-// The packed sources of a direct sum: the tree's when there is one, else packed now in input order (`packed`).
+// The packed sources of a direct sum: the tree's when there is one, else in input order, packed by the first sum over the
+// plan's inputs (`packed`: now; again for each sum, it made a small one 4 to 8 us slower).
 fmm_status directSources(Plan& P, cudaStream_t st, bool& packed)
 {
    packed = false;
-   if(P.treeReady) return FMM_OK;
+   if(P.treeReady || P.srcPacked) return FMM_OK;
    if(P.n + P.m == 0) return setError(FMM_E_INVALID, "no sources or targets set");
    FMM_TRY(P.waitDirect(st));
    packed = true;
@@ -383,6 +384,7 @@ fmm_status directDone(Plan& P, cudaStream_t st, bool packed, fmm_status s)
    {
       const cudaError_t done = s == FMM_OK ? cudaEventSynchronize(P.evPacked) : cudaStreamSynchronize(st);
       if(e == cudaSuccess) e = done;
+      P.srcPacked = s == FMM_OK && e == cudaSuccess;
    }
    if(s == FMM_OK && e != cudaSuccess) s = setError(FMM_E_CUDA, "direct sum: %s", cudaGetErrorString(e));
    return s;
@@ -472,7 +474,7 @@ fmm_status fmm_set_sources(fmm_plan* plan, const void* xyz, const void* w, const
    P.bem = false;
    P.n = n;
    P.tgtIsSrc = false;
-   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.srcPacked = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -525,7 +527,7 @@ fmm_status fmm_set_sources_async(fmm_plan* plan, const void* xyz, const void* w,
    P.bem = false;
    P.n = n;
    P.tgtIsSrc = false;
-   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.srcPacked = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -578,7 +580,7 @@ fmm_status fmm_set_bem_sources(fmm_plan* plan, const void* xyz, const void* w, c
    }
    stage.release();
    P.inputsAsync = false;
-   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.srcPacked = P.upReady = P.downReady = false;
    P.dropGraph();
    return s;
 }
@@ -596,7 +598,7 @@ fmm_status fmm_set_targets(fmm_plan* plan, const void* xyz, int64_t m, int on_de
    if(!on_device) FMM_CUDA(cudaStreamSynchronize(st));
    P.m = m;
    P.tgtIsSrc = false;
-   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.srcPacked = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -616,7 +618,7 @@ fmm_status fmm_set_targets_to_sources(fmm_plan* plan, void* stream)
    P.tgtXYZ = P.tgtXYZb.ptr;
    P.m = P.n;
    P.tgtIsSrc = true;
-   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.srcPacked = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
@@ -635,6 +637,7 @@ fmm_status fmm_build_tree(fmm_plan* plan, void* stream)
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    P.dropGraph();
+   P.srcPacked = false;   // the tree's order from here on, whether the build succeeds or not
    cudaEventRecord(P.ev[0], st);
    FMM_TRY(P.fp64 ? buildTreeT<double>(P, st) : buildTreeT<float>(P, st));
    cudaEventRecord(P.ev[1], st);
@@ -1066,7 +1069,7 @@ fmm_status fmm_batch_set_coils(fmm_plan* plan, int64_t ncoils, const int64_t* sr
       P.nCoils = int(ncoils);
       P.batch = true;
    }
-   P.treeReady = P.treeDeferred = P.upReady = P.downReady = false;
+   P.treeReady = P.treeDeferred = P.srcPacked = P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }

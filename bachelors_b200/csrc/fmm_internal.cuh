@@ -265,6 +265,7 @@ struct Plan
    // state
    bool treeReady = false, upReady = false, downReady = false;
    bool treeDeferred = false;            // fmm_direct has been called without a tree since the inputs were set
+   bool srcPacked = false;               // ... and sPos, sQ and segb hold the sources in input order
    fmm_stats stats{};
    cudaEvent_t ev[8];
    cudaEvent_t evPacked, evDirect;       // the last direct sum's sources packed (without a tree), its kernels done

@@ -175,3 +175,47 @@ def test_own_source_is_skipped_whatever_its_strength(precision, bad):
     B, A = plan.treecode(tgt[:2], 1.0, 3)
     assert rel(B, Bo[:2]) < tol and rel(A, Ao[:2]) < tol
     plan.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_sources_packed_once_follow_the_inputs(precision):
+    """The sources are packed by the first of several direct sums and again when anything they depend on changes: every
+    sum equals that of a new plan with the same inputs, bit for bit."""
+    dt = np.float32 if precision == "fp32" else np.float64
+    rng = np.random.default_rng(11)
+    n, m = 1500, 40
+    sets = [[v.astype(dt) for v in (rng.uniform(-1, 1, (n, 3)), rng.uniform(0.5, 1, n), rng.normal(size=(n, 3)))] for _ in range(2)]
+    tgts = [rng.uniform(-2, 2, (m, 3)).astype(dt) for _ in range(2)]
+
+    def fresh(s, t, coils=None):
+        plan = Plan(order=3, leaf_capacity=50, precision=precision)
+        plan.set_sources(*s)
+        plan.set_targets(t)
+        if coils:
+            plan.set_coils(*coils)
+        out = plan.direct(1.0, 1)[0].copy()
+        plan.close()
+        return out
+
+    plan = Plan(order=3, leaf_capacity=50, precision=precision)
+    plan.set_sources(*sets[0])
+    plan.set_targets(tgts[0])
+    for _ in range(3):
+        assert np.array_equal(plan.direct(1.0, 1)[0], fresh(sets[0], tgts[0]))
+    plan.set_targets(tgts[1])
+    assert np.array_equal(plan.direct(1.0, 1)[0], fresh(sets[0], tgts[1]))
+    plan.set_sources(*sets[1])
+    assert np.array_equal(plan.direct(1.0, 1)[0], fresh(sets[1], tgts[1]))
+    coils = ([0, 600, n], [0, 10, m])
+    plan.set_coils(*coils)
+    for _ in range(2):
+        assert np.array_equal(plan.direct(1.0, 1)[0], fresh(sets[1], tgts[1], coils))
+    plan.set_coils(None, None)
+    assert np.array_equal(plan.direct(1.0, 1)[0], fresh(sets[1], tgts[1]))
+    plan.solve(1.0, 1)                                   # the tree's order from here on
+    tree = plan.direct(1.0, 1)[0].copy()
+    assert rel(tree, fresh(sets[1], tgts[1]).astype(np.float64)) < (1e-12 if precision == "fp64" else 1e-5)
+    assert np.array_equal(plan.direct(1.0, 1)[0], tree)
+    plan.set_sources(*sets[0])                           # and back to the input order
+    assert np.array_equal(plan.direct(1.0, 1)[0], fresh(sets[0], tgts[1]))
+    plan.close()
