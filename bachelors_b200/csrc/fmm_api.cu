@@ -192,18 +192,19 @@ fmm_status Plan::init(const fmm_config& c)
    if(const char* e = getenv("FMM_TC_DRAINMODE")) tcDrainMode = std::min(3, std::max(0, atoi(e)));
    if(const char* e = getenv("FMM_TC_GROUP")) tcGroup = std::min(2, std::max(0, atoi(e)));
    if(const char* e = getenv("FMM_L2P_SPLIT")) l2pSplit = atoi(e) != 0;
+   if(const char* e = getenv("FMM_ROT_SHARED")) rotShared = atoi(e) != 0;
    if(const char* e = getenv("FMM_TC_TRANSLATE")) tcTranslate = atoi(e) & 3;
    if(const char* e = getenv("FMM_TC_TRDRAIN")) tcTrDrainItems = std::max(0, atoi(e));
    if(const char* e = getenv("FMM_TC_TRNP_UP")) tcTrPiecesUp = std::min(3, std::max(0, atoi(e)));
    if(const char* e = getenv("FMM_TC_TRNP_DN")) tcTrPiecesDn = std::min(3, std::max(0, atoi(e)));
 
    FMM_TRY(rootb.reserve(sizeof(RootBox)));
-   FMM_TRY(errb.reserve(2 * sizeof(int)));
+   FMM_TRY(errb.reserve(3 * sizeof(int)));
    FMM_TRY(initOffsetTables());
    root = (RootBox*)rootb.ptr;
    err = (int*)errb.ptr;
    pipeErr = err + 1;
-   FMM_CUDA(cudaMemset(errb.ptr, 0, 2 * sizeof(int)));
+   FMM_CUDA(cudaMemset(errb.ptr, 0, 3 * sizeof(int)));
    FMM_CUDA(pinnedWord(&hostErr));
    *hostErr = 0;
    for(int i = 0; i < 8; i++) cudaEventCreate(&ev[i]);
@@ -237,7 +238,7 @@ void Plan::release()
    DevBuf* bufs[] = {&segb, &srcXYZb, &srcWb, &srcJb, &tgtXYZb, &rootb, &sKeys, &tKeys, &sIdx, &tIdx, &sPos, &sQ, &tPos,
                      &cubTmp, &scratch, &lvlBounds, &lvlCnt, &lvlOff, &p2pOff, &p2pList, &parList, &m2lTargets, &m2lKeys, &errb,
                      &mult, &local, &outB, &outA, &opM2M64, &opL2L64, &opM2L64, &opM2Lbf, &multBf, &tcCounters,
-                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &directPart, &subsetPart, &nearPart, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotWs};
+                     &adjG, &adjOut, &tcPts, &tcOut, &srcSigmab, &nearCounts, &tcProfBuf, &levelState, &curlTab, &vtabUp, &vtabDn, &l2lTargets, &l2lKeys, &opM2Mbf, &opL2Lbf, &directPart, &subsetPart, &nearPart, &tcCurl, &tcSort, &rotOps, &rotQuarter, &rotTasks, &rotTiles, &rotWs};
    cudaDeviceSynchronize();   // once for all buffers
    for(DevBuf* b : bufs) b->release(true);
    for(auto& b : nodeBufs) b.release(true);

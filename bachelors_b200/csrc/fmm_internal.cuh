@@ -224,10 +224,12 @@ struct Plan
    int opOrder = -1;
    int denseOrder = -1;
    // translations through the z axis (fmm_rotate.cu): operator tables for degree cutoff rotCut, the quarter
-   // turn they are made from, partial sums of split tiles
-   DevBuf rotOps, rotQuarter, rotTasks, rotWs;
+   // turn they are made from, the M2L tiles' operators, partial sums of split tiles
+   DevBuf rotOps, rotQuarter, rotTasks, rotTiles, rotWs;
    std::vector<unsigned char> rotTaskHost;   // host copy of rotTasks (kept for the asynchronous upload)
    int rotCut = -1;
+   int rotShared = 1;                    // 0: as if there were no room for those sums
+   int rotResident = 0;                  // blocks of the M2L an SM holds (0: not asked yet)
    // tensor-core M2L tile choices (autotuned per order and leaf capacity, or set by environment)
    int tcKChunk = 0;                     // K chunk width 32 or 64 (0: 64 for BF16X3, 32 for BF16X6)
    int tcDrainFar = 8;                   // the same through the first (far) half of a tile's offsets
@@ -352,7 +354,7 @@ template <class T> fmm_status directT(Plan& P, double current, int want, cudaStr
 fmm_status buildOperators(Plan& P, cudaStream_t st);
 fmm_status buildDenseOperators(Plan& P, cudaStream_t st);
 template <class T> fmm_status ensureRotations(Plan& P, cudaStream_t st);
-template <class T> fmm_status reserveRotations(Plan& P);
+template <class T> fmm_status reserveRotations(Plan& P, cudaStream_t st);
 template <class T> fmm_status rotM2L(Plan& P, cudaStream_t st);
 template <class T> fmm_status rotM2M(Plan& P, cudaStream_t st);
 template <class T> fmm_status rotL2L(Plan& P, cudaStream_t st);

@@ -21,6 +21,8 @@
 #include <type_traits>
 #include <vector>
 
+#include <cub/cub.cuh>
+
 #include "fmm_internal.cuh"
 
 namespace fmm {
@@ -260,6 +262,7 @@ struct __align__(16) Task
    unsigned short out[4];           // output positions (0xFFFF: none)
 };
 constexpr int MAXTASK = 88;         // quarter-warp tasks of one step (p = 16)
+constexpr int MAXTILE = 100;        // target boxes of an M2L or M2M tile at most
 struct TaskTable
 {
    int n[3];                        // warp tasks (four tasks of equal K) of each step
@@ -477,7 +480,7 @@ __device__ __forceinline__ void turn(const unsigned* pairs, int nPairs, int warp
    }
 }
 
-constexpr int MAXT = 100;     // target boxes of an M2L or M2M tile at most
+constexpr int MAXT = MAXTILE;
 constexpr int MAXTL = 160;    // of an L2L tile
 template <class T>
 struct Smem   // byte offsets in the block's dynamic shared memory
@@ -529,7 +532,168 @@ __device__ __forceinline__ T boxScale(int k, bool less)
 
 struct L2LSegR { int start[9]; };
 
-// One tile of TT target boxes (blockIdx.x) and one part of its operators (blockIdx.y of gridDim.y). For every
+// The M2L operators of every tile, in order: their number, the operators and the work of those before each; over the tiles
+// the work before each tile (start[tiles]: all); and how the tiles are dealt out to the blocks: the first `whole` in turn,
+// then of the rest block b takes the work from share[b] to share[b + 1].
+struct TileOps
+{
+   int tiles, whole, blocks;
+   int* n;
+   int* before;          // [tile][316]
+   unsigned short* op;   // [tile][316]
+   int64_t* start;       // [tiles + 1]
+   int64_t* share;       // [blocks + 1]
+};
+
+// The work of an operator with n pairs in the tile, in twentieths of a full chunk: its chunks, a half chunk being one with a
+// single group of rows, and its table. (The weights that served best of those around a fit to the blocks' times; they
+// move the M2L by a few per cent.)
+template <class T>
+__device__ __forceinline__ int opWork(int n, int p)
+{
+   constexpr int CH = chunkPairs<T>();
+   const int rest = n % CH, half = sizeof(T) == 8 ? 13 : (p <= 6 ? 12 : 9);
+   return n == 0 ? 0 : 1 + 20 * (n / CH) + (3 * rest > 8 * laneRows<T>() ? 20 : (rest ? half : 0));
+}
+
+// start[] from the tiles' work at start[tile + 1], then the shares, by one block: every block's whole tiles and share together
+// are to make the same work (a block whose whole tiles alone are more than that gets an empty share).
+constexpr int TILEOPS_NT = 320;
+__device__ void tileStarts(const TileOps ops)
+{
+   typedef cub::BlockScan<int64_t, TILEOPS_NT> Scan;
+   __shared__ typename Scan::TempStorage tmp;
+   const int tid = threadIdx.x;
+   int64_t base = 0;
+   if(tid == 0) ops.start[0] = 0;
+   for(int t0 = 0; t0 < ops.tiles; t0 += TILEOPS_NT)
+   {
+      const int t = t0 + tid;
+      int64_t v = t < ops.tiles ? __ldcg(ops.start + t + 1) : 0, sum;
+      Scan(tmp).InclusiveSum(v, v, sum);
+      if(t < ops.tiles) ops.start[t + 1] = base + v;
+      base += sum;
+      __syncthreads();
+   }
+   // what each block still needs, summed up to each block's end; then scaled to the work that is left
+   const int64_t first = ops.start[ops.whole];
+   int64_t needed = 0;
+   for(int b0 = 0; b0 < ops.blocks; b0 += TILEOPS_NT)
+   {
+      const int b = b0 + tid;
+      int64_t need = 0, sum;
+      if(b < ops.blocks)
+      {
+         need = base / ops.blocks + 1;
+         for(int t = b; t < ops.whole; t += ops.blocks) need -= ops.start[t + 1] - ops.start[t];
+         if(need < 0) need = 0;
+      }
+      Scan(tmp).InclusiveSum(need, need, sum);
+      if(b < ops.blocks) ops.share[b + 1] = needed + need;
+      needed += sum;
+      __syncthreads();
+   }
+   for(int b = tid; b < ops.blocks; b += TILEOPS_NT)
+      ops.share[b + 1] = b + 1 == ops.blocks ? base : first + int64_t(double(base - first) * double(ops.share[b + 1]) / double(max(needed, int64_t(1))));
+   if(tid == 0) ops.share[0] = first;
+}
+
+// TileOps of one tile a block, a thread per operator; the last block to end (done counts them, from 0 back to 0) makes the starts.
+template <class T>
+__global__ void __launch_bounds__(TILEOPS_NT) kTileOps(const int* __restrict__ targets, int nTargets, const int* __restrict__ vtab,
+                                                       int TT, int p, const TileOps ops, unsigned* done)
+{
+   __shared__ int node[MAXTILE];
+   __shared__ int warpSum[TILEOPS_NT / 32][2];
+   const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+   const int nTile = min(TT, nTargets - tile * TT);
+   for(int t = tid; t < nTile; t += TILEOPS_NT) node[t] = targets[tile * TT + t];
+   __syncthreads();
+   int n = 0;
+   if(tid < 316)
+#pragma unroll 8
+      for(int t = 0; t < nTile; t++) n += vtab[int64_t(node[t]) * 316 + tid] >= 0;
+   // positions in the list and the work before, over the block
+   const int mine = opWork<T>(n, p);
+   const unsigned bits = __ballot_sync(0xffffffffu, n > 0);
+   int incl = mine;
+   for(int d = 1; d < 32; d <<= 1)
+   {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if(lane >= d) incl += v;
+   }
+   if(lane == 31) { warpSum[warp][0] = __popc(bits); warpSum[warp][1] = incl; }
+   __syncthreads();
+   int at = __popc(bits & ((1u << lane) - 1)), work = incl - mine, count = 0, all = 0;
+   for(int w = 0; w < TILEOPS_NT / 32; w++)
+   {
+      if(w < warp) { at += warpSum[w][0]; work += warpSum[w][1]; }
+      count += warpSum[w][0];
+      all += warpSum[w][1];
+   }
+   if(n > 0)
+   {
+      ops.op[int64_t(tile) * 316 + at] = (unsigned short)tid;
+      ops.before[int64_t(tile) * 316 + at] = work;
+   }
+   __shared__ bool last;
+   if(tid == 0)
+   {
+      ops.n[tile] = count;
+      ops.start[tile + 1] = all;
+      __threadfence();
+      last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+      __threadfence();
+   }
+   __syncthreads();
+   if(last) tileStarts(ops);
+}
+
+// the tile that holds unit w of the work (w < start[tiles])
+__device__ __forceinline__ int tileOf(const int64_t* __restrict__ start, int tiles, int64_t w)
+{
+   int a = 0, b = tiles;   // start[a] <= w < start[b]
+   while(b - a > 1)
+   {
+      const int m = (a + b) >> 1;
+      if(start[m] <= w) a = m;
+      else b = m;
+   }
+   return a;
+}
+
+// Y of the tiles that several blocks share: the slots' sums added in block order. blockIdx.x: the tile, of those behind the
+// whole ones; blockIdx.y of gridDim.y: boxes of it.
+template <class T>
+__global__ void __launch_bounds__(256) kAddParts(const int* __restrict__ targets, int nTargets, int TT, const TileOps ops, int Lp,
+                                                 const T* __restrict__ ws, T* __restrict__ Y)
+{
+   const int tile = ops.whole + blockIdx.x;
+   const int64_t a = ops.start[tile], e = ops.start[tile + 1];
+   int b0 = 0, b1 = ops.blocks;   // the first block that begins behind a
+   while(b0 < b1)
+   {
+      const int m = (b0 + b1) >> 1;
+      if(ops.share[m] > a) b1 = m;
+      else b0 = m + 1;
+   }
+   while(b1 < ops.blocks && ops.share[b1] < e) b1++;
+   if(b0 == b1) return;
+   const int nTile = min(TT, nTargets - tile * TT), n = 3 * Lp;
+   for(int t = blockIdx.y; t < nTile; t += gridDim.y)
+   {
+      T* y = Y + int64_t(targets[tile * TT + t]) * n;
+      for(int k = threadIdx.x; k < n; k += 256)
+      {
+         T s = y[k];
+#pragma unroll 8
+         for(int b = b0; b < b1; b++) s += ws[(int64_t(b) * TT + t) * n + k];
+         y[k] = s;
+      }
+   }
+}
+
+// A tile of TT target boxes and its operators, or some of them. For every
 // operator with a source for some box of the tile the pairs are taken a chunk at a time, 20 (FP64: 10) pairs of 3
 // vectors, none of them empty: their source rows are gathered into shared memory [coefficient][vector],
 // turned about z in place, then the three steps (rotation, z translation, rotation back) alternate between two
@@ -550,12 +714,20 @@ struct L2LSegR { int start[9]; };
 // In the M2M and L2L a coefficient's own term (lambda = l) is the coefficient times a power of two: it is added as
 // it is, and only the other, smaller terms go through the rotations and their rounding (with it among them the
 // 2^24-point solve at p = 16 was 8.5e-7 off, without 7.7e-7 as with the dense operators).
-// gridDim.y > 1: the parts' sums go to ws[part][3 nTargets][Lp] (zero before) for kSumParts.
+// M2L: a block takes every gridDim.x-th of the first tiles, so that those in flight are neighbours and share their sources
+// in L2, and of the rest a share of operators that evens out the blocks' work (TileOps). The block with a tile's first
+// operator adds to the rows of Y, one that begins inside a tile keeps its sums there in its slot of ws ([3 TT][Lp])
+// for kAddParts: a slot a block, whatever the tree. Without ws the grid is a block per tile.
+// (Before, every tile was split into as many equal parts as made eight rounds of blocks, up to 64 copies of the locals:
+// 0.43 to 0.57 GB, now 75 MB at most. M2L of 65,536 points and targets, FP32 p = 12 1.24 -> 1.02 ms, FP64 p = 9 1.49 -> 1.23;
+// 131,072, FP32 p = 16 5.37 -> 4.95; 2^20, p = 4 4.6 both, p = 8 11.7 -> 12.0, p = 12 24.7 both, p = 16 50.8 -> 46.0.)
+// M2M: blockIdx.y of gridDim.y parts of a tile's operators, their sums go to ws[part][3 nTargets][Lp] (zero before) for kSumParts.
 template <class T, int MODE>
 __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ targets, int nTargets,
                                                     const int* __restrict__ vtab, const int* __restrict__ parent,
-                                                    const L2LSegR seg, int TT, int p, int Lp, const TaskTable* __restrict__ tasks,
-                                                    const T* __restrict__ ops, const T* X, T* Y, T* ws)
+                                                    const L2LSegR seg, const TileOps tileOps, int TT, int p, int Lp,
+                                                    const TaskTable* __restrict__ tasks, const T* __restrict__ ops, const T* X,
+                                                    T* Y, T* ws)
 {
    constexpr int NOP = MODE == 0 ? 316 : 8;
    constexpr int RS = rowStride<T>(), CH = chunkPairs<T>(), V = laneRows<T>();
@@ -578,7 +750,18 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
       end = seg.start[blockIdx.z + 1];
       if(first >= end) return;
    }
-   const int nTile = min(TT, end - first);
+   // M2L: the tile in which this block's share begins (tiles: its share is empty)
+   auto shareTile = [&]() {
+      const int64_t w = tileOps.share[blockIdx.x];
+      return w < tileOps.share[blockIdx.x + 1] || w > tileOps.start[tileOf(tileOps.start, tileOps.tiles, w)] ? tileOf(tileOps.start, tileOps.tiles, w)
+                                                                                                          : tileOps.tiles;
+   };
+   if(MODE == 0 && blockIdx.x >= tileOps.whole)
+   {
+      first = shareTile() * TT;
+      if(first >= end) return;
+   }
+   int nTile = min(TT, end - first);
    const Smem<T> sm(p);
    T* D = reinterpret_cast<T*>(smraw);
    T* W0 = reinterpret_cast<T*>(smraw + sm.w0);
@@ -587,8 +770,6 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
    unsigned* pairs = reinterpret_cast<unsigned*>(smraw + sm.pairs);       // positions of (l, m), (l, -m), and m
    int* pads = reinterpret_cast<int*>(smraw + sm.pads);                   // order-major pad positions, their number at [MAXORDER + 1]
    unsigned short* pos = reinterpret_cast<unsigned short*>(smraw + sm.pos);   // degree-major position of k (L: none)
-   for(int t = tid; t < nTile; t += NT) tileNode[t] = targets[first + t];
-   if(tid < 10) present[tid] = 0;
    const int nTask[3] = {tasks->n[0], tasks->n[1], tasks->n[2]};
    for(int e = tid; e < 3 * MAXTASK; e += NT)
       reinterpret_cast<uint4*>(task)[e] = reinterpret_cast<const uint4*>(&tasks->t[0][0])[e];
@@ -615,224 +796,268 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
    // (a zero operator row meets these: they must be numbers)
    for(int e = tid; e < 2 * RS; e += NT) W0[L * RS + e] = T(0);
    for(int e = tid; e < RS; e += NT) W1[ordSize(p) * RS + e] = T(0);
-   __syncthreads();
-   int o0 = 0, o1 = 1;
-   if(MODE == 2)
+   // the tiles of the block's share (M2M, L2L: its one tile)
+   for(;;)
    {
-      // every box has its pair: its parent
-      if(tid == 0) { offs[0] = blockIdx.z; nSlot[0] = nTile; }
-      for(int t = tid; t < nTile; t += NT) slotS[0][t] = parent[tileNode[t]];
+      for(int t = tid; t < nTile; t += NT) tileNode[t] = targets[first + t];
+      if(MODE == 1 && tid < 10) present[tid] = 0;
       __syncthreads();
-   }
-   else
-   {
-      // a warp per box, its table row in loads that are all in flight
-      constexpr int NWORD = (NOP + 31) / 32;
-      uint32_t have[NWORD] = {};
-      for(int t = warp; t < nTile; t += NW)
+      int o0 = 0, o1 = 1;
+      bool toParts = false;   // the sums of this tile go to ws
+      if(MODE == 2)
       {
-         const int* row = vtab + int64_t(tileNode[t]) * NOP;
-         int v[NWORD];
-#pragma unroll
-         for(int w = 0; w < NWORD; w++) v[w] = lane + 32 * w < NOP ? row[lane + 32 * w] : -1;
-#pragma unroll
-         for(int w = 0; w < NWORD; w++) have[w] |= __ballot_sync(0xffffffffu, v[w] >= 0);
-      }
-      if(lane == 0)
-#pragma unroll
-         for(int w = 0; w < NWORD; w++)
-            if(have[w]) atomicOr(&present[w], have[w]);
-      __syncthreads();
-      if(warp == 0)
-      {
-         // the operators present, in order
-         int base = 0;
-         for(int w = 0; w * 32 < NOP; w++)
-         {
-            const uint32_t bits = present[w];
-            if(bits >> lane & 1) offs[base + __popc(bits & ((1u << lane) - 1))] = 32 * w + lane;
-            base += __popc(bits);
-         }
-         if(lane == 0) nOffS = base;
-      }
-      __syncthreads();
-      const int nOff = nOffS, parts = gridDim.y, part = blockIdx.y;
-      o0 = int(int64_t(nOff) * part / parts);
-      o1 = int(int64_t(nOff) * (part + 1) / parts);
-   }
-   if(o0 >= o1) return;
-   // source of the tile's box t for operator o
-   auto sourceOf = [&](int t, int o) {
-      if(t >= nTile) return -1;
-      return vtab[int64_t(tileNode[t]) * NOP + o];
-   };
-   // warp 0: the pairs of operator oi, compacted; the sources were loaded one operator earlier
-   constexpr int AH = (MAXT + 31) / 32;
-   int ahead[AH];
-   auto loadAhead = [&](int oi) {
-#pragma unroll
-      for(int h = 0; h < AH; h++) ahead[h] = sourceOf(lane + 32 * h, offs[oi]);
-   };
-   auto compact = [&](int b) {
-      int n = 0;
-#pragma unroll
-      for(int h = 0; h < AH; h++)
-      {
-         const uint32_t bits = __ballot_sync(0xffffffffu, ahead[h] >= 0);
-         if(ahead[h] >= 0)
-         {
-            const int k = n + __popc(bits & ((1u << lane) - 1));
-            slotT[b][k] = lane + 32 * h;
-            slotS[b][k] = ahead[h];
-         }
-         n += __popc(bits);
-      }
-      if(lane == 0) nSlot[b] = n;
-   };
-   const bool toParts = gridDim.y > 1 && MODE != 2;
-   T* out = toParts ? ws + (int64_t(blockIdx.y) * nTargets + first) * 3 * Lp : Y;
-   // the rows of X a chunk's vectors come from and the rows of Y (or of this part's sums) they are added to
-   auto setRows = [&](int b, int c0, int nr, int db) {
-      if(tid < nr)
-      {
-         const int t = c0 + tid / 3, cmp = tid % 3;
-         srcRow[db][tid] = 3 * slotS[b][t] + cmp;
-         dstRow[db][tid] = 3 * (MODE == 2 ? tileNode[t] : toParts ? slotT[b][t] : tileNode[slotT[b][t]]) + cmp;
-      }
-   };
-   // Gather: element copies that all stay in flight while the previous chunk's sums are added, 8 consecutive
-   // coefficients (a 32-byte sector in FP32) of 4 rows a warp.
-   const int nk8 = (L + 7) >> 3, k8 = lane & 7, r4 = lane >> 3;
-   auto gather = [&](const int* rows, int nr) {
-      const int nq = (nr + 3) >> 2;
-      for(int j = warp; j < nk8; j += NW)
-      {
-         const int k = 8 * j + k8;
-         if(k >= L) continue;
-         T* w = W0 + int(pos[k]) * RS + r4;
-         const T* src = X + k;
-#pragma unroll 4
-         for(int q = 0; q < nq; q++)
-            if(4 * q + r4 < nr) cpAsyncElem(w + 4 * q, src + int64_t(rows[4 * q + r4]) * Lp);
-      }
-   };
-   // Sums: 4 lanes of V consecutive coefficients by 8 rows a warp and item, BT items' loads in flight together.
-   const int kl = V * (lane & 3), rl = lane >> 2, nkb = (Lp + 4 * V - 1) / (4 * V);
-   typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type VT;
-   constexpr int BT = MODE == 0 ? 6 : 4;
-   auto addOut = [&](int db, int nr) {
-      const int* rows = dstRow[db];
-      const int nItems = nkb * ((nr + 7) >> 3);
-      for(int i0 = warp; i0 < nItems; i0 += BT * NW)
-      {
-         VT y[BT], id[BT];
-         T* q[BT];
-#pragma unroll
-         for(int h = 0; h < BT; h++)
-         {
-            const int it = i0 + h * NW, r = 8 * (it / nkb) + rl, k = 4 * V * (it % nkb) + kl;
-            q[h] = nullptr;
-            if(it < nItems && r < nr)
-            {
-               q[h] = out + int64_t(rows[r]) * Lp + k;
-               y[h] = *reinterpret_cast<const VT*>(q[h]);
-               if(MODE != 0) id[h] = *reinterpret_cast<const VT*>(X + int64_t(srcRow[db][r]) * Lp + k);
-            }
-         }
-#pragma unroll
-         for(int h = 0; h < BT; h++)
-         {
-            if(!q[h]) continue;
-            const int it = i0 + h * NW, r = 8 * (it / nkb) + rl, k = 4 * V * (it % nkb) + kl;
-            T* ys = reinterpret_cast<T*>(&y[h]);
-#pragma unroll
-            for(int i = 0; i < V; i++)
-            {
-               const int w = pos[k + i];
-               if(w == 0xFFFF) continue;
-               T v = W1[w * RS + r];
-               if(MODE != 0) v = fma(reinterpret_cast<const T*>(&id[h])[i], boxScale<T>(k + i, MODE == 2), v);
-               ys[i] += v;
-            }
-            *reinterpret_cast<VT*>(q[h]) = y[h];
-         }
-      }
-   };
-   if(MODE != 2 && warp == 0)
-   {
-      loadAhead(o0);
-      compact(0);
-      if(o0 + 1 < o1) loadAhead(o0 + 1);
-   }
-   __syncthreads();
-   int oi = o0, b = 0, c0 = 0, nPairs = nSlot[0], nr = 3 * min(CH, nPairs), prevRows = 0, chunk = 0;
-   setRows(0, 0, nr, 0);
-   __syncthreads();
-   const T* Z = D + B.zOff;
-   const int nTurn = p * (p + 1) / 2;
-   while(true)
-   {
-      if(c0 == 0)
-      {
-         const T* src = ops + int64_t(offs[oi]) * B.size;
-         for(int e = tid * V; e < B.size; e += NT * V) cpAsync16(D + e, src + e);
-         asm volatile("cp.async.commit_group;" ::: "memory");
-      }
-      gather(srcRow[chunk & 1], nr);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      if(chunk) addOut((chunk - 1) & 1, prevRows);
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();
-      if(MODE != 2 && c0 == 0 && warp == 0 && oi + 1 < o1)
-      {
-         compact(b ^ 1);
-         if(oi + 2 < o1) loadAhead(oi + 2);
-      }
-      for(int e = tid; e < pads[MAXORDER + 1] * RS; e += NT) W1[pads[e / RS] * RS + e % RS] = T(0);
-      if(nr > 8 * V)
-      {
-         turn<T, 2>(pairs, nTurn, warp, NW, lane, Z, W0, false);
+         // every box has its pair: its parent
+         if(tid == 0) { offs[0] = blockIdx.z; nSlot[0] = nTile; }
+         for(int t = tid; t < nTile; t += NT) slotS[0][t] = parent[tileNode[t]];
          __syncthreads();
-         runStep<T, 2>(task, nTask[0], warp, NW, lane, D, W0, W1);
-         __syncthreads();
-         runStep<T, 2>(task + MAXTASK, nTask[1], warp, NW, lane, D, W1, W0);
-         __syncthreads();
-         runStep<T, 2>(task + 2 * MAXTASK, nTask[2], warp, NW, lane, D, W0, W1);
-         __syncthreads();
-         turn<T, 2>(pairs, nTurn, warp, NW, lane, Z, W1, true);
+      }
+      else if(MODE == 0)
+      {
+         // the tile's operators, those whose work begins in the share
+         const int tile = first / TT, n = tileOps.n[tile];
+         const int64_t lo = tile < tileOps.whole ? 0 : tileOps.share[blockIdx.x] - tileOps.start[tile];
+         const int64_t hi = tile < tileOps.whole ? INT64_MAX : tileOps.share[blockIdx.x + 1] - tileOps.start[tile];
+         o1 = 0;
+         for(int e0 = 0; e0 < n; e0 += NT)
+         {
+            const int e = e0 + tid;
+            const int64_t at = e < n ? tileOps.before[int64_t(tile) * NOP + e] : INT64_MAX;
+            if(e < n) offs[e] = tileOps.op[int64_t(tile) * NOP + e];
+            o0 += __syncthreads_count(at < lo);
+            o1 += __syncthreads_count(at < hi);
+         }
+         toParts = o0 > 0;
       }
       else
       {
-         // at most one group of rows
-         turn<T, 1>(pairs, nTurn, warp, NW, lane, Z, W0, false);
+         // a warp per box, its table row in loads that are all in flight
+         constexpr int NWORD = (NOP + 31) / 32;
+         uint32_t have[NWORD] = {};
+         for(int t = warp; t < nTile; t += NW)
+         {
+            const int* row = vtab + int64_t(tileNode[t]) * NOP;
+            int v[NWORD];
+#pragma unroll
+            for(int w = 0; w < NWORD; w++) v[w] = lane + 32 * w < NOP ? row[lane + 32 * w] : -1;
+#pragma unroll
+            for(int w = 0; w < NWORD; w++) have[w] |= __ballot_sync(0xffffffffu, v[w] >= 0);
+         }
+         if(lane == 0)
+#pragma unroll
+            for(int w = 0; w < NWORD; w++)
+               if(have[w]) atomicOr(&present[w], have[w]);
          __syncthreads();
-         runStep<T, 1>(task, nTask[0], warp, NW, lane, D, W0, W1);
+         if(warp == 0)
+         {
+            // the operators present, in order
+            int base = 0;
+            for(int w = 0; w * 32 < NOP; w++)
+            {
+               const uint32_t bits = present[w];
+               if(bits >> lane & 1) offs[base + __popc(bits & ((1u << lane) - 1))] = 32 * w + lane;
+               base += __popc(bits);
+            }
+            if(lane == 0) nOffS = base;
+         }
          __syncthreads();
-         runStep<T, 1>(task + MAXTASK, nTask[1], warp, NW, lane, D, W1, W0);
-         __syncthreads();
-         runStep<T, 1>(task + 2 * MAXTASK, nTask[2], warp, NW, lane, D, W0, W1);
-         __syncthreads();
-         turn<T, 1>(pairs, nTurn, warp, NW, lane, Z, W1, true);
+         const int nOff = nOffS, parts = gridDim.y, part = blockIdx.y;
+         o0 = int(int64_t(nOff) * part / parts);
+         o1 = int(int64_t(nOff) * (part + 1) / parts);
+         toParts = parts > 1;
       }
-      // the next chunk
-      prevRows = nr;
-      chunk++;
-      c0 += CH;
-      if(c0 >= nPairs)
+      // source of the tile's box t for operator o
+      auto sourceOf = [&](int t, int o) {
+         if(t >= nTile) return -1;
+         return vtab[int64_t(tileNode[t]) * NOP + o];
+      };
+      // warp 0: the pairs of operator oi, compacted; the sources were loaded one operator earlier
+      constexpr int AH = (MAXT + 31) / 32;
+      int ahead[AH];
+      auto loadAhead = [&](int oi) {
+#pragma unroll
+         for(int h = 0; h < AH; h++) ahead[h] = sourceOf(lane + 32 * h, offs[oi]);
+      };
+      auto compact = [&](int b) {
+         int n = 0;
+#pragma unroll
+         for(int h = 0; h < AH; h++)
+         {
+            const uint32_t bits = __ballot_sync(0xffffffffu, ahead[h] >= 0);
+            if(ahead[h] >= 0)
+            {
+               const int k = n + __popc(bits & ((1u << lane) - 1));
+               slotT[b][k] = lane + 32 * h;
+               slotS[b][k] = ahead[h];
+            }
+            n += __popc(bits);
+         }
+         if(lane == 0) nSlot[b] = n;
+      };
+      T* out = !toParts ? Y : ws + (MODE == 0 ? int64_t(blockIdx.x) * TT : int64_t(blockIdx.y) * nTargets + first) * 3 * Lp;
+      if(MODE == 0 && toParts)
       {
-         c0 = 0;
-         b ^= 1;
-         if(++oi < o1) nPairs = nSlot[b];
+         for(int e = tid; e < 3 * nTile * Lp; e += NT) out[e] = T(0);
+         __syncthreads();
       }
-      if(oi < o1)
+      if(o0 < o1)
       {
-         nr = 3 * min(CH, nPairs - c0);
-         setRows(b, c0, nr, chunk & 1);
+         // the rows of X a chunk's vectors come from and the rows of Y (or of this part's sums) they are added to
+         auto setRows = [&](int b, int c0, int nr, int db) {
+            if(tid < nr)
+            {
+               const int t = c0 + tid / 3, cmp = tid % 3;
+               srcRow[db][tid] = 3 * slotS[b][t] + cmp;
+               dstRow[db][tid] = 3 * (MODE == 2 ? tileNode[t] : toParts ? slotT[b][t] : tileNode[slotT[b][t]]) + cmp;
+            }
+         };
+         // Gather: element copies that all stay in flight while the previous chunk's sums are added, 8 consecutive
+         // coefficients (a 32-byte sector in FP32) of 4 rows a warp.
+         const int nk8 = (L + 7) >> 3, k8 = lane & 7, r4 = lane >> 3;
+         auto gather = [&](const int* rows, int nr) {
+            const int nq = (nr + 3) >> 2;
+            for(int j = warp; j < nk8; j += NW)
+            {
+               const int k = 8 * j + k8;
+               if(k >= L) continue;
+               T* w = W0 + int(pos[k]) * RS + r4;
+               const T* src = X + k;
+#pragma unroll 4
+               for(int q = 0; q < nq; q++)
+                  if(4 * q + r4 < nr) cpAsyncElem(w + 4 * q, src + int64_t(rows[4 * q + r4]) * Lp);
+            }
+         };
+         // Sums: 4 lanes of V consecutive coefficients by 8 rows a warp and item, BT items' loads in flight together.
+         const int kl = V * (lane & 3), rl = lane >> 2, nkb = (Lp + 4 * V - 1) / (4 * V);
+         typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type VT;
+         constexpr int BT = MODE == 0 ? 5 : 4;
+         auto addOut = [&](int db, int nr) {
+            const int* rows = dstRow[db];
+            const int nItems = nkb * ((nr + 7) >> 3);
+            for(int i0 = warp; i0 < nItems; i0 += BT * NW)
+            {
+               VT y[BT], id[BT];
+               T* q[BT];
+#pragma unroll
+               for(int h = 0; h < BT; h++)
+               {
+                  const int it = i0 + h * NW, r = 8 * (it / nkb) + rl, k = 4 * V * (it % nkb) + kl;
+                  q[h] = nullptr;
+                  if(it < nItems && r < nr)
+                  {
+                     q[h] = out + int64_t(rows[r]) * Lp + k;
+                     y[h] = *reinterpret_cast<const VT*>(q[h]);
+                     if(MODE != 0) id[h] = *reinterpret_cast<const VT*>(X + int64_t(srcRow[db][r]) * Lp + k);
+                  }
+               }
+#pragma unroll
+               for(int h = 0; h < BT; h++)
+               {
+                  if(!q[h]) continue;
+                  const int it = i0 + h * NW, r = 8 * (it / nkb) + rl, k = 4 * V * (it % nkb) + kl;
+                  T* ys = reinterpret_cast<T*>(&y[h]);
+#pragma unroll
+                  for(int i = 0; i < V; i++)
+                  {
+                     const int w = pos[k + i];
+                     if(w == 0xFFFF) continue;
+                     T v = W1[w * RS + r];
+                     if(MODE != 0) v = fma(reinterpret_cast<const T*>(&id[h])[i], boxScale<T>(k + i, MODE == 2), v);
+                     ys[i] += v;
+                  }
+                  *reinterpret_cast<VT*>(q[h]) = y[h];
+               }
+            }
+         };
+         if(MODE != 2 && warp == 0)
+         {
+            loadAhead(o0);
+            compact(0);
+            if(o0 + 1 < o1) loadAhead(o0 + 1);
+         }
+         __syncthreads();
+         int oi = o0, b = 0, c0 = 0, nPairs = nSlot[0], nr = 3 * min(CH, nPairs), prevRows = 0, chunk = 0;
+         setRows(0, 0, nr, 0);
+         __syncthreads();
+         const T* Z = D + B.zOff;
+         const int nTurn = p * (p + 1) / 2;
+         while(true)
+         {
+            if(c0 == 0)
+            {
+               const T* src = ops + int64_t(offs[oi]) * B.size;
+               for(int e = tid * V; e < B.size; e += NT * V) cpAsync16(D + e, src + e);
+               asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            gather(srcRow[chunk & 1], nr);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if(chunk) addOut((chunk - 1) & 1, prevRows);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if(MODE != 2 && c0 == 0 && warp == 0 && oi + 1 < o1)
+            {
+               compact(b ^ 1);
+               if(oi + 2 < o1) loadAhead(oi + 2);
+            }
+            for(int e = tid; e < pads[MAXORDER + 1] * RS; e += NT) W1[pads[e / RS] * RS + e % RS] = T(0);
+            if(nr > 8 * V)
+            {
+               turn<T, 2>(pairs, nTurn, warp, NW, lane, Z, W0, false);
+               __syncthreads();
+               runStep<T, 2>(task, nTask[0], warp, NW, lane, D, W0, W1);
+               __syncthreads();
+               runStep<T, 2>(task + MAXTASK, nTask[1], warp, NW, lane, D, W1, W0);
+               __syncthreads();
+               runStep<T, 2>(task + 2 * MAXTASK, nTask[2], warp, NW, lane, D, W0, W1);
+               __syncthreads();
+               turn<T, 2>(pairs, nTurn, warp, NW, lane, Z, W1, true);
+            }
+            else
+            {
+               // at most one group of rows
+               turn<T, 1>(pairs, nTurn, warp, NW, lane, Z, W0, false);
+               __syncthreads();
+               runStep<T, 1>(task, nTask[0], warp, NW, lane, D, W0, W1);
+               __syncthreads();
+               runStep<T, 1>(task + MAXTASK, nTask[1], warp, NW, lane, D, W1, W0);
+               __syncthreads();
+               runStep<T, 1>(task + 2 * MAXTASK, nTask[2], warp, NW, lane, D, W0, W1);
+               __syncthreads();
+               turn<T, 1>(pairs, nTurn, warp, NW, lane, Z, W1, true);
+            }
+            // the next chunk
+            prevRows = nr;
+            chunk++;
+            c0 += CH;
+            if(c0 >= nPairs)
+            {
+               c0 = 0;
+               b ^= 1;
+               if(++oi < o1) nPairs = nSlot[b];
+            }
+            if(oi < o1)
+            {
+               nr = 3 * min(CH, nPairs - c0);
+               setRows(b, c0, nr, chunk & 1);
+            }
+            __syncthreads();
+            if(oi >= o1) break;
+         }
+         addOut((chunk - 1) & 1, prevRows);
       }
+      // the block's next tile
+      if(MODE != 0) break;
+      int next = first / TT;
+      if(next < tileOps.whole)
+      {
+         next += gridDim.x;
+         if(next >= tileOps.whole) next = tileOps.whole < tileOps.tiles ? shareTile() : tileOps.tiles;
+      }
+      else if(++next < tileOps.tiles && tileOps.start[next] >= tileOps.share[blockIdx.x + 1]) next = tileOps.tiles;
+      if(next >= tileOps.tiles) break;
+      first = next * TT;
+      nTile = min(TT, end - first);
       __syncthreads();
-      if(oi >= o1) break;
    }
-   addOut((chunk - 1) & 1, prevRows);
 }
 
 // Y of every target row = the parts' sums in order.
@@ -875,13 +1100,11 @@ fmm_status ensureRotations(Plan& P, cudaStream_t st)
    return FMM_OK;
 }
 
-// Boxes of a tile, into how many parts the operators of a tile are split (a part is a block; their sums meet in
-// kSumParts), and the block's threads. An M2L tile has five chunks' boxes (FP64: six): an operator has partners for about half of
-// them, so its chunks are mostly full (tiles of one chunk: M2L of 2^19 points and targets, p = 12, 9.3 ms, of five 7.5;
-// FP64, 131,072, p = 12, 4.3 and 3.6). Parts: eight rounds of resident blocks (four: 8.3 and 3.6 ms), so that small trees
-// fill the chip and larger ones have no long last round. Threads: 16 warps an SM (the registers' limit) as two blocks,
-// from p = 13 on as one; for the M2L blocks of 4 warps where three or four fit, p <= 9 in FP32 (8 warps a block at p = 4: 2.4 ms,
-// 4 warps 1.7; at p = 8 4.3 and 3.9; at p = 10, where two fit, 6.0 and 7.4).
+// Boxes of a tile, the blocks of a launch and their threads. An M2L tile has five chunks' boxes (FP64: six): an operator
+// has partners for about half of them, so its chunks are mostly full (tiles of one chunk: M2L of 2^19 points and
+// targets, p = 12, 9.3 ms, of five 7.5; FP64, 131,072, p = 12, 4.3 and 3.6). Threads: 16 warps an SM (the registers' limit)
+// as two blocks, from p = 13 on as one; for the M2L blocks of 4 warps where three or four fit, p <= 9 in FP32 (8 warps a block at
+// p = 4: 2.4 ms, 4 warps 1.7; at p = 8 4.3 and 3.9; at p = 10, where two fit, 6.0 and 7.4).
 template <class T> static int rotTile(int mode) { return rot::chunkPairs<T>() * (mode == 0 ? (sizeof(T) == 8 ? 6 : 5) : 1); }
 template <class T>
 static int rotPerSM(const Plan& P, int mode)
@@ -889,28 +1112,78 @@ static int rotPerSM(const Plan& P, int mode)
    const int fit = (227 * 1024) / (rot::Smem<T>(P.p).total + 6 * 1024);
    return fit >= 3 && mode == 0 ? std::min(fit, 4) : (fit >= 2 ? 2 : 1);
 }
-template <class T>
-static int rotParts(const Plan& P, int mode, int count)
+template <class T> static int rotTiles(int mode, int count) { return (count + rotTile<T>(mode) - 1) / rotTile<T>(mode); }
+template <class T> static int rotThreads(const Plan& P, int mode)
 {
-   const int tile = rotTile<T>(mode), tiles = (count + tile - 1) / tile;
-   if(tiles == 0) return 1;
-   return std::max(1, std::min(mode == 0 ? 64 : 8, 8 * 148 * rotPerSM<T>(P, mode) / tiles));
+   const int perSM = rotPerSM<T>(P, mode);
+   return perSM >= 3 ? 128 : 512 / perSM;
+}
+// M2L: the blocks of a launch, all resident at once (fewer in trees of a few tiles: 64 a tile)
+template <class T> static int rotBlocks(Plan& P, int tiles)
+{
+   if(P.rotResident == 0)
+   {
+      auto kern = rot::kRotTranslate<T, 0>;
+      const int smem = rot::Smem<T>(P.p).total;
+      int n = 0;
+      if(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, rotThreads<T>(P, 0), smem) != cudaSuccess)
+         cudaGetLastError();
+      P.rotResident = std::max(1, n);
+   }
+   return std::min(148 * P.rotResident, 64 * tiles);
+}
+// M2M: parts of a tile's operators, four rounds of blocks
+template <class T>
+static int rotParts(const Plan& P, int count)
+{
+   const int tiles = rotTiles<T>(1, count);
+   return tiles ? std::max(1, std::min(8, 4 * 148 * rotPerSM<T>(P, 1) / tiles)) : 1;
+}
+template <class T> static size_t rotRowBytes(const Plan& P) { return sizeof(T) * 3 * size_t(P.Lp); }
+
+// The M2L's tile lists in rotTiles. The last one to two rounds of tiles are shared, those before them whole (half a round to one
+// and a half: 2^19 points, p = 16, 15.3 ms against 13.8, as blocks whose whole tiles exceed the mean get no share).
+template <class T> static rot::TileOps rotTileOps(Plan& P)
+{
+   rot::TileOps o;
+   o.tiles = rotTiles<T>(0, P.nM2LTargets);
+   o.blocks = rotBlocks<T>(P, o.tiles);
+   o.whole = std::max(0, o.tiles / o.blocks - 1) * o.blocks;
+   o.start = (int64_t*)P.rotTiles.ptr;
+   o.share = o.start + o.tiles + 1;
+   o.before = (int*)(o.share + o.blocks + 1);
+   o.n = o.before + size_t(o.tiles) * 316;
+   o.op = (unsigned short*)(o.n + o.tiles);
+   return o;
 }
 
-// Room for the parts' sums of every launch on the current tree, so that none of them allocates.
+// What the launches on the current tree need, so that none of them allocates: the M2L's tile lists and room for the blocks' and
+// parts' sums, at most 75 MB whatever the tree and order. Without that room the M2L takes a block per tile and the M2M does not
+// split, which is slower but needs none.
 template <class T>
-fmm_status reserveRotations(Plan& P)
+fmm_status reserveRotations(Plan& P, cudaStream_t st)
 {
    const bool tc = !P.fp64 && P.cfg.m2l_mode != FMM_M2L_SIMT;   // M2L (and M2M) on the tensor cores
    if(tc && P.tcTranslations(1)) return FMM_OK;
-   size_t rows = 0;
-   auto need = [&](int mode, int count) {
-      const int parts = rotParts<T>(P, mode, count);
-      if(parts > 1) rows = std::max(rows, size_t(parts) * 3 * size_t(count));
-   };
-   if(!tc) need(0, P.nM2LTargets);
-   for(int level = 0; level + 1 < P.tree.nLevels; level++) need(1, P.parStart[level + 1] - P.parStart[level]);
-   return rows ? P.rotWs.reserve(sizeof(T) * rows * P.Lp) : FMM_OK;
+   size_t bytes = 0;
+   if(!tc && P.nM2LTargets > 0)
+   {
+      const int tiles = rotTiles<T>(0, P.nM2LTargets), blocks = rotBlocks<T>(P, tiles);
+      FMM_TRY(P.rotTiles.reserve(size_t(tiles) * (8 + 4 + 316 * 6) + 8 * size_t(blocks + 2)));
+      const rot::TileOps ops = rotTileOps<T>(P);
+      rot::kTileOps<T><<<tiles, rot::TILEOPS_NT, 0, st>>>((const int*)P.m2lTargets.ptr, P.nM2LTargets, P.lists.vtab, rotTile<T>(0),
+                                                              P.p, ops, (unsigned*)P.err + 2);
+      FMM_TRY(launched(P, "kTileOps", st));
+      bytes = rotRowBytes<T>(P) * rotTile<T>(0) * blocks;
+   }
+   for(int level = 0; level + 1 < P.tree.nLevels; level++)
+   {
+      const int count = P.parStart[level + 1] - P.parStart[level], parts = rotParts<T>(P, count);
+      if(parts > 1) bytes = std::max(bytes, rotRowBytes<T>(P) * parts * size_t(count));
+   }
+   if(bytes && P.rotShared && P.rotWs.reserve(bytes) != FMM_OK) cudaGetLastError();
+   return FMM_OK;
 }
 
 template <class T, int MODE>
@@ -919,7 +1192,7 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
 {
    const rot::Blob B(P.p);
    const size_t smem = rot::Smem<T>(P.p).total;
-   const int perSM = rotPerSM<T>(P, MODE), THREADS = perSM >= 3 ? 128 : 512 / perSM;
+   const int THREADS = rotThreads<T>(P, MODE);
    auto kern = rot::kRotTranslate<T, MODE>;
    FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
    const T* ops = (const T*)P.rotOps.ptr + size_t(B.size) * (MODE == 0 ? 16 : MODE == 1 ? 0 : 8);
@@ -930,19 +1203,35 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
       // up to eight chunks a block, which loads the octant's tables once, while that leaves four rounds of blocks
       const int chunk = rot::chunkPairs<T>(), all = seg.start[8] - seg.start[0];
       const int tl = chunk * std::max(1, std::min(rot::MAXTL / chunk, all / (chunk * 4 * 148 * rotPerSM<T>(P, MODE))));
-      kern<<<dim3((most + tl - 1) / tl, 1, 8), THREADS, smem, st>>>(targets, 0, nullptr, P.tree.parent, seg, tl, P.p, P.Lp,
-                                                                   tasks, ops, X, Y, nullptr);
+      kern<<<dim3((most + tl - 1) / tl, 1, 8), THREADS, smem, st>>>(targets, 0, nullptr, P.tree.parent, seg, rot::TileOps{}, tl, P.p,
+                                                                   P.Lp, tasks, ops, X, Y, nullptr);
       return launched(P, "kRotTranslate<L2L>", st);
    }
-   const int tiles = (count + tile - 1) / tile, parts = rotParts<T>(P, MODE, count);
+   const int tiles = rotTiles<T>(MODE, count);
+   T* ws = (T*)P.rotWs.ptr;
+   if(MODE == 0)
+   {
+      rot::TileOps tileOps = rotTileOps<T>(P);
+      if(P.rotWs.bytes < rotRowBytes<T>(P) * tile * tileOps.blocks) tileOps.whole = tileOps.blocks = tiles;
+      kern<<<tileOps.blocks, THREADS, smem, st>>>(targets, count, vtab, P.tree.parent, seg, tileOps, tile, P.p, P.Lp, tasks, ops, X, Y,
+                                                  ws);
+      FMM_TRY(launched(P, "kRotTranslate<M2L>", st));
+      const int shared = tiles - tileOps.whole;
+      if(shared == 0) return FMM_OK;
+      rot::kAddParts<T><<<dim3(shared, std::max(8, std::min(tile, 4736 / shared))), 256, 0, st>>>(targets, count, tile, tileOps, P.Lp, ws,
+                                                                                                Y);
+      return launched(P, "kAddParts", st);
+   }
    const int64_t n = 3 * int64_t(count) * P.Lp;
-   if(parts > 1) FMM_CUDA(cudaMemsetAsync(P.rotWs.ptr, 0, sizeof(T) * size_t(parts) * n, st));
-   kern<<<dim3(tiles, parts), THREADS, smem, st>>>(targets, count, vtab, P.tree.parent, seg, tile, P.p, P.Lp, tasks, ops, X, Y,
-                                                   (T*)P.rotWs.ptr);
-   FMM_TRY(launched(P, MODE == 0 ? "kRotTranslate<M2L>" : "kRotTranslate<M2M>", st));
+   int parts = rotParts<T>(P, count);
+   if(P.rotWs.bytes < sizeof(T) * size_t(parts) * n) parts = 1;
+   if(parts > 1) FMM_CUDA(cudaMemsetAsync(ws, 0, sizeof(T) * size_t(parts) * n, st));
+   kern<<<dim3(tiles, parts), THREADS, smem, st>>>(targets, count, vtab, P.tree.parent, seg, rot::TileOps{}, tile, P.p, P.Lp, tasks,
+                                                   ops, X, Y, ws);
+   FMM_TRY(launched(P, "kRotTranslate<M2M>", st));
    if(parts > 1)
    {
-      rot::kSumParts<T><<<int((n + 255) / 256), 256, 0, st>>>(targets, count, parts, P.Lp, (const T*)P.rotWs.ptr, Y);
+      rot::kSumParts<T><<<int((n + 255) / 256), 256, 0, st>>>(targets, count, parts, P.Lp, ws, Y);
       FMM_TRY(launched(P, "kSumParts", st));
    }
    return FMM_OK;
@@ -988,8 +1277,8 @@ fmm_status rotL2L(Plan& P, cudaStream_t st)
 
 template fmm_status ensureRotations<float>(Plan&, cudaStream_t);
 template fmm_status ensureRotations<double>(Plan&, cudaStream_t);
-template fmm_status reserveRotations<float>(Plan&);
-template fmm_status reserveRotations<double>(Plan&);
+template fmm_status reserveRotations<float>(Plan&, cudaStream_t);
+template fmm_status reserveRotations<double>(Plan&, cudaStream_t);
 template fmm_status rotM2L<float>(Plan&, cudaStream_t);
 template fmm_status rotM2L<double>(Plan&, cudaStream_t);
 template fmm_status rotM2M<float>(Plan&, cudaStream_t);

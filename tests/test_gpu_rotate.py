@@ -75,3 +75,59 @@ def test_degree_cutoff_is_the_tensor_cores(p, precision, cutoff):
                       m2l_degree_cutoff={"p": p, "p + 1": p + 1, "2 p": 2 * p, "none": -1}[cutoff])
     assert st["v_pairs"] > 0
     np.testing.assert_array_equal(cut, full)
+
+
+def memory_used(plan_args, xyz, w, J, tgt):
+    """Device memory a plan with a solve behind it holds, beyond its first solve of a little problem."""
+    import torch
+    plan = Plan(**plan_args)
+    plan.set_sources(xyz[:64], w[:64], J[:64])
+    plan.set_targets(tgt[:64])
+    plan.solve(1.0, 1)
+    free = torch.cuda.mem_get_info()[0]
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    plan.solve(1.0, 1)
+    torch.cuda.synchronize()
+    used = free - torch.cuda.mem_get_info()[0]
+    plan.close()
+    return used
+
+
+@pytest.mark.parametrize("p,n,leaf,precision", [(3, 250007, 2, "fp32"), (3, 150001, 2, "fp64"), (13, 60013, 3, "fp32"),
+                                                (13, 40009, 3, "fp64"), (9, 30011, 4, "fp32"), (16, 9001, 20, "fp64")])
+def test_whole_and_shared_tiles(monkeypatch, p, n, leaf, precision):
+    """Trees from a few tiles to several rounds of blocks (whole tiles, shared ones, parents and children in more tiles
+    than blocks): the same sums with every tile a block's own, and the direct sum at some targets."""
+    rng = np.random.default_rng(n)
+    dt = np.float32 if precision == "fp32" else np.float64
+    # uneven density, so that the tiles' operators differ
+    xyz = np.concatenate([rng.uniform(-1, 1, (n - n // 3, 3)), rng.normal(size=(n // 3, 3)) * 0.1 + 0.5]).astype(dt)
+    w, J = rng.uniform(0.5, 1.5, n).astype(dt), rng.normal(size=(n, 3)).astype(dt)
+    tgt = np.concatenate([xyz[::2] + dt(0.001), rng.uniform(-1, 1, (n // 2, 3)).astype(dt)]).astype(dt)
+    (B, A), st = solve(p, leaf, precision, xyz, w, J, tgt)
+    monkeypatch.setenv("FMM_ROT_SHARED", "0")
+    (Bo, Ao), _ = solve(p, leaf, precision, xyz, w, J, tgt)
+    # the same terms in another order: ~1e3 of them, 2^-24 (2^-53) each
+    tol = 1e-5 if precision == "fp32" else 1e-13
+    assert rel(B, Bo) < tol and rel(A, Ao) < tol
+    pick = rng.choice(len(tgt), 50, replace=False)
+    plan = Plan(order=2, precision=precision)
+    plan.set_sources(xyz, w, J)
+    D = plan.direct_fp64(tgt[pick])
+    plan.close()
+    assert rel(B[pick], D) < {3: 5e-2, 9: 2e-3, 13: 2e-4, 16: 1e-4}[p]
+
+
+@pytest.mark.parametrize("p,precision", [(9, "fp32"), (12, "fp32"), (9, "fp64"), (16, "fp64")])
+def test_scratch_is_bounded(monkeypatch, p, precision):
+    """The room for split sums: at most 75 MB beside what the plan needs without them (16 MB for the granularity of
+    allocations)."""
+    rng = np.random.default_rng(p)
+    n = 60000
+    xyz, w, J = rng.uniform(-1, 1, (n, 3)), rng.uniform(0.5, 1.5, n), rng.normal(size=(n, 3))
+    args = dict(order=p, leaf_capacity=20, precision=precision)
+    with_room = memory_used(args, xyz, w, J, xyz)
+    monkeypatch.setenv("FMM_ROT_SHARED", "0")
+    without = memory_used(args, xyz, w, J, xyz)
+    assert with_room - without < (75 + 16) << 20
