@@ -228,7 +228,6 @@ struct Plan
    DevBuf rotOps, rotQuarter, rotTasks, rotTiles, rotWs;
    std::vector<unsigned char> rotTaskHost;   // host copy of rotTasks (kept for the asynchronous upload)
    int rotCut = -1;
-   int rotShared = 1;                    // 0: as if there were no room for those sums
    int rotResident = 0;                  // blocks of the M2L an SM holds (0: not asked yet)
    // tensor-core M2L tile choices (autotuned per order and leaf capacity, or set by environment)
    int tcKChunk = 0;                     // K chunk width 32 or 64 (0: 64 for BF16X3, 32 for BF16X6)
@@ -325,6 +324,16 @@ struct Plan
       return FMM_OK;
    }
 
+   // Room that a faster form of a phase needs and its plain form does not: false when there is none (out of memory, or
+   // splitSums = 0, as if), and the plain form runs.
+   int splitSums = 1;
+   bool roomFor(DevBuf& b, size_t bytes)
+   {
+      if(splitSums && b.reserve(bytes) == FMM_OK) return true;
+      cudaGetLastError();
+      return false;
+   }
+
    fmm_status init(const fmm_config& c);
    void release();
    fmm_status ensureNodes(int64_t cap, cudaStream_t st = 0);
@@ -347,6 +356,7 @@ inline fmm_status launched(Plan& P, const char* name, cudaStream_t st)
 template <class T> fmm_status buildTreeT(Plan& P, cudaStream_t st);
 template <class T> fmm_status packSourcesT(Plan& P, cudaStream_t st);   // sPos, sQ in input order, coil segments uploaded
 int nearParts(const Plan& P);         // blocks a leaf's direct list is split into
+inline size_t nearPartBytes(const Plan& P, int parts) { return sizeof(double) * 6 * size_t(parts) * size_t(P.m); }
 template <class T> fmm_status upwardT(Plan& P, cudaStream_t st);
 template <class T> fmm_status downwardT(Plan& P, cudaStream_t st);
 template <class T> fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st);

@@ -1609,8 +1609,8 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
       else FMM_TRY(runL2P(kL2PWarp<T, false>, l2pWarpSmem<T, false>(P.p)));
       FMM_TRY(launched(P, "kL2PWarp", st));
    }
-   const int parts = split ? nearParts(P) : 1;
-   if(parts > 1) FMM_TRY(P.nearPart.reserve(sizeof(double) * 6 * size_t(parts) * size_t(P.m)));
+   int parts = split ? nearParts(P) : 1;
+   if(P.nearPart.bytes < nearPartBytes(P, parts)) parts = 1;   // (reserved at tree build)
    auto run = [&](auto kernel) -> fmm_status {
       FMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
       kernel<<<dim3(int(N), parts), NT, shm, st>>>(P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr,
@@ -1651,8 +1651,8 @@ static fmm_status launchDirect(Plan& P, DevBuf& partBuf, int coils, int maxT, in
    const int blocks = (maxT + NT - 1) / NT;
    if(blocks == 0) return FMM_OK;
    const int64_t wantParts = (8 * 148 + int64_t(blocks) * coils - 1) / (int64_t(blocks) * coils);
-   const int parts = int(std::max<int64_t>(1, std::min<int64_t>(wantParts, maxS / 512)));
-   if(parts > 1) FMM_TRY(partBuf.reserve(sizeof(U) * 6 * size_t(parts) * size_t(m)));
+   int parts = int(std::max<int64_t>(1, std::min<int64_t>(wantParts, maxS / 512)));
+   if(parts > 1 && !P.roomFor(partBuf, sizeof(U) * 6 * size_t(parts) * size_t(m))) parts = 1;
    U* part = (U*)partBuf.ptr;
    auto run = [&](auto kern) {
       kern<<<dim3(blocks, coils, parts), NT, 0, st>>>((const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, int(P.n), tgt, m, sseg, tseg,

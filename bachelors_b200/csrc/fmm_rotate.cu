@@ -1182,7 +1182,7 @@ fmm_status reserveRotations(Plan& P, cudaStream_t st)
       const int count = P.parStart[level + 1] - P.parStart[level], parts = rotParts<T>(P, count);
       if(parts > 1) bytes = std::max(bytes, rotRowBytes<T>(P) * parts * size_t(count));
    }
-   if(bytes && P.rotShared && P.rotWs.reserve(bytes) != FMM_OK) cudaGetLastError();
+   if(bytes) P.roomFor(P.rotWs, bytes);
    return FMM_OK;
 }
 

@@ -1544,7 +1544,7 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
    }
    // room for split sums, so that no later phase allocates
    const int parts = nearParts(P);
-   if(parts > 1) FMM_TRY(P.nearPart.reserve(sizeof(double) * 6 * size_t(parts) * size_t(m)));
+   if(parts > 1) P.roomFor(P.nearPart, nearPartBytes(P, parts));
    return reserveRotations<T>(P, st);
 }
 

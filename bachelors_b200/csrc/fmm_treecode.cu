@@ -463,17 +463,20 @@ fmm_status treecodeT(Plan& P, double current, int want, const void* pts, int64_t
    int W = 1;
    while(W < 32 && 2 * W <= dense && m / (2 * W) >= 2 * 148) W *= 2;
    const int* order = nullptr;
+   size_t tmp = 0;
+   unsigned* k = nullptr;
    if(W > 1)
    {
-      // keys, sorted keys, indexes, sorted indexes
-      FMM_TRY(P.tcSort.reserve(sizeof(unsigned) * 4 * size_t(m)));
-      unsigned* k = (unsigned*)P.tcSort.ptr;
+      // keys, sorted keys, indexes, sorted indexes, then the sort's scratch; without room for them every point walks alone
+      cub::DeviceRadixSort::SortPairs(nullptr, tmp, k, k, (int*)nullptr, (int*)nullptr, int(m), 0, 30, st);
+      if(!P.roomFor(P.tcSort, sizeof(unsigned) * 4 * size_t(m)) || !P.roomFor(P.cubTmp, tmp)) W = 1;
+   }
+   if(W > 1)
+   {
+      k = (unsigned*)P.tcSort.ptr;
       int* ix = (int*)(k + 2 * m);
       kQueryKeys<T><<<int((m + 255) / 256), 256, 0, st>>>((const T*)pts, m, P.root, k, ix);
       FMM_TRY(launched(P, "kQueryKeys", st));
-      size_t tmp = 0;
-      cub::DeviceRadixSort::SortPairs(nullptr, tmp, k, k + m, ix, ix + m, int(m), 0, 30, st);
-      FMM_TRY(P.cubTmp.reserve(tmp));
       tmp = P.cubTmp.bytes;
       FMM_CUDA(cub::DeviceRadixSort::SortPairs(P.cubTmp.ptr, tmp, k, k + m, ix, ix + m, int(m), 0, 30, st));
       order = ix + m;

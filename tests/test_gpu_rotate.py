@@ -106,7 +106,7 @@ def test_whole_and_shared_tiles(monkeypatch, p, n, leaf, precision):
     w, J = rng.uniform(0.5, 1.5, n).astype(dt), rng.normal(size=(n, 3)).astype(dt)
     tgt = np.concatenate([xyz[::2] + dt(0.001), rng.uniform(-1, 1, (n // 2, 3)).astype(dt)]).astype(dt)
     (B, A), st = solve(p, leaf, precision, xyz, w, J, tgt)
-    monkeypatch.setenv("FMM_ROT_SHARED", "0")
+    monkeypatch.setenv("FMM_SPLIT_SUMS", "0")
     (Bo, Ao), _ = solve(p, leaf, precision, xyz, w, J, tgt)
     # the same terms in another order: ~1e3 of them, 2^-24 (2^-53) each
     tol = 1e-5 if precision == "fp32" else 1e-13
@@ -128,6 +128,6 @@ def test_scratch_is_bounded(monkeypatch, p, precision):
     xyz, w, J = rng.uniform(-1, 1, (n, 3)), rng.uniform(0.5, 1.5, n), rng.normal(size=(n, 3))
     args = dict(order=p, leaf_capacity=20, precision=precision)
     with_room = memory_used(args, xyz, w, J, xyz)
-    monkeypatch.setenv("FMM_ROT_SHARED", "0")
+    monkeypatch.setenv("FMM_SPLIT_SUMS", "0")
     without = memory_used(args, xyz, w, J, xyz)
     assert with_room - without < (75 + 16) << 20
