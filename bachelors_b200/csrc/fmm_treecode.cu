@@ -25,8 +25,7 @@
 // harmonic). With a thread per point walking alone, evaluating value and gradient by dual numbers and reading
 // its boxes' multipoles itself, the few points near the sources kept their warps for the whole call. Measured, that ->
 // this, 262,144 sources, p = 10, FP32: leaves of 1000, 65,536 points 23.4 -> 2.65 ms, 1,000 points 16.6 -> 0.45 ms, one
-// point 0.39 -> 0.03 ms; leaves of 100, 65,536 points 11.5 -> 7.3 ms, 10,000 points 8.3 -> 3.6 ms; FP64, leaves of 1000,
-// 65,536 points 40 -> 3.2 ms.
+// point 0.39 -> 0.03 ms; leaves of 100, 65,536 points 11.5 -> 3.9 ms; FP64, leaves of 1000, 65,536 points 40 -> 3.5 ms.
 #include <cub/cub.cuh>
 
 #include "fmm_internal.cuh"
@@ -152,7 +151,7 @@ struct TcSmem
       farM = take(4 * TC_NT);
       nearN = take(4 * TC_NT);
       nearM = take(4 * TC_NT);
-      pts = take(8 * 3 * 32);
+      pts = take(8 * (3 * 32 + 2));
       src = take(8 * 8 * TC_SRC);            // also the warps' sums at the end: [TC_WARPS][32][6]
       warp0 = b;
       // per warp: the curl expansion [(p + 2)^2][4] and the potential's [(p + 1)^2][4]
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(TC_NT) kTreecode(Tree t, const RootBox* __rest
    unsigned* farM = reinterpret_cast<unsigned*>(smraw + sm.farM);
    int* nearN = reinterpret_cast<int*>(smraw + sm.nearN);
    unsigned* nearM = reinterpret_cast<unsigned*>(smraw + sm.nearM);
-   double* P = reinterpret_cast<double*>(smraw + sm.pts);       // [3][32]
+   double* P = reinterpret_cast<double*>(smraw + sm.pts);       // [3][32], then the root's side and its inverse
    double* S = reinterpret_cast<double*>(smraw + sm.src);       // [TC_SRC][8]
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    V4* Cs = reinterpret_cast<V4*>(smraw + sm.warp0 + warp * sm.perWarp);
@@ -200,6 +199,7 @@ __global__ void __launch_bounds__(TC_NT) kTreecode(Tree t, const RootBox* __rest
       for(int d = 0; d < 3; d++) P[32 * d + tid] = double(pts[3 * src + d]);
    }
    const RootBox rb = rootp[0];
+   if(tid == 0) { P[96] = 2.0 * rb.H; P[97] = 1.0 / (2.0 * rb.H); }
    const unsigned all = nq == 32 ? 0xffffffffu : (1u << nq) - 1u;
    int count = 0;
    for(int r = t.levelStart[0]; r < t.levelStart[1]; r++)
@@ -211,11 +211,15 @@ __global__ void __launch_bounds__(TC_NT) kTreecode(Tree t, const RootBox* __rest
    const double x = P[j], y = P[32 + j], z = P[64 + j];
    double A[3] = {0, 0, 0}, B[3] = {0, 0, 0};
    const T eps = T(1e-3);   // the reference's math::eps for the central differences
+   // (the side is the root's times a power of two, so neither it nor its inverse takes a division)
+   auto power2 = [](int e) { return __longlong_as_double((long long)(1023 + e) << 52); };
    auto centre = [&](int node, double& h, double& cx, double& cy, double& cz) {
-      h = 2.0 * rb.H / double(int64_t(1) << t.level[node]);
+      const int level = t.level[node];
+      h = P[96] * power2(-level);
       cx = rb.center[0] - rb.H + (double(t.ix[node]) + 0.5) * h;
       cy = rb.center[1] - rb.H + (double(t.iy[node]) + 0.5) * h;
       cz = rb.center[2] - rb.H + (double(t.iz[node]) + 0.5) * h;
+      return level;
    };
    while(count > 0)
    {
@@ -283,8 +287,8 @@ __global__ void __launch_bounds__(TC_NT) kTreecode(Tree t, const RootBox* __rest
             }
          __syncwarp();
          double h, cx, cy, cz;
-         centre(box, h, cx, cy, cz);
-         const double dx = x - cx, dy = y - cy, dz = z - cz, ih = 1.0 / h;
+         const double ih = P[97] * power2(centre(box, h, cx, cy, cz));
+         const double dx = x - cx, dy = y - cy, dz = z - cz;
          T b[3] = {T(0), T(0), T(0)}, a[3] = {T(0), T(0), T(0)};
          // (for m = 0 the imaginary part is zero, so its k1 = k0 term adds nothing)
          auto addA = [&](int k0, int k1, T re, T im) {
@@ -457,11 +461,19 @@ fmm_status treecodeT(Plan& P, double current, int want, const void* pts, int64_t
       FMM_CUDA(cudaMemcpyAsync(P.tcCurl.ptr, P.tcCurlHost.data(), bytes, cudaMemcpyHostToDevice, st));
       P.tcCurlOrder = P.p;
    }
-   // Points a block: as many as share a leaf's neighbourhood on average, so that a block's points want mostly the
-   // same boxes; few points, or points sparse among the leaves, walk alone (then a point has 256 threads).
-   const int64_t dense = m / std::max<int64_t>(1, P.tree.nNodes);
+   // Points a block (W): neighbours want mostly the same boxes, and a far box is prepared once for the block's points; few
+   // points, or points sparse among the boxes, walk alone (then a point has 256 threads). W grows while the block's
+   // points meet up to 32 times as many boxes and 592 blocks (2 points), 296 (4, 8), 1184 (16, 32) remain, or while every box has
+   // a point of its own and 296 blocks remain (few large leaves: the near sums fill the lanes). Measured over orders
+   // 1-16, leaves of 10-1000, 300-300,000 points, both precisions: on average within 3 % of the best W (the second
+   // condition alone 35 %), e.g. 65,536 points, 65,536 sources in leaves of 30, p = 10, FP32: W = 8 4.6 ms, 32 3.1.
+   const int64_t nodes = std::max<int64_t>(1, P.tree.nNodes);
    int W = 1;
-   while(W < 32 && 2 * W <= dense && m / (2 * W) >= 2 * 148) W *= 2;
+   auto grow = [&](int w) {
+      const int64_t blocks = m / w;
+      return (w <= 32 * m / nodes && blocks >= (w == 2 ? 592 : (w <= 8 ? 296 : 1184))) || (w <= m / nodes && blocks >= 296);
+   };
+   while(W < 32 && grow(2 * W)) W *= 2;
    const int* order = nullptr;
    size_t tmp = 0;
    unsigned* k = nullptr;

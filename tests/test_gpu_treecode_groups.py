@@ -80,3 +80,9 @@ def test_calls_on_two_streams(precision):
     assert all(idle)
     for a, b in zip(one, two):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("p,cap,m", [(1, 10, 40009), (5, 20, 20011), (9, 30, 1301)])
+def test_groups_over_many_boxes(p, cap, m):
+    """Groups larger than the points a box has: most boxes want few of a block's points."""
+    test_groups_equal_single_points(p, cap, m, {})
