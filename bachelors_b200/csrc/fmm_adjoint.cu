@@ -357,7 +357,7 @@ fmm_status adjointT(Plan& P, Plan& A, double current, const void* g, void* dJ, v
    const int p = A.p;
    const int L = nharm(p), L1 = nharm(p - 1), L2 = nharm(p >= 2 ? p - 2 : 0);
    size_t shm = ((sizeof(T) * (3 * L + 3 * L1 + 9 * L2) + 31) & ~size_t(31)) + 2 * sizeof(V4) * NT;
-   FMM_CUDA(cudaFuncSetAttribute(kAdjointEval<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+   FMM_CUDA(allowShared(kAdjointEval<T, NT>));
    const double scale = REF_MU0 / (4 * REF_PI) * current;
    kAdjointEval<T, NT><<<int(A.tree.nNodes), NT, shm, st>>>(
       A.tree, A.root, p, A.Lp, (const T*)A.local.ptr, (const V4*)A.tPos.ptr, (const V4*)A.sPos.ptr,

@@ -235,7 +235,7 @@ fmm_status bemP2MT(Plan& P, cudaStream_t st)
    typedef typename Vec4<T>::type V4;
    const int64_t N = P.tree.nNodes;
    const size_t shm = sizeof(double) * 3 * size_t(P.L) * BEM_P2M_WARPS;
-   FMM_CUDA(cudaFuncSetAttribute(kP2MBem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+   FMM_CUDA(allowShared(kP2MBem<T>));
    kP2MBem<T><<<int((N + BEM_P2M_WARPS - 1) / BEM_P2M_WARPS), 32 * BEM_P2M_WARPS, shm, st>>>(
       P.tree, P.root, P.p, P.Lp, (const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, (T*)P.mult.ptr);
    return launched(P, "kP2MBem", st);

@@ -90,6 +90,16 @@ void poolFree(void* ptr);
 cudaError_t pinnedWord(int** word);   // a page-locked host word, and back
 void pinnedWordFree(int* word);
 
+// Lets a kernel be launched with any dynamic shared memory up to SHARED_LIMIT (227 KB less room for its static part). The
+// attribute belongs to the process: set to each launch's own size, two threads' plans of different orders took each
+// other's away between the setting and the launch (cudaErrorInvalidValue), so it is the same whoever sets it.
+constexpr size_t SHARED_LIMIT = 227 * 1024 - 6 * 1024;
+template <class K>
+inline cudaError_t allowShared(K* kernel)
+{
+   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SHARED_LIMIT));
+}
+
 // A growable device allocation.
 struct DevBuf
 {

@@ -1508,7 +1508,7 @@ fmm_status upwardT(Plan& P, cudaStream_t st)
       auto kern = split ? kP2MWarp<T, true> : kP2MWarp<T, false>;
       const int warps = split ? P2MW_SPLIT_WARPS : P2MW_WARPS;
       const size_t shw = p2mWarpSmem<T>(P.p, Lp, warps);
-      if(shw > 48 * 1024) FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shw)));
+      if(shw > 48 * 1024) FMM_CUDA(allowShared(kern));
       // tensor-core M2M plans: the leaves' multipoles also leave as the M2M's operand pieces
       int np = 0;
       if(sizeof(T) == 4 && P.tcTranslations(1) && P.tcDrainMode != 0) np = m2mPieces(P);
@@ -1589,7 +1589,7 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
       // BEM: the far field sum_k L_k R_k (the A form of the L2P), then the BEM kernel's near field and
       // the 1 / (4 pi) of calcBEM (fast_multipole_solver.cpp:233-250; no current factor there)
       const size_t sh = l2pWarpSmem<T, true>(P.p);
-      if(sh > 48 * 1024) FMM_CUDA(cudaFuncSetAttribute(kL2PWarp<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh)));
+      if(sh > 48 * 1024) FMM_CUDA(allowShared(kL2PWarp<T, true>));
       kL2PWarp<T, true><<<walkBlocks(kL2PWarp<T, true>, 32 * L2PW_WARPS, sh, N), 32 * L2PW_WARPS, sh, st>>>(
          P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr, (const int*)P.tIdx.ptr,
          (const CurlEntry<T>*)P.curlTab.ptr, 2, (T*)P.outB.ptr, (T*)P.outA.ptr);
@@ -1599,7 +1599,7 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
    if(split)
    {
       auto runL2P = [&](auto kernel, size_t sh) -> fmm_status {
-         if(sh > 48 * 1024) FMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh)));
+         if(sh > 48 * 1024) FMM_CUDA(allowShared(kernel));
          kernel<<<walkBlocks(kernel, 32 * L2PW_WARPS, sh, N), 32 * L2PW_WARPS, sh, st>>>(
             P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr, (const int*)P.tIdx.ptr,
             (const CurlEntry<T>*)P.curlTab.ptr, want, (T*)P.outB.ptr, (T*)P.outA.ptr);
@@ -1612,7 +1612,7 @@ fmm_status evaluateT(Plan& P, double current, int want, cudaStream_t st)
    int parts = split ? nearParts(P) : 1;
    if(P.nearPart.bytes < nearPartBytes(P, parts)) parts = 1;   // (reserved at tree build)
    auto run = [&](auto kernel) -> fmm_status {
-      FMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+      if(shm > 48 * 1024) FMM_CUDA(allowShared(kernel));
       kernel<<<dim3(int(N), parts), NT, shm, st>>>(P.tree, P.root, P.p, P.Lp, (const T*)P.local.ptr, (const V4*)P.tPos.ptr,
                                       (const V4*)P.sPos.ptr, (const V4*)P.sQ.ptr, (const int*)P.p2pOff.ptr,
                                       (const int*)P.p2pList.ptr, (const int*)P.tIdx.ptr, scaleB, scaleA, want,

@@ -1126,7 +1126,7 @@ template <class T> static int rotBlocks(Plan& P, int tiles)
       auto kern = rot::kRotTranslate<T, 0>;
       const int smem = rot::Smem<T>(P.p).total;
       int n = 0;
-      if(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      if(allowShared(kern) != cudaSuccess ||
          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, rotThreads<T>(P, 0), smem) != cudaSuccess)
          cudaGetLastError();
       P.rotResident = std::max(1, n);
@@ -1194,7 +1194,7 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
    const size_t smem = rot::Smem<T>(P.p).total;
    const int THREADS = rotThreads<T>(P, MODE);
    auto kern = rot::kRotTranslate<T, MODE>;
-   FMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+   FMM_CUDA(allowShared(kern));
    const T* ops = (const T*)P.rotOps.ptr + size_t(B.size) * (MODE == 0 ? 16 : MODE == 1 ? 0 : 8);
    const rot::TaskTable* tasks = (const rot::TaskTable*)P.rotTasks.ptr + (MODE == 0 ? 0 : 1);
    const int tile = rotTile<T>(MODE);

@@ -494,11 +494,11 @@ void launchTranslateAll(T* r, const T* a, const T* b, int64_t count, int p, cuda
    // p = 13 78 81 (128) 88 80 (512); p = 16 106 122 (128) 127 123 (512); p = 19 134 179 (128) 190 178 (512); FP64: p = 13 85 91
    // (128) 98 90 (512).
    const int64_t few = p < 2 ? 2048 : (p < 13 ? 0 : 448);
-   if(count > few && seamItemsSmem<T>(L) <= 227 * 1024 && (count + SEAM_ITEMS - 1) / SEAM_ITEMS <= INT32_MAX)
+   if(count > few && seamItemsSmem<T>(L) <= SHARED_LIMIT && (count + SEAM_ITEMS - 1) / SEAM_ITEMS <= INT32_MAX)
    {
       const size_t smem = seamItemsSmem<T>(L);
       if(smem > 48 * 1024)
-         cudaFuncSetAttribute(kTranslateItems<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+         allowShared(kTranslateItems<T>);
       kTranslateItems<T><<<unsigned((count + SEAM_ITEMS - 1) / SEAM_ITEMS), 32 * SEAM_WARPS, smem, st>>>(r, a, b, count, p);
       return;
    }

@@ -494,7 +494,7 @@ fmm_status treecodeT(Plan& P, double current, int want, const void* pts, int64_t
       order = ix + m;
    }
    const TcSmem<T> sm(P.p, (want & 2) || (flags & 2));
-   FMM_CUDA(cudaFuncSetAttribute(kTreecode<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm.total));
+   FMM_CUDA(allowShared(kTreecode<T>));
    kTreecode<T><<<unsigned((m + W - 1) / W), TC_NT, sm.total, st>>>(
       P.tree, P.root, P.p, P.Lp, (const T*)P.mult.ptr, (const CurlTerm<T>*)P.tcCurl.ptr, (const V4*)P.sPos.ptr,
       (const V4*)P.sQ.ptr, (const T*)pts, order, m, W, flags, scaleB, scaleA, want, P.bem ? 1 : 0, (T*)outB, (T*)outA);
