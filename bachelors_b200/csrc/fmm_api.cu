@@ -65,7 +65,8 @@ DevicePool* devicePool()
       props.location.type = cudaMemLocationTypeDevice;
       props.location.id = dev;
       if(cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) { d.pool = nullptr; return; }
-      uint64_t keep = POOL_KEEP;
+      // (nothing is given back at synchronisations, which every allocation has one of: poolTrim does)
+      uint64_t keep = UINT64_MAX;
       if(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
          cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking) != cudaSuccess)
       {
@@ -116,7 +117,13 @@ cudaError_t poolAlloc(void** ptr, size_t bytes)
    DevicePool* d = devicePool();
    if(!d) return cudaErrorNotSupported;
    cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, d->pool, d->stream);
-   if(e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
+   if(e != cudaSuccess)
+   {
+      cudaGetLastError();
+      return e == cudaErrorMemoryAllocation ? e : cudaErrorNotSupported;
+   }
+   e = cudaStreamSynchronize(d->stream);
+   if(e != cudaSuccess) cudaFreeAsync(*ptr, d->stream);
    return e;
 }
 
@@ -124,6 +131,17 @@ void poolFree(void* ptr)
 {
    DevicePool* d = devicePool();
    if(d) cudaFreeAsync(ptr, d->stream);
+}
+
+void poolTrim(size_t keep)
+{
+   DevicePool* d = devicePool();
+   uint64_t reserved = 0, used = 0;
+   if(!d || cudaStreamSynchronize(d->stream) != cudaSuccess ||   // the frees of this and other threads so far
+      cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+      return;
+   if(reserved > used + keep) cudaMemPoolTrimTo(d->pool, used + keep);
 }
 
 fmm_status Plan::ensureNodes(int64_t cap, cudaStream_t st)
@@ -243,6 +261,7 @@ void Plan::release()
    for(DevBuf* b : bufs) b->release(true);
    for(auto& b : nodeBufs) b.release(true);
    for(auto& b : listBufs) b.release(true);
+   poolTrim(POOL_KEEP);
    if(hostErr) pinnedWordFree(hostErr);
    hostErr = nullptr;
    err = pipeErr = nullptr;
@@ -1331,8 +1350,8 @@ fmm_status fmm_add_vectors(const float* a, const float* b, float* c, int64_t n)
       if(e != cudaSuccess) s = setError(FMM_E_CUDA, "fmm_add_vectors: %s", cudaGetErrorString(e));
    }
    da.release();
-   db.release();
-   dc.release();
+   db.release(true);
+   dc.release(true);
    return s;
 }
 

@@ -79,14 +79,16 @@ extern __constant__ int d_m2lIndex[NOFF];   // offset index (0..342) -> M2L slot
 extern __constant__ int d_m2lOffset[316];   // M2L slot -> offset index
 extern __constant__ int d_m2lFarFirst[316]; // M2L slots by decreasing offset length
 
-// Small device blocks (up to POOL_BLOCK bytes) come from a memory pool of the library, one per device, which keeps at most
-// POOL_KEEP bytes of freed blocks for later plans (the driver returns the rest): a plan has about fifty of them, and
-// cudaMalloc and cudaFree took ~5 ms for each plan a call creates and drops. A block is handed out after its pool's stream
+// Small device blocks (up to POOL_BLOCK bytes) come from a memory pool of the library, one per device: a plan has about fifty
+// of them, and cudaMalloc and cudaFree took ~5 ms for each plan a call creates and drops. Beside the blocks in use the
+// pool keeps at most POOL_KEEP bytes of freed ones for later plans and buffers (poolTrim, after a plan's or a buffer's
+// release), and gives them all back before an allocation fails. A block is handed out after its pool's stream
 // has been waited for, so any stream may use it, and taken back after the device has been waited for (as cudaFree
 // does); the pool's own calls are safe from several threads. Larger blocks, and devices without memory pools, use cudaMalloc.
 constexpr size_t POOL_BLOCK = size_t(8) << 20, POOL_KEEP = size_t(128) << 20;
 cudaError_t poolAlloc(void** ptr, size_t bytes);   // cudaErrorNotSupported: no pool on the current device
 void poolFree(void* ptr);
+void poolTrim(size_t keep);   // gives freed blocks beyond `keep` bytes back to the device
 cudaError_t pinnedWord(int** word);   // a page-locked host word, and back
 void pinnedWordFree(int* word);
 
@@ -111,10 +113,18 @@ struct DevBuf
       if(want <= bytes) return FMM_OK;
       release();
       size_t b = std::max<size_t>(want, 256);
-      cudaError_t e = cudaErrorNotSupported;
-      if(b <= POOL_BLOCK) e = poolAlloc(&ptr, b);
-      pooled = e == cudaSuccess;
-      if(e == cudaErrorNotSupported) e = cudaMalloc(&ptr, b);
+      auto get = [&]() {
+         cudaError_t e = b <= POOL_BLOCK ? poolAlloc(&ptr, b) : cudaErrorNotSupported;
+         pooled = e == cudaSuccess;
+         return e == cudaErrorNotSupported ? cudaMalloc(&ptr, b) : e;
+      };
+      cudaError_t e = get();
+      if(e == cudaErrorMemoryAllocation)
+      {
+         cudaGetLastError();
+         poolTrim(0);
+         e = get();
+      }
       if(e != cudaSuccess)
       {
          cudaGetLastError();
@@ -131,6 +141,7 @@ struct DevBuf
       {
          if(!idle) cudaDeviceSynchronize();
          poolFree(ptr);
+         if(!idle && bytes >= (size_t(1) << 20)) poolTrim(POOL_KEEP);   // (small ones wait for the next)
       }
       else if(ptr) cudaFree(ptr);
       ptr = nullptr;
