@@ -75,16 +75,18 @@ __host__ __device__ inline int ordBase(int p, int m)   // first position of orde
 __host__ __device__ inline int ordPos(int p, int l, int m) { return ordBase(p, m) + l - (m < 0 ? -m : m); }
 __host__ __device__ inline int ordSize(int p) { return ordBase(p, p + 1); }
 
-// D^ of the quarter turn about x that takes e_z to e_y, degree blocks [2l+1][2l+1] one after the other, by
+// D^ of the quarter turn about x that takes e_z to e_y, degree blocks [2l+1][2l+1] up to degree p one after the other, by
 // integrating products of the orthonormal harmonics over the sphere (Gauss-Legendre x trapezoid, exact for
-// these degrees): R_i(Q x) against R_j(x).
+// these degrees): R_i(Q x) against R_j(x). A product of two harmonics of one degree is even, so the points below the
+// equator are left out. Made once for an order (p = 16 1 ms, p = 8 0.05).
 static int quarterOff(int l) { return l * (4 * l * l - 1) / 3; }   // sum of (2i+1)^2, i < l
-static const std::vector<double>& quarterTurn()
+static const std::vector<double>& quarterTurn(int p)
 {
-   static std::vector<double> tab;
-   static std::once_flag once;
-   std::call_once(once, [] {
-      const int p = MAXORDER, L = nharm(p), nz = p + 1, na = 2 * p + 1;
+   static std::vector<double> tabs[MAXORDER + 1];
+   static std::once_flag once[MAXORDER + 1];
+   std::vector<double>& tab = tabs[p];
+   std::call_once(once[p], [&] {
+      const int L = nharm(p), nz = p + 1, na = 2 * p + 2;
       // Gauss-Legendre nodes by Newton's method on P_nz
       std::vector<double> zs(nz), ws(nz);
       for(int i = 0; i < nz; i++)
@@ -140,14 +142,14 @@ static const std::vector<double>& quarterTurn()
       };
       tab.assign(quarterOff(p + 1), 0.0);
       std::vector<double> a(L), b(L);
-      for(int i = 0; i < nz; i++)
+      for(int i = 0; i < (nz + 1) / 2; i++)   // (the nodes come in decreasing order; an odd number's middle one is the equator)
          for(int j = 0; j < na; j++)
          {
             const double s = std::sqrt(1 - zs[i] * zs[i]), f = 2 * M_PI * j / na;
             const double x = s * std::cos(f), y = s * std::sin(f), z = zs[i];
             harm(x, y, z, b.data());
             harm(x, z, -y, a.data());   // Q x: e_z -> e_y, e_y -> -e_z
-            const double w = ws[i] * 2 * M_PI / na / (4 * M_PI);
+            const double w = ws[i] / (2 * i + 1 == nz ? 2 : 1) / na;
             for(int l = 0; l <= p; l++)
                for(int u = 0; u <= 2 * l; u++)
                   for(int v = 0; v <= 2 * l; v++)
@@ -1076,17 +1078,19 @@ __global__ void kSumParts(const int* __restrict__ targets, int nTargets, int par
 
 }  // namespace rot
 
-// The rotation tables of the plan's order, all 332 operators: the full M2L operator, or with m2l_truncate the terms up
-// to l + lambda = p. (fmm_config.m2l_tc_degree_cutoff is the tensor-core M2L's: here a cutoff would save nothing.)
+// The rotation tables of the plan's order: the full M2L operator, or with m2l_truncate the terms up to l + lambda = p.
+// (fmm_config.m2l_tc_degree_cutoff is the tensor-core M2L's: here a cutoff would save nothing.) Tensor-core M2L plans take
+// the M2M's and L2L's operators alone.
 template <class T>
 fmm_status ensureRotations(Plan& P, cudaStream_t st)
 {
    const int cut = P.cfg.m2l_truncate ? P.p : 2 * P.p;
    if(P.rotCut == cut) return FMM_OK;
+   const int count = !P.fp64 && P.cfg.m2l_mode != FMM_M2L_SIMT ? 16 : 16 + 316;
    const rot::Blob B(P.p);
-   const std::vector<double>& q = rot::quarterTurn();
+   const std::vector<double>& q = rot::quarterTurn(P.p);
    FMM_TRY(P.rotQuarter.reserve(sizeof(double) * q.size()));
-   FMM_TRY(P.rotOps.reserve(sizeof(T) * size_t(B.size) * (16 + 316)));
+   FMM_TRY(P.rotOps.reserve(sizeof(T) * size_t(B.size) * count));
    // the step tasks of the M2L and of the M2M / L2L
    P.rotTaskHost.resize(2 * sizeof(rot::TaskTable));
    for(int mode = 0; mode < 2; mode++)
@@ -1094,7 +1098,7 @@ fmm_status ensureRotations(Plan& P, cudaStream_t st)
    FMM_TRY(P.rotTasks.reserve(P.rotTaskHost.size()));
    FMM_CUDA(cudaMemcpyAsync(P.rotTasks.ptr, P.rotTaskHost.data(), P.rotTaskHost.size(), cudaMemcpyHostToDevice, st));
    FMM_CUDA(cudaMemcpyAsync(P.rotQuarter.ptr, q.data(), sizeof(double) * q.size(), cudaMemcpyHostToDevice, st));
-   rot::kBuildRotations<T><<<16 + 316, 256, 0, st>>>(P.p, cut, (const double*)P.rotQuarter.ptr, (T*)P.rotOps.ptr);
+   rot::kBuildRotations<T><<<count, 256, 0, st>>>(P.p, cut, (const double*)P.rotQuarter.ptr, (T*)P.rotOps.ptr);
    FMM_TRY(launched(P, "kBuildRotations", st));
    P.rotCut = cut;
    return FMM_OK;
