@@ -1247,11 +1247,15 @@ fmm_status fmm_get_stats(const fmm_plan* plan, fmm_stats* stats)
    if(!plan || !stats) return setError(FMM_E_INVALID, "null argument");
    const Plan& P = plan->P;
    DeviceGuard g(P.cfg.device);
+   bool noTree = false;
    if(P.treeDeferred && !P.treeReady)
    {
-      // the tree fmm_direct left out, on the default stream after everything queued so far
+      // the tree fmm_direct left out, on the default stream after everything queued so far and before whatever follows on
+      // any other. Reading statistics does not fail for it: without the tree its figures are zero.
       FMM_CUDA(cudaDeviceSynchronize());
-      FMM_TRY(buildDeferredTree(const_cast<fmm_plan*>(plan), nullptr));
+      noTree = buildDeferredTree(const_cast<fmm_plan*>(plan), nullptr) != FMM_OK;
+      if(noTree) cudaGetLastError();
+      FMM_CUDA(cudaStreamSynchronize(nullptr));
    }
    fmm_stats s{};
    if(P.downReady) cudaEventSynchronize(P.ev[5]);
@@ -1266,10 +1270,13 @@ fmm_status fmm_get_stats(const fmm_plan* plan, fmm_stats* stats)
       cudaEventSynchronize(P.ev[7]);
       s.ms_adjoint = elapsed(P.ev[6], P.ev[7]);
    }
-   s.nodes = P.tree.nNodes;
-   s.levels = P.tree.nLevels;
-   s.p2p_pairs = P.nP2P;
-   s.v_pairs = P.nV;
+   if(!noTree)
+   {
+      s.nodes = P.tree.nNodes;
+      s.levels = P.tree.nLevels;
+      s.p2p_pairs = P.nP2P;
+      s.v_pairs = P.nV;
+   }
    if(P.treeReady && P.nearCounts.ptr)
    {
       unsigned long long c[2] = {0, 0};

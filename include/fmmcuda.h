@@ -262,6 +262,9 @@ fmm_status fmm_graph_launch(fmm_plan* plan, double current, void* out_B, void* o
  * A graph captured earlier is dropped (it holds the old limit). */
 fmm_status fmm_set_wait_limit(fmm_plan* plan, double seconds);
 
+/* The last solve's phase times and tree. After fmm_direct on a plan without a tree (fmm_direct needs none) it waits for the
+ * device, builds the tree on the default stream and waits for it, so the plan counts as in use; if the tree cannot be
+ * built, its figures are zero. */
 fmm_status fmm_get_stats(const fmm_plan* plan, fmm_stats* stats);
 
 /* Operator tables, for verification. kind 0 = M2M (index = child octant 0..7), 1 = L2L

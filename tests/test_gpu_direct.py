@@ -219,3 +219,33 @@ def test_sources_packed_once_follow_the_inputs(precision):
     plan.set_sources(*sets[0])                           # and back to the input order
     assert np.array_equal(plan.direct(1.0, 1)[0], fresh(sets[0], tgts[1]))
     plan.close()
+
+
+def test_statistics_between_streams():
+    """stats() after a direct sum builds the tree on the default stream; the phases then go on at once on another
+    stream, and the sum still running on a third keeps its result."""
+    import torch
+    rng = np.random.default_rng(12)
+    n, m = 60001, 3001
+    xyz, w, J, tgt = _cuda(rng.uniform(-1, 1, (n, 3)), rng.uniform(0.5, 1, n), rng.normal(size=(n, 3)),
+                           rng.uniform(-2, 2, (m, 3)), dtype=torch.float64)
+    plan = Plan(order=4, leaf_capacity=60, precision="fp64")
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    want, alone = plan.solve(1.0, 1)[0].clone(), None
+    for _ in range(2):
+        plan.set_targets(tgt)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            D = plan.direct(1.0, 1)[0]
+        st = plan.stats()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            plan.upward()
+            plan.downward()
+            B = plan.evaluate(1.0, 1)[0]
+        torch.cuda.synchronize()
+        assert st["nodes"] > 1 and st["leaves"] > 1 and st["p2p_pairs"] > 0
+        assert torch.equal(B, want)
+        assert alone is None or torch.equal(D, alone)
+        alone = D.clone()
+    plan.close()
