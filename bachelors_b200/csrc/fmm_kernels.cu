@@ -672,8 +672,8 @@ __global__ void __launch_bounds__(32 * (SPLIT ? P2MW_SPLIT_WARPS : P2MW_WARPS), 
                {
                   if(j > p + 1) break;
                   const ulonglong2 kk = ldsPair(AB + 2 * (j * P2MW_U + u));
-               const T ka = __longlong_as_double(kk.x), kb = __longlong_as_double(kk.y);
-               const T ke = __longlong_as_double(ldsOne(EE + j * P2MW_U + u));
+                  const T ka = __longlong_as_double(kk.x), kb = __longlong_as_double(kk.y);
+                  const T ke = __longlong_as_double(ldsOne(EE + j * P2MW_U + u));
                   const T az = ka * z, br = kb * r2;
                   const T az2 = ka * z2, br2 = kb * r22;
                   const T cre = ke * bdr + br * bre + az * are;
@@ -1684,7 +1684,7 @@ fmm_status directT(Plan& P, double current, int want, cudaStream_t st)
       maxT = std::max(maxT, P.tgtOff[c + 1] - P.tgtOff[c]);
       maxS = std::max(maxS, P.srcOff[c + 1] - P.srcOff[c]);
    }
-   const int* seg = (const int*)P.segb.ptr;   // srcOff then tgtOff, uploaded by the tree build
+   const int* seg = (const int*)P.segb.ptr;   // srcOff then tgtOff, uploaded by the tree build or with the packed sources
    return launchDirect<T, T>(P, P.directPart, P.nCoils, maxT, maxS, (const T*)P.tgtXYZ, int(P.m), seg, seg + P.nCoils + 1, scaleB, scaleA,
                              want, (T*)P.outB.ptr, (T*)P.outA.ptr, st);
 }
