@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <array>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <string>
@@ -50,6 +51,7 @@ struct DevicePool
    std::once_flag once;
    cudaMemPool_t pool = nullptr;
    cudaStream_t stream = nullptr;
+   std::atomic<int64_t> used{0}, most{0};   // bytes handed out; what the pool may hold: the most of them, less what was trimmed
 };
 DevicePool* devicePool()
 {
@@ -124,24 +126,35 @@ cudaError_t poolAlloc(void** ptr, size_t bytes)
    }
    e = cudaStreamSynchronize(d->stream);
    if(e != cudaSuccess) cudaFreeAsync(*ptr, d->stream);
+   else
+   {
+      const int64_t now = d->used += int64_t(bytes);
+      int64_t most = d->most;
+      while(now > most && !d->most.compare_exchange_weak(most, now)) {}
+   }
    return e;
 }
 
-void poolFree(void* ptr)
+void poolFree(void* ptr, size_t bytes)
 {
    DevicePool* d = devicePool();
-   if(d) cudaFreeAsync(ptr, d->stream);
+   if(!d) return;
+   cudaFreeAsync(ptr, d->stream);
+   d->used -= int64_t(bytes);
 }
 
 void poolTrim(size_t keep)
 {
    DevicePool* d = devicePool();
+   // (what the pool holds is at most a chunk more than the most it has handed out: no need to ask after every small plan)
+   if(!d || (keep > 0 && d->most - d->used <= int64_t(keep))) return;
    uint64_t reserved = 0, used = 0;
-   if(!d || cudaStreamSynchronize(d->stream) != cudaSuccess ||   // the frees of this and other threads so far
+   if(cudaStreamSynchronize(d->stream) != cudaSuccess ||   // the frees of this and other threads so far
       cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
       cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
       return;
    if(reserved > used + keep) cudaMemPoolTrimTo(d->pool, used + keep);
+   d->most = d->used + int64_t(std::min<uint64_t>(keep, reserved > used ? reserved - used : 0));
 }
 
 fmm_status Plan::ensureNodes(int64_t cap, cudaStream_t st)
@@ -226,8 +239,6 @@ fmm_status Plan::init(const fmm_config& c)
    FMM_CUDA(pinnedWord(&hostErr));
    *hostErr = 0;
    for(int i = 0; i < 8; i++) cudaEventCreate(&ev[i]);
-   cudaEventCreateWithFlags(&evPacked, cudaEventDisableTiming);
-   cudaEventCreateWithFlags(&evDirect, cudaEventDisableTiming);
    eventsMade = true;
    return FMM_OK;
 }
@@ -266,11 +277,10 @@ void Plan::release()
    hostErr = nullptr;
    err = pipeErr = nullptr;
    if(eventsMade)
-   {
       for(int i = 0; i < 8; i++) cudaEventDestroy(ev[i]);
-      cudaEventDestroy(evPacked);
-      cudaEventDestroy(evDirect);
-   }
+   if(evDirect) cudaEventDestroy(evDirect);
+   evDirect = nullptr;
+   directQueued = false;
    eventsMade = false;
 }
 
@@ -371,43 +381,35 @@ fmm_status downwardPhase(Plan& P, cudaStream_t st)
 }
 
 // The packed sources of a direct sum: the tree's when there is one, else in input order, packed by the first sum over the
-// plan's inputs (`packed`: now; again for each sum, it made a small one 4 to 8 us slower).
-fmm_status directSources(Plan& P, cudaStream_t st, bool& packed)
+// plan's inputs (again for each sum, it made a small one 4 to 8 us slower).
+fmm_status directSources(Plan& P, cudaStream_t st)
 {
-   packed = false;
    if(P.treeReady || P.srcPacked) return FMM_OK;
    if(P.n + P.m == 0) return setError(FMM_E_INVALID, "no sources or targets set");
-   FMM_TRY(P.waitDirect(st));
-   packed = true;
    FMM_TRY(P.fp64 ? packSourcesT<double>(P, st) : packSourcesT<float>(P, st));
-   FMM_CUDA(cudaEventRecord(P.evPacked, st));
-   P.treeDeferred = true;
+   P.srcPacked = P.treeDeferred = true;
    P.upReady = P.downReady = false;
    P.dropGraph();
    return FMM_OK;
 }
 
-// Ends a direct sum of status s. The next call may be on another stream: whatever puts the packed sources in another
-// order waits for this sum (waitDirect); and the inputs, which the packing reads, may change as soon as the host goes
-// on, so it waits for the packing (not for the sum, which is queued behind it). A sum that a caller captures into a
-// graph of its own leaves no event: the replays are the caller's to order.
-fmm_status directDone(Plan& P, cudaStream_t st, bool packed, fmm_status s)
+// Runs `sum`, a direct sum queued on st, behind the one before it, and leaves the event that the next call waits for on
+// its own stream if it would change what the sum reads (Plan::waitDirect). A sum that a caller captures into a
+// graph of its own does neither: the replays are the caller's to order.
+template <class F>
+fmm_status queueDirect(Plan& P, cudaStream_t st, F&& sum)
 {
    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-   cudaError_t e = cudaStreamIsCapturing(st, &cap);
-   if(e == cudaSuccess && cap == cudaStreamCaptureStatusNone)
-   {
-      e = cudaEventRecord(P.evDirect, st);
-      P.directQueued = e == cudaSuccess;
-   }
-   if(packed)
-   {
-      const cudaError_t done = s == FMM_OK ? cudaEventSynchronize(P.evPacked) : cudaStreamSynchronize(st);
-      if(e == cudaSuccess) e = done;
-      P.srcPacked = s == FMM_OK && e == cudaSuccess;
-   }
-   if(s == FMM_OK && e != cudaSuccess) s = setError(FMM_E_CUDA, "direct sum: %s", cudaGetErrorString(e));
-   return s;
+   if(cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+   if(cap != cudaStreamCaptureStatusNone)
+      return P.treeReady || P.srcPacked ? sum() : setError(FMM_E_INVALID, "a direct sum under capture: run one, or fmm_build_tree, before");
+   FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
+   FMM_TRY(P.waitDirect(st));
+   if(!P.evDirect) FMM_CUDA(cudaEventCreateWithFlags(&P.evDirect, cudaEventDisableTiming));
+   const fmm_status s = sum();
+   const cudaError_t e = cudaEventRecord(P.evDirect, st);
+   P.directQueued = e == cudaSuccess;
+   return s == FMM_OK && e != cudaSuccess ? setError(FMM_E_CUDA, "direct sum: %s", cudaGetErrorString(e)) : s;
 }
 
 double elapsed(cudaEvent_t a, cudaEvent_t b)
@@ -485,6 +487,7 @@ fmm_status fmm_set_sources(fmm_plan* plan, const void* xyz, const void* w, const
    cudaStream_t st = (cudaStream_t)stream;
    size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    FMM_TRY(P.waitSourceInputs(st));   // copies of an earlier fmm_set_sources_async into the same buffers
+   FMM_TRY(P.waitDirect(st));
    FMM_TRY(copyIn(P.srcXYZb, xyz, es * 3 * n, on_device, st, &P.srcXYZ));
    FMM_TRY(copyIn(P.srcWb, w, es * n, on_device, st, &P.srcW));
    P.hasJ = J != nullptr;
@@ -532,7 +535,8 @@ fmm_status fmm_set_sources_async(fmm_plan* plan, const void* xyz, const void* w,
       FMM_CUDA(cudaEventCreateWithFlags(&P.evPos, cudaEventDisableTiming));
       FMM_CUDA(cudaEventCreateWithFlags(&P.evInputs, cudaEventDisableTiming));
    }
-   // the copies follow the work queued on `stream` so far (it may still read the previous sources)
+   // the copies follow the work queued on `stream` so far (it may still read the previous sources) and the last direct sum
+   FMM_TRY(P.waitDirect(st));
    FMM_CUDA(cudaEventRecord(P.evPrev, st));
    FMM_CUDA(cudaStreamWaitEvent(P.copyStream, P.evPrev, 0));
    if(n) FMM_CUDA(cudaMemcpyAsync(P.srcXYZb.ptr, xyz, es * 3 * n, cudaMemcpyHostToDevice, P.copyStream));
@@ -563,6 +567,7 @@ fmm_status fmm_set_bem_sources(fmm_plan* plan, const void* xyz, const void* w, c
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
+   FMM_TRY(P.waitDirect(st));
    const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    FMM_TRY(copyIn(P.srcXYZb, xyz, es * 3 * n, on_device, st, &P.srcXYZ));
    FMM_TRY(copyIn(P.srcWb, w, es * n, on_device, st, &P.srcW));
@@ -614,6 +619,7 @@ fmm_status fmm_set_targets(fmm_plan* plan, const void* xyz, int64_t m, int on_de
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    size_t es = P.fp64 ? sizeof(double) : sizeof(float);
+   FMM_TRY(P.waitDirect(st));
    FMM_TRY(copyIn(P.tgtXYZb, xyz, es * 3 * m, on_device, st, &P.tgtXYZ));
    if(!on_device) FMM_CUDA(cudaStreamSynchronize(st));
    P.m = m;
@@ -631,6 +637,7 @@ fmm_status fmm_set_targets_to_sources(fmm_plan* plan, void* stream)
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourcePoints(st));   // fmm_set_sources_async copies in flight
+   FMM_TRY(P.waitDirect(st));
    const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    const size_t bytes = es * 3 * size_t(P.n);
    FMM_TRY(P.tgtXYZb.reserve(std::max<size_t>(bytes, 16)));
@@ -756,10 +763,8 @@ fmm_status fmm_direct(fmm_plan* plan, double current, int want, void* out_B, voi
       return setError(FMM_E_INVALID, "a plan with BEM sources sums the BEM integral into out_A (want = 2)");
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
-   FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   bool packed = false;
-   auto sum = [&]() -> fmm_status {
-      FMM_TRY(directSources(P, st, packed));
+   return queueDirect(P, st, [&]() -> fmm_status {
+      FMM_TRY(directSources(P, st));
       size_t es = P.fp64 ? sizeof(double) : sizeof(float);
       size_t bytes = es * 3 * std::max<int64_t>(P.m, 1);
       if(want & 1) FMM_TRY(P.outB.reserve(bytes));
@@ -768,8 +773,7 @@ fmm_status fmm_direct(fmm_plan* plan, double current, int want, void* out_B, voi
       if(want & 1) FMM_TRY(copyOut(out_B, P.outB, es * 3 * P.m, on_device, st));
       if(want & 2) FMM_TRY(copyOut(out_A, P.outA, es * 3 * P.m, on_device, st));
       return FMM_OK;
-   };
-   return directDone(P, st, packed, sum());
+   });
 }
 
 fmm_status fmm_direct_fp64_subset(fmm_plan* plan, double current, const double* tgt, int64_t k, double* out_B)
@@ -780,11 +784,9 @@ fmm_status fmm_direct_fp64_subset(fmm_plan* plan, double current, const double* 
       return setError(FMM_E_INVALID, "fmm_direct_fp64_subset: explicit targets belong to no coil of a batched plan");
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = 0;
-   FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
    DevBuf t, o;
-   bool packed = false;
-   auto sum = [&]() -> fmm_status {
-      FMM_TRY(directSources(P, st, packed));
+   const fmm_status s = queueDirect(P, st, [&]() -> fmm_status {
+      FMM_TRY(directSources(P, st));
       FMM_TRY(t.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
       FMM_TRY(o.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
       FMM_CUDA(cudaMemcpyAsync(t.ptr, tgt, sizeof(double) * 3 * k, cudaMemcpyHostToDevice, st));
@@ -792,8 +794,7 @@ fmm_status fmm_direct_fp64_subset(fmm_plan* plan, double current, const double* 
       FMM_CUDA(cudaMemcpyAsync(out_B, o.ptr, sizeof(double) * 3 * k, cudaMemcpyDeviceToHost, st));
       FMM_CUDA(cudaStreamSynchronize(st));
       return FMM_OK;
-   };
-   const fmm_status s = directDone(P, st, packed, sum());
+   });
    t.release();
    o.release();
    return s;
@@ -1133,6 +1134,7 @@ fmm_status fmm_update_sources(fmm_plan* plan, const void* w, const void* J, int 
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
+   FMM_TRY(P.waitDirect(st));
    const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    if(P.n)
    {

@@ -87,7 +87,7 @@ extern __constant__ int d_m2lFarFirst[316]; // M2L slots by decreasing offset le
 // does); the pool's own calls are safe from several threads. Larger blocks, and devices without memory pools, use cudaMalloc.
 constexpr size_t POOL_BLOCK = size_t(8) << 20, POOL_KEEP = size_t(128) << 20;
 cudaError_t poolAlloc(void** ptr, size_t bytes);   // cudaErrorNotSupported: no pool on the current device
-void poolFree(void* ptr);
+void poolFree(void* ptr, size_t bytes);
 void poolTrim(size_t keep);   // gives freed blocks beyond `keep` bytes back to the device
 cudaError_t pinnedWord(int** word);   // a page-locked host word, and back
 void pinnedWordFree(int* word);
@@ -140,7 +140,7 @@ struct DevBuf
       if(ptr && pooled)
       {
          if(!idle) cudaDeviceSynchronize();
-         poolFree(ptr);
+         poolFree(ptr, bytes);
          if(!idle && bytes >= (size_t(1) << 20)) poolTrim(POOL_KEEP);   // (small ones wait for the next)
       }
       else if(ptr) cudaFree(ptr);
@@ -290,7 +290,7 @@ struct Plan
    bool srcPacked = false;               // ... and sPos, sQ and segb hold the sources in input order
    fmm_stats stats{};
    cudaEvent_t ev[8];
-   cudaEvent_t evPacked, evDirect;       // the last direct sum's sources packed (without a tree), its kernels done
+   cudaEvent_t evDirect = nullptr;       // the last direct sum's kernels done
    bool directQueued = false;            // evDirect has been recorded
    bool eventsMade = false;
 
@@ -331,7 +331,8 @@ struct Plan
    bool inputsAsync = false;
    fmm_status waitSourcePoints(cudaStream_t st) { return waitCopy(st, evPos); }
    fmm_status waitSourceInputs(cudaStream_t st) { return waitCopy(st, evInputs); }
-   // before the packed sources change: a direct sum on another stream may still read them
+   // before the inputs or the packed sources change, and before another sum takes the packed sources and the buffers for
+   // split sums and outputs: a direct sum on another stream may still be using them
    fmm_status waitDirect(cudaStream_t st)
    {
       const cudaError_t e = directQueued ? cudaStreamWaitEvent(st, evDirect, 0) : cudaSuccess;
