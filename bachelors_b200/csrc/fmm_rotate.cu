@@ -577,6 +577,11 @@ __device__ void tileStarts(const TileOps ops)
       base += sum;
       __syncthreads();
    }
+   if(ops.whole == 0)
+   {
+      for(int b = tid; b <= ops.blocks; b += TILEOPS_NT) ops.share[b] = base / ops.blocks * b + base % ops.blocks * b / ops.blocks;
+      return;
+   }
    // what each block still needs, summed up to each block's end; then scaled to the work that is left
    const int64_t first = ops.start[ops.whole];
    int64_t needed = 0;
@@ -613,8 +618,14 @@ __global__ void __launch_bounds__(TILEOPS_NT) kTileOps(const int* __restrict__ t
    __syncthreads();
    int n = 0;
    if(tid < 316)
-#pragma unroll 8
-      for(int t = 0; t < nTile; t++) n += vtab[int64_t(node[t]) * 316 + tid] >= 0;
+      for(int t0 = 0; t0 < nTile; t0 += 50)
+      {
+         int v[50];   // loads that are all in flight: a small tree waits for this one block
+#pragma unroll
+         for(int u = 0; u < 50; u++) v[u] = t0 + u < nTile ? vtab[int64_t(node[t0 + u]) * 316 + tid] : -1;
+#pragma unroll
+         for(int u = 0; u < 50; u++) n += v[u] >= 0;
+      }
    // positions in the list and the work before, over the block
    const int mine = opWork<T>(n, p);
    const unsigned bits = __ballot_sync(0xffffffffu, n > 0);
@@ -665,31 +676,36 @@ __device__ __forceinline__ int tileOf(const int64_t* __restrict__ start, int til
 }
 
 // Y of the tiles that several blocks share: the slots' sums added in block order. blockIdx.x: the tile, of those behind the
-// whole ones; blockIdx.y of gridDim.y: boxes of it.
+// whole ones; blockIdx.y of gridDim.y: boxes of it. Bound by latency where tiles are few (16 slots' loads in flight).
 template <class T>
-__global__ void __launch_bounds__(256) kAddParts(const int* __restrict__ targets, int nTargets, int TT, const TileOps ops, int Lp,
+__global__ void __launch_bounds__(512) kAddParts(const int* __restrict__ targets, int nTargets, int TT, const TileOps ops, int Lp,
                                                  const T* __restrict__ ws, T* __restrict__ Y)
 {
    const int tile = ops.whole + blockIdx.x;
    const int64_t a = ops.start[tile], e = ops.start[tile + 1];
-   int b0 = 0, b1 = ops.blocks;   // the first block that begins behind a
-   while(b0 < b1)
+   int b0 = 0, b1 = 0;   // the blocks that begin inside the tile
+   for(int c = 0; c < ops.blocks; c += blockDim.x)
    {
-      const int m = (b0 + b1) >> 1;
-      if(ops.share[m] > a) b1 = m;
-      else b0 = m + 1;
+      const int64_t at = c + int(threadIdx.x) < ops.blocks ? ops.share[c + threadIdx.x] : INT64_MAX;
+      b0 += __syncthreads_count(at <= a);
+      b1 += __syncthreads_count(at < e);
    }
-   while(b1 < ops.blocks && ops.share[b1] < e) b1++;
-   if(b0 == b1) return;
+   if(b0 >= b1) return;
    const int nTile = min(TT, nTargets - tile * TT), n = 3 * Lp;
    for(int t = blockIdx.y; t < nTile; t += gridDim.y)
    {
       T* y = Y + int64_t(targets[tile * TT + t]) * n;
-      for(int k = threadIdx.x; k < n; k += 256)
+      for(int k = threadIdx.x; k < n; k += blockDim.x)
       {
          T s = y[k];
-#pragma unroll 8
-         for(int b = b0; b < b1; b++) s += ws[(int64_t(b) * TT + t) * n + k];
+         for(int b = b0; b < b1; b += 16)
+         {
+            T v[16];
+#pragma unroll
+            for(int u = 0; u < 16; u++) v[u] = b + u < b1 ? ws[(int64_t(b + u) * TT + t) * n + k] : T(0);
+#pragma unroll
+            for(int u = 0; u < 16; u++) s += v[u];
+         }
          y[k] = s;
       }
    }
@@ -1222,8 +1238,9 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
       FMM_TRY(launched(P, "kRotTranslate<M2L>", st));
       const int shared = tiles - tileOps.whole;
       if(shared == 0) return FMM_OK;
-      rot::kAddParts<T><<<dim3(shared, std::max(8, std::min(tile, 4736 / shared))), 256, 0, st>>>(targets, count, tile, tileOps, P.Lp, ws,
-                                                                                                Y);
+      const int n = 3 * P.Lp, rounds = (n + 511) / 512, threads = ((n + rounds - 1) / rounds + 31) / 32 * 32;
+      rot::kAddParts<T><<<dim3(shared, std::max(8, std::min(tile, 4736 / shared))), threads, 0, st>>>(targets, count, tile, tileOps,
+                                                                                                    P.Lp, ws, Y);
       return launched(P, "kAddParts", st);
    }
    const int64_t n = 3 * int64_t(count) * P.Lp;
