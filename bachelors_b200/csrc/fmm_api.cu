@@ -278,9 +278,9 @@ void Plan::release()
    err = pipeErr = nullptr;
    if(eventsMade)
       for(int i = 0; i < 8; i++) cudaEventDestroy(ev[i]);
-   if(evDirect) cudaEventDestroy(evDirect);
-   evDirect = nullptr;
-   directQueued = false;
+   if(evReads) cudaEventDestroy(evReads);
+   evReads = nullptr;
+   readsQueued = false;
    eventsMade = false;
 }
 
@@ -393,23 +393,22 @@ fmm_status directSources(Plan& P, cudaStream_t st)
    return FMM_OK;
 }
 
-// Runs `sum`, a direct sum queued on st, behind the one before it, and leaves the event that the next call waits for on
-// its own stream if it would change what the sum reads (Plan::waitDirect). A sum that a caller captures into a
-// graph of its own does neither: the replays are the caller's to order.
+// Runs a direct sum or treecode query, queued on st behind the one before it, and leaves the event that the next call waits
+// for on its own stream if it would change what this one reads or uses (Plan::waitReads). Captured into a
+// graph of the caller's (`capturable`) it does neither: the replays are the caller's to order.
 template <class F>
-fmm_status queueDirect(Plan& P, cudaStream_t st, F&& sum)
+fmm_status queueRead(Plan& P, cudaStream_t st, bool capturable, const char* what, F&& run)
 {
    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
    if(cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-   if(cap != cudaStreamCaptureStatusNone)
-      return P.treeReady || P.srcPacked ? sum() : setError(FMM_E_INVALID, "a direct sum under capture: run one, or fmm_build_tree, before");
+   if(cap != cudaStreamCaptureStatusNone) return capturable ? run() : setError(FMM_E_INVALID, "%s: not under capture", what);
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   FMM_TRY(P.waitDirect(st));
-   if(!P.evDirect) FMM_CUDA(cudaEventCreateWithFlags(&P.evDirect, cudaEventDisableTiming));
-   const fmm_status s = sum();
-   const cudaError_t e = cudaEventRecord(P.evDirect, st);
-   P.directQueued = e == cudaSuccess;
-   return s == FMM_OK && e != cudaSuccess ? setError(FMM_E_CUDA, "direct sum: %s", cudaGetErrorString(e)) : s;
+   FMM_TRY(P.waitReads(st));
+   if(!P.evReads) FMM_CUDA(cudaEventCreateWithFlags(&P.evReads, cudaEventDisableTiming));
+   const fmm_status s = run();
+   const cudaError_t e = cudaEventRecord(P.evReads, st);
+   P.readsQueued = e == cudaSuccess;
+   return s == FMM_OK && e != cudaSuccess ? setError(FMM_E_CUDA, "%s: %s", what, cudaGetErrorString(e)) : s;
 }
 
 double elapsed(cudaEvent_t a, cudaEvent_t b)
@@ -487,7 +486,7 @@ fmm_status fmm_set_sources(fmm_plan* plan, const void* xyz, const void* w, const
    cudaStream_t st = (cudaStream_t)stream;
    size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    FMM_TRY(P.waitSourceInputs(st));   // copies of an earlier fmm_set_sources_async into the same buffers
-   FMM_TRY(P.waitDirect(st));
+   FMM_TRY(P.waitReads(st));
    FMM_TRY(copyIn(P.srcXYZb, xyz, es * 3 * n, on_device, st, &P.srcXYZ));
    FMM_TRY(copyIn(P.srcWb, w, es * n, on_device, st, &P.srcW));
    P.hasJ = J != nullptr;
@@ -536,7 +535,7 @@ fmm_status fmm_set_sources_async(fmm_plan* plan, const void* xyz, const void* w,
       FMM_CUDA(cudaEventCreateWithFlags(&P.evInputs, cudaEventDisableTiming));
    }
    // the copies follow the work queued on `stream` so far (it may still read the previous sources) and the last direct sum
-   FMM_TRY(P.waitDirect(st));
+   FMM_TRY(P.waitReads(st));
    FMM_CUDA(cudaEventRecord(P.evPrev, st));
    FMM_CUDA(cudaStreamWaitEvent(P.copyStream, P.evPrev, 0));
    if(n) FMM_CUDA(cudaMemcpyAsync(P.srcXYZb.ptr, xyz, es * 3 * n, cudaMemcpyHostToDevice, P.copyStream));
@@ -567,7 +566,7 @@ fmm_status fmm_set_bem_sources(fmm_plan* plan, const void* xyz, const void* w, c
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   FMM_TRY(P.waitDirect(st));
+   FMM_TRY(P.waitReads(st));
    const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    FMM_TRY(copyIn(P.srcXYZb, xyz, es * 3 * n, on_device, st, &P.srcXYZ));
    FMM_TRY(copyIn(P.srcWb, w, es * n, on_device, st, &P.srcW));
@@ -619,7 +618,7 @@ fmm_status fmm_set_targets(fmm_plan* plan, const void* xyz, int64_t m, int on_de
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    size_t es = P.fp64 ? sizeof(double) : sizeof(float);
-   FMM_TRY(P.waitDirect(st));
+   FMM_TRY(P.waitReads(st));
    FMM_TRY(copyIn(P.tgtXYZb, xyz, es * 3 * m, on_device, st, &P.tgtXYZ));
    if(!on_device) FMM_CUDA(cudaStreamSynchronize(st));
    P.m = m;
@@ -637,7 +636,7 @@ fmm_status fmm_set_targets_to_sources(fmm_plan* plan, void* stream)
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourcePoints(st));   // fmm_set_sources_async copies in flight
-   FMM_TRY(P.waitDirect(st));
+   FMM_TRY(P.waitReads(st));
    const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    const size_t bytes = es * 3 * size_t(P.n);
    FMM_TRY(P.tgtXYZb.reserve(std::max<size_t>(bytes, 16)));
@@ -681,6 +680,7 @@ fmm_status fmm_upward(fmm_plan* plan, void* stream)
    if(!P.treeReady) return setError(FMM_E_INVALID, "fmm_upward: tree not built");
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
+   FMM_TRY(P.waitReads(st));
    FMM_TRY(pipeBegin(P, st));
    FMM_TRY(upwardPhase(P, st));
    return pipeCheck(P, st, "fmm_upward");
@@ -763,7 +763,7 @@ fmm_status fmm_direct(fmm_plan* plan, double current, int want, void* out_B, voi
       return setError(FMM_E_INVALID, "a plan with BEM sources sums the BEM integral into out_A (want = 2)");
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
-   return queueDirect(P, st, [&]() -> fmm_status {
+   return queueRead(P, st, P.treeReady || P.srcPacked, "fmm_direct without a tree or a sum before it", [&]() -> fmm_status {
       FMM_TRY(directSources(P, st));
       size_t es = P.fp64 ? sizeof(double) : sizeof(float);
       size_t bytes = es * 3 * std::max<int64_t>(P.m, 1);
@@ -785,7 +785,7 @@ fmm_status fmm_direct_fp64_subset(fmm_plan* plan, double current, const double* 
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = 0;
    DevBuf t, o;
-   const fmm_status s = queueDirect(P, st, [&]() -> fmm_status {
+   const fmm_status s = queueRead(P, st, false, "fmm_direct_fp64_subset", [&]() -> fmm_status {
       FMM_TRY(directSources(P, st));
       FMM_TRY(t.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
       FMM_TRY(o.reserve(sizeof(double) * 3 * std::max<int64_t>(k, 1)));
@@ -874,35 +874,33 @@ fmm_status fmm_treecode(fmm_plan* plan, double current, int want, const void* pt
    if(m == 0) return FMM_OK;
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
-   FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
-   const size_t bytes = es * 3 * size_t(m);
-   const void* dPts = pts;
-   void* dB = out_B;
-   void* dA = out_A;
-   if(!on_device)
-   {
-      FMM_TRY(P.tcPts.reserve(bytes));
-      FMM_TRY(P.tcOut.reserve(2 * bytes));
-      FMM_CUDA(cudaMemcpyAsync(P.tcPts.ptr, pts, bytes, cudaMemcpyHostToDevice, st));
-      dPts = P.tcPts.ptr;
-      dB = (want & 1) ? P.tcOut.ptr : nullptr;
-      dA = (want & 2) ? (char*)P.tcOut.ptr + bytes : nullptr;
-   }
-   fmm_status s = P.fp64 ? treecodeT<double>(P, current, want, dPts, m, dB, dA, flags, st)
-                         : treecodeT<float>(P, current, want, dPts, m, dB, dA, flags, st);
-   cudaError_t e = cudaSuccess;
-   if(s == FMM_OK && !on_device)
-   {
-      if(want & 1) e = cudaMemcpyAsync(out_B, dB, bytes, cudaMemcpyDeviceToHost, st);
-      if(e == cudaSuccess && (want & 2)) e = cudaMemcpyAsync(out_A, dA, bytes, cudaMemcpyDeviceToHost, st);
-   }
-   // The points' order, the curl table and the staging belong to the plan: nothing of this call is in flight when the
-   // next one, on whatever stream, takes them (nor when the caller reuses the points or reads the results elsewhere).
-   const cudaError_t done = cudaStreamSynchronize(st);
-   if(e == cudaSuccess) e = done;
-   if(s == FMM_OK && e != cudaSuccess) s = setError(FMM_E_CUDA, "fmm_treecode: %s", cudaGetErrorString(e));
-   return s;
+   // The points' order, the sort's scratch, the curl table and the staging belong to the plan, and the query reads its tree:
+   // queueRead keeps the next call, on whatever stream, off them.
+   return queueRead(P, st, false, "fmm_treecode", [&]() -> fmm_status {
+      const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
+      const size_t bytes = es * 3 * size_t(m);
+      const void* dPts = pts;
+      void* dB = out_B;
+      void* dA = out_A;
+      if(!on_device)
+      {
+         FMM_TRY(P.tcPts.reserve(bytes));
+         FMM_TRY(P.tcOut.reserve(2 * bytes));
+         FMM_CUDA(cudaMemcpyAsync(P.tcPts.ptr, pts, bytes, cudaMemcpyHostToDevice, st));
+         dPts = P.tcPts.ptr;
+         dB = (want & 1) ? P.tcOut.ptr : nullptr;
+         dA = (want & 2) ? (char*)P.tcOut.ptr + bytes : nullptr;
+      }
+      FMM_TRY(P.fp64 ? treecodeT<double>(P, current, want, dPts, m, dB, dA, flags, st)
+                     : treecodeT<float>(P, current, want, dPts, m, dB, dA, flags, st));
+      if(!on_device)
+      {
+         if(want & 1) FMM_CUDA(cudaMemcpyAsync(out_B, dB, bytes, cudaMemcpyDeviceToHost, st));
+         if(want & 2) FMM_CUDA(cudaMemcpyAsync(out_A, dA, bytes, cudaMemcpyDeviceToHost, st));
+         FMM_CUDA(cudaStreamSynchronize(st));
+      }
+      return FMM_OK;
+   });
 }
 
 fmm_status fmm_adjoint_direct(fmm_plan* plan, double current, const void* dL_dB, void* dL_dJ, void* dL_dx,
@@ -977,6 +975,7 @@ fmm_status fmm_autotune(fmm_plan* plan, fmm_tuning* out, void* stream)
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
+   FMM_TRY(P.waitReads(st));
    P.dropGraph();
    FMM_TRY(pipeBegin(P, st));
    cudaEvent_t e0, e1;
@@ -1134,7 +1133,7 @@ fmm_status fmm_update_sources(fmm_plan* plan, const void* w, const void* J, int 
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    FMM_TRY(P.waitSourceInputs(st));   // fmm_set_sources_async copies in flight
-   FMM_TRY(P.waitDirect(st));
+   FMM_TRY(P.waitReads(st));
    const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
    if(P.n)
    {
@@ -1212,6 +1211,7 @@ fmm_status fmm_graph_launch(fmm_plan* plan, double current, void* out_B, void* o
    DeviceGuard g(P.cfg.device);
    cudaStream_t st = (cudaStream_t)stream;
    const size_t es = P.fp64 ? sizeof(double) : sizeof(float);
+   FMM_TRY(P.waitReads(st));
    FMM_TRY(pipeBegin(P, st));
    FMM_CUDA(cudaGraphLaunch(P.graphExec, st));
    const int64_t cnt = 3 * P.m;

@@ -290,8 +290,8 @@ struct Plan
    bool srcPacked = false;               // ... and sPos, sQ and segb hold the sources in input order
    fmm_stats stats{};
    cudaEvent_t ev[8];
-   cudaEvent_t evDirect = nullptr;       // the last direct sum's kernels done
-   bool directQueued = false;            // evDirect has been recorded
+   cudaEvent_t evReads = nullptr;        // behind the last direct sum or treecode query (and so all before it)
+   bool readsQueued = false;             // evReads has been recorded
    bool eventsMade = false;
 
    int64_t launches = 0;      // kernels this plan launched (all phases, cumulative)
@@ -331,12 +331,12 @@ struct Plan
    bool inputsAsync = false;
    fmm_status waitSourcePoints(cudaStream_t st) { return waitCopy(st, evPos); }
    fmm_status waitSourceInputs(cudaStream_t st) { return waitCopy(st, evInputs); }
-   // before the inputs or the packed sources change, and before another sum takes the packed sources and the buffers for
-   // split sums and outputs: a direct sum on another stream may still be using them
-   fmm_status waitDirect(cudaStream_t st)
+   // Before the inputs, the packed sources, the tree or the multipoles change, and before another sum or query takes the
+   // buffers of the last: it may still be running on another stream.
+   fmm_status waitReads(cudaStream_t st)
    {
-      const cudaError_t e = directQueued ? cudaStreamWaitEvent(st, evDirect, 0) : cudaSuccess;
-      if(e != cudaSuccess) return setError(FMM_E_CUDA, "waiting for a direct sum: %s", cudaGetErrorString(e));
+      const cudaError_t e = readsQueued ? cudaStreamWaitEvent(st, evReads, 0) : cudaSuccess;
+      if(e != cudaSuccess) return setError(FMM_E_CUDA, "waiting for a direct sum or query: %s", cudaGetErrorString(e));
       return FMM_OK;
    }
    fmm_status waitCopy(cudaStream_t st, cudaEvent_t ev)

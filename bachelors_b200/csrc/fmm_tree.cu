@@ -1174,7 +1174,7 @@ fmm_status buildTreeT(Plan& P, cudaStream_t st)
    const int threads = 256;
    // the key keeps ceil(log2(coils)) bits above the Morton bits
    const int K = P.nCoils;
-   FMM_TRY(P.waitDirect(st));
+   FMM_TRY(P.waitReads(st));
    FMM_TRY(uploadCoils(P, st));
    int* dSrcOff = (int*)P.segb.ptr;
    int* dTgtOff = dSrcOff + K + 1;

@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(TC_NT) kTreecode(Tree t, const RootBox* __rest
                double* d = S + 8 * tid;
                d[0] = double(a.x); d[1] = double(a.y); d[2] = double(a.z); d[3] = double(b.w);
                d[4] = double(b.x); d[5] = double(b.y); d[6] = double(b.z);
-               odd = !(isfinite(b.x) && isfinite(b.y) && isfinite(b.z) && isfinite(b.w));
+               odd = !isfinite(b.x + b.y + b.z + b.w);   // (or a sum out of range, which only costs)
             }
             // Coincident points are skipped: by a factor of zero, but in a tile with a strength that is no number the sum
             // goes from one such point to the next.

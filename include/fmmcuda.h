@@ -167,8 +167,9 @@ fmm_status fmm_solve(fmm_plan* plan, double current, int want, void* out_B, void
  * FMM_TREECODE_REFERENCE_NEAR drops such leaves (they contribute nothing there), FMM_TREECODE_FD_CURL takes B
  * by central differences of A with step 1e-3. The reference's tree uses root centre 0 and half-width 3 and
  * splits a box holding `cap` points: configure root_center / root_half_width and leaf_capacity = cap - 1.
- * Outputs in point input order, the plan's element type; not available on a batched plan. The call waits for
- * its results, with device pointers too: calls on different streams may follow one another without more ado. */
+ * Outputs in point input order, the plan's element type; not available on a batched plan. With
+ * device pointers the call queues its work on `stream`; later calls of the plan, on whatever stream, wait for it where they
+ * would change what it reads. */
 #define FMM_TREECODE_REFERENCE_NEAR 1
 #define FMM_TREECODE_FD_CURL 2
 fmm_status fmm_treecode(fmm_plan* plan, double current, int want, const void* pts, int64_t m, void* out_B, void* out_A,

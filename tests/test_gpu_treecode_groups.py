@@ -54,8 +54,8 @@ def test_points_on_sources_and_far_away(precision, tol):
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
 def test_calls_on_two_streams(precision):
     """Queries of different sizes, one after the other on two streams without a wait by the caller: the plan's scratch
-    (the points' order, the curl table) is never one call's while another's kernel reads it. The results are complete
-    when a call returns and equal those of the same calls on one stream, bit for bit."""
+    (the points' order, the curl table) is never one call's while another's kernel reads it. The results equal those
+    of the same calls on one stream, bit for bit."""
     import torch
     dt = torch.float32 if precision == "fp32" else torch.float64
     xyz, w, J = (torch.tensor(v, dtype=dt, device="cuda") for v in G.torus(64, 24, 12, 2.0, 0.5))
@@ -65,21 +65,63 @@ def test_calls_on_two_streams(precision):
         s = MultipoleSolver((xyz, w, J), quadratureOctreeLeafCapacity=500, order=8, precision=precision)
         s.calcMultipoleExpansionsAtLeaves()
         torch.cuda.synchronize()
-        out, idle = [], []
+        out = []
         for i, p in enumerate(pts):
             with torch.cuda.stream(streams[i % len(streams)]):
                 out.append(s.calcB(1.0, p))
-                idle.append(streams[i % len(streams)].query())
         torch.cuda.synchronize()
         out = [v.cpu().numpy() for v in out]
         s.plan.close()
-        return out, idle
+        return out
 
-    one, _ = queries([torch.cuda.current_stream()])
-    two, idle = queries([torch.cuda.Stream(), torch.cuda.Stream()])
-    assert all(idle)
-    for a, b in zip(one, two):
+    for a, b in zip(queries([torch.cuda.current_stream()]), queries([torch.cuda.Stream(), torch.cuda.Stream()])):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("then", ["new sources", "new strengths", "graph", "direct", "autotune"])
+def test_next_call_on_another_stream(precision, then):
+    """A query still running on one stream when the plan's next call comes on another and changes the sources, the
+    tree or the multipoles: the query's result stays what it is alone, bit for bit."""
+    import torch
+    dt = torch.float32 if precision == "fp32" else torch.float64
+    cuda = lambda a: torch.tensor(a, dtype=dt, device="cuda")
+    xyz, w, J = (cuda(v) for v in G.torus(64, 24, 12, 2.0, 0.5))
+    rng = np.random.default_rng(4)
+    other = [cuda(rng.uniform(-1, 1, (3001, 3))), cuda(rng.uniform(1, 2, 3001)), cuda(rng.normal(size=(3001, 3)))]
+    pts, tgt = cuda(G.uniform_points(50021, -3, 3, 1)), cuda(G.uniform_points(300, -3, 3, 2))
+    plan = Plan(order=8, leaf_capacity=300, precision=precision)
+    plan.set_sources(xyz, w, J)
+    plan.set_targets(tgt)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(2):
+        plan.set_sources(xyz, w, J)
+        plan.set_targets(tgt)
+        plan.solve(1.0, 1)
+        if then == "graph":
+            plan.graph_capture(1)
+        alone = plan.treecode(pts, 1.0, 1)[0].clone()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            got = plan.treecode(pts, 1.0, 1)[0]
+        with torch.cuda.stream(b):
+            if then == "new sources":
+                plan.set_sources(*other)
+                plan.build_tree()
+                plan.upward()
+            elif then == "new strengths":
+                plan.update_sources(w * 3, J)
+                plan.upward()
+            elif then == "graph":
+                plan.graph_launch(1.0)
+            elif then == "direct":
+                plan.set_targets(tgt + 1)
+                plan.direct(1.0, 1)
+            else:
+                plan.autotune()
+        torch.cuda.synchronize()
+        assert torch.equal(got, alone)
+    plan.close()
 
 
 @pytest.mark.parametrize("p,cap,m", [(1, 10, 40009), (5, 20, 20011), (9, 30, 1301)])
