@@ -78,7 +78,7 @@ __host__ __device__ inline int ordSize(int p) { return ordBase(p, p + 1); }
 // D^ of the quarter turn about x that takes e_z to e_y, degree blocks [2l+1][2l+1] up to degree p one after the other, by
 // integrating products of the orthonormal harmonics over the sphere (Gauss-Legendre x trapezoid, exact for
 // these degrees): R_i(Q x) against R_j(x). A product of two harmonics of one degree is even, so the points below the
-// equator are left out. Made once for an order (p = 16 1 ms, p = 8 0.05).
+// equator are left out. Made once for an order (p = 16 1.3 ms, p = 8 0.1).
 static int quarterOff(int l) { return l * (4 * l * l - 1) / 3; }   // sum of (2i+1)^2, i < l
 static const std::vector<double>& quarterTurn(int p)
 {
@@ -735,12 +735,12 @@ __global__ void __launch_bounds__(512) kAddParts(const int* __restrict__ targets
 // M2L: a block takes every gridDim.x-th of the first tiles, so that those in flight are neighbours and share their sources
 // in L2, and of the rest a share of operators that evens out the blocks' work (TileOps). The block with a tile's first
 // operator adds to the rows of Y, one that begins inside a tile keeps its sums there in its slot of ws ([3 TT][Lp])
-// for kAddParts: a slot a block, whatever the tree. Without ws the grid is a block per tile.
+// for kAddParts: a slot a block, whatever the tree. Without SHARED the grid is a block per tile.
 // (Before, every tile was split into as many equal parts as made eight rounds of blocks, up to 64 copies of the locals:
 // 0.43 to 0.57 GB, now 75 MB at most. M2L of 65,536 points and targets, FP32 p = 12 1.24 -> 1.02 ms, FP64 p = 9 1.49 -> 1.23;
-// 131,072, FP32 p = 16 5.37 -> 4.95; 2^20, p = 4 4.6 both, p = 8 11.7 -> 12.0, p = 12 24.7 both, p = 16 50.8 -> 46.0.)
+// 131,072, FP32 p = 16 5.37 -> 4.95; 2^20, p = 4 4.6 both, p = 8 11.7 -> 12.0, p = 12 24.8 both, p = 16 51.0 -> 46.1.)
 // M2M: blockIdx.y of gridDim.y parts of a tile's operators, their sums go to ws[part][3 nTargets][Lp] (zero before) for kSumParts.
-template <class T, int MODE>
+template <class T, int MODE, bool SHARED = false>
 __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ targets, int nTargets,
                                                     const int* __restrict__ vtab, const int* __restrict__ parent,
                                                     const L2LSegR seg, const TileOps tileOps, int TT, int p, int Lp,
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
       return w < tileOps.share[blockIdx.x + 1] || w > tileOps.start[tileOf(tileOps.start, tileOps.tiles, w)] ? tileOf(tileOps.start, tileOps.tiles, w)
                                                                                                           : tileOps.tiles;
    };
-   if(MODE == 0 && blockIdx.x >= tileOps.whole)
+   if(SHARED && blockIdx.x >= tileOps.whole)
    {
       first = shareTile() * TT;
       if(first >= end) return;
@@ -833,8 +833,9 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
       {
          // the tile's operators, those whose work begins in the share
          const int tile = first / TT, n = tileOps.n[tile];
-         const int64_t lo = tile < tileOps.whole ? 0 : tileOps.share[blockIdx.x] - tileOps.start[tile];
-         const int64_t hi = tile < tileOps.whole ? INT64_MAX : tileOps.share[blockIdx.x + 1] - tileOps.start[tile];
+         const bool all = !SHARED || tile < tileOps.whole;
+         const int64_t lo = all ? 0 : tileOps.share[blockIdx.x] - tileOps.start[tile];
+         const int64_t hi = all ? INT64_MAX : tileOps.share[blockIdx.x + 1] - tileOps.start[tile];
          o1 = 0;
          for(int e0 = 0; e0 < n; e0 += NT)
          {
@@ -844,7 +845,7 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
             o0 += __syncthreads_count(at < lo);
             o1 += __syncthreads_count(at < hi);
          }
-         toParts = o0 > 0;
+         toParts = SHARED && o0 > 0;
       }
       else
       {
@@ -912,7 +913,7 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
          if(lane == 0) nSlot[b] = n;
       };
       T* out = !toParts ? Y : ws + (MODE == 0 ? int64_t(blockIdx.x) * TT : int64_t(blockIdx.y) * nTargets + first) * 3 * Lp;
-      if(MODE == 0 && toParts)
+      if(SHARED && toParts)
       {
          for(int e = tid; e < 3 * nTile * Lp; e += NT) out[e] = T(0);
          __syncthreads();
@@ -947,7 +948,7 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
          // Sums: 4 lanes of V consecutive coefficients by 8 rows a warp and item, BT items' loads in flight together.
          const int kl = V * (lane & 3), rl = lane >> 2, nkb = (Lp + 4 * V - 1) / (4 * V);
          typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type VT;
-         constexpr int BT = MODE == 0 ? 5 : 4;
+         constexpr int BT = MODE != 0 ? 4 : (SHARED ? 5 : 6);   // (6 would spill beside the loop over tiles)
          auto addOut = [&](int db, int nr) {
             const int* rows = dstRow[db];
             const int nItems = nkb * ((nr + 7) >> 3);
@@ -1063,7 +1064,7 @@ __global__ void __launch_bounds__(512) kRotTranslate(const int* __restrict__ tar
          addOut((chunk - 1) & 1, prevRows);
       }
       // the block's next tile
-      if(MODE != 0) break;
+      if(!SHARED) break;
       int next = first / TT;
       if(next < tileOps.whole)
       {
@@ -1143,7 +1144,7 @@ template <class T> static int rotBlocks(Plan& P, int tiles)
 {
    if(P.rotResident == 0)
    {
-      auto kern = rot::kRotTranslate<T, 0>;
+      auto kern = rot::kRotTranslate<T, 0, true>;
       const int smem = rot::Smem<T>(P.p).total;
       int n = 0;
       if(allowShared(kern) != cudaSuccess ||
@@ -1214,7 +1215,7 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
    const size_t smem = rot::Smem<T>(P.p).total;
    const int THREADS = rotThreads<T>(P, MODE);
    auto kern = rot::kRotTranslate<T, MODE>;
-   FMM_CUDA(allowShared(kern));
+   if(MODE != 0) FMM_CUDA(allowShared(kern));
    const T* ops = (const T*)P.rotOps.ptr + size_t(B.size) * (MODE == 0 ? 16 : MODE == 1 ? 0 : 8);
    const rot::TaskTable* tasks = (const rot::TaskTable*)P.rotTasks.ptr + (MODE == 0 ? 0 : 1);
    const int tile = rotTile<T>(MODE);
@@ -1231,13 +1232,19 @@ static fmm_status launchRot(Plan& P, cudaStream_t st, const int* targets, int co
    T* ws = (T*)P.rotWs.ptr;
    if(MODE == 0)
    {
-      rot::TileOps tileOps = rotTileOps<T>(P);
-      if(P.rotWs.bytes < rotRowBytes<T>(P) * tile * tileOps.blocks) tileOps.whole = tileOps.blocks = tiles;
-      kern<<<tileOps.blocks, THREADS, smem, st>>>(targets, count, vtab, P.tree.parent, seg, tileOps, tile, P.p, P.Lp, tasks, ops, X, Y,
-                                                  ws);
-      FMM_TRY(launched(P, "kRotTranslate<M2L>", st));
-      const int shared = tiles - tileOps.whole;
-      if(shared == 0) return FMM_OK;
+      const rot::TileOps tileOps = rotTileOps<T>(P);
+      auto run = [&](auto kernel, int grid) -> fmm_status {
+         FMM_CUDA(allowShared(kernel));
+         kernel<<<grid, THREADS, smem, st>>>(targets, count, vtab, P.tree.parent, seg, tileOps, tile, P.p, P.Lp, tasks, ops, X, Y, ws);
+         return launched(P, "kRotTranslate<M2L>", st);
+      };
+      // A block per tile where the last round of blocks counts for little against the registers that the loop over tiles
+      // costs, or without room for the slots. In shares / a block per tile, ms: one block an SM (p = 16) 2^21 points, 8 rounds,
+      // 74 / 78, 2^22, 17 rounds, 213 / 206, 2^24 669 / 621; two (p = 12) 2^20, 2 rounds, 25 / 29, 2^21, 4 rounds, 43.4 / 42.4,
+      // 2^22 117 / 111; four (p = 8) 2^21, 2 rounds, 19 / 22, 2^22, 4 rounds, 54.9 / 54.6, 2^23 75 / 71.
+      const int shared = tiles - tileOps.whole, perTile = P.rotResident == 1 ? 12 : 4;
+      if(tiles >= perTile * tileOps.blocks || P.rotWs.bytes < rotRowBytes<T>(P) * tile * tileOps.blocks) return run(rot::kRotTranslate<T, 0>, tiles);
+      FMM_TRY(run(rot::kRotTranslate<T, 0, true>, tileOps.blocks));
       const int n = 3 * P.Lp, rounds = (n + 511) / 512, threads = ((n + rounds - 1) / rounds + 31) / 32 * 32;
       rot::kAddParts<T><<<dim3(shared, std::max(8, std::min(tile, 4736 / shared))), threads, 0, st>>>(targets, count, tile, tileOps,
                                                                                                     P.Lp, ws, Y);
