@@ -689,9 +689,10 @@ kM2LTc(const int* __restrict__ targets, int nTargets, const int* __restrict__ vt
       // The whole warp runs the loop and one lane issues: every operand of an MMA (stage descriptors, the item's
       // program from the kernel's parameters) is then a uniform value. An MMA of N columns takes max(45, N / 2)
       // cycles; issued by one thread with widths read from shared memory it took 105-120 whatever N, for the moves into
-      // the uniform registers. What bounds the tile now is the shared memory: per offset at p = 16 the MMAs read 290 KB
-      // and the copies write 225 KB, 4.0k cycles at 128 B a cycle, of the 6.2k a (tile, offset) step takes (7.6k before;
-      // M2L of 2^24 points 112 -> 95 ms, of 2^20, p = 12, 3.76 -> 3.1 ms).
+      // the uniform registers. A (tile, offset) step at p = 16 takes 6.2k cycles (7.6k before; M2L of 2^24 points 112 -> 95 ms, of
+      // 2^20, p = 12, 3.76 -> 3.1 ms): the MMAs need 2.3k, the shared memory's traffic by byte counts 4.0k (290 KB read by
+      // the MMAs, 225 KB written by the copies); no unit is above half of its peak (L1 and shared memory 50 %, tensor
+      // memory 39 %, tensor pipe 36 % of the active cycles), the rest is the hand-over between the roles.
       {
          const uint32_t el = electOne();
          const int nItemsU = __shfl_sync(0xffffffffu, nItems, 0), nOffU = __shfl_sync(0xffffffffu, nOff, 0);
